@@ -148,7 +148,7 @@ static int engine_alloc(Engine& E) {
     const int ncell = (E.K.nx + 1) * (E.K.nz + 1);
     if ((rc = ialloc(E, &E.nempty, (size_t)ncell))) return rc;
     if (E.cfg.discrete_types && (rc = ialloc(E, &E.count1, (size_t)ncell))) return rc;
-    if ((rc = dalloc(E, &E.red, (size_t)(4 * (E.K.nz + 1) + 64)))) return rc;
+    if ((rc = dalloc(E, &E.red, (size_t)(8 * (E.K.nz + 1) + 64)))) return rc;
     if ((rc = dalloc(E, &E.dscal, 32))) return rc;
     CK(cudaMallocHost(&E.hscal, 64 * sizeof(double)));
     CK(cudaMalloc(&E.derr, sizeof(int)));

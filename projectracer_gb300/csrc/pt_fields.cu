@@ -3,7 +3,8 @@
 //
 // Compiled with --fmad=false: every operation rounds exactly as the reference's Fortran
 // expression (same association order), so these kernels reproduce the CPU oracle bit for bit and
-// the data-dependent smoother loop counts match.  All are HBM-bound stencils or reductions.
+// the data-dependent smoother loop counts match (the statistics are the exception: their sums run
+// in a fixed tree, not in the reference's serial order).  All are HBM-bound stencils or reductions.
 #include <cmath>
 #include <cstring>
 
@@ -394,68 +395,74 @@ int stability_dt(Engine& E, double* dt) {
     return 0;
 }
 
-// --- statistics (basics.f90:363-462), summed in the reference's serial order --------------
-// per row k: trapezoid integrals in x of T, C, u^2+w^2, RaT/conduct/vis (integrate1Dx 494-515)
-__global__ void k_stats_rows(const double* T, const double* C, const double* u, const double* w,
-                             const double* cd, const double* vis, Geo g, double* rows) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nx = cK.nx, nz = cK.nz;
-    if (k > nz) return;
-    double fT = 0, fC = 0, fV = 0, fR = 0;
-    double pT = T[g.at(0, k)], pC = C[g.at(0, k)];
-    double pu = u[g.at(0, k)], pw = w[g.at(0, k)];
-    double pV = pu * pu + pw * pw, pR = cK.RaT / cd[g.at(0, k)] / vis[g.at(0, k)];
-    for (int i = 0; i < nx; i++) {
-        double qT = T[g.at(i + 1, k)], qC = C[g.at(i + 1, k)];
-        double qu = u[g.at(i + 1, k)], qw = w[g.at(i + 1, k)];
-        double qV = qu * qu + qw * qw, qR = cK.RaT / cd[g.at(i + 1, k)] / vis[g.at(i + 1, k)];
-        fT = fT + 0.5 * (pT * 1.0 + qT * 1.0) * cK.dr;
-        fC = fC + 0.5 * (pC * 1.0 + qC * 1.0) * cK.dr;
-        fV = fV + 0.5 * (pV * 1.0 + qV * 1.0) * cK.dr;
-        fR = fR + 0.5 * (pR * 1.0 + qR * 1.0) * cK.dr;
-        pT = qT; pC = qC; pV = qV; pR = qR;
+// Sums of the stats row, in two launches: a CTA per grid row, then one CTA over the rows.  Both
+// are latency-bound at small grids; the row pass reads six FP64 fields once (25 MB at 1024x512) and
+// divides twice per node on the narrow FP64 pipe.  A thread walks its row in strides of the CTA,
+// and the partial sums meet in a fixed tree, so a row's columns are coalesced and the result does
+// not depend on the launch.  The trapezoid rule is taken as (sum f - (f_first + f_last) / 2) dr,
+// which needs each node's value once.  One thread per row and one thread for the tail took
+// 20.7 ms at 1024x512 and 1.5 ms at 128x128 (GB300, host time of the call); this takes 0.16 and 0.06 ms.
+constexpr int kStatsRow = 7;  // per row: T, C, u^2+w^2, Ra/conduct/vis, empty, fewest, most tracers
+constexpr int kStatsThreads = 256;
+
+// sums of q < NS values and extrema of two more (fewest, most) over the CTA, in thread 0
+template <int NS, int NT>
+__device__ __forceinline__ void stats_block(double (&a)[NS], int& lo, int& hi) {
+    __shared__ double sh[NT / 32][NS];
+    __shared__ int slo[NT / 32], shi[NT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NS; q++)
+        for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+        for (int q = 0; q < NS; q++) sh[warp][q] = a[q];
+        slo[warp] = lo;
+        shi[warp] = hi;
     }
-    rows[4 * k + 0] = fT;
-    rows[4 * k + 1] = fC;
-    rows[4 * k + 2] = fV;
-    rows[4 * k + 3] = fR;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < NT / 32; w++) {
+            for (int q = 0; q < NS; q++) a[q] += sh[w][q];
+            lo = min(lo, slo[w]);
+            hi = max(hi, shi[w]);
+        }
 }
 
-// single-thread tail: z integrals, fluxes, strain maximum, tracer counts
-__global__ void k_stats_tail(const double* rows, const double* T, const double* u, const double* w,
-                             const double* cd, const double* E1, const int32_t* nempty, Geo g,
-                             double* out, int kent, int direct) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int nx = cK.nx, nz = cK.nz;
-    double I[4] = {0, 0, 0, 0}, Ient = 0.0;
-    for (int k = 0; k < nz; k++)
-        for (int q = 0; q < 4; q++) I[q] = I[q] + 0.5 * (rows[4 * k + q] * 1.0 + rows[4 * (k + 1) + q] * 1.0) * cK.ds;
-    for (int k = kent; k < nz; k++) Ient = Ient + 0.5 * (rows[4 * k + 1] * 1.0 + rows[4 * (k + 1) + 1] * 1.0) * cK.ds;
-    // surface / bottom fluxes
-    double Nu_top = 0.0, Tb = 0.0, Nu_b = 0.0, mob = 0.0;
-    double pst = 0, psb = 0, pT0 = 0, pm = 0;
-    for (int i = 0; i <= nx; i++) {
-        double t1 = 0.0, t2 = 0.0;
-        for (int j = -2; j <= 2; j++) t1 = t1 + cK.D1[3 + j] * T[g.at(i, nz + j)];
-        for (int j = -2; j <= 2; j++) t2 = t2 + cK.D1[3 + j] * T[g.at(i, j)];
-        double tzs = qdiv(t1, cK.ds, cK.inv_ds), tzb = qdiv(t2, cK.ds, cK.inv_ds);  // (the reference's / 1.0 is exact)
-        double st = -(cd[g.at(i, nz)] * tzs), sb = -(cd[g.at(i, 0)] * tzb), t0 = T[g.at(i, 0)];
-        double uu = u[g.at(i, nz)], ww = w[g.at(i, nz)];
-        double m = uu * uu + ww * ww;
-        if (i > 0) {
-            Nu_top = Nu_top + 0.5 * (pst * 1.0 + st * 1.0) * cK.dr;
-            Nu_b = Nu_b + 0.5 * (psb * 1.0 + sb * 1.0) * cK.dr;
-            Tb = Tb + 0.5 * (pT0 * 1.0 + t0 * 1.0) * cK.dr;
-            mob = mob + 0.5 * (pm * 1.0 + m * 1.0) * cK.dr;
-        }
-        pst = st; psb = sb; pT0 = t0; pm = m;
+__global__ void __launch_bounds__(kStatsThreads) k_stats_rows(const double* T, const double* C, const double* u,
+                                                              const double* w, const double* cd, const double* vis,
+                                                              const int32_t* nempty, Geo g, double* rows) {
+    const int k = blockIdx.x, nx = cK.nx;
+    double a[5] = {0, 0, 0, 0, 0};  // T, C, u^2+w^2, Ra/conduct/vis, empty
+    int lo = 0x7fffffff, hi = -0x7fffffff;
+    for (int i = threadIdx.x; i <= nx; i += kStatsThreads) {
+        const size_t o = g.at(i, k);
+        const double end = (i == 0 || i == nx) ? 0.5 : 1.0;
+        const double uu = u[o], ww = w[o];
+        a[0] += end * T[o];
+        a[1] += end * C[o];
+        a[2] += end * (uu * uu + ww * ww);
+        a[3] += end * (cK.RaT / cd[o] / vis[o]);
+        const int n = nempty[(size_t)k * (nx + 1) + i];
+        a[4] += n == 0 ? 1.0 : 0.0;
+        lo = min(lo, n);
+        hi = max(hi, n);
     }
-    // strain-rate invariant on the top row: from the multigrid's psi (compute_strain_rate_invariant_direct,
-    // momentum.f90:73-92), or for the direct solve from the velocities (compute_strain_rate_invariant,
-    // momentum.f90:1-34)
-    double smax = -1.0 / 0.0;
-    for (int i = 0; i <= nx && direct; i++) {
-        const int k = nz;
+    stats_block<5, kStatsThreads>(a, lo, hi);
+    if (threadIdx.x != 0) return;
+    double* r = rows + (size_t)kStatsRow * k;
+    for (int q = 0; q < 4; q++) r[q] = a[q] * cK.dr;
+    r[4] = a[4];
+    r[5] = (double)lo;
+    r[6] = (double)hi;
+}
+
+// the strain-rate invariant of the top row at column i
+__device__ __forceinline__ double stats_strain(const double* u, const double* w, const double* E1, Geo g, int i,
+                                               int direct) {
+    const int k = cK.nz;
+    if (direct) {
         double ur = 0, us = 0, wr = 0, ws = 0;
         for (int j = -2; j <= 2; j++) ur = ur + cK.D1[3 + j] * u[g.at(i + j, k)];
         ur = ur / cK.dr;
@@ -466,30 +473,61 @@ __global__ void k_stats_tail(const double* rows, const double* T, const double* 
         for (int j = -2; j <= 2; j++) ws = ws + cK.D1[3 + j] * w[g.at(i, k + j)];
         ws = ws / cK.ds;
         const double ux = ur / 1.0, uz = us / 1.0, wx = wr / 1.0, wz = ws / 1.0;
-        const double s = pow(0.5 * (2.0 * (ux * ux + wz * wz) + (uz + wx) * (uz + wx)), 0.5);
+        return pow(0.5 * (2.0 * (ux * ux + wz * wz) + (uz + wx) * (uz + wx)), 0.5);
+    }
+    double Sxx = 0, Szz = 0, Sxz = 0;
+    for (int j = -2; j <= 2; j++) Sxx = Sxx + cK.D2[3 + j] * E1[g.at(i + j, k)];
+    Sxx = qdiv(Sxx, cK.dr2, cK.inv_dr2);
+    for (int j = -2; j <= 2; j++) Szz = Szz + cK.D2[3 + j] * E1[g.at(i, k + j)];
+    Szz = qdiv(Szz, cK.ds2, cK.inv_ds2);
+    for (int k2 = -2; k2 <= 2; k2++)
+        for (int i2 = -2; i2 <= 2; i2++) Sxz = Sxz + cK.Drs[i2 + 2][k2 + 2] * E1[g.at(i + i2, k + k2)];
+    Sxz = Sxz / (cK.dr * cK.ds);
+    return pow(2.0 * (Sxz * Sxz) + 0.5 * ((Szz - Sxx) * (Szz - Sxx)), 0.5);
+}
+
+// z integrals of the row sums, the fluxes and velocities of the top and bottom rows, the strain
+// maximum of the top row (from the multigrid's psi: compute_strain_rate_invariant_direct,
+// momentum.f90:73-92; for the direct solve from the velocities: compute_strain_rate_invariant,
+// momentum.f90:1-34) and the tracer counts
+constexpr int kStatsTail = 512;
+__global__ void __launch_bounds__(kStatsTail) k_stats_tail(const double* rows, const double* T, const double* u,
+                                                           const double* w, const double* cd, const double* E1, Geo g,
+                                                           double* out, int kent, int direct) {
+    const int nx = cK.nx, nz = cK.nz, tid = threadIdx.x;
+    double a[10] = {};  // row integrals T, C, v^2, Ra; C from kent up; Nu_top, T bottom, Nu_bot, mobility; empty
+    int lo = 0x7fffffff, hi = -0x7fffffff;
+    for (int k = tid; k <= nz; k += kStatsTail) {
+        const double* r = rows + (size_t)kStatsRow * k;
+        const double end = (k == 0 || k == nz) ? 0.5 : 1.0;
+        for (int q = 0; q < 4; q++) a[q] += end * r[q];
+        if (k >= kent) a[4] += ((k == kent && kent < nz) || k == nz ? (kent < nz ? 0.5 : 0.0) : 1.0) * r[1];
+        a[9] += r[4];
+        lo = min(lo, (int)r[5]);
+        hi = max(hi, (int)r[6]);
+    }
+    double smax = -1.0 / 0.0;
+    for (int i = tid; i <= nx; i += kStatsTail) {
+        const double end = (i == 0 || i == nx) ? 0.5 : 1.0;
+        double t1 = 0.0, t2 = 0.0;
+        for (int j = -2; j <= 2; j++) t1 = t1 + cK.D1[3 + j] * T[g.at(i, nz + j)];
+        for (int j = -2; j <= 2; j++) t2 = t2 + cK.D1[3 + j] * T[g.at(i, j)];
+        const double tzs = qdiv(t1, cK.ds, cK.inv_ds), tzb = qdiv(t2, cK.ds, cK.inv_ds);
+        const double uu = u[g.at(i, nz)], ww = w[g.at(i, nz)];
+        a[5] += end * -(cd[g.at(i, nz)] * tzs);
+        a[6] += end * T[g.at(i, 0)];
+        a[7] += end * -(cd[g.at(i, 0)] * tzb);
+        a[8] += end * (uu * uu + ww * ww);
+        const double s = stats_strain(u, w, E1, g, i, direct);
         if (s > smax) smax = s;
     }
-    for (int i = 0; i <= nx && !direct; i++) {
-        int k = nz;
-        double Sxx = 0, Szz = 0, Sxz = 0;
-        for (int j = -2; j <= 2; j++) Sxx = Sxx + cK.D2[3 + j] * E1[g.at(i + j, k)];
-        Sxx = qdiv(Sxx, cK.dr2, cK.inv_dr2);
-        for (int j = -2; j <= 2; j++) Szz = Szz + cK.D2[3 + j] * E1[g.at(i, k + j)];
-        Szz = qdiv(Szz, cK.ds2, cK.inv_ds2);
-        for (int k2 = -2; k2 <= 2; k2++)
-            for (int i2 = -2; i2 <= 2; i2++) Sxz = Sxz + cK.Drs[i2 + 2][k2 + 2] * E1[g.at(i + i2, k + k2)];
-        Sxz = Sxz / (cK.dr * cK.ds);
-        double s = pow(2.0 * (Sxz * Sxz) + 0.5 * ((Szz - Sxx) * (Szz - Sxx)), 0.5);
-        if (s > smax) smax = s;
-    }
-    int empty = 0, tmin = 0x7fffffff, tmax = -0x7fffffff;
-    for (int q = 0; q < (nx + 1) * (nz + 1); q++) {
-        int n = nempty[q];
-        if (n == 0) empty++;
-        if (n < tmin) tmin = n;
-        if (n > tmax) tmax = n;
-    }
-    double q1, q2, q3, q4, d;
+    for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+    __shared__ double ssm[kStatsTail / 32];
+    if ((tid & 31) == 0) ssm[tid >> 5] = smax;
+    stats_block<10, kStatsTail>(a, lo, hi);  // (its barrier orders ssm too)
+    if (tid != 0) return;
+    for (int q = 1; q < kStatsTail / 32; q++) smax = fmax(smax, ssm[q]);
+    double d, q1, q2, q3, q4;
     d = 0; for (int j = -2; j <= 2; j++) d = d + cK.D1[3 + j] * T[g.at(0, nz + j)];
     q1 = -qdiv(cd[g.at(0, nz)] * d, cK.ds, cK.inv_ds);
     d = 0; for (int j = -2; j <= 2; j++) d = d + cK.D1[3 + j] * T[g.at(nx, nz + j)];
@@ -498,24 +536,22 @@ __global__ void k_stats_tail(const double* rows, const double* T, const double* 
     q3 = -qdiv(cd[g.at(nx, 0)] * d, cK.ds, cK.inv_ds);
     d = 0; for (int j = -2; j <= 2; j++) d = d + cK.D1[3 + j] * T[g.at(0, j)];
     q4 = -qdiv(cd[g.at(0, 0)] * d, cK.ds, cK.inv_ds);
-    out[0] = I[0];   // integral of T
-    out[1] = I[1];   // integral of C
-    out[2] = I[2];   // integral of u^2+w^2
-    out[3] = I[3];   // integral of RaT/conduct/vis
-    out[4] = Ient;
-    out[5] = Nu_top; out[6] = Tb; out[7] = Nu_b; out[8] = mob; out[9] = smax;
+    for (int q = 0; q < 5; q++) out[q] = a[q] * cK.ds;  // integrals of T, C, u^2+w^2, Ra/conduct/vis, C above kent
+    for (int q = 5; q < 9; q++) out[q] = a[q] * cK.dr;  // Nu_top, T bottom, Nu_bot, mobility
+    out[9] = smax;
     out[10] = q1; out[11] = q2; out[12] = q3; out[13] = q4;
-    out[14] = (double)empty; out[15] = (double)tmin; out[16] = (double)tmax;
+    out[14] = a[9]; out[15] = (double)lo; out[16] = (double)hi;
 }
 
 int stats(Engine& E, pt_stats_row* o) {
     double* rows = E.red;
     int nz = E.K.nz;
     const double* C = E.cfg.comp ? E.Cnew : E.T;
-    PT_COUNT(), k_stats_rows<<<nblk(nz + 1, 64), 64, 0, E.st>>>(E.T, C, E.u, E.w, E.cond, E.vis[1], E.g1, rows);
-    double* out = rows + 4 * (nz + 1) + 8;
-    PT_COUNT(), k_stats_tail<<<1, 32, 0, E.st>>>(rows, E.T, E.u, E.w, E.cond, E.err[1], E.nempty, E.g1, out, E.kent,
-                                                  E.cfg.direct);
+    PT_COUNT(), k_stats_rows<<<nz + 1, kStatsThreads, 0, E.st>>>(E.T, C, E.u, E.w, E.cond, E.vis[1], E.nempty, E.g1,
+                                                                 rows);
+    double* out = rows + kStatsRow * (nz + 1) + 8;
+    PT_COUNT(), k_stats_tail<<<1, kStatsTail, 0, E.st>>>(rows, E.T, E.u, E.w, E.cond, E.err[1], E.g1, out, E.kent,
+                                                         E.cfg.direct);
     CKL("stats");
     CK(cudaMemcpyAsync(E.hscal, out, 17 * sizeof(double), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
