@@ -13,10 +13,12 @@
 // coefficient fields are rounded to FP32 once per solve.  Residuals that feed a coarser level use
 // FP64 arithmetic on the FP32 correction: for smooth modes the biharmonic stencil cancels by many
 // orders of magnitude on the fine levels.  Each iteration is two captured CUDA graphs.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <utility>
 
+#include "pt_cluster.cuh"
 #include "pt_consts.cuh"
 #include "pt_exact.cuh"
 
@@ -415,6 +417,344 @@ __global__ void k_res_to_f32(float* out, const double* in, size_t n) {
     if (q < n) out[q] = (float)in[q];
 }
 
+// ---------------------------------------------------------------- levels in one cluster
+// A stretch of the cycle on levels that fit one cluster (pt_cluster.cuh): per visit the restriction
+// or the prolongation that enters it, the RKC1 stages in increment form, and the residual that the
+// next coarser level restricts; the coarsest level by the explicit inverse.
+// A thread owns one node for a whole visit and keeps what belongs to it in registers: the 29 weights
+// of A there (the operator with its five coefficient fields folded in once per visit), F0, Y0 and D_{j-2}.
+// A stage is then 29 shared loads and 29 multiply-adds per thread.  With one to eight warps per
+// scheduler it is bound by the latency of that chain and of one exchange, so one node per thread and
+// 32 warps rather than two nodes and 16: the same 1,024 nodes a CTA with half the chain.
+struct FLevel {
+    Geo g;
+    float *e, *rhs, *res;
+    const float* coef[6];  // vis, vx, vz, vxz, vxxmzz, dt_stream
+    float h[10];           // 1/dr^2, 2/dr^3, 1/dr^4, the same in z, 2/(dr^2 ds^2), 4/(dr ds), 2/(dr ds^2), 2/(dr^2 ds)
+    int solo;              // >= 0: walked by every CTA alone, its arrays at this float of the solo area
+};
+struct FRun {
+    FLevel L[PT_MAXLEV];
+    cl::Visit v[cl::kMaxVisits];
+    int nv, N, ivis, ngc, solo, coarse_solo;  // solo: floats of the solo levels' arrays
+    float sz;
+    float mew[64], vv[64], mewtc[64];
+    const double* r1;  // FP64 residual that level 2 restricts
+    const double *G, *RowB;
+};
+// warps' turns of a level (32 columns of a row): at most one a warp
+__host__ __device__ inline int cluster_tiles(int nx, int nz) {
+    return cl::Strip::segments(nx) * cl::Strip::rows_per_cta(nz);
+}
+__host__ __device__ inline int cluster_tiles_alone(int nx, int nz) { return cl::Strip::segments(nx) * (nz - 1); }
+
+// The points of A's stencil: a 5 x 5 block, then (-3,0), (3,0), (0,-3), (0,3)
+constexpr int kPts = 29;
+__host__ __device__ constexpr int pt_dx(int p) { return p < 25 ? p % 5 - 2 : p == 25 ? -3 : p == 26 ? 3 : 0; }
+__host__ __device__ constexpr int pt_dz(int p) { return p < 25 ? p / 5 - 2 : p == 27 ? -3 : p == 28 ? 3 : 0; }
+__host__ __device__ constexpr int pt_index(int dx, int dz) {  // -1: not a point of the stencil
+    return dx >= -2 && dx <= 2 && dz >= -2 && dz <= 2 ? (dz + 2) * 5 + dx + 2
+           : dz == 0 && dx == -3 ? 25 : dz == 0 && dx == 3 ? 26 : dx == 0 && dz == -3 ? 27 : dx == 0 && dz == 3 ? 28 : -1;
+}
+// the finite-difference weights (exact_stencils_setup compares the engine's with them)
+__host__ __device__ constexpr float fd1(int j) { return (j == -2 ? 1.f : j == -1 ? -8.f : j == 1 ? 8.f : j == 2 ? -1.f : 0.f) / 12.f; }
+__host__ __device__ constexpr float fd2(int j) { return (j == 0 ? -30.f : j == 1 || j == -1 ? 16.f : -1.f) / 12.f; }
+__host__ __device__ constexpr float fd3(int j) {
+    return (j < 0 ? 1.f : -1.f) * (j == 0 ? 0.f : j == 1 || j == -1 ? 13.f : j == 2 || j == -2 ? -8.f : 1.f) / 8.f;
+}
+__host__ __device__ constexpr float fd4(int j) {
+    return (j == 0 ? 56.f : j == 1 || j == -1 ? -39.f : j == 2 || j == -2 ? 12.f : -1.f) / 6.f;
+}
+
+// The weights of A at node (i, k) from its coefficients (vis, vxxmzz, vxz, vx, vz in c) and the level's
+// spacings h.  The ghost cells' share is folded onto the nodes that they mirror (antisymmetric across
+// the side walls, sign sz across top and bottom; every mirror node of a stencil lies in the stencil),
+// so that the windows hold no images.
+__device__ __forceinline__ void make_weights(float (&w)[kPts], const float (&c)[5], const float* h, int i, int k, int nx,
+                                             int nz, float sz) {
+    const float x2 = c[1] * h[0], x3 = c[3] * h[1], x4 = c[0] * h[2], z2 = c[1] * h[3], z3 = c[4] * h[4], z4 = c[0] * h[5];
+    const float xxzz = c[0] * h[6], xz = c[2] * h[7], xzz = c[3] * h[8], xxz = c[4] * h[9];
+#pragma unroll
+    for (int z = -2; z <= 2; z++) {
+        const float even = fd2(z) * xxzz + fd1(z) * xxz, odd = fd1(z) * xz + fd2(z) * xzz;
+#pragma unroll
+        for (int x = -2; x <= 2; x++) w[pt_index(x, z)] = fd2(x) * even + fd1(x) * odd;
+    }
+#pragma unroll
+    for (int j = -3; j <= 3; j++) {
+        const float ax = fd4(j) * x4 + fd3(j) * x3, az = fd4(j) * z4 + fd3(j) * z3;
+        if (j == -3 || j == 3) {
+            w[pt_index(j, 0)] = ax;
+            w[pt_index(0, j)] = az;
+        } else {
+            w[pt_index(j, 0)] += ax + fd2(j) * x2;
+            w[pt_index(0, j)] += az - fd2(j) * z2;
+        }
+    }
+    if (__any_sync(0xffffffffu, i <= 2 || i >= nx - 2)) {
+#pragma unroll
+        for (int z = -2; z <= 2; z++) {
+            if (i == 1) w[pt_index(0, z)] -= w[pt_index(-2, z)];
+            if (i == nx - 1) w[pt_index(0, z)] -= w[pt_index(2, z)];
+        }
+        if (i == 1) w[pt_index(1, 0)] -= w[pt_index(-3, 0)];
+        if (i == 2) w[pt_index(-1, 0)] -= w[pt_index(-3, 0)];
+        if (i == nx - 1) w[pt_index(-1, 0)] -= w[pt_index(3, 0)];
+        if (i == nx - 2) w[pt_index(1, 0)] -= w[pt_index(3, 0)];
+    }
+    if (k <= 2 || k >= nz - 2) {
+#pragma unroll
+        for (int x = -2; x <= 2; x++) {
+            if (k == 1) w[pt_index(x, 0)] += sz * w[pt_index(x, -2)];
+            if (k == nz - 1) w[pt_index(x, 0)] += sz * w[pt_index(x, 2)];
+        }
+        if (k == 1) w[pt_index(0, 1)] += sz * w[pt_index(0, -3)];
+        if (k == 2) w[pt_index(0, -1)] += sz * w[pt_index(0, -3)];
+        if (k == nz - 1) w[pt_index(0, -1)] += sz * w[pt_index(0, 3)];
+        if (k == nz - 2) w[pt_index(0, 1)] += sz * w[pt_index(0, 3)];
+    }
+}
+
+// the residual at node (i, k) in FP64 arithmetic on the correction in window y
+__device__ __noinline__ float cluster_residual64(const FRun& P, int l, const float* y, int W, int i, int k, float rhs) {
+    const FLevel& L = P.L[l];  // y: the node's cell
+    const FOp op{L.coef[0], L.coef[1], L.coef[2], L.coef[3], L.coef[4], nullptr, nullptr};
+    const double a = apply_A_ld<double>(
+        [&](int dx, int dz) {
+            const int ii = mirror_idx(i + dx, L.g.nx), kk = mirror_idx(k + dz, L.g.nz);
+            const float v = y[(kk - k) * W + ii - i];
+            return (ii != i + dx ? -v : v) * (kk != k + dz ? P.sz : 1.0f);
+        },
+        l, op, L.g.at(i, k), P.ivis);
+    return (float)((double)rhs - a);
+}
+
+// where a level's arrays of a visit lie
+struct FView {
+    float *e, *rhs, *res;
+    Geo g;
+};
+__host__ __device__ inline size_t solo_floats(const Geo& g) { return (size_t)(g.nx + 2 * GH + 1) * (size_t)(g.nz + 2 * GH + 1); }
+__device__ __forceinline__ FView level_view(const FRun& P, int l, float* solo) {
+    const FLevel& L = P.L[l];
+    if (L.solo < 0) return FView{L.e, L.rhs, L.res, L.g};
+    const int n = (int)solo_floats(L.g);
+    float* a = solo + L.solo;
+    return FView{a, a + n, a + 2 * n, Geo{L.g.nx, L.g.nz, L.g.nx + 2 * GH + 1}};
+}
+__device__ __forceinline__ float restricted(const FRun& P, int l, const FView& f, int i, int k) {
+    return l == 2 ? restrict_node(P.r1, P.L[1].g, i, k) : restrict_node((const float*)f.res, f.g, i, k);
+}
+
+// the coarsest level: x = G b in FP64 as in k_coarse_apply_mixed, a warp per row of G over the cluster,
+// or, solo, over each CTA from its own copy of G and the row factors behind b
+__device__ __noinline__ void cluster_coarse(const FRun& P, int l, double* b, float* solo) {
+    const FView V = level_view(P, l, solo), F = level_view(P, l - 1, solo);
+    const Geo g = V.g;
+    const int N1 = g.nz + 1, nn = (g.nx + 1) * N1, nk = g.nz - 1, ni = (g.nx - 1) * nk;
+    const double *G = P.coarse_solo ? b + P.ngc : P.G, *RowB = P.coarse_solo ? G + (size_t)nn * nn : P.RowB;
+    if (P.coarse_solo) {
+        cl::copy_wait();
+        __syncthreads();
+    }
+    for (int q = threadIdx.x; q < nn; q += cl::kThreads) {
+        const int ip = q / N1, kp = q - ip * N1;
+        double x = 0.0;
+        if (ip > 0 && ip < g.nx && kp > 0 && kp < g.nz) x = (double)restricted(P, l, F, ip, kp) * RowB[q];
+        b[q] = x;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, first = P.coarse_solo ? 0 : (int)cl::rank(), ctas = P.coarse_solo ? 1 : cl::kCtas;
+    for (int r = first * cl::kWarps + (threadIdx.x >> 5); r < ni; r += ctas * cl::kWarps) {
+        const int ip = r / nk + 1, kp = r - (ip - 1) * nk + 1, p = ip * N1 + kp;
+        const double* row = G + (size_t)p * nn;
+        double a = 0.0;
+        for (int q = lane; q < nn; q += 32) a = fma(row[q], b[q], a);
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) V.e[g.at(ip, kp)] = (float)a;  // (its walls stay zero, its images are not read)
+    }
+}
+
+// the thread's place in a visit
+struct FPlace {
+    int i, k, up, down, bytes, m;  // node; readers of its row; bytes received a stage; its window cell
+    bool alone, busy, on;          // busy: the warp has nodes, on: the thread has one
+    size_t oc;                     // the node in the global coefficient fields
+    cl::Strip s;
+};
+__device__ __forceinline__ FPlace place_visit(const FRun& P, int n, int c) {
+    const FLevel& L = P.L[P.v[n].level];
+    FPlace p;
+    p.alone = L.solo >= 0;
+    p.s.set(L.g.nz, c, p.alone);
+    // a warp has 32 columns of one row; t / segs by the reciprocal, exact for 16 warps
+    const int t = threadIdx.x >> 5, segs = cl::Strip::segments(L.g.nx);
+    const int r = (int)(((float)t + 0.5f) * __frcp_rn((float)segs));
+    p.i = (t - r * segs) * 32 + (int)(threadIdx.x & 31) + 1;
+    p.k = p.s.k0 + r;
+    p.busy = r < p.s.rows;
+    p.on = p.busy && p.i <= L.g.nx - 1;
+    p.up = p.busy ? p.s.readers_up(r) : 0;
+    p.down = p.busy ? p.s.readers_down(r) : 0;
+    p.bytes = p.s.rows_received(L.g.nz) * (L.g.nx - 1) * (int)sizeof(float);
+    p.m = p.busy ? p.s.at(min(p.i, L.g.nx - 1), p.k) : cl::kReach * cl::kPitch + cl::kReach;  // idle: anywhere inside
+    p.oc = p.on ? L.g.at(p.i, p.k) : 0;
+    return p;
+}
+// clears the two windows that a visit will use, and starts the loads that no visit writes to
+__device__ __forceinline__ void open_visit(const FRun& P, int n, const FPlace& p, float* win, float (&cv)[5], float& dt) {
+    const FLevel& L = P.L[P.v[n].level];
+    if (p.on) {
+        cv[0] = L.coef[0][p.oc];
+        dt = L.coef[5][p.oc];
+        if (P.ivis != 0) {
+            cv[1] = L.coef[4][p.oc];
+            cv[2] = L.coef[3][p.oc];
+            cv[3] = L.coef[1][p.oc];
+            cv[4] = L.coef[2][p.oc];
+        }
+    }
+    const int cols = L.g.nx + 2 * cl::kReach + 1, rows = p.s.R + 2 * cl::kReach;
+    for (int r = threadIdx.x >> 5; r < rows; r += cl::kWarps)
+        for (int q = threadIdx.x & 31; q < cols; q += 32) win[r * cl::kPitch + q] = win[cl::kWindow + r * cl::kPitch + q] = 0.0f;
+}
+
+__global__ void __launch_bounds__(cl::kThreads, 1) k_cycle_cluster_f(const __grid_constant__ FRun P) {
+    // four windows (two a visit, the next visit's cleared while this one's are in use), the coarsest
+    // right-hand side, the solo levels' arrays
+    extern __shared__ __align__(16) float sm[];
+    __shared__ uint64_t bars[2];
+    __shared__ float4 cheb[64];  // per stage: mew, vv, mewt c
+    double* const coarse = reinterpret_cast<double*>(sm + 4 * cl::kWindow);
+    float* const solo = reinterpret_cast<float*>(coarse + P.ngc + (P.coarse_solo ? P.ngc * (P.ngc + 1) : 0));
+    if (threadIdx.x < 64) cheb[threadIdx.x] = make_float4(P.mew[threadIdx.x], P.vv[threadIdx.x], P.mewtc[threadIdx.x], 0.0f);
+    for (int q = threadIdx.x; q < P.solo; q += cl::kThreads) solo[q] = 0.0f;
+    const int c = (int)cl::rank();
+    cl::Exchange ex;
+    ex.init(bars);
+    pdl_begin();
+    if (P.coarse_solo) {  // the inverse and the row factors, on their way while the first levels run
+        double* G = coarse + P.ngc;
+        for (int q = threadIdx.x; q < P.ngc * (P.ngc + 1); q += cl::kThreads)
+            cl::copy8(G + q, q < P.ngc * P.ngc ? P.G + q : P.RowB + (q - P.ngc * P.ngc));
+    }
+    FPlace p{};
+    float cv[5] = {}, dt = 0.0f;
+    bool open = false;  // the visit's windows are cleared and its coefficients on their way
+    for (int n = 0; n < P.nv; n++) {
+        const int l = P.v[n].level, fl = P.v[n].flags;
+        const bool more = n + 1 < P.nv && !(P.v[n + 1].flags & cl::kCoarse);
+        if (fl & cl::kCoarse) {
+            cluster_coarse(P, l, coarse, solo);
+            open = more;
+            if (more) {
+                p = place_visit(P, n + 1, c);
+                open_visit(P, n + 1, p, sm + (n + 1 & 1) * 2 * cl::kWindow, cv, dt);
+            }
+            if (P.coarse_solo && p.alone) __syncthreads();
+            else cl::sync();
+            continue;
+        }
+        float* const win = sm + (n & 1) * 2 * cl::kWindow;
+        if (!open) {
+            p = place_visit(P, n, c);
+            open_visit(P, n, p, win, cv, dt);
+            cl::sync();  // every window is cleared and every mbarrier ready
+        }
+        const FView V = level_view(P, l, solo);
+        const Geo g = V.g;
+        const bool zero = fl & (cl::kRestrict | cl::kZero), alone = p.alone, on = p.on;
+        const size_t o = on ? g.at(p.i, p.k) : 0;
+        float rhs = 0.0f, y0 = 0.0f;
+        if (on) {
+            if (fl & cl::kRestrict) {
+                rhs = restricted(P, l, level_view(P, l - 1, solo), p.i, p.k);
+                V.rhs[o] = rhs;
+            } else {
+                rhs = V.rhs[o];
+            }
+            if (!zero) {
+                y0 = V.e[o];
+                if (fl & cl::kProlong) {
+                    const FView C = level_view(P, l + 1, solo);
+                    y0 += prolong_value(C.e, C.g, p.i, p.k);
+                }
+            }
+        }
+        float w[kPts];
+        make_weights(w, cv, P.L[l].h, p.i, p.k, g.nx, g.nz, P.sz);
+        ex.bytes = (uint32_t)p.bytes;
+        cl::Outlet<float> out;
+        out.set(p.s, win, bars, p.m, p.up, p.down);
+        const float* const m = win + p.m;
+        float A = 0.0f, own = 0.0f;
+        auto apply = [&](int q) {  // A of window q at the node, and the window's value there
+            const float* x = m + q * cl::kWindow;
+            float a[3] = {};
+#pragma unroll
+            for (int j = 0; j < kPts; j++) {
+                const float v = x[pt_dz(j) * cl::kPitch + pt_dx(j)];
+                a[j % 3] += w[j] * v;
+                if (j == pt_index(0, 0)) own = v;
+            }
+            A = (a[0] + a[1]) + a[2];
+        };
+        auto publish = [&](int q, float v) {
+            if (on) {
+                win[q * cl::kWindow + p.m] = v;
+                if (p.up | p.down) out.put_remote(q, v);
+            }
+            if (alone) __syncthreads();
+            else ex.arrive(q);
+        };
+        int cur = 0;  // the window of D_{j-1}
+        if (!zero) {
+            publish(0, y0);
+            if (p.busy) apply(0);
+            cur = 1;
+        }
+        const float F0 = rhs - A;
+        float d = cheb[1].z * dt * F0, old = 0.0f;
+        publish(cur, d);
+        for (int j = 2; j <= P.N; j++) {
+            if (p.busy) {
+                const float4 ch = cheb[j];
+                apply(cur);
+                d = ch.x * own + ch.z * dt * (F0 - A) + ch.y * old;
+                old = own;
+            }
+            if (j < P.N) {
+                cur ^= 1;
+                publish(cur, d);
+            }
+        }
+        d = ex.ok ? y0 + d : __int_as_float(0x7fc00000);  // a wait ran out: NaN, which the host reports
+        if (on) {
+            // with its images where a kernel outside this one applies A to it
+            if (l == 1) store_ghosts_f(V.e, g, p.i, p.k, g.nx, g.nz, d, P.sz);
+            else V.e[o] = d;
+        }
+        if (fl & cl::kResidual) {  // FP32 after a zero start, FP64 arithmetic otherwise (see k_residual_f)
+            cur ^= 1;
+            publish(cur, d);
+            if (zero) {
+                if (p.busy) apply(cur);
+                if (on) V.res[o] = rhs - A;
+            } else if (on) {
+                V.res[o] = cluster_residual64(P, l, m + cur * cl::kWindow, cl::kPitch, p.i, p.k, rhs);
+            }
+        }
+        open = more;
+        if (more) {
+            p = place_visit(P, n + 1, c);
+            open_visit(P, n + 1, p, sm + (n + 1 & 1) * 2 * cl::kWindow, cv, dt);
+        }
+        // the correction and the residual are in place, the next windows clear
+        if (alone && (more ? p.alone : n + 1 < P.nv && P.coarse_solo)) __syncthreads();
+        else cl::sync();
+    }
+}
+
 // writes value v of interior node (i,k) of the FP64 iterate and its free-slip ghost images (the
 // per-node form of enforceBCs_stream: antisymmetric across the side walls, sign sz across top and
 // bottom; wall nodes and their images are zero and are not written)
@@ -712,6 +1052,140 @@ static int bcs_f(Engine& E, int l, float* f) {
                       E.st, f, g, g.nx, g.nz, E.cfg.Vbc == 0 ? -1.f : 1.f);
 }
 
+// ---- levels in one cluster: which ones, and a stretch of the schedule as one launch
+// shared memory of a launch whose solo levels take that many floats
+static size_t cluster_bytes(const Engine& E, size_t solo) {
+    const size_t n = E.ccoarse ? (size_t)E.ngc : 0;  // the coarsest right-hand side; solo: its inverse and row factors
+    return sizeof(float) * (4 * (size_t)cl::kWindow + solo) + sizeof(double) * (n + (E.coarse_solo ? n * (n + 1) : 0));
+}
+static int cluster_setup_f(Engine& E) {
+    E.ctop = E.grids + 1;
+    E.csolo = E.grids + 1;
+    E.cl1 = E.ccoarse = E.coarse_solo = false;
+    if (E.cfg.Nmulti != 1 || !E.res_int) return 0;  // (res_int: the stencils are the rationals of fd1..fd4)
+    // a level goes to the cluster when each of its nodes finds a thread: 16 CTAs x 16 warps x 32 columns,
+    // 8,192 nodes
+    auto fits = [&](int l) {
+        const Geo& g = E.gl[l];
+        return cluster_tiles(g.nx, g.nz) <= cl::kWarps && g.nx + 2 * cl::kReach + 1 <= cl::kPitch;
+    };
+    if (cudaFuncSetAttribute(k_cycle_cluster_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::kMaxSmem) ||
+        cudaFuncSetAttribute(k_cycle_cluster_f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
+        return fail(PT_ERR_CUDA, "cluster kernel attributes");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {cl::kCtas, 1, 1};
+    cfg.gridDim = dim3(cl::kCtas);
+    cfg.blockDim = dim3(cl::kThreads);
+    cfg.dynamicSmemBytes = cl::kMaxSmem;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, k_cycle_cluster_f, &cfg) != cudaSuccess || fit < 1) {
+        (void)cudaGetLastError();  // no room for a cluster of this size: the per-stage kernels run
+        return 0;
+    }
+    while (E.ctop > 2 && (E.ctop - 1 == E.grids || fits(E.ctop - 1))) E.ctop--;
+    if (E.ctop >= E.grids) E.ctop = E.grids + 1;  // nothing but the coarsest level
+    E.cl1 = fits(1);
+    // the coarse solve inside the cluster: n^2 FP64 products on 16 SMs against 152 and a launch
+    E.ccoarse = E.Ginv && E.ngc <= 700;
+    E.coarse_solo = E.ccoarse && E.ngc <= 90;  // n^2 products on one SM against one exchange
+    // levels whose nodes fit one CTA's threads, 512 nodes, need no exchange between CTAs: each CTA
+    // walks them for itself.  The way back up must be in the same launch.
+    E.csolo = E.grids;
+    size_t solo = 3 * solo_floats(E.gl[E.grids]);
+    if (E.ccoarse)
+        while (E.csolo - 1 > E.ctop) {
+            const Geo& g = E.gl[E.csolo - 1];
+            if (cluster_tiles_alone(g.nx, g.nz) > cl::kWarps || cluster_bytes(E, solo + 3 * solo_floats(g)) > cl::kMaxSmem) break;
+            solo += 3 * solo_floats(g);
+            E.csolo--;
+        }
+    return 0;
+}
+
+static int launch_run_f(Engine& E, FRun& R, bool coarse_smoother, const double* r1) {
+    const double* kmew = coarse_smoother ? E.mew_c : E.K.mew;
+    const double* kvv = coarse_smoother ? E.vv_c : E.K.vv;
+    const double* kmewt = coarse_smoother ? E.mewt_c : E.K.mewt;
+    R.N = coarse_smoother ? E.nstageC : E.cfg.nstageS;
+    R.ivis = E.cfg.ivis;
+    R.sz = E.cfg.Vbc == 0 ? -1.f : 1.f;
+    for (int j = 1; j <= R.N; j++) {
+        R.mew[j] = (float)kmew[j];
+        R.vv[j] = (float)kvv[j];
+        R.mewtc[j] = (float)(kmewt[j] * E.cfg.c_2);
+    }
+    int a = PT_MAXLEV, b = 0;
+    for (int n = 0; n < R.nv; n++)
+        if (!(R.v[n].flags & cl::kCoarse)) {
+            a = std::min<int>(a, R.v[n].level);
+            b = std::max<int>(b, R.v[n].level);
+        }
+    for (int l = 1; l <= E.grids; l++) {
+        FLevel& L = R.L[l];
+        L.g = E.gl[l];
+        L.e = E.ferr[l];
+        L.rhs = E.fRHS[l];
+        L.res = E.fres[l];
+        for (int q = 0; q < 6; q++) L.coef[q] = E.fcoef[l][q];
+        const LevConst& K = E.L[l];
+        const double h[10] = {1.0 / K.dr2, 2.0 / K.dr3, 1.0 / K.dr4, 1.0 / K.ds2, 2.0 / K.ds3, 1.0 / K.ds4,
+                              2.0 / K.dr2ds2, 4.0 / K.drds, 2.0 / K.drds2, 2.0 / K.dr2ds};
+        for (int q = 0; q < 10; q++) L.h[q] = (float)h[q];
+        L.solo = -1;
+        // only in a run that walks the whole way down and up: a solo level's arrays last for one launch
+        const bool mine = l < E.grids ? l >= a && l <= b : E.coarse_solo;
+        if (l >= E.csolo && mine && E.ccoarse && coarse_smoother) {
+            L.solo = R.solo;
+            R.solo += 3 * (int)solo_floats(L.g);
+        }
+    }
+    R.coarse_solo = E.coarse_solo && coarse_smoother;
+    R.r1 = r1;
+    R.G = E.Ginv;
+    R.RowB = E.RowB;
+    R.ngc = E.ccoarse && coarse_smoother ? E.ngc : 0;
+    const size_t bytes = cluster_bytes(E, (size_t)R.solo);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {cl::kCtas, 1, 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(cl::kCtas);
+    cfg.blockDim = dim3(cl::kThreads);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = E.st;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    PT_COUNT();
+    return cuda_check(cudaLaunchKernelEx(&cfg, k_cycle_cluster_f, R), "k_cycle_cluster_f");
+}
+
+// the entries p.. of the schedule that one cluster can walk, as one launch; *last receives the last
+// of them
+static int cluster_run_f(Engine& E, int p, const double* r1, int* last) {
+    FRun R{};
+    const int* multi = E.mmulti;
+    for (; p <= E.mnsteps && R.nv < cl::kMaxVisits; p++) {
+        const int l = multi[p];
+        if (l < E.ctop || (l == E.grids && !E.ccoarse)) break;
+        cl::Visit& v = R.v[R.nv++];
+        v.level = (signed char)l;
+        if (l == E.grids) v.flags = cl::kCoarse;
+        else {
+            if (multi[p - 1] < l) v.flags |= cl::kRestrict;
+            else if (R.nv > 1) v.flags |= cl::kProlong;  // (a run's first visit finds it done)
+            if (multi[p + 1] > l) v.flags |= cl::kResidual;
+        }
+        *last = p;
+    }
+    return launch_run_f(E, R, true, r1);
+}
+
 // FP32 iterate_stream on the correction of level l, RKC1 in increment form (k_rkc_first_f).
 // zero: the correction is zero on entry (first visit after a descent); want_res: the residual is
 // needed (the next step descends).
@@ -735,6 +1209,14 @@ static int smooth_f(Engine& E, int l, bool zero, bool want_res, bool restrict_in
     float* e = E.ferr[l];
     float* F0 = E.fS0[l];
     const double c = E.cfg.c_2;  // Nmulti = 1: one pass with c = c_2
+    if (l == 1 && zero && !want_res && E.cl1) {
+        GraphTimer gt(E, 1, N);
+        FRun R{};
+        R.nv = 1;
+        R.v[0].level = 1;
+        R.v[0].flags = cl::kZero;
+        return launch_run_f(E, R, false, nullptr);
+    }
     for (int n = 1; n <= E.cfg.Nmulti; n++) {
         GraphTimer gt(E, 1, (l == 1 && zero) ? N : 0);
         float* Dm1 = E.fS1[l];
@@ -827,13 +1309,18 @@ static int mixed_part(Engine& E, int part, int slot = -1) {
     const int grids = E.grids, nsteps = E.mnsteps;
     const int* multi = E.mmulti;
     for (int p = 2; p <= nsteps; p++) {
+        if (multi[p] >= E.ctop && (multi[p] < grids || E.ccoarse)) {
+            if ((rc = cluster_run_f(E, p, r1, &p))) return rc;
+            if (!(multi[p + 1] < multi[p])) continue;  // a coarser level follows
+        }
         const int l = multi[p];
         const Geo& g = E.gl[l];
+        const bool done = l >= E.ctop && (l < grids || E.ccoarse);  // visited by the cluster: its way up is left
         // the reference's schedules visit level 1 only at their first step; the pre-smoothing of
         // part 0 is already in x, so the cycle's level-1 correction is the closing prolongation
         if (l == 1) return fail(PT_ERR_CONFIG, "mixed-precision cycle: schedule revisits level 1");
         const bool descend = multi[p - 1] < multi[p];
-        if (descend && l == grids) {  // (above the coarsest level the restriction is fused into smooth_f)
+        if (!done && descend && l == grids) {  // (above the coarsest level the restriction is fused into smooth_f)
             const Geo& gf = E.gl[l - 1];
             dim3 gr(nblk(g.nx - 1, 128), g.nz - 1);
             // the correction of level l restarts from zero: cleared by the first smoothing stage
@@ -846,7 +1333,8 @@ static int mixed_part(Engine& E, int part, int slot = -1) {
                                 (const float*)E.fres[l - 1], g, gf, g.nx, g.nz);
             if (rc) return rc;
         }
-        if (l < grids) {
+        if (done) {
+        } else if (l < grids) {
             if ((rc = smooth_f(E, l, descend, multi[p + 1] > multi[p], descend, r1))) return rc;
         } else if ((rc = coarse_solve_f(E))) {
             return rc;
@@ -1154,7 +1642,7 @@ int mixed_alloc(Engine& E) {
             E.bytes_allocated += n * sizeof(float);
         }
     }
-    return 0;
+    return cluster_setup_f(E);
 }
 
 }  // namespace pt
