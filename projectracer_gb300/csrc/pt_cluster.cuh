@@ -10,9 +10,9 @@
 // (asynchronous stores to distributed shared memory, counted by an mbarrier of the receiver), so a
 // stage waits for its neighbours' rows only and moves no global data.  Full-width strips rather than
 // 2D blocks: the neighbours of a strip are known from the row alone, for strips of one row too.
-// Measured per FP32 stage: 0.4-0.55 us (a cluster barrier per stage instead of the counted stores:
-// 0.7-1.3 us).  The levels below 1 of a V-cycle with 8 stages a visit: 128x128 148 -> 58 us, 256x128
-// 93 -> 51 us.
+// Measured per FP32 stage: 0.55-0.75 us (a cluster barrier per stage instead of the counted stores:
+// 1.3 us); the part of a V-cycle below level 1, 8 stages a visit: 128x128 148 -> 77 us, 256x128
+// 93 -> 62 us.  FP64 stages with exact sums: 1.5-1.7 us (4.2 with a kernel per stage).
 #pragma once
 #include <cstdint>
 
@@ -177,6 +177,18 @@ struct Visit {
 };
 enum { kRestrict = 1, kProlong = 2, kZero = 4, kResidual = 8, kCoarse = 16 };
 constexpr int kMaxVisits = 48;
+
+// the launch of one cluster; at: one attribute
+static inline void cluster_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, size_t smem, cudaStream_t st) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {kCtas, 1, 1};
+    cfg.gridDim = dim3(kCtas);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+}
 
 }  // namespace cl
 }  // namespace pt

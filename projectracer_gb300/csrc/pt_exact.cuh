@@ -52,6 +52,20 @@ __device__ __forceinline__ double i64_to_double_scaled(long long v, int e2) {
     return __longlong_as_double((long long)(sgn | (ex << 52) | (mant & 0xFFFFFFFFFFFFFull)));
 }
 
+// the double with bits b as round(S 2^s), |.| < 2^62, for a tile whose largest biased exponent is emax
+// (zero in a tile that holds Inf/NaN)
+__device__ __forceinline__ long long fixed_point(unsigned long long b, int emax) {
+    const int e = (int)((b >> 52) & 0x7FF);
+    if (e == 0 || emax == 0x7FF) return 0;
+    const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    const int sh = emax - 9 - e;  // X = m 2^-sh
+    unsigned long long a;
+    if (sh <= 0) a = m << (-sh);
+    else if (sh < 64) a = (m + (1ull << (sh - 1))) >> sh;
+    else a = 0;
+    return (b >> 63) ? -(long long)a : (long long)a;
+}
+
 struct HL {
     long long h, l;
 };
@@ -100,18 +114,7 @@ __device__ __forceinline__ int load_tile_fx(int2 (*X)[TG::W], int* emax_s, const
     for (int q = 0; q < PER; q++) {
         const int idx = tid + TG::NT * q;
         if (idx >= NT) break;
-        const unsigned long long b = raw[q];
-        const int e = (int)((b >> 52) & 0x7FF);
-        long long v = 0;
-        if (e != 0 && emax != 0x7FF) {
-            const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-            const int sh = emax - 9 - e;  // X = m 2^-sh, |X| < 2^62
-            unsigned long long a;
-            if (sh <= 0) a = m << (-sh);
-            else if (sh < 64) a = (m + (1ull << (sh - 1))) >> sh;
-            else a = 0;
-            v = (b >> 63) ? -(long long)a : (long long)a;
-        }
+        const long long v = fixed_point(raw[q], emax);
         const long long h = v >> 31;  // floor
         X[idx / kRfW][idx % kRfW] = make_int2((int)h, (int)(v - (h << 31)));
     }

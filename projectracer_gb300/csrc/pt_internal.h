@@ -131,7 +131,7 @@ struct Engine {
     float *ferr[PT_MAXLEV] = {}, *fS0[PT_MAXLEV] = {}, *fS1[PT_MAXLEV] = {}, *fS2[PT_MAXLEV] = {},
           *fRHS[PT_MAXLEV] = {}, *fres[PT_MAXLEV] = {};
     float* fcoef[PT_MAXLEV][6] = {};  // vis, vx, vz, vxz, vxxmzz, dt_stream in FP32
-    // levels ctop.. of the mixed cycle run in one thread-block cluster (pt_cluster.cuh), the coarsest
+    // levels ctop.. of the cycle run in one thread-block cluster (pt_cluster.cuh), the coarsest
     // solve too (ccoarse); level 1's smoothing as well on small grids (cl1).  Levels csolo.. are small
     // enough for one CTA, the coarsest solve with coarse_solo
     int ctop = PT_MAXLEV, csolo = PT_MAXLEV;

@@ -14,8 +14,10 @@
 #include <cstring>
 #include <vector>
 
+#include "pt_cluster.cuh"
 #include "pt_consts.cuh"
 #include "pt_exact.cuh"
+#include "pt_launch.cuh"
 
 namespace pt {
 
@@ -259,14 +261,17 @@ static int smoother_vis(Engine& E, const VisCtx& C, int l, int interpolate, VisS
 }
 
 // restrict_coefficients / restrict: full weighting onto coarse interior nodes
-__global__ void k_restrict(double* out, const double* in, Geo gc, Geo gf, int nxc, int nzc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1;
-    if (i > nxc - 1) return;
+__device__ __forceinline__ double restrict_at(const double* in, Geo gf, int i, int k) {
     int ii = 2 * i, kk = 2 * k;
     double corners = (in[gf.at(ii - 1, kk - 1)] + in[gf.at(ii - 1, kk + 1)] + in[gf.at(ii + 1, kk + 1)] + in[gf.at(ii + 1, kk - 1)]) / 16.0;
     double sides = (in[gf.at(ii - 1, kk)] + in[gf.at(ii, kk - 1)] + in[gf.at(ii + 1, kk)] + in[gf.at(ii, kk + 1)]) / 8.0;
     double centre = in[gf.at(ii, kk)] / 4.0;
-    out[gc.at(i, k)] = corners + sides + centre;
+    return corners + sides + centre;
+}
+__global__ void k_restrict(double* out, const double* in, Geo gc, Geo gf, int nxc, int nzc) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1;
+    if (i > nxc - 1) return;
+    out[gc.at(i, k)] = restrict_at(in, gf, i, k);
 }
 
 // viscosityBCs_initialize (iterative_solver.f90:636-664)
@@ -451,6 +456,7 @@ __global__ void __launch_bounds__(TG::NT) k_rkc_stage_fx(double* __restrict__ ou
                                                          double mewtc, int first, int ivis, double sz, ResFxK K) {
     __shared__ int2 X[TG::HT][TG::W];
     __shared__ int emax_s;
+    pdl_begin();
     const LevConst& L = cL[l];
     const int i0 = blockIdx.x * TG::TX + 1, k0 = blockIdx.y * TG::TZ + 1;
     const int emax = load_tile_fx<TG>(X, &emax_s, S1, g, i0, k0, L.nx, L.nz);
@@ -475,6 +481,7 @@ __global__ void __launch_bounds__(TG::NT) k_residual_fx64(double* __restrict__ r
                                                           StreamOp op, Geo g, int l, int ivis, ResFxK K) {
     __shared__ int2 X[TG::HT][TG::W];
     __shared__ int emax_s;
+    pdl_begin();
     const LevConst& L = cL[l];
     const int i0 = blockIdx.x * TG::TX + 1, k0 = blockIdx.y * TG::TZ + 1;
     const int emax = load_tile_fx<TG>(X, &emax_s, S, g, i0, k0, L.nx, L.nz);
@@ -530,8 +537,8 @@ static StreamOp stream_op(Engine& E, int l) {
 }
 
 // one RKC1 stage / one residual on level l: the exact-sum kernels when the stencils allow them
-static void launch_stage(Engine& E, int l, double* out, const double* S1, const double* S2, const double* S0,
-                         const StreamOp& op, double cS0, double mew, double vv, double mewtc, int first, double sz) {
+static int launch_stage(Engine& E, int l, double* out, const double* S1, const double* S2, const double* S0,
+                        const StreamOp& op, double cS0, double mew, double vv, double mewtc, int first, double sz) {
     const Geo& g = E.gl[l];
     const int ivis = E.cfg.ivis;
     if (E.res_int) {
@@ -539,35 +546,33 @@ static void launch_stage(Engine& E, int l, double* out, const double* S1, const 
         if (use_big_tiles(g.nx, g.nz)) {
             dim3 blk(TileBig::TX, TileBig::TY), grd(nblk(g.nx - 1, TileBig::TX), nblk(g.nz - 1, TileBig::TZ));
             auto kern = sq ? k_rkc_stage_fx<true, TileBig> : k_rkc_stage_fx<false, TileBig>;
-            PT_COUNT(), kern<<<grd, blk, 0, E.st>>>(out, S1, S2, S0, op, g, l, cS0, mew, vv, mewtc, first, ivis, sz,
-                                                    E.resfx[l]);
-        } else {
-            dim3 blk(TileSmall::TX, TileSmall::TY), grd(nblk(g.nx - 1, TileSmall::TX), nblk(g.nz - 1, TileSmall::TZ));
-            auto kern = sq ? k_rkc_stage_fx<true, TileSmall> : k_rkc_stage_fx<false, TileSmall>;
-            PT_COUNT(), kern<<<grd, blk, 0, E.st>>>(out, S1, S2, S0, op, g, l, cS0, mew, vv, mewtc, first, ivis, sz,
-                                                    E.resfx[l]);
+            return launch_pdl("k_rkc_stage_fx", kern, grd, blk, 0, E.st, out, S1, S2, S0, op, g, l, cS0, mew, vv, mewtc,
+                              first, ivis, sz, E.resfx[l]);
         }
-    } else {
-        dim3 gs(nblk(g.nx - 1, 128), g.nz - 1);
-        PT_COUNT(), k_rkc_stage<<<gs, 128, 0, E.st>>>(out, S1, S2, S0, op, g, l, cS0, mew, vv, mewtc, first, ivis, sz);
+        dim3 blk(TileSmall::TX, TileSmall::TY), grd(nblk(g.nx - 1, TileSmall::TX), nblk(g.nz - 1, TileSmall::TZ));
+        auto kern = sq ? k_rkc_stage_fx<true, TileSmall> : k_rkc_stage_fx<false, TileSmall>;
+        return launch_pdl("k_rkc_stage_fx", kern, grd, blk, 0, E.st, out, S1, S2, S0, op, g, l, cS0, mew, vv, mewtc, first,
+                          ivis, sz, E.resfx[l]);
     }
+    dim3 gs(nblk(g.nx - 1, 128), g.nz - 1);
+    PT_COUNT(), k_rkc_stage<<<gs, 128, 0, E.st>>>(out, S1, S2, S0, op, g, l, cS0, mew, vv, mewtc, first, ivis, sz);
+    return 0;
 }
-static void launch_residual(Engine& E, int l, double* res, const double* S, const StreamOp& op) {
+static int launch_residual(Engine& E, int l, double* res, const double* S, const StreamOp& op) {
     const Geo& g = E.gl[l];
     if (E.res_int) {
         const bool sq = E.resfx[l].square;
         if (use_big_tiles(g.nx, g.nz)) {
             dim3 blk(TileBig::TX, TileBig::TY), grd(nblk(g.nx - 1, TileBig::TX), nblk(g.nz - 1, TileBig::TZ));
             auto kern = sq ? k_residual_fx64<true, TileBig> : k_residual_fx64<false, TileBig>;
-            PT_COUNT(), kern<<<grd, blk, 0, E.st>>>(res, S, op, g, l, E.cfg.ivis, E.resfx[l]);
-        } else {
-            dim3 blk(TileSmall::TX, TileSmall::TY), grd(nblk(g.nx - 1, TileSmall::TX), nblk(g.nz - 1, TileSmall::TZ));
-            auto kern = sq ? k_residual_fx64<true, TileSmall> : k_residual_fx64<false, TileSmall>;
-            PT_COUNT(), kern<<<grd, blk, 0, E.st>>>(res, S, op, g, l, E.cfg.ivis, E.resfx[l]);
+            return launch_pdl("k_residual_fx64", kern, grd, blk, 0, E.st, res, S, op, g, l, E.cfg.ivis, E.resfx[l]);
         }
-    } else {
-        PT_COUNT(), k_residual<<<dim3(nblk(g.nx - 1, 128), g.nz - 1), 128, 0, E.st>>>(res, S, op, g, l, E.cfg.ivis);
+        dim3 blk(TileSmall::TX, TileSmall::TY), grd(nblk(g.nx - 1, TileSmall::TX), nblk(g.nz - 1, TileSmall::TZ));
+        auto kern = sq ? k_residual_fx64<true, TileSmall> : k_residual_fx64<false, TileSmall>;
+        return launch_pdl("k_residual_fx64", kern, grd, blk, 0, E.st, res, S, op, g, l, E.cfg.ivis, E.resfx[l]);
     }
+    PT_COUNT(), k_residual<<<dim3(nblk(g.nx - 1, 128), g.nz - 1), 128, 0, E.st>>>(res, S, op, g, l, E.cfg.ivis);
+    return 0;
 }
 
 // iterate_stream (RKC1 = 1, splitting = 0) + compute_residual.  The last stage writes straight
@@ -588,39 +593,374 @@ static int iterate_stream(Engine& E, int l, int want_sum) {
         const double* S0 = E.err[l];
         GraphTimer gt(E, 0, (l == 1 && want_sum) ? N : 0);
         int cur = 0;
-        launch_stage(E, l, buf[cur], S0, nullptr, nullptr, op, 0, 0, 0, E.K.mewt[1] * c, 1, sz);
+        const double* none = nullptr;
+        if (int rc = launch_stage(E, l, buf[cur], S0, none, none, op, 0, 0, 0, E.K.mewt[1] * c, 1, sz)) return rc;
         const double* Sm1 = buf[cur];
         const double* Sm2 = S0;
         for (int j = 2; j <= N; j++) {
             int nxt = (cur + 1) % 3;
             if (buf[nxt] == Sm2) nxt = (nxt + 1) % 3;
             double* out = (j == N) ? E.err[l] : buf[nxt];
-            launch_stage(E, l, out, Sm1, Sm2, S0, op, E.K.cc[j], E.K.mew[j], E.K.vv[j], E.K.mewt[j] * c, 0, sz);
+            if (int rc = launch_stage(E, l, out, Sm1, Sm2, S0, op, E.K.cc[j], E.K.mew[j], E.K.vv[j], E.K.mewt[j] * c, 0, sz))
+                return rc;
             Sm2 = Sm1;
             Sm1 = out;
             cur = nxt;
         }
         CKL("k_rkc_stage");
     }
-    launch_residual(E, l, E.res[l], E.err[l], op);
+    if (int rc = launch_residual(E, l, E.res[l], E.err[l], op)) return rc;
     CKL("k_residual");
     if (want_sum) return reduce_sum_abs_interior(E, E.res[l], g.nx, g.nz, g.pitch, E.dscal + 8);
     return 0;
 }
 
 // prolong (iterative_solver.f90:343-396): bilinear coarse correction added to the finer level
+__device__ __forceinline__ double prolong_at(const double* C, Geo gc, int i, int k) {
+    if (!(i & 1) && !(k & 1)) return C[gc.at(i / 2, k / 2)];
+    if (!(i & 1)) return (C[gc.at(i / 2, (k - 1) / 2)] + C[gc.at(i / 2, (k + 1) / 2)]) / 2.0;
+    if (!(k & 1)) return (C[gc.at((i - 1) / 2, k / 2)] + C[gc.at((i + 1) / 2, k / 2)]) / 2.0;
+    return (C[gc.at((i - 1) / 2, (k - 1) / 2)] + C[gc.at((i + 1) / 2, (k - 1) / 2)] + C[gc.at((i + 1) / 2, (k + 1) / 2)] +
+            C[gc.at((i - 1) / 2, (k + 1) / 2)]) / 4.0;
+}
 __global__ void k_prolong(double* F, const double* C, Geo gf, Geo gc, int nxf, int nzf) {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1;
     if (i > nxf - 1) return;
-    double add;
-    if (!(i & 1) && !(k & 1)) add = C[gc.at(i / 2, k / 2)];
-    else if (!(i & 1)) add = (C[gc.at(i / 2, (k - 1) / 2)] + C[gc.at(i / 2, (k + 1) / 2)]) / 2.0;
-    else if (!(k & 1)) add = (C[gc.at((i - 1) / 2, k / 2)] + C[gc.at((i + 1) / 2, k / 2)]) / 2.0;
-    else
-        add = (C[gc.at((i - 1) / 2, (k - 1) / 2)] + C[gc.at((i + 1) / 2, (k - 1) / 2)] +
-               C[gc.at((i + 1) / 2, (k + 1) / 2)] + C[gc.at((i - 1) / 2, (k + 1) / 2)]) / 4.0;
-    size_t o = gf.at(i, k);
-    F[o] = F[o] + add;
+    const size_t o = gf.at(i, k);
+    F[o] = F[o] + prolong_at(C, gc, i, k);
+}
+
+// ------------------------------------------------------------------ levels in one cluster
+// A stretch of the FP64 cycle on levels that fit one cluster (pt_cluster.cuh): the entering restriction
+// or prolongation, the RKC1 stages, the residual that the next coarser level restricts; the coarsest
+// level by the explicit inverse.  The stencil sums are exact, as in k_rkc_stage_fx.  A stage has three
+// parts, each with the split that keeps its chain short (a few warps an SM: latency is the bound, at
+// the upper end the FP64 pipe with its two lanes a clock an SM):
+//   * the CTA takes the largest exponent of its window and writes the window, images included, as
+//     62-bit fixed point X = Xh 2^31 + Xl (each thread keeps its few cells' places for the visit);
+//   * warps form the derivative groups, five warps (or, with more tiles than that leaves warps for,
+//     two) to a tile of 32 nodes: integer multiply-adds with constant weights, one rounding of the
+//     78-bit sum to FP64 by integer operations, as adding its two exact halves would round it, and the
+//     product with the node's coefficient; one more warp the rest of the recurrence;
+//   * a thread a node adds these up and publishes the value.
+// An FP64 instruction keeps a scheduler's pipe busy for some 64 cycles, so the products and the
+// recurrence go to the warps that have room beside their integer work.
+struct DLevel {
+    Geo g;
+    double *e, *rhs, *res;
+    const double *vis, *vx, *vz, *vxz, *vxxmzz, *dtst;
+    ResFxK K;
+};
+struct DRun {
+    DLevel L[PT_MAXLEV];
+    cl::Visit v[cl::kMaxVisits];
+    int nv, N, ivis, ngc;
+    double sz;
+    double cc[64], mew[64], vv[64], mewtc[64];
+    const double *G, *RowB;
+};
+constexpr int kDOwn = cl::kThreads / 2, kDGroups = 10;  // nodes of a CTA at most; derivative groups at most
+constexpr int kDTiles = kDOwn / 32, kDParts = 5;         // its tiles; warps to a tile at most
+constexpr int kDCells = 5;  // window cells of a thread at most: 8 rows of 263, with strips of two rows
+static size_t cluster_bytes_d(int ngc) {
+    return sizeof(double) * (2 * (size_t)cl::kWindow + (kDGroups + kDParts + 5) * (size_t)kDOwn + (size_t)ngc) +
+           sizeof(int2) * (size_t)cl::kWindow;
+}
+
+// integer weight of the point (dx, dz) in derivative group g (tile_apply_A's sums; SQUARE: combined)
+__host__ __device__ constexpr int id1(int j) { return j == -2 ? 1 : j == -1 ? -8 : j == 1 ? 8 : j == 2 ? -1 : 0; }
+__host__ __device__ constexpr int id2(int j) { return j == 0 ? -30 : j == 1 || j == -1 ? 16 : j == 2 || j == -2 ? -1 : 0; }
+__host__ __device__ constexpr int id3(int j) {
+    return j == -3 ? 1 : j == -2 ? -8 : j == -1 ? 13 : j == 1 ? -13 : j == 2 ? 8 : j == 3 ? -1 : 0;
+}
+__host__ __device__ constexpr int id4(int j) {
+    return j == 0 ? 56 : j == 1 || j == -1 ? -39 : j == 2 || j == -2 ? 12 : -1;
+}
+template <bool SQUARE>
+__host__ __device__ constexpr int group_weight(int g, int dx, int dz) {
+    const int x4 = dz == 0 ? id4(dx) : 0, z4 = dx == 0 ? id4(dz) : 0, x2 = dz == 0 ? id2(dx) : 0, z2 = dx == 0 ? id2(dz) : 0;
+    const int x3 = dz == 0 ? id3(dx) : 0, z3 = dx == 0 ? id3(dz) : 0;
+    const int i11 = id1(dx) * id1(dz), i12 = id1(dx) * id2(dz), i21 = id2(dx) * id1(dz), i22 = id2(dx) * id2(dz);
+    if (SQUARE)
+        return g == 0 ? 24 * (x4 + z4) + 2 * i22 : g == 1 ? x2 - z2 : g == 2 ? i11 : g == 3 ? 18 * x3 + i12 : 18 * z3 + i21;
+    return g == 0 ? x4 : g == 1 ? z4 : g == 2 ? i22 : g == 3 ? x2 : g == 4 ? z2 : g == 5 ? i11 : g == 6 ? x3 : g == 7 ? i12
+           : g == 8 ? z3 : i21;
+}
+
+// (h 2^31 + l) 2^-s rounded once to FP64 (|h|, |l| < 2^52, result normal or zero); s = 1084 - emax
+__device__ __forceinline__ double hl_rounded(long long h, long long l, int emax) {
+    long long hi = h + (l >> 31);  // hi 2^31 + lo, 0 <= lo < 2^31
+    unsigned lo = (unsigned)l & 0x7FFFFFFFu;
+    const bool neg = hi < 0;
+    if (neg) {
+        hi = lo ? ~hi : -hi;
+        lo = (0x80000000u - lo) & 0x7FFFFFFFu;
+    }
+    if (hi == 0) {
+        if (lo == 0) return 0.0;
+        hi = (long long)lo;  // as hi 2^31 with the exponent 31 lower
+        lo = 0;
+        emax -= 31;
+    }
+    // the 64 leading bits of the sum, and whether any bit below them is set
+    const int lz = __clzll(hi);
+    unsigned long long A = (unsigned long long)hi << lz;
+    bool sticky = false;
+    if (lz >= 31) {
+        A |= (unsigned long long)lo << (lz - 31);
+    } else {
+        A |= lo >> (31 - lz);
+        sticky = (lo & ((1u << (31 - lz)) - 1u)) != 0;
+    }
+    unsigned long long q = A >> 11;
+    const unsigned rem = (unsigned)A & 0x7FFu;
+    if (rem > 0x400u || (rem == 0x400u && (sticky || (q & 1ull)))) q++;
+    const long long ex = 1023 + 52 + 42 - lz - (1084 - emax);
+    if (ex <= 0) return 0.0;  // below the normal range (S itself near underflow)
+    return __longlong_as_double((long long)(((unsigned long long)neg << 63) | (((unsigned long long)(ex - 1) << 52) + q)));
+}
+
+// sum of derivative group G at cell x of the fixed-point window, rounded
+template <bool SQUARE, int G>
+__device__ __forceinline__ double group_sum(const int2* x, int emax) {
+    long long h[2] = {0, 0}, l[2] = {0, 0};
+    int n = 0;
+#pragma unroll
+    for (int dz = -3; dz <= 3; dz++)
+#pragma unroll
+        for (int dx = -3; dx <= 3; dx++) {
+            const bool block = dx >= -2 && dx <= 2 && dz >= -2 && dz <= 2;
+            const int w = block || dx == 0 || dz == 0 ? group_weight<SQUARE>(G, dx, dz) : 0;
+            if (w == 0) continue;
+            const int2 v = x[dz * cl::kPitch + dx];
+            h[n & 1] += (long long)w * v.x;
+            l[n & 1] += (long long)w * v.y;
+            n++;
+        }
+    return hl_rounded(h[0] + h[1], l[0] + l[1], emax);
+}
+// groups G .. G + N - 1, each times its coefficient (w: kDOwn apart)
+template <bool SQUARE, int G, int N>
+__device__ __forceinline__ double group_part(const int2* x, int emax, const double* w) {
+    double a = w[G * kDOwn] * group_sum<SQUARE, G>(x, emax);
+    if constexpr (N > 1) a += group_part<SQUARE, G + 1, N - 1>(x, emax, w);
+    return a;
+}
+
+template <bool SQUARE>
+__global__ void __launch_bounds__(cl::kThreads, 1) k_cycle_cluster_d(const __grid_constant__ DRun P) {
+    constexpr int NG = SQUARE ? 5 : 10;
+    extern __shared__ __align__(16) double dm[];
+    __shared__ uint64_t bars[2];
+    __shared__ double cheb[64][4];
+    __shared__ int emax_s[cl::kWarps];
+    // of each node: the coefficients of its groups, its parts of a stage's sum, then S0, dt rhs, dt
+    // and a stage's recurrence without A and its factor of A
+    double *const W = dm + 2 * cl::kWindow, *const D = W + kDGroups * kDOwn, *const S0s = D + kDParts * kDOwn;
+    double *const drhs = S0s + kDOwn, *const dts = drhs + kDOwn;
+    double *const B = dts + kDOwn, *const M = B + kDOwn, *const cb = M + kDOwn;  // cb: the coarsest right-hand side
+    int2* const X = reinterpret_cast<int2*>(cb + P.ngc);
+    if (threadIdx.x < 64) {
+        cheb[threadIdx.x][0] = P.cc[threadIdx.x];
+        cheb[threadIdx.x][1] = P.mew[threadIdx.x];
+        cheb[threadIdx.x][2] = P.vv[threadIdx.x];
+        cheb[threadIdx.x][3] = P.mewtc[threadIdx.x];
+    }
+    const int c = (int)cl::rank(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    cl::Exchange ex;
+    ex.init(bars);
+    for (int n = 0; n < P.nv; n++) {
+        const int l = P.v[n].level, fl = P.v[n].flags;
+        const DLevel& L = P.L[l];
+        const Geo g = L.g;
+        if (fl & cl::kCoarse) {  // x = G b, a warp per row over the cluster (k_coarse_apply's sums)
+            const Geo gf = P.L[l - 1].g;
+            const int N1 = g.nz + 1, nn = (g.nx + 1) * N1, nk = g.nz - 1, ni = (g.nx - 1) * nk;
+            for (int q = threadIdx.x; q < nn; q += cl::kThreads) {
+                const int ip = q / N1, kp = q - ip * N1;
+                cb[q] = ip > 0 && ip < g.nx && kp > 0 && kp < g.nz ? restrict_at(P.L[l - 1].res, gf, ip, kp) * P.RowB[q] : 0.0;
+            }
+            __syncthreads();
+            for (int r = c * cl::kWarps + warp; r < ni; r += cl::kCtas * cl::kWarps) {
+                const int ip = r / nk + 1, kp = r - (ip - 1) * nk + 1;
+                const double* row = P.G + (size_t)(ip * N1 + kp) * nn;
+                double a = 0.0;
+                for (int q = lane; q < nn; q += 32) a += row[q] * cb[q];
+                for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                if (lane == 0) L.e[g.at(ip, kp)] = a;  // (its walls stay zero, its images are not read)
+            }
+            cl::sync();
+            continue;
+        }
+        cl::Strip s;
+        s.set(g.nz, c, false);
+        const int segs = cl::Strip::segments(g.nx), tiles = s.rows * segs, cols = g.nx + 2 * cl::kReach + 1;
+        const float inv_segs = __frcp_rn((float)segs);
+        // cell of lane's node in tile t (32 columns of a row); lanes past the row take its last node
+        auto tile_cell = [&](int t) {
+            const int r = (int)(((float)t + 0.5f) * inv_segs);
+            return s.at(min((t - r * segs) * 32 + lane + 1, g.nx - 1), s.k0 + r);
+        };
+        // the thread's node: its coefficients, right-hand side and place
+        const int r = (int)(((float)warp + 0.5f) * inv_segs), i = (warp - r * segs) * 32 + lane + 1, k = s.k0 + r;
+        const bool on = warp < tiles && i <= g.nx - 1;
+        const size_t o = on ? g.at(i, k) : 0;
+        const int m = on ? s.at(i, k) : 0;
+        double rhs = 0.0, S0 = 0.0;
+        if (on) {
+            double w[NG];
+            const double* K = L.K.k;
+            const double vis = L.vis[o];
+            double c1 = 0.0, c2 = 0.0, c3 = 0.0, c4 = 0.0;
+            if (P.ivis != 0) {
+                c1 = L.vxxmzz[o];
+                c2 = L.vxz[o];
+                c3 = L.vx[o];
+                c4 = L.vz[o];
+            }
+            const double dt = L.dtst[o];
+            if (!(fl & cl::kZero)) S0 = L.e[o];
+            if (fl & cl::kRestrict) {
+                rhs = restrict_at(P.L[l - 1].res, P.L[l - 1].g, i, k);
+                L.rhs[o] = rhs;
+            } else {
+                rhs = L.rhs[o];
+            }
+            if (fl & cl::kProlong) S0 = S0 + prolong_at(P.L[l + 1].e, P.L[l + 1].g, i, k);
+            if constexpr (SQUARE) {
+                w[0] = K[0] * vis; w[1] = K[1] * c1; w[2] = K[2] * c2; w[3] = K[3] * c3; w[4] = K[4] * c4;
+            } else {
+                w[0] = K[0] * vis; w[1] = K[1] * vis; w[2] = 2.0 * K[2] * vis; w[3] = K[3] * c1; w[4] = -K[4] * c1;
+                w[5] = 4.0 * K[5] * c2; w[6] = 2.0 * K[6] * c3; w[7] = 2.0 * K[7] * c3; w[8] = 2.0 * K[8] * c4;
+                w[9] = 2.0 * K[9] * c4;
+            }
+#pragma unroll
+            for (int G = 0; G < NG; G++) W[G * kDOwn + threadIdx.x] = w[G];
+            S0s[threadIdx.x] = S0;
+            drhs[threadIdx.x] = dt * rhs;
+            dts[threadIdx.x] = dt;
+        }
+        // the thread's window cells: where each goes (upper half) and where it comes from, with the sign
+        // of the image; -1 where the window stays zero (walls, rows past the images)
+        int place[kDCells];
+        {
+            const int cells = s.rows ? (s.rows + 2 * cl::kReach) * cols : 0;
+            const float inv_cols = __frcp_rn((float)cols);
+#pragma unroll
+            for (int q = 0; q < kDCells; q++) {
+                const int cell = (int)threadIdx.x + q * cl::kThreads;
+                place[q] = -1;
+                if (cell >= cells) continue;
+                const int wr = (int)(((float)cell + 0.5f) * inv_cols), wc = cell - wr * cols;
+                const int ci = wc - cl::kReach, ck = s.k0 - cl::kReach + wr;
+                const int mi = mirror_idx(ci, g.nx), mk = mirror_idx(ck, g.nz);
+                if (mi <= 0 || mi >= g.nx || mk <= 0 || mk >= g.nz) continue;
+                const int neg = (mi != ci) != (mk != ck && P.sz < 0.0);
+                place[q] = (wr * cl::kPitch + wc) << 16 | s.at(mi, mk) << 1 | neg;
+            }
+        }
+        for (int q = threadIdx.x; q < (s.R + 2 * cl::kReach) * cl::kPitch; q += cl::kThreads) X[q] = make_int2(0, 0);
+        ex.bytes = (uint32_t)(s.rows_received(g.nz) * (g.nx - 1)) * (uint32_t)sizeof(double);
+        cl::Outlet<double> out;
+        out.set(s, dm, bars, m, on ? s.readers_up(r) : 0, on ? s.readers_down(r) : 0);
+        cl::sync();  // every CTA has left its windows of the last visit (and, the first time, its mbarriers are ready)
+        auto publish = [&](int q, double v) {
+            if (on) {
+                dm[q * cl::kWindow + m] = v;
+                if (out.up | out.down) out.put_remote(q, v);
+            }
+            ex.arrive(q);
+        };
+        // the parts of A of window q at every node of the strip, into D
+        const bool fine = tiles * kDParts <= cl::kWarps;
+        // the warp's part (part major: the long ones go to different schedulers), its tile's nodes
+        const int part = warp < tiles ? 0 : fine ? warp / max(tiles, 1) : 1, part_tile = warp - part * tiles;
+        const bool has_part = tiles > 0 && part_tile < tiles && part < (fine ? kDParts : 2);
+        const int part_cell = has_part ? tile_cell(part_tile) : 0, part_node = has_part ? part_tile * 32 + lane : 0;
+        const int ncell = (s.rows ? (s.rows + 2 * cl::kReach) * cols : 0) > cl::kThreads ? kDCells : 1;
+        auto groups = [&](int q) {
+            unsigned long long b[kDCells];
+            int em = 0;
+#pragma unroll
+            for (int j = 0; j < kDCells; j++) {
+                if (j >= ncell) break;
+                b[j] = 0;
+                if (place[j] >= 0)
+                    b[j] = (unsigned long long)__double_as_longlong(dm[q * cl::kWindow + (place[j] >> 1 & 0x7FFF)]);
+                em = max(em, (int)(b[j] >> 52) & 0x7FF);
+            }
+            em = __reduce_max_sync(0xffffffffu, em);
+            if (lane == 0) emax_s[warp] = em;
+            __syncthreads();
+            const int emax = __reduce_max_sync(0xffffffffu, emax_s[lane & (cl::kWarps - 1)]);
+#pragma unroll
+            for (int j = 0; j < kDCells; j++) {
+                if (j >= ncell) break;
+                if (place[j] >= 0) {
+                    const long long f = fixed_point(b[j], emax), v = place[j] & 1 ? -f : f, h = v >> 31;  // floor
+                    X[place[j] >> 16] = make_int2((int)h, (int)(v - (h << 31)));
+                }
+            }
+            __syncthreads();
+            if (has_part) {
+                const int2* x = X + part_cell;
+                const double* w = W + part_node;
+                double d;
+                if (fine) {
+                    switch (part) {
+                        case 0: d = group_part<SQUARE, SQUARE ? 0 : 0, SQUARE ? 1 : 2>(x, emax, w); break;
+                        case 1: d = group_part<SQUARE, SQUARE ? 1 : 2, SQUARE ? 1 : 2>(x, emax, w); break;
+                        case 2: d = group_part<SQUARE, SQUARE ? 2 : 4, SQUARE ? 1 : 2>(x, emax, w); break;
+                        case 3: d = group_part<SQUARE, SQUARE ? 3 : 6, SQUARE ? 1 : 2>(x, emax, w); break;
+                        default: d = group_part<SQUARE, SQUARE ? 4 : 8, SQUARE ? 1 : 2>(x, emax, w);
+                    }
+                } else if (part == 0) {
+                    d = group_part<SQUARE, 0, SQUARE ? 2 : 5>(x, emax, w);
+                } else {
+                    d = group_part<SQUARE, SQUARE ? 2 : 5, SQUARE ? 3 : 5>(x, emax, w);
+                }
+                D[part * kDOwn + part_node] = emax == 0x7FF ? __longlong_as_double(0x7FF8000000000000ll) : d;
+            }
+        };
+        auto sum = [&]() {  // A at the thread's node
+            const double* d = D + threadIdx.x;
+            return fine ? ((d[0] + d[kDOwn]) + (d[2 * kDOwn] + d[3 * kDOwn])) + d[4 * kDOwn] : d[0] + d[kDOwn];
+        };
+        // what a stage adds to the sum, by the last warps, whose parts are the short ones or none
+        const int spare = cl::kWarps - 1 - warp, spare_cell = spare < tiles ? tile_cell(spare) : 0;
+        publish(0, S0);
+        int cur = 0;
+        for (int j = 1; j <= P.N; j++) {
+            const bool last = j == P.N;
+            groups(cur);
+            if (spare < tiles) {  // cc S0 + mew S_{j-1} + vv S_{j-2} + mewt c dt rhs (stage 1: S0 + ..)
+                const int q = spare * 32 + lane, cell = spare_cell;
+                double base = dm[cur * cl::kWindow + cell];
+                if (j > 1) base = fma(cheb[j][1], base, fma(cheb[j][2], dm[(cur ^ 1) * cl::kWindow + cell], cheb[j][0] * S0s[q]));
+                B[q] = fma(cheb[j][3], drhs[q], base);
+                M[q] = -cheb[j][3] * dts[q];
+            }
+            __syncthreads();
+            double v = 0.0;
+            if (on) {
+                v = fma(M[threadIdx.x], sum(), B[threadIdx.x]);
+                if (last) {
+                    if (!ex.ok) v = __longlong_as_double(0x7FF8000000000000ll);  // a wait ran out: NaN, reported by the host
+                    L.e[o] = v;
+                }
+            }
+            if (!last || (fl & cl::kResidual)) {
+                cur ^= 1;
+                publish(cur, v);
+            }
+        }
+        if (fl & cl::kResidual) {
+            groups(cur);
+            __syncthreads();
+            if (on) L.res[o] = rhs - sum();
+        }
+        cl::sync();  // the correction and the residual are in global memory
+    }
 }
 
 static int prolong(Engine& E, int lc) {
@@ -1112,14 +1452,14 @@ int coarse_band_solve(Engine& E) {
 }
 
 int residual_level1_nosum(Engine& E) {
-    launch_residual(E, 1, E.res[1], E.err[1], stream_op(E, 1));
+    if (int rc = launch_residual(E, 1, E.res[1], E.err[1], stream_op(E, 1))) return rc;
     CKL("k_residual");
     return 0;
 }
 
 int residual_level1(Engine& E) {
     const Geo& g = E.gl[1];
-    launch_residual(E, 1, E.res[1], E.err[1], stream_op(E, 1));
+    if (int rc = launch_residual(E, 1, E.res[1], E.err[1], stream_op(E, 1))) return rc;
     CKL("k_residual");
     return reduce_sum_abs_interior(E, E.res[1], g.nx, g.nz, g.pitch, E.dscal + 8);
 }
@@ -1166,6 +1506,82 @@ int mg_setup_solve(Engine& E) {
     return 0;
 }
 
+// levels ctop.. run in one cluster, where their nodes fit its arrays and the coarsest solve is a small
+// product with the explicit inverse
+static int cluster_setup_d(Engine& E) {
+    E.ctop = E.grids + 1;
+    if (E.cfg.precision != PT_PREC_FP64 || E.cfg.Nmulti != 1 || !E.res_int || !E.Ginv || E.ngc > 700) return 0;
+    const size_t bytes = cluster_bytes_d(E.ngc);
+    for (auto k : {k_cycle_cluster_d<true>, k_cycle_cluster_d<false>}) {
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
+            return fail(PT_ERR_CUDA, "cluster kernel attributes");
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        cl::cluster_launch(cfg, at, bytes, E.st);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess || fit < 1) {
+            (void)cudaGetLastError();  // no room for a cluster of this size: the per-stage kernels run
+            return 0;
+        }
+    }
+    auto fits = [&](int l) {
+        const Geo& g = E.gl[l];
+        const int R = cl::Strip::rows_per_cta(g.nz);
+        const int cols = g.nx + 2 * cl::kReach + 1;
+        return R * cl::Strip::segments(g.nx) <= kDTiles && cols <= cl::kPitch &&
+               (R + 2 * cl::kReach) * cols <= kDCells * cl::kThreads;
+    };
+    E.ctop = E.grids;
+    while (E.ctop > 2 && fits(E.ctop - 1)) E.ctop--;
+    if (E.ctop == E.grids) E.ctop = E.grids + 1;  // nothing but the coarsest level
+    return 0;
+}
+
+// the entries p.. of the schedule on levels ctop.. as one launch; *last receives the last of them
+static int cluster_run_d(Engine& E, const int* multi, int nsteps, int p, int* last) {
+    DRun R{};
+    for (; p <= nsteps && multi[p] >= E.ctop && R.nv < cl::kMaxVisits; p++) {
+        const int l = multi[p];
+        cl::Visit& v = R.v[R.nv++];
+        v.level = (signed char)l;
+        if (l == E.grids) {
+            v.flags = cl::kCoarse;
+        } else {
+            if (multi[p - 1] < l) {
+                v.flags |= cl::kRestrict;
+                if (E.cfg.mg_scheme == PT_MG_CORRECTION) v.flags |= cl::kZero;
+            } else {
+                v.flags |= cl::kProlong;
+            }
+            if (multi[p + 1] > l) v.flags |= cl::kResidual;
+        }
+        *last = p;
+    }
+    for (int l = 1; l <= E.grids; l++) {
+        const StreamOp op = stream_op(E, l);
+        R.L[l] = DLevel{E.gl[l], E.err[l], E.RHS[l], E.res[l], op.vis, op.vx, op.vz, op.vxz, op.vxxmzz, op.dtst, E.resfx[l]};
+    }
+    R.N = E.cfg.nstageS;
+    R.ivis = E.cfg.ivis;
+    R.ngc = E.ngc;
+    R.sz = E.cfg.Vbc == 0 ? -1.0 : 1.0;
+    for (int j = 1; j <= R.N; j++) {
+        R.cc[j] = E.K.cc[j];
+        R.mew[j] = E.K.mew[j];
+        R.vv[j] = E.K.vv[j];
+        R.mewtc[j] = E.K.mewt[j] * E.cfg.c_2;
+    }
+    R.G = E.Ginv;
+    R.RowB = E.RowB;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cl::cluster_launch(cfg, at, cluster_bytes_d(E.ngc), E.st);
+    PT_COUNT();
+    return cuda_check(cudaLaunchKernelEx(&cfg, E.resfx[1].square ? k_cycle_cluster_d<true> : k_cycle_cluster_d<false>, R),
+                      "k_cycle_cluster_d");
+}
+
 // One multigrid cycle of the reference's schedule, split where the reference tests convergence
 // (after the level-1 smoothing pass, iterative_solver.f90:313-315).  Part A: level-1 smoothing,
 // residual and sum|r|.  Part B: the rest of the schedule (restrict, coarse visits, coarse solve,
@@ -1179,6 +1595,10 @@ static int cycle_part(Engine& E, int part) {
     const int* multi = v ? E.mmulti : E.multi;
     if (part == 0) return iterate_stream(E, 1, 1);
     for (int p = 2; p <= nsteps; p++) {
+        if (multi[p] >= E.ctop) {  // (the way out is up: the coarsest level is among them)
+            if ((rc = cluster_run_d(E, multi, nsteps, p, &p)) || (rc = prolong(E, multi[p]))) return rc;
+            continue;
+        }
         const int level = multi[p];
         if (multi[p - 1] < multi[p]) {
             if ((rc = compute_RHS(E, level))) return rc;
@@ -1348,7 +1768,7 @@ int mg_alloc(Engine& E) {
         CK(cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)inv_smem(E.ngc, E.kl, E.ku)));
     }
-    return 0;
+    return cluster_setup_d(E);
 }
 
 // ------------------------------------------------------------------ learned-guess support
@@ -1401,7 +1821,7 @@ int coarse_scale_fit(Engine& E, double* alpha) {
                                                                                    gc.nz, 1 << (L - 1));
     CKL("k_inject");
     if (int rc = enforce_bcs_stream(E, L, E.err[L])) return rc;
-    launch_residual(E, L, E.res[L], E.err[L], stream_op(E, L));
+    if (int rc = launch_residual(E, L, E.res[L], E.err[L], stream_op(E, L))) return rc;
     PT_COUNT(), k_fit_rows<<<gc.nz - 1, 128, 0, E.st>>>(E.RHS[L], E.res[L], gc, gc.nx, E.red);
     CKL("coarse_scale_fit");
     std::vector<double> part(2 * (size_t)(gc.nz - 1));

@@ -21,35 +21,9 @@
 #include "pt_cluster.cuh"
 #include "pt_consts.cuh"
 #include "pt_exact.cuh"
+#include "pt_launch.cuh"
 
 namespace pt {
-
-// Programmatic dependent launch: every kernel of the mixed cycle starts by waiting for its
-// predecessor grid (griddepcontrol.wait returns once that grid has completed and its writes are
-// visible; it is a no-op for a kernel launched without the attribute) and then lets its own
-// successor be scheduled.  The successor's launch latency hides behind this kernel's run, which
-// matters on the coarse levels where each stage kernel lasts a couple of microseconds.
-__device__ __forceinline__ void pdl_begin() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-template <typename... KArgs, typename... Args>
-static int launch_pdl(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                      Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    PT_COUNT();
-    return cuda_check(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...), what);
-}
 
 // Per-level stencils with the grid spacing folded in (FP32 and FP64 copies): no division and no
 // FP64->FP32 conversion in the kernels (both run on the FP64 pipe of this part).
@@ -423,7 +397,7 @@ __global__ void k_res_to_f32(float* out, const double* in, size_t n) {
 // next coarser level restricts; the coarsest level by the explicit inverse.
 // A thread owns one node for a whole visit and keeps what belongs to it in registers: the 29 weights
 // of A there (the operator with its five coefficient fields folded in once per visit), F0, Y0 and D_{j-2}.
-// A stage is then 29 shared loads and 29 multiply-adds per thread.  With one to eight warps per
+// A stage is then 29 shared loads, 28 differences and 29 multiply-adds per thread.  With one to eight warps per
 // scheduler it is bound by the latency of that chain and of one exchange, so one node per thread and
 // 32 warps rather than two nodes and 16: the same 1,024 nodes a CTA with half the chain.
 struct FLevel {
@@ -467,7 +441,10 @@ __host__ __device__ constexpr float fd4(int j) {
 }
 
 // The weights of A at node (i, k) from its coefficients (vis, vxxmzz, vxz, vx, vz in c) and the level's
-// spacings h.  The ghost cells' share is folded onto the nodes that they mirror (antisymmetric across
+// spacings h.  A is applied to differences from the node's own value, which for a smooth correction are
+// exact and small: on the values themselves the rounding of the weights, a factor h k larger, would
+// swamp A of a smooth mode.  The weights of a stencil add up to zero, so the middle one takes what
+// folding adds to the sum.  The ghost cells' share is folded onto the nodes that they mirror (antisymmetric across
 // the side walls, sign sz across top and bottom; every mirror node of a stencil lies in the stencil),
 // so that the windows hold no images.
 __device__ __forceinline__ void make_weights(float (&w)[kPts], const float (&c)[5], const float* h, int i, int k, int nx,
@@ -491,28 +468,36 @@ __device__ __forceinline__ void make_weights(float (&w)[kPts], const float (&c)[
             w[pt_index(0, j)] += az - fd2(j) * z2;
         }
     }
+    float folded = 0.0f;  // what folding adds to the sum of the weights
+    auto fold = [&](bool yes, int to, int from, float sign) {
+        if (!yes) return;
+        const float x = sign * w[from];
+        w[to] += x;
+        folded += x;
+    };
     if (__any_sync(0xffffffffu, i <= 2 || i >= nx - 2)) {
 #pragma unroll
         for (int z = -2; z <= 2; z++) {
-            if (i == 1) w[pt_index(0, z)] -= w[pt_index(-2, z)];
-            if (i == nx - 1) w[pt_index(0, z)] -= w[pt_index(2, z)];
+            fold(i == 1, pt_index(0, z), pt_index(-2, z), -1.0f);
+            fold(i == nx - 1, pt_index(0, z), pt_index(2, z), -1.0f);
         }
-        if (i == 1) w[pt_index(1, 0)] -= w[pt_index(-3, 0)];
-        if (i == 2) w[pt_index(-1, 0)] -= w[pt_index(-3, 0)];
-        if (i == nx - 1) w[pt_index(-1, 0)] -= w[pt_index(3, 0)];
-        if (i == nx - 2) w[pt_index(1, 0)] -= w[pt_index(3, 0)];
+        fold(i == 1, pt_index(1, 0), pt_index(-3, 0), -1.0f);
+        fold(i == 2, pt_index(-1, 0), pt_index(-3, 0), -1.0f);
+        fold(i == nx - 1, pt_index(-1, 0), pt_index(3, 0), -1.0f);
+        fold(i == nx - 2, pt_index(1, 0), pt_index(3, 0), -1.0f);
     }
     if (k <= 2 || k >= nz - 2) {
 #pragma unroll
         for (int x = -2; x <= 2; x++) {
-            if (k == 1) w[pt_index(x, 0)] += sz * w[pt_index(x, -2)];
-            if (k == nz - 1) w[pt_index(x, 0)] += sz * w[pt_index(x, 2)];
+            fold(k == 1, pt_index(x, 0), pt_index(x, -2), sz);
+            fold(k == nz - 1, pt_index(x, 0), pt_index(x, 2), sz);
         }
-        if (k == 1) w[pt_index(0, 1)] += sz * w[pt_index(0, -3)];
-        if (k == 2) w[pt_index(0, -1)] += sz * w[pt_index(0, -3)];
-        if (k == nz - 1) w[pt_index(0, -1)] += sz * w[pt_index(0, 3)];
-        if (k == nz - 2) w[pt_index(0, 1)] += sz * w[pt_index(0, 3)];
+        fold(k == 1, pt_index(0, 1), pt_index(0, -3), sz);
+        fold(k == 2, pt_index(0, -1), pt_index(0, -3), sz);
+        fold(k == nz - 1, pt_index(0, -1), pt_index(0, 3), sz);
+        fold(k == nz - 2, pt_index(0, 1), pt_index(0, 3), sz);
     }
+    w[pt_index(0, 0)] = folded;
 }
 
 // the residual at node (i, k) in FP64 arithmetic on the correction in window y
@@ -690,13 +675,11 @@ __global__ void __launch_bounds__(cl::kThreads, 1) k_cycle_cluster_f(const __gri
         float A = 0.0f, own = 0.0f;
         auto apply = [&](int q) {  // A of window q at the node, and the window's value there
             const float* x = m + q * cl::kWindow;
-            float a[3] = {};
+            own = *x;
+            float a[3] = {w[pt_index(0, 0)] * own, 0.0f, 0.0f};
 #pragma unroll
-            for (int j = 0; j < kPts; j++) {
-                const float v = x[pt_dz(j) * cl::kPitch + pt_dx(j)];
-                a[j % 3] += w[j] * v;
-                if (j == pt_index(0, 0)) own = v;
-            }
+            for (int j = 0; j < kPts; j++)
+                if (j != pt_index(0, 0)) a[j % 3] += w[j] * (x[pt_dz(j) * cl::kPitch + pt_dx(j)] - own);
             A = (a[0] + a[1]) + a[2];
         };
         auto publish = [&](int q, float v) {

@@ -49,3 +49,38 @@ def test_cluster_levels_contract_like_the_fp64_cycle(kind, nx, nz, grids, cycle,
     assert abs(out[PT_PREC_MIXED][0] - out[PT_PREC_FP64][0]) <= 1 + out[PT_PREC_FP64][0] // 10
     assert rel_err(out[PT_PREC_MIXED][1], out[PT_PREC_FP64][1]) < 1e-4
     assert np.isfinite(out[PT_PREC_MIXED][1]).all()
+
+
+@pytest.mark.parametrize("kind,nx,nz,grids,cycle,vbc,scheme", [
+    ("iso", 32, 32, 3, PT_CYCLE_REFERENCE, 0, 0),    # level 2 of 16x16: strips of one row, one CTA idle
+    ("chem", 96, 48, 3, PT_CYCLE_REFERENCE, 1, 0),   # rigid walls, two rows a strip, coarsest solve over the cluster
+    ("chem", 128, 128, 6, PT_CYCLE_REFERENCE, 0, 0),  # stale corrections kept between visits
+    ("depth", 256, 64, 4, PT_CYCLE_REFERENCE, 0, 1),  # four column segments
+    ("depth", 48, 256, 4, PT_CYCLE_V, 1, 1),          # tall: eight rows a strip
+    ("chem", 112, 80, 4, PT_CYCLE_REFERENCE, 0, 0),   # unequal spacings: ten derivative groups
+])
+def test_fp64_cluster_levels_match_the_reference_rounding(kind, nx, nz, grids, cycle, vbc, scheme):
+    """The same solve with the reference's FP64 stencils, which runs a kernel per stage and the banded
+    substitutions: the same outcome in the same number of cycles (the reference's stale corrections do
+    not converge everywhere), and psi, or without convergence the first residuals, to the reference's
+    rounding: 64 eps / h^4 of each stencil against the operator's smallest eigenvalue,
+    (pi^2 (1 + 1 / aspect^2))^2."""
+    cfg, _ = small_case(kind, nx=nx, nz=nz, tpc=4)
+    cfg.aspect = 1.1 * nx / nz if nx == 112 else nx / nz
+    cfg.grids, cfg.mg_cycle, cfg.Vbc, cfg.mg_scheme = grids, cycle, vbc, scheme
+    cfg.tolerance, cfg.max_cycles = 1e-7, 100
+    st = make_state(cfg, 9, noise=1e-3 if cfg.ivis else 0.0)
+    out = []
+    for rounding in (0, 1):
+        c = cfg.copy()
+        c.reference_rounding = rounding
+        e = eng.Engine(c)
+        e.upload(st)
+        try:
+            out.append((e.solve_psi()["cycles"], e.get(eng.F_SF)))
+        except eng.PtError as ex:
+            out.append((ex.code, np.array(e.residuals()[:8])))  # before rounding grows with a diverging cycle
+        e.close()
+    assert out[0][0] == out[1][0]
+    bound = 64 * 1.1e-16 * max(nx / cfg.aspect, nz) ** 4 / (np.pi**2 * (1 + cfg.aspect**-2)) ** 2
+    assert rel_err(out[0][1], out[1][1]) < bound
