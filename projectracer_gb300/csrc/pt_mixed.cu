@@ -102,13 +102,20 @@ __device__ __forceinline__ const Stencil<float>& stencil<float>(int l) { return 
 template <>
 __device__ __forceinline__ const Stencil<double>& stencil<double>(int l) { return cSD[l]; }
 
-// A S (no right-hand side) at a node, in arithmetic T with the folded stencils of level l
-// (FP32: the smoother stages; FP64: residuals); ld(dx, dz) returns S at offset (dx, dz) from the
-// node (global memory or values held in registers: the same operations in the same order either
-// way), o is the node's index into the coefficient fields
-template <typename T, typename Ld, typename Op>
-__device__ __forceinline__ T apply_A_ld(const Ld& ld, int l, const Op& op, size_t o, int ivis) {
-    const Stencil<T>& C = stencil<T>(l);
+// The points of A's stencil: a 5 x 5 block, then (-3,0), (3,0), (0,-3), (0,3)
+constexpr int kPts = 29;
+__host__ __device__ constexpr int pt_dx(int p) { return p < 25 ? p % 5 - 2 : p == 25 ? -3 : p == 26 ? 3 : 0; }
+__host__ __device__ constexpr int pt_dz(int p) { return p < 25 ? p / 5 - 2 : p == 27 ? -3 : p == 28 ? 3 : 0; }
+__host__ __device__ constexpr int pt_index(int dx, int dz) {
+    return dx >= -2 && dx <= 2 && dz >= -2 && dz <= 2 ? (dz + 2) * 5 + dx + 2 : dx == -3 ? 25 : dx == 3 ? 26 : dz == -3 ? 27 : 28;
+}
+
+// A S (no right-hand side) at a node, in arithmetic T (FP32: the smoother stages; FP64: residuals), from
+// the folded stencils C of its level (stencil<T>, or CompactStencil's registers), ld(dx, dz) = S at
+// offset (dx, dz) from the node (global memory, or values held in registers or shared memory) and the
+// node's coefficients: the same operations in the same order in every form
+template <typename T, typename St, typename Ld>
+__device__ __forceinline__ T apply_A_core(const St& C, const Ld& ld, T vis, T vx, T vz, T vxz, T vxxmzz, int ivis) {
     T sx[7], sz[7];
 #pragma unroll
     for (int j = 0; j < 7; j++) {
@@ -117,11 +124,15 @@ __device__ __forceinline__ T apply_A_ld(const Ld& ld, int l, const Op& op, size_
     }
     T Sxx = 0, Sxxx = 0, Sxxxx = 0, Szz = 0, Szzz = 0, Szzzz = 0;
 #pragma unroll
-    for (int j = 0; j < 5; j++) { Sxx += C.x2[j] * sx[j + 1]; Szz += C.z2[j] * sz[j + 1]; }
+    for (int j = 0; j < 5; j++) { Sxx += C.x2(j) * sx[j + 1]; Szz += C.z2(j) * sz[j + 1]; }
 #pragma unroll
     for (int j = 0; j < 7; j++) {
-        Sxxx += C.x3[j] * sx[j]; Sxxxx += C.x4[j] * sx[j];
-        Szzz += C.z3[j] * sz[j]; Szzzz += C.z4[j] * sz[j];
+        if (j != 3 || !St::kZeros) {
+            Sxxx += C.x3(j) * sx[j];
+            Szzz += C.z3(j) * sz[j];
+        }
+        Sxxxx += C.x4(j) * sx[j];
+        Szzzz += C.z4(j) * sz[j];
     }
     T Sxz = 0, Sxxz = 0, Sxzz = 0, Sxxzz = 0;
 #pragma unroll
@@ -130,19 +141,52 @@ __device__ __forceinline__ T apply_A_ld(const Ld& ld, int l, const Op& op, size_
 #pragma unroll
         for (int ii = 0; ii < 5; ii++) {
             T v = (kk == 2) ? sx[ii + 1] : (T)ld(ii - 2, kk - 2);
-            d1 += C.i1[ii] * v;
-            d2 += C.i2[ii] * v;
+            if (ii != 2 || !St::kZeros) d1 += C.i1(ii) * v;
+            d2 += C.i2(ii) * v;
         }
-        Sxz += C.o_xz[kk] * d1;
-        Sxzz += C.o_xzz[kk] * d1;
-        Sxxz += C.o_xxz[kk] * d2;
-        Sxxzz += C.o_xxzz[kk] * d2;
+        if (kk != 2 || !St::kZeros) {
+            Sxz += C.o_xz(kk) * d1;
+            Sxxz += C.o_xxz(kk) * d2;
+        }
+        Sxzz += C.o_xzz(kk) * d1;
+        Sxxzz += C.o_xxzz(kk) * d2;
     }
-    T r = (T)op.vis[o] * (Sxxxx + Szzzz + (T)2 * Sxxzz);
+    T r = vis * (Sxxxx + Szzzz + (T)2 * Sxxzz);
     if (ivis != 0)
-        r += (T)op.vxxmzz[o] * (Sxx - Szz) + (T)4 * (T)op.vxz[o] * Sxz + (T)2 * (T)op.vx[o] * (Sxxx + Sxzz) +
-             (T)2 * (T)op.vz[o] * (Szzz + Sxxz);
+        r += vxxmzz * (Sxx - Szz) + (T)4 * vxz * Sxz + (T)2 * vx * (Sxxx + Sxzz) + (T)2 * vz * (Szzz + Sxxz);
     return r;
+}
+
+template <typename T>
+struct LevelStencil {  // the constant tables, every weight read and multiplied
+    static constexpr bool kZeros = false;
+    const Stencil<T>& s;
+    __device__ __forceinline__ T x2(int j) const { return s.x2[j]; }
+    __device__ __forceinline__ T x3(int j) const { return s.x3[j]; }
+    __device__ __forceinline__ T x4(int j) const { return s.x4[j]; }
+    __device__ __forceinline__ T z2(int j) const { return s.z2[j]; }
+    __device__ __forceinline__ T z3(int j) const { return s.z3[j]; }
+    __device__ __forceinline__ T z4(int j) const { return s.z4[j]; }
+    __device__ __forceinline__ T i1(int j) const { return s.i1[j]; }
+    __device__ __forceinline__ T i2(int j) const { return s.i2[j]; }
+    __device__ __forceinline__ T o_xz(int j) const { return s.o_xz[j]; }
+    __device__ __forceinline__ T o_xzz(int j) const { return s.o_xzz[j]; }
+    __device__ __forceinline__ T o_xxz(int j) const { return s.o_xxz[j]; }
+    __device__ __forceinline__ T o_xxzz(int j) const { return s.o_xxzz[j]; }
+};
+
+// o is the node's index into the coefficient fields
+template <typename T, typename Ld, typename Op>
+__device__ __forceinline__ T apply_A_ld(const Ld& ld, int l, const Op& op, size_t o, int ivis) {
+    const LevelStencil<T> C{stencil<T>(l)};
+    T vx = 0, vz = 0, vxz = 0, vxxmzz = 0;
+    if (ivis != 0) {
+        vx = (T)op.vx[o];
+        vz = (T)op.vz[o];
+        vxz = (T)op.vxz[o];
+        vxxmzz = (T)op.vxxmzz[o];
+    }
+    return apply_A_core<T>(C, ld, (T)op.vis[o], vx, vz, vxz, vxxmzz, ivis);
 }
 
 // A S at node (i,k) of the array S in global memory
@@ -395,16 +439,60 @@ __global__ void k_res_to_f32(float* out, const double* in, size_t n) {
 // A stretch of the cycle on levels that fit one cluster (pt_cluster.cuh): per visit the restriction
 // or the prolongation that enters it, the RKC1 stages in increment form, and the residual that the
 // next coarser level restricts; the coarsest level by the explicit inverse.
-// A thread owns one node for a whole visit and keeps what belongs to it in registers: the 29 weights
-// of A there (the operator with its five coefficient fields folded in once per visit), F0, Y0 and D_{j-2}.
-// A stage is then 29 shared loads, 28 differences and 29 multiply-adds per thread.  With one to eight warps per
-// scheduler it is bound by the latency of that chain and of one exchange, so one node per thread and
-// 32 warps rather than two nodes and 16: the same 1,024 nodes a CTA with half the chain.
+// A thread owns one node for a whole visit and keeps its coefficients, F0, Y0 and D_{j-2} in registers,
+// the level's stencils beside them; a stage is 29 shared loads and the operations of apply_A_core, which
+// round as in the per-stage kernels: the results are the same bits.  With one to four warps per
+// scheduler a stage is bound by the latency of that chain and of one exchange, so one node per thread and
+// 16 warps.  The part of a cycle below level 1 at 128x128: 148 us with a kernel per stage, 77 here.  (The
+// five coefficient fields folded into 29 weights of each node halve the
+// operations, 58 us, but their rounding changes the iterates of a solve.)
+// The folded stencils of a level in 30 registers: the one-dimensional D1 and D2 as constants, the others
+// by their (anti)symmetry, zero weights left out.  compact_stencil checks that it holds the very numbers
+// of the constant tables, so that A rounds here as in the per-stage kernels.
+struct CompactStencil {
+    static constexpr bool kZeros = true;
+    float a2x[3], a3x[3], a4x[4], a2z[3], a3z[3], a4z[4], axz[2], axzz[3], axxz[2], axxzz[3];
+    static constexpr int m5(int j) { return j < 3 ? j : 4 - j; }
+    static constexpr int m7(int j) { return j < 4 ? j : 6 - j; }
+    __host__ __device__ __forceinline__ float x2(int j) const { return a2x[m5(j)]; }
+    __host__ __device__ __forceinline__ float z2(int j) const { return a2z[m5(j)]; }
+    __host__ __device__ __forceinline__ float x3(int j) const { return j < 3 ? a3x[j] : j == 3 ? 0.f : -a3x[m7(j)]; }
+    __host__ __device__ __forceinline__ float z3(int j) const { return j < 3 ? a3z[j] : j == 3 ? 0.f : -a3z[m7(j)]; }
+    __host__ __device__ __forceinline__ float x4(int j) const { return a4x[m7(j)]; }
+    __host__ __device__ __forceinline__ float z4(int j) const { return a4z[m7(j)]; }
+    __host__ __device__ __forceinline__ float i1(int j) const {
+        return j == 0 ? (float)(1.0 / 12.0) : j == 1 ? (float)(-8.0 / 12.0) : j == 2 ? 0.f : j == 3 ? (float)(8.0 / 12.0)
+                                                                                         : (float)(-1.0 / 12.0);
+    }
+    __host__ __device__ __forceinline__ float i2(int j) const {
+        return j == 2 ? -2.5f : j == 1 || j == 3 ? (float)(16.0 / 12.0) : (float)(-1.0 / 12.0);
+    }
+    __host__ __device__ __forceinline__ float o_xz(int j) const { return j < 2 ? axz[j] : j == 2 ? 0.f : -axz[4 - j]; }
+    __host__ __device__ __forceinline__ float o_xxz(int j) const { return j < 2 ? axxz[j] : j == 2 ? 0.f : -axxz[4 - j]; }
+    __host__ __device__ __forceinline__ float o_xzz(int j) const { return axzz[m5(j)]; }
+    __host__ __device__ __forceinline__ float o_xxzz(int j) const { return axxzz[m5(j)]; }
+};
+static bool compact_stencil(const Stencil<float>& s, CompactStencil& c) {
+    for (int j = 0; j < 3; j++) {
+        c.a2x[j] = s.x2[j]; c.a2z[j] = s.z2[j]; c.a3x[j] = s.x3[j]; c.a3z[j] = s.z3[j];
+        c.axzz[j] = s.o_xzz[j]; c.axxzz[j] = s.o_xxzz[j];
+    }
+    for (int j = 0; j < 4; j++) { c.a4x[j] = s.x4[j]; c.a4z[j] = s.z4[j]; }
+    for (int j = 0; j < 2; j++) { c.axz[j] = s.o_xz[j]; c.axxz[j] = s.o_xxz[j]; }
+    bool same = true;
+    for (int j = 0; j < 5; j++)
+        same = same && c.x2(j) == s.x2[j] && c.z2(j) == s.z2[j] && c.i1(j) == s.i1[j] && c.i2(j) == s.i2[j] &&
+               c.o_xz(j) == s.o_xz[j] && c.o_xxz(j) == s.o_xxz[j] && c.o_xzz(j) == s.o_xzz[j] && c.o_xxzz(j) == s.o_xxzz[j];
+    for (int j = 0; j < 7; j++)
+        same = same && c.x3(j) == s.x3[j] && c.z3(j) == s.z3[j] && c.x4(j) == s.x4[j] && c.z4(j) == s.z4[j];
+    return same;
+}
+
 struct FLevel {
     Geo g;
     float *e, *rhs, *res;
     const float* coef[6];  // vis, vx, vz, vxz, vxxmzz, dt_stream
-    float h[10];           // 1/dr^2, 2/dr^3, 1/dr^4, the same in z, 2/(dr^2 ds^2), 4/(dr ds), 2/(dr ds^2), 2/(dr^2 ds)
+    CompactStencil st;
     int solo;              // >= 0: walked by every CTA alone, its arrays at this float of the solo area
 };
 struct FRun {
@@ -422,82 +510,31 @@ __host__ __device__ inline int cluster_tiles(int nx, int nz) {
 }
 __host__ __device__ inline int cluster_tiles_alone(int nx, int nz) { return cl::Strip::segments(nx) * (nz - 1); }
 
-// The points of A's stencil: a 5 x 5 block, then (-3,0), (3,0), (0,-3), (0,3)
-constexpr int kPts = 29;
-__host__ __device__ constexpr int pt_dx(int p) { return p < 25 ? p % 5 - 2 : p == 25 ? -3 : p == 26 ? 3 : 0; }
-__host__ __device__ constexpr int pt_dz(int p) { return p < 25 ? p / 5 - 2 : p == 27 ? -3 : p == 28 ? 3 : 0; }
-__host__ __device__ constexpr int pt_index(int dx, int dz) {  // -1: not a point of the stencil
-    return dx >= -2 && dx <= 2 && dz >= -2 && dz <= 2 ? (dz + 2) * 5 + dx + 2
-           : dz == 0 && dx == -3 ? 25 : dz == 0 && dx == 3 ? 26 : dx == 0 && dz == -3 ? 27 : dx == 0 && dz == 3 ? 28 : -1;
-}
-// the finite-difference weights (exact_stencils_setup compares the engine's with them)
-__host__ __device__ constexpr float fd1(int j) { return (j == -2 ? 1.f : j == -1 ? -8.f : j == 1 ? 8.f : j == 2 ? -1.f : 0.f) / 12.f; }
-__host__ __device__ constexpr float fd2(int j) { return (j == 0 ? -30.f : j == 1 || j == -1 ? 16.f : -1.f) / 12.f; }
-__host__ __device__ constexpr float fd3(int j) {
-    return (j < 0 ? 1.f : -1.f) * (j == 0 ? 0.f : j == 1 || j == -1 ? 13.f : j == 2 || j == -2 ? -8.f : 1.f) / 8.f;
-}
-__host__ __device__ constexpr float fd4(int j) {
-    return (j == 0 ? 56.f : j == 1 || j == -1 ? -39.f : j == 2 || j == -2 ? 12.f : -1.f) / 6.f;
-}
-
-// The weights of A at node (i, k) from its coefficients (vis, vxxmzz, vxz, vx, vz in c) and the level's
-// spacings h.  A is applied to differences from the node's own value, which for a smooth correction are
-// exact and small: on the values themselves the rounding of the weights, a factor h k larger, would
-// swamp A of a smooth mode.  The weights of a stencil add up to zero, so the middle one takes what
-// folding adds to the sum.  The ghost cells' share is folded onto the nodes that they mirror (antisymmetric across
-// the side walls, sign sz across top and bottom; every mirror node of a stencil lies in the stencil),
-// so that the windows hold no images.
-__device__ __forceinline__ void make_weights(float (&w)[kPts], const float (&c)[5], const float* h, int i, int k, int nx,
-                                             int nz, float sz) {
-    const float x2 = c[1] * h[0], x3 = c[3] * h[1], x4 = c[0] * h[2], z2 = c[1] * h[3], z3 = c[4] * h[4], z4 = c[0] * h[5];
-    const float xxzz = c[0] * h[6], xz = c[2] * h[7], xzz = c[3] * h[8], xxz = c[4] * h[9];
-#pragma unroll
-    for (int z = -2; z <= 2; z++) {
-        const float even = fd2(z) * xxzz + fd1(z) * xxz, odd = fd1(z) * xz + fd2(z) * xzz;
-#pragma unroll
-        for (int x = -2; x <= 2; x++) w[pt_index(x, z)] = fd2(x) * even + fd1(x) * odd;
-    }
-#pragma unroll
-    for (int j = -3; j <= 3; j++) {
-        const float ax = fd4(j) * x4 + fd3(j) * x3, az = fd4(j) * z4 + fd3(j) * z3;
-        if (j == -3 || j == 3) {
-            w[pt_index(j, 0)] = ax;
-            w[pt_index(0, j)] = az;
-        } else {
-            w[pt_index(j, 0)] += ax + fd2(j) * x2;
-            w[pt_index(0, j)] += az - fd2(j) * z2;
-        }
-    }
-    float folded = 0.0f;  // what folding adds to the sum of the weights
-    auto fold = [&](bool yes, int to, int from, float sign) {
-        if (!yes) return;
-        const float x = sign * w[from];
-        w[to] += x;
-        folded += x;
-    };
+// The cells around a node with the images of ghost cells put in (antisymmetric across the side walls,
+// sign sz across top and bottom): every node that a stencil's ghost cell mirrors lies in the stencil.
+__device__ __forceinline__ void put_images(float (&v)[kPts], int i, int k, int nx, int nz, float sz) {
     if (__any_sync(0xffffffffu, i <= 2 || i >= nx - 2)) {
 #pragma unroll
         for (int z = -2; z <= 2; z++) {
-            fold(i == 1, pt_index(0, z), pt_index(-2, z), -1.0f);
-            fold(i == nx - 1, pt_index(0, z), pt_index(2, z), -1.0f);
+            if (i == 1) v[pt_index(-2, z)] = -v[pt_index(0, z)];
+            if (i == nx - 1) v[pt_index(2, z)] = -v[pt_index(0, z)];
         }
-        fold(i == 1, pt_index(1, 0), pt_index(-3, 0), -1.0f);
-        fold(i == 2, pt_index(-1, 0), pt_index(-3, 0), -1.0f);
-        fold(i == nx - 1, pt_index(-1, 0), pt_index(3, 0), -1.0f);
-        fold(i == nx - 2, pt_index(1, 0), pt_index(3, 0), -1.0f);
+        if (i == 1) v[pt_index(-3, 0)] = -v[pt_index(1, 0)];
+        if (i == 2) v[pt_index(-3, 0)] = -v[pt_index(-1, 0)];
+        if (i == nx - 1) v[pt_index(3, 0)] = -v[pt_index(-1, 0)];
+        if (i == nx - 2) v[pt_index(3, 0)] = -v[pt_index(1, 0)];
     }
-    if (k <= 2 || k >= nz - 2) {
+    if (k <= 2 || k >= nz - 2) {  // (a warp has one row)
 #pragma unroll
         for (int x = -2; x <= 2; x++) {
-            fold(k == 1, pt_index(x, 0), pt_index(x, -2), sz);
-            fold(k == nz - 1, pt_index(x, 0), pt_index(x, 2), sz);
+            if (k == 1) v[pt_index(x, -2)] = sz * v[pt_index(x, 0)];
+            if (k == nz - 1) v[pt_index(x, 2)] = sz * v[pt_index(x, 0)];
         }
-        fold(k == 1, pt_index(0, 1), pt_index(0, -3), sz);
-        fold(k == 2, pt_index(0, -1), pt_index(0, -3), sz);
-        fold(k == nz - 1, pt_index(0, -1), pt_index(0, 3), sz);
-        fold(k == nz - 2, pt_index(0, 1), pt_index(0, 3), sz);
+        if (k == 1) v[pt_index(0, -3)] = sz * v[pt_index(0, 1)];
+        if (k == 2) v[pt_index(0, -3)] = sz * v[pt_index(0, -1)];
+        if (k == nz - 1) v[pt_index(0, 3)] = sz * v[pt_index(0, -1)];
+        if (k == nz - 2) v[pt_index(0, 3)] = sz * v[pt_index(0, 1)];
     }
-    w[pt_index(0, 0)] = folded;
 }
 
 // the residual at node (i, k) in FP64 arithmetic on the correction in window y
@@ -666,8 +703,7 @@ __global__ void __launch_bounds__(cl::kThreads, 1) k_cycle_cluster_f(const __gri
                 }
             }
         }
-        float w[kPts];
-        make_weights(w, cv, P.L[l].h, p.i, p.k, g.nx, g.nz, P.sz);
+        const CompactStencil st = P.L[l].st;
         ex.bytes = (uint32_t)p.bytes;
         cl::Outlet<float> out;
         out.set(p.s, win, bars, p.m, p.up, p.down);
@@ -675,12 +711,13 @@ __global__ void __launch_bounds__(cl::kThreads, 1) k_cycle_cluster_f(const __gri
         float A = 0.0f, own = 0.0f;
         auto apply = [&](int q) {  // A of window q at the node, and the window's value there
             const float* x = m + q * cl::kWindow;
-            own = *x;
-            float a[3] = {w[pt_index(0, 0)] * own, 0.0f, 0.0f};
+            float v[kPts];
 #pragma unroll
-            for (int j = 0; j < kPts; j++)
-                if (j != pt_index(0, 0)) a[j % 3] += w[j] * (x[pt_dz(j) * cl::kPitch + pt_dx(j)] - own);
-            A = (a[0] + a[1]) + a[2];
+            for (int j = 0; j < kPts; j++) v[j] = x[pt_dz(j) * cl::kPitch + pt_dx(j)];
+            own = v[pt_index(0, 0)];
+            put_images(v, p.i, p.k, g.nx, g.nz, P.sz);
+            A = apply_A_core<float>(st, [&](int dx, int dz) { return v[pt_index(dx, dz)]; }, cv[0], cv[3], cv[4], cv[2],
+                                    cv[1], P.ivis);
         };
         auto publish = [&](int q, float v) {
             if (on) {
@@ -696,14 +733,16 @@ __global__ void __launch_bounds__(cl::kThreads, 1) k_cycle_cluster_f(const __gri
             if (p.busy) apply(0);
             cur = 1;
         }
-        const float F0 = rhs - A;
+        const float F0 = zero ? rhs : rhs - A;
         float d = cheb[1].z * dt * F0, old = 0.0f;
         publish(cur, d);
         for (int j = 2; j <= P.N; j++) {
             if (p.busy) {
                 const float4 ch = cheb[j];
                 apply(cur);
-                d = ch.x * own + ch.z * dt * (F0 - A) + ch.y * old;
+                const float F = F0 - A;
+                d = ch.x * own + ch.z * dt * F;
+                if (j > 2) d += ch.y * old;
                 old = own;
             }
             if (j < P.N) {
@@ -1045,7 +1084,13 @@ static int cluster_setup_f(Engine& E) {
     E.ctop = E.grids + 1;
     E.csolo = E.grids + 1;
     E.cl1 = E.ccoarse = E.coarse_solo = false;
-    if (E.cfg.Nmulti != 1 || !E.res_int) return 0;  // (res_int: the stencils are the rationals of fd1..fd4)
+    if (E.cfg.Nmulti != 1) return 0;
+    for (int l = 1; l < E.grids; l++) {
+        Stencil<float> f;
+        make_stencil(E, l, f);
+        CompactStencil c;
+        if (!compact_stencil(f, c)) return 0;
+    }
     // a level goes to the cluster when each of its nodes finds a thread: 16 CTAs x 16 warps x 32 columns,
     // 8,192 nodes
     auto fits = [&](int l) {
@@ -1114,10 +1159,11 @@ static int launch_run_f(Engine& E, FRun& R, bool coarse_smoother, const double* 
         L.rhs = E.fRHS[l];
         L.res = E.fres[l];
         for (int q = 0; q < 6; q++) L.coef[q] = E.fcoef[l][q];
-        const LevConst& K = E.L[l];
-        const double h[10] = {1.0 / K.dr2, 2.0 / K.dr3, 1.0 / K.dr4, 1.0 / K.ds2, 2.0 / K.ds3, 1.0 / K.ds4,
-                              2.0 / K.dr2ds2, 4.0 / K.drds, 2.0 / K.drds2, 2.0 / K.dr2ds};
-        for (int q = 0; q < 10; q++) L.h[q] = (float)h[q];
+        if (l < E.grids) {
+            Stencil<float> f;
+            make_stencil(E, l, f);
+            compact_stencil(f, L.st);
+        }
         L.solo = -1;
         // only in a run that walks the whole way down and up: a solo level's arrays last for one launch
         const bool mine = l < E.grids ? l >= a && l <= b : E.coarse_solo;
