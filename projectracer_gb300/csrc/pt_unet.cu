@@ -1,6 +1,7 @@
-// pt_unet.cu -- learned psi guess (no reference counterpart): BF16 implicit-GEMM convolutions
-// on the tcgen05 tensor cores (pt_tc.cuh), their self-check entry point, and the U-Net built on
-// them.
+// pt_unet.cu -- learned psi guess (no reference counterpart): the U-Net whose convolutions run on the
+// tcgen05 tensor cores (pt_conv.cuh), the GEMM tile's self-check entry point, and the engine side.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -10,14 +11,13 @@
 
 #include "pt_internal.h"
 #include "../../include/ptgpu_unet.h"
-#include "pt_tc.cuh"
+#include "pt_conv.cuh"
 #include <cuda_bf16.h>
 
 namespace pt {
 
 // plain GEMM problem: C (M x N, FP32) = A (M x K) * B (N x K)^T, BF16 row-major operands
 struct GemmProb {
-    static constexpr int kGather = tc::kGatherElem;
     int M, N, K, Ntile, kc_split;
     const uint16_t* A;
     const uint16_t* B;
@@ -33,263 +33,124 @@ struct GemmProb {
 static inline unsigned nblk(size_t n, unsigned b) { return (unsigned)((n + b - 1) / b); }
 
 // ============================================================================ U-Net kernels
+using tc::PadGeo;
 __device__ __forceinline__ uint16_t f2bf(float f) { return __bfloat16_as_ushort(__float2bfloat16_rn(f)); }
 __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
-
-// The input of a convolution as seen by its im2col gather, at the convolution's resolution
-// (B x H x W): mode 0 one BF16 NHWC tensor; mode 1 a tensor at 2H x 2W averaged over 2x2 (pooling);
-// mode 2 the concatenation of a tensor at H/2 x W/2 read nearest-neighbour (upsampling, channels
-// 0..C0-1) and a skip tensor at H x W (channels C0..C0+C1-1).
-struct InView {
-    const uint16_t* t0;
-    const uint16_t* t1;
-    int B, H, W, C0, C1, mode;
-    __host__ __device__ int C() const { return C0 + C1; }
-    __device__ __forceinline__ float get(int b, int y, int x, int c) const {
-        if (mode == 0) return bf2f(t0[(((size_t)b * H + y) * W + x) * C0 + c]);
-        if (mode == 1) {
-            const size_t W2 = 2 * (size_t)W;
-            const uint16_t* q = t0 + (((size_t)b * 2 * H + 2 * y) * W2 + 2 * x) * C0 + c;
-            const float s = ((bf2f(q[0]) + bf2f(q[C0])) + bf2f(q[W2 * C0])) + bf2f(q[W2 * C0 + C0]);
-            return s * 0.25f;
-        }
-        if (c < C0) return bf2f(t0[(((size_t)b * (H >> 1) + (y >> 1)) * (W >> 1) + (x >> 1)) * C0 + c]);
-        return bf2f(t1[(((size_t)b * H + y) * W + x) * C1 + (c - C0)]);
-    }
-};
-
-// pixel p of a B x H x W grid shifted by tap (3x3, row-major taps); false outside the grid
-__device__ __forceinline__ bool tap_pixel(int p, int tap, int H, int W, int& b, int& y, int& x) {
-    x = p % W;
-    const int r = p / W;
-    y = r % H;
-    b = r / H;
-    y += tap / 3 - 1;
-    x += tap % 3 - 1;
-    return y >= 0 && y < H && x >= 0 && x < W;
-}
-
-// 8 BF16 values from one 16-byte-aligned address
+// 8 BF16 values at a 16-byte-aligned address
 __device__ __forceinline__ uint4 ld8(const uint16_t* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) { return (uint32_t)lo | ((uint32_t)hi << 16); }
-
-// channels c..c+7 of a view at pixel (b, y, x) as 8 BF16 values (c, C0 and C1 multiples of 8):
-// one 16-byte load, or four averaged in the order of InView::get for a pooled view
-__device__ __forceinline__ uint4 view_load8(const InView& in, int b, int y, int x, int c) {
-    if (in.mode == 0) return ld8(in.t0 + (((size_t)b * in.H + y) * in.W + x) * in.C0 + c);
-    if (in.mode == 2) {
-        if (c < in.C0) return ld8(in.t0 + (((size_t)b * (in.H >> 1) + (y >> 1)) * (in.W >> 1) + (x >> 1)) * in.C0 + c);
-        return ld8(in.t1 + (((size_t)b * in.H + y) * in.W + x) * in.C1 + (c - in.C0));
-    }
-    const size_t W2 = 2 * (size_t)in.W;
-    const uint16_t* q = in.t0 + (((size_t)b * 2 * in.H + 2 * y) * W2 + 2 * x) * in.C0 + c;
-    const uint4 a = ld8(q), bq = ld8(q + in.C0), cq = ld8(q + W2 * in.C0), d = ld8(q + W2 * in.C0 + in.C0);
-    const uint32_t* pa = &a.x;
-    const uint32_t* pb = &bq.x;
-    const uint32_t* pc = &cq.x;
-    const uint32_t* pd = &d.x;
-    uint32_t o[4];
+__device__ __forceinline__ void st8(uint16_t* p, const uint16_t (&h)[8]) {
+    uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        uint16_t h[2];
+    for (int j = 0; j < 4; j++) w[j] = (uint32_t)h[2 * j] | ((uint32_t)h[2 * j + 1] << 16);
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int sh = 16 * e;
-            const float sum = ((bf2f((uint16_t)(pa[j] >> sh)) + bf2f((uint16_t)(pb[j] >> sh))) +
-                               bf2f((uint16_t)(pc[j] >> sh))) + bf2f((uint16_t)(pd[j] >> sh));
-            h[e] = f2bf(sum * 0.25f);
-        }
-        o[j] = pack2(h[0], h[1]);
-    }
-    return make_uint4(o[0], o[1], o[2], o[3]);
+    for (int j = 0; j < 8; j++) f[j] = bf2f((uint16_t)(w[j >> 1] >> (16 * (j & 1))));
 }
 
-// channels c..c+7 of dZ (the ReLU-masked gradient, BF16) at flat index idx = pixel * C + c
-__device__ __forceinline__ uint4 dz_load8(const float* dY, const uint16_t* Y, size_t idx) {
-    const float4 g0 = *reinterpret_cast<const float4*>(dY + idx), g1 = *reinterpret_cast<const float4*>(dY + idx + 4);
-    const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+constexpr int kImCols = 64;  // columns of the first layer's im2col rows: 36 values (tap, channel), zeros
+
+// the network input, NCHW FP32, as im2col rows in BF16 at the padded positions: 8 columns a thread
+// (columns 40..63 stay zero from allocation)
+__global__ void k_im2col(uint16_t* __restrict__ o, const float* __restrict__ x, PadGeo g) {
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x, n = (size_t)g.B * g.H * g.W;
+    if (q >= 5 * n) return;
+    const int j = (int)(q / n);
+    size_t r = q - j * n;
+    const int px = (int)(r % g.W);
+    r /= g.W;
+    const int py = (int)(r % g.H), b = (int)(r / g.H);
     uint16_t h[8];
-    if (Y) {
-        const uint4 m = ld8(Y + idx);
-        const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint16_t yb = (uint16_t)(mm[j >> 1] >> (16 * (j & 1)));
-            h[j] = bf2f(yb) > 0.f ? f2bf(g[j]) : (uint16_t)0;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++) h[j] = f2bf(g[j]);
+    for (int e = 0; e < 8; e++) {
+        const int tap = 2 * j + e / 4, c = e % 4, y = py + tap / 3 - 1, xx = px + tap % 3 - 1;
+        float v = 0.f;
+        if (tap < 9 && y >= 0 && y < g.H && xx >= 0 && xx < g.W) v = x[(((size_t)b * 4 + c) * g.H + y) * g.W + xx];
+        h[e] = f2bf(v);
     }
-    return make_uint4(pack2(h[0], h[1]), pack2(h[2], h[3]), pack2(h[4], h[5]), pack2(h[6], h[7]));
+    st8(o + g.at(b, py, px) * kImCols + 8 * j, h);
 }
 
-// forward: out[p][co] = relu(sum_{tap,ci} in(p+tap)[ci] w[co][tap][ci] + bias[co]) in BF16.
-// K = 9 cin, ordered (tap, ci): with cin a multiple of 8 the 8 values of a gather_a8 are 8
-// consecutive channels of one pixel (one 16-byte load of an NHWC tensor, four for a pooled view),
-// and those of a gather_b8 8 consecutive weights; the first layer (cin = 4) gathers element-wise.
-struct ConvFwd {
-    static constexpr int kGather = tc::kGatherRow;
-    int M, N, K, Ntile, kc_split;
-    InView in;
-    const uint16_t* w;
-    const float* bias;
+// pixel and channel octet of element q of a batch's real pixels, pixels within octets of a row adjacent
+__device__ __forceinline__ bool octet(size_t q, const PadGeo& g, int C, int& b, int& y, int& x, int& c) {
+    const int noct = C >> 3;
+    c = (int)(q % noct) * 8;
+    size_t r = q / noct;
+    x = (int)(r % g.W);
+    r /= g.W;
+    y = (int)(r % g.H);
+    b = (int)(r / g.H);
+    return b < g.B;
+}
+
+// 2x2 average of a tensor at twice the resolution, ((a+b)+c)+d in FP32
+__global__ void k_pool(uint16_t* __restrict__ o, const uint16_t* __restrict__ in, PadGeo g, PadGeo gf, int C) {
+    int b, y, x, c;
+    if (!octet((size_t)blockIdx.x * blockDim.x + threadIdx.x, g, C, b, y, x, c)) return;
+    const uint16_t* p = in + gf.at(b, 2 * y, 2 * x) * C + c;
+    const size_t row = (size_t)gf.Wp() * C;
+    float a[8], e[8], d[8], f[8];
+    unpack8(ld8(p), a);
+    unpack8(ld8(p + C), e);
+    unpack8(ld8(p + row), d);
+    unpack8(ld8(p + row + C), f);
+    uint16_t h[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) h[j] = f2bf((((a[j] + e[j]) + d[j]) + f[j]) * 0.25f);
+    st8(o + g.at(b, y, x) * C + c, h);
+}
+
+// epilogue of the forward GEMM: bias, ReLU, BF16; the nearest-neighbour upsampled copy beside it
+// where the next layer reads that
+struct FwdEpi {
     uint16_t* out;
-    int relu;
-    __device__ __forceinline__ uint16_t gather_a(int p, int k) const {
-        if (p >= M || k >= K) return 0;
-        const int cin = in.C(), tap = k / cin, ci = k - tap * cin;
-        int b, y, x;
-        if (!tap_pixel(p, tap, in.H, in.W, b, y, x)) return 0;
-        return f2bf(in.get(b, y, x, ci));
-    }
-    __device__ __forceinline__ uint16_t gather_b(int co, int k) const {
-        return (co < N && k < K) ? w[(size_t)co * K + k] : (uint16_t)0;
-    }
-    __device__ __forceinline__ uint4 gather_a8(int p, int k0) const {
-        const int cin = in.C();
-        if ((cin & 7) || (in.C0 & 7) || k0 + 8 > K) {
-            uint16_t v[8];
+    const float* bias;
+    int C;
+    uint16_t* up;
+    PadGeo gup;
+    __device__ __forceinline__ void operator()(int p, int b, int y, int x, int c0, const float (&v)[32]) const {
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = gather_a(p, k0 + j);
-            return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-        }
-        if (p >= M) return make_uint4(0u, 0u, 0u, 0u);
-        const int tap = k0 / cin, ci = k0 - tap * cin;
-        int b, y, x;
-        if (!tap_pixel(p, tap, in.H, in.W, b, y, x)) return make_uint4(0u, 0u, 0u, 0u);
-        return view_load8(in, b, y, x, ci);
-    }
-    __device__ __forceinline__ uint4 gather_b8(int co, int k0) const {
-        if ((K & 7) || co >= N || k0 + 8 > K) {
-            uint16_t v[8];
+        for (int j = 0; j < 32; j += 8) {
+            uint16_t h[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = gather_b(co, k0 + j);
-            return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+            for (int e = 0; e < 8; e++) h[e] = f2bf(fmaxf(v[j + e] + bias[c0 + j + e], 0.f));
+            st8(out + (size_t)p * C + c0 + j, h);
+            if (up)
+                for (int q = 0; q < 4; q++) st8(up + gup.at(b, 2 * y + (q >> 1), 2 * x + (q & 1)) * C + c0 + j, h);
         }
-        return ld8(w + (size_t)co * K + k0);
     }
-    __device__ __forceinline__ void store(int p, int co, int, float v) const {
-        v += bias[co];
-        if (relu) v = fmaxf(v, 0.f);
-        out[(size_t)p * N + co] = f2bf(v);
+};
+// epilogue of the backward-data GEMM: the view's gradient in FP32 at the padded positions
+struct DxEpi {
+    float* dx;
+    int N;
+    __device__ __forceinline__ void operator()(int p, int, int, int, int c0, const float (&v)[32]) const {
+        float* o = dx + (size_t)p * N + c0;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
 };
 
-// gradient w.r.t. the pre-activation of a layer, as a BF16 GEMM operand: dY masked by Y > 0
-__device__ __forceinline__ uint16_t dz_bf(const float* dY, const uint16_t* Y, size_t idx) {
-    const float g = dY[idx];
-    if (Y && !(bf2f(Y[idx]) > 0.f)) return 0;
-    return f2bf(g);
-}
-
-// backward data: dX[q][ci] = sum_{t,co} dZ[q + tap t][co] w[co][8 - t][ci]  (FP32 out).  K is
-// ordered (t, co): a gather_a8 takes 8 consecutive channels of dZ at one shifted pixel (two 16-byte
-// loads of dY, one of the ReLU mask), a gather_b8 8 consecutive weights of wbd[ci][t][co] =
-// w[co][8 - t][ci], the layout k_w_bwd_layout writes before the GEMM.
-struct ConvBwdData {
-    static constexpr int kGather = tc::kGatherRow;
-    int M, N, K, Ntile, kc_split;  // M pixels, N = Cin, K = 9 Cout
-    int H, W, Cout;
-    const float* dY;
-    const uint16_t* Y;
-    const uint16_t* w;
-    const uint16_t* wbd;
-    float* dX;
-    __device__ __forceinline__ uint4 gather_a8(int q, int k0) const {
-        if ((Cout & 7) || k0 + 8 > K) {
-            uint16_t v[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = gather_a(q, k0 + j);
-            return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-        }
-        if (q >= M) return make_uint4(0u, 0u, 0u, 0u);
-        const int t = k0 / Cout, co = k0 - t * Cout;
-        int b, y, x;
-        if (!tap_pixel(q, t, H, W, b, y, x)) return make_uint4(0u, 0u, 0u, 0u);
-        return dz_load8(dY, Y, (((size_t)b * H + y) * W + x) * Cout + co);
-    }
-    __device__ __forceinline__ uint4 gather_b8(int ci, int k0) const {
-        if ((K & 7) || ci >= N || k0 + 8 > K) {
-            uint16_t v[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = gather_b(ci, k0 + j);
-            return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-        }
-        return ld8(wbd + (size_t)ci * K + k0);
-    }
-    __device__ __forceinline__ uint16_t gather_a(int q, int k) const {
-        if (q >= M || k >= K) return 0;
-        const int t = k / Cout, co = k - t * Cout;
-        int b, y, x;
-        if (!tap_pixel(q, t, H, W, b, y, x)) return 0;
-        return dz_bf(dY, Y, (((size_t)b * H + y) * W + x) * Cout + co);
-    }
-    __device__ __forceinline__ uint16_t gather_b(int ci, int k) const {
-        if (ci >= N || k >= K) return 0;
-        const int t = k / Cout, co = k - t * Cout;
-        return w[((size_t)co * 9 + (8 - t)) * N + ci];
-    }
-    __device__ __forceinline__ void store(int q, int ci, int, float v) const { dX[(size_t)q * N + ci] = v; }
+// the convolutions' weights in the layouts that only the GEMMs use: wbd[ci][t][co] = w[co][8 - t][ci] (the
+// K order of the backward-data GEMM), and the first layer's rows padded to the im2col width
+struct PackArgs {
+    int cin[14], cout[14];
+    size_t woff[14];
 };
-
-// backward weights (split over pixels): part[z][tap*Cin + ci][co] = sum_{p in split z} in(p+tap)[ci] dZ[p][co]
-struct ConvBwdW {
-    static constexpr int kGather = tc::kGatherCol;
-    int M, N, K, Ntile, kc_split;  // M = 9 Cin, N = Cout, K = pixels
-    InView in;
-    const float* dY;
-    const uint16_t* Y;
-    float* part;
-    __device__ __forceinline__ uint16_t gather_a(int kk, int p) const {
-        if (kk >= M || p >= K) return 0;
-        const int cin = in.C(), tap = kk / cin, ci = kk - tap * cin;
-        int b, y, x;
-        if (!tap_pixel(p, tap, in.H, in.W, b, y, x)) return 0;
-        return f2bf(in.get(b, y, x, ci));
-    }
-    __device__ __forceinline__ uint16_t gather_b(int co, int p) const {
-        return (co < N && p < K) ? dz_bf(dY, Y, (size_t)p * N + co) : (uint16_t)0;
-    }
-    // A[kk0..kk0+7][p]: channels ci..ci+7 of the input at pixel p shifted by the rows' tap
-    __device__ __forceinline__ uint4 gather_col_a(int kk0, int p) const {
-        const int cin = in.C();
-        if ((cin & 7) || (in.C0 & 7)) {
-            uint16_t v[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = gather_a(kk0 + j, p);
-            return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+__global__ void k_pack_weights(uint16_t* __restrict__ wbd, uint16_t* __restrict__ w0, const uint16_t* __restrict__ w,
+                               PackArgs a) {
+    const int l = blockIdx.y, cin = a.cin[l], cout = a.cout[l];
+    const uint16_t* wl = w + a.woff[l];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < cin * 9 * cout; q += gridDim.x * blockDim.x) {
+        if (l == 0) {
+            w0[q / 36 * kImCols + q % 36] = wl[q];
+        } else {
+            const int co = q % cout, t = q / cout % 9, ci = q / (9 * cout);
+            wbd[a.woff[l] + q] = wl[((size_t)co * 9 + (8 - t)) * cin + ci];
         }
-        if (kk0 >= M || p >= K) return make_uint4(0u, 0u, 0u, 0u);
-        const int tap = kk0 / cin, ci = kk0 - tap * cin;
-        int b, y, x;
-        if (!tap_pixel(p, tap, in.H, in.W, b, y, x)) return make_uint4(0u, 0u, 0u, 0u);
-        return view_load8(in, b, y, x, ci);
     }
-    // B[co0..co0+7][p]: channels co0..co0+7 of dZ at pixel p
-    __device__ __forceinline__ uint4 gather_col_b(int co0, int p) const {
-        if (N & 7) {
-            uint16_t v[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = gather_b(co0 + j, p);
-            return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-        }
-        if (co0 >= N || p >= K) return make_uint4(0u, 0u, 0u, 0u);
-        return dz_load8(dY, Y, (size_t)p * N + co0);
-    }
-    __device__ __forceinline__ void store(int kk, int co, int z, float v) const {
-        part[((size_t)z * M + kk) * N + co] = v;
-    }
-};
-
-// wbd[ci][t][co] = w[co][8 - t][ci]: the weights in the K order of the backward-data GEMM
-__global__ void k_w_bwd_layout(uint16_t* __restrict__ wbd, const uint16_t* __restrict__ w, int cin, int cout) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (size_t)cin * 9 * cout) return;
-    const int co = (int)(q % cout);
-    const int t = (int)((q / cout) % 9);
-    const int ci = (int)(q / ((size_t)cout * 9));
-    wbd[q] = w[((size_t)co * 9 + (8 - t)) * cin + ci];
 }
 
 // dW[co][kk] = sum_z part[z][kk][co], z ascending
@@ -302,68 +163,127 @@ __global__ void k_wgrad_reduce(float* dW, const float* part, int nsplit, int M, 
     dW[(size_t)co * M + kk] = s;
 }
 
-// db[co] = sum_p dZ[p][co] (block per channel, fixed-order tree)
-__global__ void k_bias_grad(float* db, const float* dY, const uint16_t* Y, int P, int C) {
-    __shared__ float sh[256];
-    const int co = blockIdx.x;
-    float s = 0.f;
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
-        const size_t idx = (size_t)p * C + co;
-        if (!Y || bf2f(Y[idx]) > 0.f) s += dY[idx];
+// Gradient of a layer's pre-activation as a GEMM operand, dZ = dY masked by Y > 0 in BF16, and per-block
+// partial sums of its bias gradient (of the FP32 dY).  dY is where the gradient of the view that read
+// the layer's output comes from:
+//   plain   the view's gradient itself
+//   pooled  the skip connection's share plus a quarter of the pooled pixel's
+//   up      the sum of the four fine pixels, ((a+b)+c)+d
+//   out     the output layer: dy w[c]; the partial sums of its own weights' gradients too
+// One pass over the tensor, bound by its bytes (FP32 in, two BF16 tensors in and out).
+enum { kDzPlain = 0, kDzPooled, kDzUp, kDzOut };
+constexpr int kDzThreads = 256;
+struct DzArgs {
+    PadGeo g, g2;  // of the layer, and of the other resolution (pooled: coarse, up: fine)
+    int C;
+    const uint16_t* Y;
+    uint16_t* dZ;
+    const float* dx;  // gradient of the view (out: dy)
+    int ldx;          // its channels
+    const float* skip;  // pooled: the skip connection's view gradient, its channels and the offset in them
+    int lds, offs;
+    const float* w;  // out: weights
+    float* part;     // [block][C], out: [block][2 C + 1] with the weights' and the bias' sums behind
+};
+template <int MODE>
+__global__ void __launch_bounds__(kDzThreads) k_dz(DzArgs a) {
+    constexpr int NV = MODE == kDzOut ? 2 : 1;
+    __shared__ float sh[NV * 8][kDzThreads + 1];
+    __shared__ float shb[kDzThreads];
+    const int noct = a.C >> 3;
+    const size_t total = (size_t)a.g.B * a.g.H * a.g.W * noct;
+    float sum[8] = {}, wsum[8] = {}, bsum = 0.f;
+    // the stride is a multiple of noct: a thread keeps its channels
+    for (size_t q = (size_t)blockIdx.x * kDzThreads + threadIdx.x; q < total; q += (size_t)gridDim.x * kDzThreads) {
+        int b, y, x, c;
+        octet(q, a.g, a.C, b, y, x, c);
+        const size_t p = a.g.at(b, y, x);
+        float g[8], act[8];
+        unpack8(ld8(a.Y + p * a.C + c), act);
+        auto load = [&](const float* f, float (&v)[8]) {
+            const float4 u = *reinterpret_cast<const float4*>(f), w = *reinterpret_cast<const float4*>(f + 4);
+            v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
+        };
+        if (MODE == kDzPlain) {
+            load(a.dx + p * a.ldx + c, g);
+        } else if (MODE == kDzPooled) {
+            float d[8];
+            load(a.skip + p * a.lds + a.offs + c, g);
+            load(a.dx + a.g2.at(b, y >> 1, x >> 1) * a.ldx + c, d);
+#pragma unroll
+            for (int j = 0; j < 8; j++) g[j] += 0.25f * d[j];
+        } else if (MODE == kDzUp) {
+            const float* f = a.dx + a.g2.at(b, 2 * y, 2 * x) * a.ldx + c;
+            const size_t row = (size_t)a.g2.Wp() * a.ldx;
+            float d[8], e[8], h[8];
+            load(f, g);
+            load(f + a.ldx, d);
+            load(f + row, e);
+            load(f + row + a.ldx, h);
+#pragma unroll
+            for (int j = 0; j < 8; j++) g[j] = ((g[j] + d[j]) + e[j]) + h[j];
+        } else {
+            const float dy = a.dx[((size_t)b * a.g.H + y) * a.g.W + x];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                g[j] = dy * a.w[c + j];
+                wsum[j] += dy * act[j];
+            }
+            if (c == 0) bsum += dy;
+        }
+        uint16_t h[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const bool pos = act[j] > 0.f;
+            h[j] = pos ? f2bf(g[j]) : (uint16_t)0;
+            if (pos) sum[j] += g[j];
+        }
+        st8(a.dZ + p * a.C + c, h);
     }
-    sh[threadIdx.x] = s;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        sh[j][threadIdx.x] = sum[j];
+        if (NV == 2) sh[8 * (NV - 1) + j][threadIdx.x] = wsum[j];
+    }
+    shb[threadIdx.x] = bsum;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[co] = sh[0];
-}
-
-// adjoints of the input views: add dXg (P x C at the view's resolution) into the sources' grads
-__global__ void k_adj_plain(float* g0, const float* dX, size_t n) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) g0[q] += dX[q];
-}
-__global__ void k_adj_pool(float* g0, const float* dX, int B, int H, int W, int C) {  // g0 at 2H x 2W
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n = (size_t)B * 4 * H * W * C;
-    if (q >= n) return;
-    const int c = (int)(q % C);
-    size_t r = q / C;
-    const int x2 = (int)(r % (2 * W));
-    r /= (2 * W);
-    const int y2 = (int)(r % (2 * H));
-    const int b = (int)(r / (2 * H));
-    g0[q] += 0.25f * dX[(((size_t)b * H + (y2 >> 1)) * W + (x2 >> 1)) * C + c];
-}
-__global__ void k_adj_upcat(float* g0, float* g1, const float* dX, int B, int H, int W, int C0, int C1) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n0 = (size_t)B * (H / 2) * (W / 2) * C0, n1 = (size_t)B * H * W * C1;
-    const int C = C0 + C1;
-    if (q < n0) {  // coarse source: sum of its 2x2 fine pixels, fixed order
-        const int c = (int)(q % C0);
-        size_t r = q / C0;
-        const int x = (int)(r % (W / 2));
-        r /= (W / 2);
-        const int y = (int)(r % (H / 2));
-        const int b = (int)(r / (H / 2));
-        const size_t f = (((size_t)b * H + 2 * y) * W + 2 * x) * C + c;
-        g0[q] += ((dX[f] + dX[f + C]) + dX[f + (size_t)W * C]) + dX[f + (size_t)W * C + C];
-    } else if (q < n0 + n1) {
-        const size_t u = q - n0;
-        const int c = (int)(u % C1);
-        const size_t p = u / C1;
-        g1[u] += dX[p * C + C0 + c];
+    // threads of equal channels, in ascending order
+    const int nout = NV * a.C + (MODE == kDzOut ? 1 : 0);
+    for (int o = threadIdx.x; o < nout; o += kDzThreads) {
+        float s = 0.f;
+        if (o == NV * a.C) {
+            for (int t = 0; t < kDzThreads; t++) s += shb[t];
+        } else {
+            const int v = o / a.C, c = o - v * a.C;
+            for (int t = c >> 3; t < kDzThreads; t += noct) s += sh[8 * v + (c & 7)][t];
+        }
+        a.part[(size_t)blockIdx.x * nout + o] = s;
     }
 }
+// out[c] = sum over blocks of part[block][off + c]: a warp a column, fixed order
+__global__ void k_colsum(float* out, const float* part, int blocks, int ld, int off, int n) {
+    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= n) return;
+    float s = 0.f;
+    for (int b = lane; b < blocks; b += 32) s += part[(size_t)b * ld + off + c];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[c] = s;
+}
 
-// 1x1 output convolution (linear, FP32 out) and its backward
-__global__ void k_out_fwd(float* y, const uint16_t* d, const float* w, const float* b, int P, int C) {
+// 1x1 output convolution (linear, FP32 out)
+__global__ void k_out_fwd(float* y, const uint16_t* d, const float* w, const float* b, PadGeo g) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
+    if (p >= g.B * g.H * g.W) return;
+    const int x = p % g.W, r = p / g.W;
+    const uint16_t* in = d + g.at(r / g.H, r % g.H, x) * 32;
     float s = b[0];
-    for (int c = 0; c < C; c++) s += bf2f(d[(size_t)p * C + c]) * w[c];
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) {
+        float f[8];
+        unpack8(ld8(in + c), f);
+#pragma unroll
+        for (int j = 0; j < 8; j++) s += f[j] * w[c + j];
+    }
     y[p] = s;
 }
 // loss = mean (y - t)^2; dy = 2 (y - t) / P; per-block partial sums of (y - t)^2
@@ -384,28 +304,6 @@ __global__ void k_mse(float* dy, float* lpart, const float* y, const float* t, i
     }
     if (threadIdx.x == 0) lpart[blockIdx.x] = sh[0];
 }
-__global__ void k_out_bwd_data(float* gd, const float* dy, const float* w, int P, int C) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (size_t)P * C) return;
-    gd[q] = dy[q / C] * w[q % C];
-}
-// dw[c] = sum_p dy[p] d[p][c] (block per c), db = sum_p dy[p] (block C)
-__global__ void k_out_bwd_w(float* dw, float* db, const float* dy, const uint16_t* d, int P, int C) {
-    __shared__ float sh[256];
-    const int c = blockIdx.x;
-    float s = 0.f;
-    for (int p = threadIdx.x; p < P; p += blockDim.x) s += c < C ? dy[p] * bf2f(d[(size_t)p * C + c]) : dy[p];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        if (c < C) dw[c] = sh[0];
-        else db[0] = sh[0];
-    }
-}
 
 // Adam on FP32 master weights, with the BF16 copy used by the convolution GEMMs
 __global__ void k_adam(float* w, float* m, float* v, uint16_t* wbf, const float* g, size_t n, float lr, float b1,
@@ -425,27 +323,32 @@ __global__ void k_to_bf16(uint16_t* o, const float* i, size_t n) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n) o[q] = f2bf(i[q]);
 }
-// NCHW FP32 -> NHWC BF16
-__global__ void k_input_nhwc(uint16_t* o, const float* i, int B, int C, int H, int W) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n = (size_t)B * C * H * W;
-    if (q >= n) return;
-    const int c = (int)(q % C);
-    size_t r = q / C;
-    const int x = (int)(r % W);
-    r /= W;
-    const int y = (int)(r % H);
-    const int b = (int)(r / H);
-    o[q] = f2bf(i[(((size_t)b * C + c) * H + y) * W + x]);
-}
 
 // ============================================================================ U-Net host side
 // 4 levels, base width 32, 3x3 convolutions with ReLU, 2x2 average pooling, nearest upsampling
-// with skip concatenation, 1x1 linear output.  Activations BF16 NHWC; FP32 master weights with
-// BF16 copies for the tensor-core GEMMs; FP32 gradients; Adam.
+// with skip concatenation, 1x1 linear output.  Activations BF16 in the padded layout of pt_conv.cuh;
+// FP32 master weights with BF16 copies for the tensor-core GEMMs; FP32 gradients; Adam.
 struct UConv {
-    int src0, src1, mode, cin, cout, level, out;  // src -1 = network input
-    size_t woff, boff;                             // in the flat parameter vector
+    int src0, src1, mode, cin, cout, level, out;  // src -1 = network input; mode 1 pools src0, 2 upsamples
+                                                  // it and appends src1
+    size_t woff, boff;                            // in the flat parameter vector
+};
+
+// a layer's GEMMs for the current batch size
+struct ConvPlan {
+    CUtensorMap A[2], B[2];
+    tc::ConvArgs a;
+    dim3 grid;
+};
+struct WgradPlan {
+    CUtensorMap A, B;
+    tc::WgradArgs a;
+    dim3 grid;
+};
+struct LayerPlan {
+    ConvPlan fwd, bwd;
+    WgradPlan wg[2];
+    int nwg = 0, nsplit = 0;
 };
 
 struct UNet {
@@ -454,18 +357,20 @@ struct UNet {
     int tch[14] = {}, tlev[14] = {};
     size_t nparams = 0, out_w = 0, out_b = 0;
     float *w32 = nullptr, *m = nullptr, *v = nullptr, *g = nullptr;
-    uint16_t* wbf = nullptr;
-    uint16_t* wbd = nullptr;  // one layer's weights in the backward-data K order (k_w_bwd_layout)
+    uint16_t *wbf = nullptr, *wbd = nullptr, *w0 = nullptr;  // BF16 weights, k_pack_weights' layouts
     int step = 0;
-    uint16_t* act[14] = {};
-    float* grad[14] = {};
-    uint16_t* x0 = nullptr;
-    float *xin = nullptr, *y = nullptr, *dy = nullptr, *tgt = nullptr, *lpart = nullptr, *dXg = nullptr,
-          *part = nullptr;
-    size_t part_cap = 0, dxg_cap = 0;
+    // padded tensors: im2col input, activations, their pooled and upsampled copies, masked gradients
+    uint16_t *im = nullptr, *act[14] = {}, *pool[14] = {}, *up[14] = {}, *dz[14] = {};
+    float *dx = nullptr, *dxcat[14] = {};  // a view's gradient; of the concatenated views, kept for the skips
+    float *xin = nullptr, *y = nullptr, *dy = nullptr, *tgt = nullptr, *lpart = nullptr, *part = nullptr,
+          *bpart = nullptr;
+    size_t part_cap = 0;
+    int planB = 0;  // batch size of the plans
+    LayerPlan plan[14];
     int* derr = nullptr;
     cudaStream_t st = nullptr;
     std::vector<void*> owned;
+    PadGeo geo(int level, int B) const { return PadGeo{B, H >> level, W >> level}; }
 };
 
 static uint64_t splitmix(uint64_t& s) {
@@ -488,10 +393,24 @@ static int ualloc(UNet& U, T** p, size_t n) {
     return 0;
 }
 
-// split of a weight-gradient GEMM over pixels: about two CTAs per SM in total
-static void wsplit(int Mw, int P, int* per, int* ns) {
-    const int gx = (Mw + 127) / 128, chunks = (P + 63) / 64;
-    const int n0 = std::max(1, std::min(chunks, 304 / gx));
+static int pack_weights(UNet& U) {
+    PackArgs a{};
+    for (int l = 0; l < 14; l++) {
+        a.cin[l] = U.L[l].cin;
+        a.cout[l] = U.L[l].cout;
+        a.woff[l] = U.L[l].woff;
+    }
+    k_pack_weights<<<dim3(64, 14), 256, 0, U.st>>>(U.wbd, U.w0, U.wbf, a);
+    return cuda_check(cudaGetLastError(), "k_pack_weights");
+}
+
+// Splits of a layer's weight gradient over the positions: about two CTAs per SM in all, and at least
+// eight chunks each; and its weight tiles' columns
+static int wgrad_ntile(int cout) { return std::min(cout, 128); }
+static void wgrad_splits(const UConv& c, size_t positions, int* per, int* ns) {
+    const int chunks = (int)((positions + tc::kWgradK - 1) / tc::kWgradK);
+    const int rows = c.src0 < 0 ? 1 : (9 * c.cin + tc::kTileM - 1) / tc::kTileM, tiles = rows * (c.cout / wgrad_ntile(c.cout));
+    const int n0 = std::max(1, std::min((chunks + 7) / 8, (304 + tiles - 1) / tiles));
     *per = (chunks + n0 - 1) / n0;
     *ns = (chunks + *per - 1) / *per;
 }
@@ -517,19 +436,18 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
         U.tch[c.out] = c.cout;
         U.tlev[c.out] = c.level;
     }
-    for (auto& c : U.L)  // ConvFwd::gather_b8 reads 16-byte-aligned rows of the BF16 weights
+    for (auto& c : U.L)  // the weight boxes start on 16-byte boundaries
         if (c.woff % 8) return fail(PT_ERR_CONFIG, "U-Net: weight offsets must be multiples of 8");
     U.out_w = off;
     off += 32;
     U.out_b = off;
     off += 1;
     U.nparams = off;
+    if (U.geo(0, maxB).positions() > (size_t)INT32_MAX / 2) return fail(PT_ERR_ARG, "U-Net: batch of grids too large");
     int rc;
-    size_t wmax = 0;
-    for (auto& c : U.L) wmax = std::max(wmax, (size_t)c.cout * 9 * c.cin);
     if ((rc = ualloc(U, &U.w32, off)) || (rc = ualloc(U, &U.m, off)) || (rc = ualloc(U, &U.v, off)) ||
-        (rc = ualloc(U, &U.g, off)) || (rc = ualloc(U, &U.wbf, off)) || (rc = ualloc(U, &U.wbd, wmax)) ||
-        (rc = ualloc(U, &U.derr, 1)))
+        (rc = ualloc(U, &U.g, off)) || (rc = ualloc(U, &U.wbf, off)) || (rc = ualloc(U, &U.wbd, off)) ||
+        (rc = ualloc(U, &U.w0, 32 * kImCols)) || (rc = ualloc(U, &U.derr, 1)))
         return rc;
     // He-normal initialisation from a portable generator; biases zero
     std::vector<float> h(off, 0.f);
@@ -542,84 +460,192 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
     CK(cudaMemcpyAsync(U.w32, h.data(), sizeof(float) * off, cudaMemcpyHostToDevice, U.st));
     k_to_bf16<<<nblk(off, 256), 256, 0, U.st>>>(U.wbf, U.w32, off);
     CK(cudaGetLastError());
-    // activations and gradients for maxB samples
-    const size_t P0 = (size_t)maxB * H * W;
-    for (int t = 0; t < 14; t++) {
-        const size_t n = (P0 >> (2 * U.tlev[t])) * U.tch[t];
-        if ((rc = ualloc(U, &U.act[t], n)) || (rc = ualloc(U, &U.grad[t], n))) return rc;
-    }
-    if ((rc = ualloc(U, &U.x0, P0 * 4)) || (rc = ualloc(U, &U.xin, P0 * 4)) || (rc = ualloc(U, &U.y, P0)) ||
-        (rc = ualloc(U, &U.dy, P0)) || (rc = ualloc(U, &U.tgt, P0)) || (rc = ualloc(U, &U.lpart, P0 / 256 + 1)))
-        return rc;
-    // workspaces: the largest view gradient, and the largest split-K partial buffer
-    size_t dxg = 0, part = 0;
+    if ((rc = pack_weights(U))) return rc;
+    // tensors for maxB samples; their padding stays zero from here on
+    auto n = [&](int level, int ch) { return U.geo(level, maxB).positions() * (size_t)ch; };
+    size_t dx = 0, part = 0, bpart = 0;
     for (auto& c : U.L) {
-        const size_t P = P0 >> (2 * c.level);
-        dxg = std::max(dxg, P * (size_t)c.cin);
+        if ((rc = ualloc(U, &U.act[c.out], n(c.level, c.cout))) || (rc = ualloc(U, &U.dz[c.out], n(c.level, c.cout))))
+            return rc;
+        if (c.mode == 1 && (rc = ualloc(U, &U.pool[c.src0], n(c.level, c.cin)))) return rc;
+        if (c.mode == 2) {
+            if ((rc = ualloc(U, &U.up[c.src0], n(c.level, U.tch[c.src0]))) ||
+                (rc = ualloc(U, &U.dxcat[c.out], n(c.level, c.cin))))
+                return rc;
+        } else {
+            dx = std::max(dx, n(c.level, c.cin));
+        }
         int per, ns;
-        wsplit(9 * c.cin, (int)P, &per, &ns);
-        part = std::max(part, (size_t)ns * 9 * c.cin * c.cout);
+        for (int B = 1; B <= maxB; B++) {  // (a smaller batch may have more splits)
+            wgrad_splits(c, U.geo(c.level, B).positions(), &per, &ns);
+            part = std::max(part, (size_t)ns * 9 * c.cin * c.cout);
+        }
     }
-    U.dxg_cap = dxg;
+    bpart = (size_t)4 * 152 * 256;
     U.part_cap = part;
-    if ((rc = ualloc(U, &U.dXg, dxg)) || (rc = ualloc(U, &U.part, part))) return rc;
-    const int smax = (int)tc::smem_bytes(256);
-    CK(cudaFuncSetAttribute(tc::k_tc_gemm<ConvFwd>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-    CK(cudaFuncSetAttribute(tc::k_tc_gemm<ConvBwdData>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-    CK(cudaFuncSetAttribute(tc::k_tc_gemm<ConvBwdW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+    const size_t P0 = (size_t)maxB * H * W;
+    if ((rc = ualloc(U, &U.im, n(0, kImCols))) || (rc = ualloc(U, &U.xin, P0 * 4)) || (rc = ualloc(U, &U.y, P0)) ||
+        (rc = ualloc(U, &U.dy, P0)) || (rc = ualloc(U, &U.tgt, P0)) || (rc = ualloc(U, &U.lpart, P0 / 256 + 1)) ||
+        (rc = ualloc(U, &U.dx, dx)) || (rc = ualloc(U, &U.part, part)) || (rc = ualloc(U, &U.bpart, bpart)))
+        return rc;
+    const int smax = (int)tc::conv_smem_bytes(256);
+    CK(cudaFuncSetAttribute(tc::k_conv_gemm<FwdEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+    CK(cudaFuncSetAttribute(tc::k_conv_gemm<DxEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+    CK(cudaFuncSetAttribute(tc::k_wgrad_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::wgrad_smem_bytes(128)));
     return 0;
 }
 
-static int ntile_for(int n) {
-    const int tiles = (n + 255) / 256;
-    const int t = (n + tiles - 1) / tiles;
-    return (t + 15) / 16 * 16;
+// 2D tensor map of a row-major BF16 array [rows][C], boxes of boxc (64 or 32) x boxr, swizzled by the box
+// row's bytes; rows outside the array read as zero
+static int tensor_map(CUtensorMap* m, const uint16_t* base, size_t C, size_t rows, int boxc, int boxr) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Encode encode = nullptr;
+    if (!encode) {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        CK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q));
+        if (!f) return fail(PT_ERR_CUDA, "cuTensorMapEncodeTiled is not in this driver");
+        encode = reinterpret_cast<Encode>(f);
+    }
+    const cuuint64_t dims[2] = {C, rows}, strides[1] = {C * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)boxc, (cuuint32_t)boxr}, es[2] = {1, 1};
+    const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(base), dims, strides, box, es,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              boxc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : fail(PT_ERR_CUDA, "U-Net: tensor map");
 }
 
-template <class Prob>
-static int run_gemm(UNet& U, Prob p, int nsplit) {
-    dim3 grid((p.M + tc::kTileM - 1) / tc::kTileM, (p.N + p.Ntile - 1) / p.Ntile, nsplit);
-    tc::k_tc_gemm<Prob><<<grid, tc::kThreads, tc::smem_bytes(p.Ntile), U.st>>>(p, U.derr);
-    CK(cudaGetLastError());
-    return 0;
-}
-
-static InView view_of(const UNet& U, const UConv& c, int B) {
-    InView v{};
-    v.B = B;
-    v.H = U.H >> c.level;
-    v.W = U.W >> c.level;
-    v.mode = c.mode;
+// the sources of a layer's view as padded tensors
+static int view_sources(const UNet& U, const UConv& c, const uint16_t* (&t)[2], int (&C)[2]) {
+    C[1] = 0;
+    t[1] = nullptr;
     if (c.src0 < 0) {
-        v.t0 = U.x0;
-        v.C0 = 4;
-    } else {
-        v.t0 = U.act[c.src0];
-        v.C0 = U.tch[c.src0];
+        t[0] = U.im;
+        C[0] = kImCols;
+        return 1;
     }
-    if (c.mode == 2) {
-        v.t1 = U.act[c.src1];
-        v.C1 = U.tch[c.src1];
+    t[0] = c.mode == 1 ? U.pool[c.src0] : c.mode == 2 ? U.up[c.src0] : U.act[c.src0];
+    C[0] = U.tch[c.src0];
+    if (c.mode != 2) return 1;
+    t[1] = U.act[c.src1];
+    C[1] = U.tch[c.src1];
+    return 2;
+}
+
+// one convolution GEMM: sources t (C channels each), weights w [N][Ktot], over the positions of g.  The
+// column tile is the largest that still gives every SM a CTA (at least 32 columns).
+static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* const* t, const int* C, const uint16_t* w,
+                     int N) {
+    tc::ConvArgs& a = P.a;
+    a.g = g;
+    a.taps = taps;
+    a.nsrc = nsrc;
+    a.N = N;
+    a.Ktot = 0;
+    for (int s = 0; s < 2; s++) {
+        a.C[s] = C[s];
+        a.bw[s] = C[s] % 64 == 0 && C[s] > 0 ? 64 : 32;
+        a.Ktot += taps * C[s];
     }
-    return v;
+    a.first = g.Wp();
+    a.last = (int)((size_t)g.B * g.Hp() * g.Wp());
+    const int mt = (a.last - a.first + tc::kTileM - 1) / tc::kTileM;
+    int nt = 1;
+    while (N / nt > 256 || N % nt || (N / nt) % 32) nt++;
+    for (int f = nt + 1; f <= N / 32 && mt * nt < 152; f++)
+        if (N % f == 0 && (N / f) % 32 == 0) nt = f;
+    a.Ntile = N / nt;
+    P.grid = dim3(mt, nt);
+    int rc;
+    for (int s = 0; s < 2; s++) {
+        const int q = s < nsrc ? s : 0;
+        if ((rc = tensor_map(&P.A[s], t[q], C[q], g.positions(), a.bw[q], tc::kTileM)) ||
+            (rc = tensor_map(&P.B[s], w, a.Ktot, N, a.bw[q], a.Ntile)))
+            return rc;
+    }
+    return 0;
+}
+
+static int plan_batch(UNet& U, int B) {
+    if (U.planB == B) return 0;
+    U.planB = 0;
+    int rc;
+    for (size_t li = 0; li < U.L.size(); li++) {
+        const UConv& c = U.L[li];
+        LayerPlan& P = U.plan[li];
+        const PadGeo g = U.geo(c.level, B);
+        const uint16_t* t[2];
+        int C[2];
+        const int ns = view_sources(U, c, t, C);
+        const bool first = c.src0 < 0;
+        if ((rc = plan_conv(P.fwd, g, first ? 1 : 9, ns, t, C, first ? U.w0 : U.wbf + c.woff, c.cout))) return rc;
+        const uint16_t* z[2] = {U.dz[c.out], nullptr};
+        const int Cz[2] = {c.cout, 0};
+        if (!first && (rc = plan_conv(P.bwd, g, 9, 1, z, Cz, U.wbd + c.woff, c.cin))) return rc;
+        int per;
+        wgrad_splits(c, g.positions(), &per, &P.nsplit);
+        if ((size_t)P.nsplit * 9 * c.cin * c.cout > U.part_cap) return fail(PT_ERR_STATE, "U-Net: split workspace too small");
+        P.nwg = ns;
+        for (int s = 0; s < ns; s++) {
+            WgradPlan& w = P.wg[s];
+            tc::WgradArgs& a = w.a;
+            a.g = g;
+            a.taps = first ? 1 : 9;
+            a.C = C[s];
+            a.bwA = C[s] % 64 == 0 ? 64 : 32;
+            a.c_off = s ? C[0] : 0;
+            a.cin = first ? 9 * c.cin : c.cin;
+            a.kk_max = 9 * c.cin;
+            a.N = c.cout;
+            a.Ntile = wgrad_ntile(c.cout);
+            a.bwB = c.cout % 64 == 0 ? 64 : 32;
+            a.per = per;
+            a.chunks = (int)((g.positions() + tc::kWgradK - 1) / tc::kWgradK);
+            a.part = U.part;
+            const int blocks = a.taps * (a.C / a.bwA), ablk = tc::kTileM / a.bwA;
+            w.grid = dim3((blocks + ablk - 1) / ablk, c.cout / a.Ntile, P.nsplit);
+            if ((rc = tensor_map(&w.A, t[s], C[s], g.positions(), a.bwA, tc::kWgradK)) ||
+                (rc = tensor_map(&w.B, U.dz[c.out], c.cout, g.positions(), a.bwB, tc::kWgradK)))
+                return rc;
+        }
+    }
+    U.planB = B;
+    return 0;
+}
+
+template <class E>
+static int run_conv(UNet& U, const ConvPlan& P, const E& e) {
+    tc::k_conv_gemm<E><<<P.grid, tc::kConvThreads, tc::conv_smem_bytes(P.a.Ntile), U.st>>>(P.A[0], P.A[1], P.B[0], P.B[1],
+                                                                                       P.a, e, U.derr);
+    return cuda_check(cudaGetLastError(), "k_conv_gemm");
 }
 
 // network input already in U.xin (device, NCHW FP32); output in U.y ([B][H][W] FP32).
 // ev (optional): 15 CUDA events recorded around the 14 convolution GEMMs
 static int unet_forward(UNet& U, int B, cudaEvent_t* ev = nullptr) {
     const size_t P0 = (size_t)B * U.H * U.W;
-    k_input_nhwc<<<nblk(P0 * 4, 256), 256, 0, U.st>>>(U.x0, U.xin, B, 4, U.H, U.W);
+    int rc;
+    if ((rc = plan_batch(U, B))) return rc;
+    k_im2col<<<nblk(P0 * 5, 256), 256, 0, U.st>>>(U.im, U.xin, U.geo(0, B));
     CK(cudaGetLastError());
     int li = 0;
     if (ev) CK(cudaEventRecord(ev[0], U.st));
     for (auto& c : U.L) {
-        const InView v = view_of(U, c, B);
-        const int P = B * v.H * v.W;
-        ConvFwd f{P, c.cout, 9 * c.cin, ntile_for(c.cout), 0, v, U.wbf + c.woff, U.w32 + c.boff, U.act[c.out], 1};
-        if (int rc = run_gemm(U, f, 1)) return rc;
-        if (ev) CK(cudaEventRecord(ev[++li], U.st));
+        if (c.mode == 1) {
+            const PadGeo g = U.geo(c.level, B);
+            const size_t n = (size_t)B * g.H * g.W * (c.cin / 8);
+            k_pool<<<nblk(n, 256), 256, 0, U.st>>>(U.pool[c.src0], U.act[c.src0], g, U.geo(c.level - 1, B), c.cin);
+            CK(cudaGetLastError());
+        }
+        const FwdEpi e{U.act[c.out], U.w32 + c.boff, c.cout, U.up[c.out], U.geo(c.level > 0 ? c.level - 1 : 0, B)};
+        if ((rc = run_conv(U, U.plan[li].fwd, e))) return rc;
+        li++;
+        if (ev) CK(cudaEventRecord(ev[li], U.st));
     }
-    k_out_fwd<<<nblk(P0, 256), 256, 0, U.st>>>(U.y, U.act[13], U.w32 + U.out_w, U.w32 + U.out_b, (int)P0, 32);
+    k_out_fwd<<<nblk(P0, 128), 128, 0, U.st>>>(U.y, U.act[13], U.w32 + U.out_w, U.w32 + U.out_b, U.geo(0, B));
     CK(cudaGetLastError());
     return 0;
 }
@@ -632,54 +658,72 @@ static int gemm_error(UNet& U) {
     return 0;
 }
 
+// dZ of the layer that produced tensor t from where its gradient lies, and that layer's bias gradient
+template <int MODE>
+static int run_dz(UNet& U, int t, int B, DzArgs a) {
+    const UConv& c = U.L[t];  // (tensor t is layer t's output)
+    a.g = U.geo(c.level, B);
+    a.C = c.cout;
+    a.Y = U.act[t];
+    a.dZ = U.dz[t];
+    a.part = U.bpart;
+    const size_t oct = (size_t)B * a.g.H * a.g.W * (c.cout / 8);
+    const int blocks = (int)std::min<size_t>(nblk(oct, 4 * kDzThreads), 4 * 152);
+    k_dz<MODE><<<blocks, kDzThreads, 0, U.st>>>(a);
+    const int ld = MODE == kDzOut ? 2 * c.cout + 1 : c.cout;
+    k_colsum<<<nblk(c.cout, 4), 128, 0, U.st>>>(U.g + c.boff, U.bpart, blocks, ld, 0, c.cout);
+    if (MODE == kDzOut)  // (the output layer's weights and bias lie next to each other)
+        k_colsum<<<nblk(c.cout + 1, 4), 128, 0, U.st>>>(U.g + U.out_w, U.bpart, blocks, ld, c.cout, c.cout + 1);
+    return cuda_check(cudaGetLastError(), "k_dz");
+}
+
 // gradients of the MSE loss against U.tgt into U.g; loss on the host
 static int unet_backward(UNet& U, int B, float* loss) {
     const int P0 = B * U.H * U.W;
     const int nb = (int)nblk(P0, 256);
+    int rc;
     k_mse<<<nb, 256, 0, U.st>>>(U.dy, U.lpart, U.y, U.tgt, P0);
-    for (int t = 0; t < 14; t++)
-        CK(cudaMemsetAsync(U.grad[t], 0, sizeof(float) * ((size_t)P0 >> (2 * U.tlev[t])) * U.tch[t], U.st));
-    k_out_bwd_data<<<nblk((size_t)P0 * 32, 256), 256, 0, U.st>>>(U.grad[13], U.dy, U.w32 + U.out_w, P0, 32);
-    k_out_bwd_w<<<33, 256, 0, U.st>>>(U.g + U.out_w, U.g + U.out_b, U.dy, U.act[13], P0, 32);
     CK(cudaGetLastError());
+    DzArgs o{};
+    o.dx = U.dy;
+    o.w = U.w32 + U.out_w;
+    if ((rc = run_dz<kDzOut>(U, 13, B, o))) return rc;
     for (int li = (int)U.L.size() - 1; li >= 0; li--) {
         const UConv& c = U.L[li];
-        const InView v = view_of(U, c, B);
-        const int P = B * v.H * v.W;
-        const float* dY = U.grad[c.out];
-        const uint16_t* Y = U.act[c.out];
-        // weights: split over pixels, then a fixed-order reduction of the splits
+        const LayerPlan& P = U.plan[li];
+        // weights: split over positions, then a fixed-order reduction of the splits
         const int Mw = 9 * c.cin;
-        int per, ns;
-        wsplit(Mw, P, &per, &ns);
-        if ((size_t)ns * Mw * c.cout > U.part_cap) return fail(PT_ERR_STATE, "U-Net: split workspace too small");
-        ConvBwdW bw{Mw, c.cout, P, ntile_for(c.cout), per, v, dY, Y, U.part};
-        if (int rc = run_gemm(U, bw, ns)) return rc;
-        k_wgrad_reduce<<<nblk((size_t)Mw * c.cout, 256), 256, 0, U.st>>>(U.g + c.woff, U.part, ns, Mw, c.cout);
-        k_bias_grad<<<c.cout, 256, 0, U.st>>>(U.g + c.boff, dY, Y, P, c.cout);
+        for (int s = 0; s < P.nwg; s++)
+            tc::k_wgrad_gemm<<<P.wg[s].grid, tc::kConvThreads, tc::wgrad_smem_bytes(P.wg[s].a.Ntile), U.st>>>(
+                P.wg[s].A, P.wg[s].B, P.wg[s].a, U.derr);
+        k_wgrad_reduce<<<nblk((size_t)Mw * c.cout, 256), 256, 0, U.st>>>(U.g + c.woff, U.part, P.nsplit, Mw, c.cout);
         CK(cudaGetLastError());
         if (c.src0 < 0) continue;  // the network input needs no gradient
-        if ((size_t)P * c.cin > U.dxg_cap) return fail(PT_ERR_STATE, "U-Net: view-gradient workspace too small");
-        const size_t nw = (size_t)c.cin * 9 * c.cout;
-        k_w_bwd_layout<<<nblk(nw, 256), 256, 0, U.st>>>(U.wbd, U.wbf + c.woff, c.cin, c.cout);
-        ConvBwdData bd{P, c.cin, 9 * c.cout, ntile_for(c.cin), 0, v.H, v.W, c.cout, dY, Y, U.wbf + c.woff, U.wbd,
-                       U.dXg};
-        if (int rc = run_gemm(U, bd, 1)) return rc;
+        float* dx = c.mode == 2 ? U.dxcat[c.out] : U.dx;
+        if ((rc = run_conv(U, P.bwd, DxEpi{dx, c.cin}))) return rc;
+        DzArgs a{};
+        a.dx = dx;
+        a.ldx = c.cin;
         if (c.mode == 0) {
-            const size_t n = (size_t)P * c.cin;
-            k_adj_plain<<<nblk(n, 256), 256, 0, U.st>>>(U.grad[c.src0], U.dXg, n);
-        } else if (c.mode == 1) {
-            const size_t n = (size_t)B * 4 * v.H * v.W * c.cin;
-            k_adj_pool<<<nblk(n, 256), 256, 0, U.st>>>(U.grad[c.src0], U.dXg, B, v.H, v.W, c.cin);
-        } else {
-            const size_t n = (size_t)B * (v.H / 2) * (v.W / 2) * v.C0 + (size_t)P * v.C1;
-            k_adj_upcat<<<nblk(n, 256), 256, 0, U.st>>>(U.grad[c.src0], U.grad[c.src1], U.dXg, B, v.H, v.W, v.C0, v.C1);
+            rc = run_dz<kDzPlain>(U, c.src0, B, a);
+        } else if (c.mode == 2) {
+            a.g2 = U.geo(c.level, B);
+            rc = run_dz<kDzUp>(U, c.src0, B, a);
+        } else {  // the skip connection's share was left by the layer that concatenates this tensor
+            a.g2 = U.geo(c.level, B);
+            for (auto& q : U.L)
+                if (q.src1 == c.src0) {
+                    a.skip = U.dxcat[q.out];
+                    a.lds = q.cin;
+                    a.offs = U.tch[q.src0];
+                }
+            rc = run_dz<kDzPooled>(U, c.src0, B, a);
         }
-        CK(cudaGetLastError());
+        if (rc) return rc;
     }
     std::vector<float> lp(nb);
     CK(cudaMemcpyAsync(lp.data(), U.lpart, sizeof(float) * nb, cudaMemcpyDeviceToHost, U.st));
-    if (int rc = gemm_error(U)) return rc;
+    if ((rc = gemm_error(U))) return rc;
     double sum = 0.0;
     for (float a : lp) sum += a;
     if (loss) *loss = (float)(sum / P0);
@@ -692,7 +736,7 @@ static int unet_adam(UNet& U, float lr) {
     const float c1 = 1.f - std::pow(b1, (float)U.step), c2 = 1.f - std::pow(b2, (float)U.step);
     k_adam<<<nblk(U.nparams, 256), 256, 0, U.st>>>(U.w32, U.m, U.v, U.wbf, U.g, U.nparams, lr, b1, b2, 1e-8f, c1, c2);
     CK(cudaGetLastError());
-    return 0;
+    return pack_weights(U);
 }
 
 // ============================================================================ engine side
@@ -892,6 +936,7 @@ int pt_unet_set_params(pt_unet* net, const float* host) {
     CK(cudaMemcpyAsync(U.w32, host, sizeof(float) * U.nparams, cudaMemcpyHostToDevice, U.st));
     k_to_bf16<<<nblk(U.nparams, 256), 256, 0, U.st>>>(U.wbf, U.w32, U.nparams);
     CK(cudaGetLastError());
+    if (int rc = pack_weights(U)) return rc;
     CK(cudaStreamSynchronize(U.st));
     return 0;
 }

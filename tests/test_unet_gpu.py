@@ -96,3 +96,40 @@ def test_unet_adam_reduces_loss_and_weights_round_trip(tmp_path):
     assert np.array_equal(net.forward(x), net2.forward(x))
     net2.close()
     net.close()
+
+
+@pytest.mark.parametrize("nz,nx,B", [(8, 8, 1), (24, 40, 3), (16, 136, 2), (56, 16, 5)])
+def test_unet_ragged_grids_match_the_oracle(nz, nx, B):
+    """Grids whose rows and pixel counts fill no tile of 128 positions, the smallest one among them
+    (the bounds of test_unet_forward_and_gradients_match_cpu_oracle: BF16 rounding of the same points)."""
+    import oracle.unet_ref as ur
+
+    net = _Net(nz, nx, B, 5)
+    rng = np.random.default_rng(nz + nx)
+    x, t = _smooth_batch(rng, B, nz, nx)
+    p = net.params().astype(np.float64)
+    y_ref, _ = ur.forward(p, x)
+    assert np.max(np.abs(net.forward(x) - y_ref)) <= 1e-2 * np.max(np.abs(y_ref))
+    loss, g = net.gradients(x, t)
+    loss_ref, g_ref = ur.gradients(p, x, t)
+    assert abs(loss - loss_ref) <= 1e-2 * loss_ref
+    offs, out_w, out_b, total = ur.layout()
+    for li, (wo, bo) in enumerate(offs):
+        for a, b in ((wo, bo), (bo, bo + ur.SPEC[li][4])):
+            assert np.linalg.norm(g[a:b] - g_ref[a:b]) < 3e-2 * max(np.linalg.norm(g_ref[a:b]), 1e-30), (li, a == wo)
+    assert np.allclose(g[out_w:total], g_ref[out_w:total], rtol=1e-2, atol=1e-2 * np.abs(g_ref[out_w:total]).max())
+    net.close()
+
+
+def test_unet_batches_below_the_maximum_see_nothing_of_earlier_ones():
+    nz, nx = 24, 40
+    rng = np.random.default_rng(1)
+    x, t = _smooth_batch(rng, 4, nz, nx)
+    net = _Net(nz, nx, 4, 3)
+    net.gradients(1e3 * x, t)
+    fresh = _Net(nz, nx, 2, 3)
+    assert np.array_equal(net.forward(x[:2]), fresh.forward(x[:2]))
+    a, b = net.gradients(x[:2], t[:2]), fresh.gradients(x[:2], t[:2])
+    assert a[0] == b[0] and np.array_equal(a[1], b[1])
+    net.close()
+    fresh.close()
