@@ -9,7 +9,7 @@
 //   * k_conv_gemm (forward, backward-data): a CTA computes 128 positions x Ntile columns.  One thread
 //     issues the TMA loads of a chunk (one tap, 64 or 32 channels: A box and weight box, K-major,
 //     128- or 64-byte swizzle), one the MMAs (K = 16 each, taps and channels in ascending order, so an
-//     output's sum does not depend on the tiling), through kConvStages stages with full/empty mbarriers;
+//     output's sum does not depend on the tiling), through a ring of stages with full/empty mbarriers;
 //     four warps read the accumulator from tensor memory and store.
 //   * k_wgrad_gemm: M = 128 rows of (tap, input channel), N = output channels, K = positions.  Both
 //     operands are the same boxes read with their channels as the leading dimension (MN-major).
@@ -22,8 +22,7 @@
 namespace pt {
 namespace tc {
 
-constexpr int kConvStages = 4, kConvThreads = 192;  // warps 0-3: epilogue, 4: TMA, 5: MMA
-constexpr int kMaxBlocks = 4;                       // operand boxes of a weight-gradient stage
+constexpr int kMaxStages = 10, kConvThreads = 192;  // warps 0-3: epilogue, 4: TMA, 5: MMA
 
 // shared-memory descriptor with a swizzle: layout 2 = 128-byte, 4 = 64-byte; strides in bytes
 __device__ __forceinline__ uint64_t smem_desc_sw(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
@@ -79,6 +78,7 @@ struct PadGeo {
 struct ConvArgs {
     PadGeo g;
     int taps, nsrc, C[2], bw[2], Ktot, N, Ntile, first, last;  // positions first .. last - 1
+    int stages, abytes, bbytes;                               // pipeline depth; operand bytes of a stage
 };
 
 // one role's failure ends the CTA: waits that follow return at once
@@ -89,8 +89,16 @@ __device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
-__host__ __device__ constexpr size_t conv_stage_bytes(int ntile) { return 16384 + (size_t)ntile * 128; }
-__host__ __device__ constexpr size_t conv_smem_bytes(int ntile) { return kConvStages * conv_stage_bytes(ntile) + 1024; }
+// Pipeline depth for stages of sbytes in a grid of `ctas`: with a CTA per SM at most, as deep as the
+// shared memory allows, since a chunk's load latency (1-2 us) is all there is; with more, four stages, so
+// that several CTAs share an SM and one's prologue and epilogue run beside the others' loads.
+static inline int conv_stages(size_t sbytes, size_t ctas, int chunks) {
+    const int most = (int)((220 * 1024) / sbytes);
+    int s = ctas <= 152 ? most : 4;
+    s = s < most ? s : most;
+    s = s < chunks ? s : chunks;
+    return s < kMaxStages ? (s > 1 ? s : 1) : kMaxStages;
+}
 
 // Epilogue E: void operator()(int p, int col0, const float (&v)[32]) for columns col0 .. col0 + 31 of
 // position p (called for real pixels with their coordinates)
@@ -101,17 +109,18 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
                                                             const __grid_constant__ CUtensorMap mapB1, ConvArgs a, E epi,
                                                             int* err) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t full[kConvStages], empty[kConvStages], done;
+    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
     __shared__ uint32_t tslot;
     __shared__ int bad;
     unsigned char* const smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int p0 = a.first + blockIdx.x * kTileM, n0 = blockIdx.y * a.Ntile;
     const uint32_t ncols = tmem_cols(a.Ntile);
-    const size_t sbytes = conv_stage_bytes(a.Ntile);
+    const int S = a.stages;
+    const size_t sbytes = (size_t)(a.abytes + a.bbytes);
     if (tid == 0) {
         bad = 0;
-        for (int s = 0; s < kConvStages; s++) {
+        for (int s = 0; s < S; s++) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
@@ -124,33 +133,55 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
     tc_fence_after();
     const uint32_t taddr = tslot;
     const int nb0 = a.C[0] / a.bw[0], nb1 = a.nsrc > 1 ? a.C[1] / a.bw[1] : 0, nblk = nb0 + nb1, chunks = a.taps * nblk;
+    // One thread each drives the loads and the MMAs, so a chunk's instructions are a serial chain: counters
+    // instead of divisions (with them a chunk took 0.6 us).
     if (warp == 4 && lane == 0) {
-        int k = 0;
-        for (int c = 0; c < chunks; c++) {
-            const int st = c % kConvStages, use = c / kConvStages;
-            if (use > 0 && !conv_wait(empty + st, (use - 1) & 1, &bad)) break;
-            const int tap = c / nblk, blk = c - tap * nblk, src = blk >= nb0;
-            const int shift = a.taps == 1 ? 0 : (tap / 3 - 1) * a.g.Wp() + (tap % 3 - 1);
-            const int bw = a.bw[src], ch = (src ? blk - nb0 : blk) * bw;
-            unsigned char* sa = smem + st * sbytes;
-            mbar_expect(full + st, (uint32_t)((kTileM + a.Ntile) * bw * 2));
-            tma_load_2d(sa, src ? &mapA1 : &mapA0, ch, p0 + shift, full + st);
-            tma_load_2d(sa + 16384, bw == a.bw[0] ? &mapB0 : &mapB1, k, n0, full + st);
-            k += bw;
+        int k = 0, st = 0, dx = -1, shift = a.taps == 1 ? 0 : -a.g.Wp() - 1;
+        uint32_t parity = 1;  // of the stage's previous use; the first wait for a stage passes
+        bool go = true;
+        for (int tap = 0; tap < a.taps && go; tap++) {
+            for (int blk = 0; blk < nblk; blk++) {
+                if (!conv_wait(empty + st, parity, &bad)) {
+                    go = false;
+                    break;
+                }
+                const int src = blk >= nb0, bw = a.bw[src], ch = (src ? blk - nb0 : blk) * bw;
+                unsigned char* sa = smem + st * sbytes;
+                mbar_expect(full + st, (uint32_t)((kTileM + a.Ntile) * bw * 2));
+                tma_load_2d(sa, src ? &mapA1 : &mapA0, ch, p0 + shift, full + st);
+                tma_load_2d(sa + a.abytes, bw == a.bw[0] ? &mapB0 : &mapB1, k, n0, full + st);
+                k += bw;
+                if (++st == S) {
+                    st = 0;
+                    parity ^= 1u;
+                }
+            }
+            shift += dx < 1 ? 1 : a.g.Wp() - 2;
+            dx = dx < 1 ? dx + 1 : -1;
         }
     } else if (warp == 5 && lane == 0) {
         const uint32_t idesc = idesc_bf16(a.Ntile);
+        const uint64_t d64 = smem_desc_sw(0, 16, 1024, 2u), d32 = smem_desc_sw(0, 16, 512, 4u);
+        int st = 0, blk = 0;
+        uint32_t parity = 0, acc = 0;
         for (int c = 0; c < chunks; c++) {
-            const int st = c % kConvStages;
-            if (!conv_wait(full + st, (c / kConvStages) & 1, &bad)) break;
+            if (!conv_wait(full + st, parity, &bad)) break;
             tc_fence_after();
-            const int blk = c % nblk, bw = a.bw[blk >= nb0];
-            const uint32_t sa = smem_u32(smem + st * sbytes), sb = sa + 16384;
-            const uint32_t layout = bw == 64 ? 2u : 4u, sbo = bw == 64 ? 1024u : 512u;
-            for (int s = 0; s < bw / 16; s++)
-                mma_bf16(taddr, smem_desc_sw(sa + s * 32, 16, sbo, layout), smem_desc_sw(sb + s * 32, 16, sbo, layout),
-                         idesc, (c > 0 || s > 0) ? 1u : 0u);
+            const bool wide = a.bw[blk >= nb0] == 64;
+            const uint32_t sa = smem_u32(smem) + (uint32_t)(st * sbytes);
+            const uint64_t da = (wide ? d64 : d32) + (sa >> 4), db = da + (uint32_t)(a.abytes >> 4);
+#pragma unroll
+            for (int s = 0; s < 4; s++) {
+                if (s >= 2 && !wide) break;
+                mma_bf16(taddr, da + 2 * s, db + 2 * s, idesc, acc);  // 16 channels further: 32 bytes
+                acc = 1u;
+            }
             mma_commit(empty + st);
+            if (++blk == nblk) blk = 0;
+            if (++st == S) {
+                st = 0;
+                parity ^= 1u;
+            }
         }
         mma_commit(&done);
     }
@@ -171,7 +202,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
     __syncthreads();
     if (bad && tid == 0) {
         atomicOr(err, 1);
-        for (int s = 0; s < kConvStages; s++) mbar_wait(full + s, 0);  // copies still in flight (bounded)
+        for (int s = 0; s < S; s++) mbar_wait(full + s, 0);  // copies still in flight (bounded)
     }
     if (warp == 5) tmem_dealloc(taddr, ncols);
 }
@@ -182,13 +213,11 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
 struct WgradArgs {
     PadGeo g;
     int taps, C, bwA, c_off, cin, N, Ntile, bwB, per, chunks;  // per: chunks of 64 positions a split, of `chunks`
-    int kk_max;                                                // rows kk >= kk_max are not stored (im2col padding)
+    int kk_max;  // rows kk >= kk_max are not stored (im2col padding)
+    int stages, abytes, bbytes;
     float* part;
 };
 constexpr int kWgradK = 64;
-__host__ __device__ constexpr size_t wgrad_smem_bytes(int ntile) {
-    return kConvStages * (16384 + (size_t)ntile * 128) + 1024;
-}
 // instruction descriptor with both operands MN-major
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) { return idesc_bf16(n) | (1u << 15) | (1u << 16); }
 
@@ -196,17 +225,18 @@ __global__ void __launch_bounds__(kConvThreads) k_wgrad_gemm(const __grid_consta
                                                              const __grid_constant__ CUtensorMap mapB, WgradArgs a,
                                                              int* err) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t full[kConvStages], empty[kConvStages], done;
+    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
     __shared__ uint32_t tslot;
     __shared__ int bad;
     unsigned char* const smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.y * a.Ntile;
     const uint32_t ncols = tmem_cols(a.Ntile);
-    const size_t sbytes = 16384 + (size_t)a.Ntile * 128;
+    const int S = a.stages;
+    const size_t sbytes = (size_t)(a.abytes + a.bbytes);
     if (tid == 0) {
         bad = 0;
-        for (int s = 0; s < kConvStages; s++) {
+        for (int s = 0; s < S; s++) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
@@ -220,35 +250,52 @@ __global__ void __launch_bounds__(kConvThreads) k_wgrad_gemm(const __grid_consta
     const uint32_t taddr = tslot;
     const int cbeg = blockIdx.z * a.per, cend = min(a.chunks, cbeg + a.per), n = max(0, cend - cbeg);
     const int ablk = kTileM / a.bwA, nch = a.C / a.bwA, blocks = a.taps * nch, bblk = a.Ntile / a.bwB;
-    const uint32_t abytes = (uint32_t)(kWgradK * a.bwA * 2), bbytes = (uint32_t)(kWgradK * a.bwB * 2);
+    const uint32_t abox = (uint32_t)(kWgradK * a.bwA * 2), bbox = (uint32_t)(kWgradK * a.bwB * 2);
     if (warp == 4 && lane == 0) {
-        for (int c = 0; c < n; c++) {
-            const int st = c % kConvStages, use = c / kConvStages;
-            if (use > 0 && !conv_wait(empty + st, (use - 1) & 1, &bad)) break;
+        int ch[4], shift[4];  // of the A blocks; past the last one: loaded, not stored
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int blk = min((int)blockIdx.x * ablk + q, blocks - 1), tap = blk / nch;
+            ch[q] = (blk - tap * nch) * a.bwA;
+            shift[q] = a.taps == 1 ? 0 : (tap / 3 - 1) * a.g.Wp() + (tap % 3 - 1);
+        }
+        int st = 0, p = cbeg * kWgradK;
+        uint32_t parity = 1;  // of the stage's previous use; the first wait for a stage passes
+        for (int c = 0; c < n; c++, p += kWgradK) {
+            if (!conv_wait(empty + st, parity, &bad)) break;
             unsigned char* sa = smem + st * sbytes;
-            const int p = (cbeg + c) * kWgradK;
-            mbar_expect(full + st, (uint32_t)ablk * abytes + (uint32_t)bblk * bbytes);
-            for (int q = 0; q < ablk; q++) {
-                const int blk = min((int)blockIdx.x * ablk + q, blocks - 1);  // past the last: loaded, not stored
-                const int tap = blk / nch, ch = (blk - tap * nch) * a.bwA;
-                const int shift = a.taps == 1 ? 0 : (tap / 3 - 1) * a.g.Wp() + (tap % 3 - 1);
-                tma_load_2d(sa + q * abytes, &mapA, ch, p + shift, full + st);
+            mbar_expect(full + st, (uint32_t)ablk * abox + (uint32_t)bblk * bbox);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (q < ablk) tma_load_2d(sa + q * abox, &mapA, ch[q], p + shift[q], full + st);
+            for (int q = 0; q < bblk; q++) tma_load_2d(sa + a.abytes + q * bbox, &mapB, n0 + q * a.bwB, p, full + st);
+            if (++st == S) {
+                st = 0;
+                parity ^= 1u;
             }
-            for (int q = 0; q < bblk; q++) tma_load_2d(sa + 16384 + q * bbytes, &mapB, n0 + q * a.bwB, p, full + st);
         }
     } else if (warp == 5 && lane == 0) {
         const uint32_t idesc = idesc_bf16_mn(a.Ntile);
-        const uint32_t la = a.bwA == 64 ? 2u : 4u, lb = a.bwB == 64 ? 2u : 4u;
         const uint32_t ra = (uint32_t)a.bwA * 2, rb = (uint32_t)a.bwB * 2;  // bytes of a position's block row
+        const uint64_t da0 = smem_desc_sw(0, abox, 8 * ra, a.bwA == 64 ? 2u : 4u);
+        const uint64_t db0 = smem_desc_sw(0, bbox, 8 * rb, a.bwB == 64 ? 2u : 4u);
+        int st = 0;
+        uint32_t parity = 0, acc = 0;
         for (int c = 0; c < n; c++) {
-            const int st = c % kConvStages;
-            if (!conv_wait(full + st, (c / kConvStages) & 1, &bad)) break;
+            if (!conv_wait(full + st, parity, &bad)) break;
             tc_fence_after();
-            const uint32_t sa = smem_u32(smem + st * sbytes), sb = sa + 16384;
-            for (int s = 0; s < kWgradK / 16; s++)
-                mma_bf16(taddr, smem_desc_sw(sa + s * 16 * ra, abytes, 8 * ra, la),
-                         smem_desc_sw(sb + s * 16 * rb, bbytes, 8 * rb, lb), idesc, (c > 0 || s > 0) ? 1u : 0u);
+            const uint32_t sa = smem_u32(smem) + (uint32_t)(st * sbytes);
+            const uint64_t da = da0 + (sa >> 4), db = db0 + ((sa + (uint32_t)a.abytes) >> 4);
+#pragma unroll
+            for (int s = 0; s < kWgradK / 16; s++) {
+                mma_bf16(taddr, da + s * ra, db + s * rb, idesc, acc);  // 16 positions further
+                acc = 1u;
+            }
             mma_commit(empty + st);
+            if (++st == S) {
+                st = 0;
+                parity ^= 1u;
+            }
         }
         mma_commit(&done);
     }
@@ -274,7 +321,7 @@ __global__ void __launch_bounds__(kConvThreads) k_wgrad_gemm(const __grid_consta
     __syncthreads();
     if (bad && tid == 0) {
         atomicOr(err, 1);
-        for (int s = 0; s < kConvStages; s++) mbar_wait(full + s, 0);  // copies still in flight (bounded)
+        for (int s = 0; s < S; s++) mbar_wait(full + s, 0);  // copies still in flight (bounded)
     }
     if (warp == 5) tmem_dealloc(taddr, ncols);
 }

@@ -153,13 +153,23 @@ __global__ void k_pack_weights(uint16_t* __restrict__ wbd, uint16_t* __restrict_
     }
 }
 
-// dW[co][kk] = sum_z part[z][kk][co], z ascending
-__global__ void k_wgrad_reduce(float* dW, const float* part, int nsplit, int M, int N) {
+// dW[co][kk] = sum_z part[z][kk][co], z ascending (loads of eight splits in flight); with two sources
+// the rows' channels below c0 have nsplit0 partial sums, the others nsplit1
+__global__ void k_wgrad_reduce(float* dW, const float* part, int nsplit0, int nsplit1, int c0, int cin, int M, int N) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= M * N) return;
-    const int kk = q / N, co = q % N;
+    const int kk = q / N, co = q % N, nsplit = kk % cin < c0 ? nsplit0 : nsplit1;
+    const size_t ld = (size_t)M * N;
     float s = 0.f;
-    for (int z = 0; z < nsplit; z++) s += part[((size_t)z * M + kk) * N + co];
+    int z = 0;
+    for (; z + 8 <= nsplit; z += 8) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = part[(size_t)(z + j) * ld + q];
+#pragma unroll
+        for (int j = 0; j < 8; j++) s += v[j];
+    }
+    for (; z < nsplit; z++) s += part[(size_t)z * ld + q];
     dW[(size_t)co * M + kk] = s;
 }
 
@@ -348,7 +358,7 @@ struct WgradPlan {
 struct LayerPlan {
     ConvPlan fwd, bwd;
     WgradPlan wg[2];
-    int nwg = 0, nsplit = 0;
+    int nwg = 0, nsplit[2] = {};
 };
 
 struct UNet {
@@ -404,12 +414,12 @@ static int pack_weights(UNet& U) {
     return cuda_check(cudaGetLastError(), "k_pack_weights");
 }
 
-// Splits of a layer's weight gradient over the positions: about two CTAs per SM in all, and at least
-// eight chunks each; and its weight tiles' columns
+// Weight tiles' columns, and the splits over the positions of the weight gradient of a source of C channels:
+// about two CTAs per SM in all, and at least eight chunks each
 static int wgrad_ntile(int cout) { return std::min(cout, 128); }
-static void wgrad_splits(const UConv& c, size_t positions, int* per, int* ns) {
+static void wgrad_splits(int taps, int C, int cout, size_t positions, int* per, int* ns) {
     const int chunks = (int)((positions + tc::kWgradK - 1) / tc::kWgradK);
-    const int rows = c.src0 < 0 ? 1 : (9 * c.cin + tc::kTileM - 1) / tc::kTileM, tiles = rows * (c.cout / wgrad_ntile(c.cout));
+    const int tiles = (taps * C + tc::kTileM - 1) / tc::kTileM * (cout / wgrad_ntile(cout));
     const int n0 = std::max(1, std::min((chunks + 7) / 8, (304 + tiles - 1) / tiles));
     *per = (chunks + n0 - 1) / n0;
     *ns = (chunks + *per - 1) / *per;
@@ -475,11 +485,14 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
         } else {
             dx = std::max(dx, n(c.level, c.cin));
         }
-        int per, ns;
-        for (int B = 1; B <= maxB; B++) {  // (a smaller batch may have more splits)
-            wgrad_splits(c, U.geo(c.level, B).positions(), &per, &ns);
-            part = std::max(part, (size_t)ns * 9 * c.cin * c.cout);
-        }
+        const int C0 = c.src0 < 0 ? kImCols : U.tch[c.src0], C1 = c.mode == 2 ? U.tch[c.src1] : 0;
+        for (int B = 1; B <= maxB; B++)  // (a smaller batch may have more splits)
+            for (int C : {C0, C1}) {
+                int per, ns;
+                if (C == 0) continue;
+                wgrad_splits(c.src0 < 0 ? 1 : 9, C, c.cout, U.geo(c.level, B).positions(), &per, &ns);
+                part = std::max(part, (size_t)ns * 9 * c.cin * c.cout);
+            }
     }
     bpart = (size_t)4 * 152 * 256;
     U.part_cap = part;
@@ -488,10 +501,10 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
         (rc = ualloc(U, &U.dy, P0)) || (rc = ualloc(U, &U.tgt, P0)) || (rc = ualloc(U, &U.lpart, P0 / 256 + 1)) ||
         (rc = ualloc(U, &U.dx, dx)) || (rc = ualloc(U, &U.part, part)) || (rc = ualloc(U, &U.bpart, bpart)))
         return rc;
-    const int smax = (int)tc::conv_smem_bytes(256);
+    const int smax = 221 * 1024;  // conv_stages' bound and the alignment
     CK(cudaFuncSetAttribute(tc::k_conv_gemm<FwdEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     CK(cudaFuncSetAttribute(tc::k_conv_gemm<DxEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-    CK(cudaFuncSetAttribute(tc::k_wgrad_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::wgrad_smem_bytes(128)));
+    CK(cudaFuncSetAttribute(tc::k_wgrad_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     return 0;
 }
 
@@ -559,6 +572,10 @@ static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* 
         if (N % f == 0 && (N / f) % 32 == 0) nt = f;
     a.Ntile = N / nt;
     P.grid = dim3(mt, nt);
+    const int bw = nsrc > 1 ? std::max(a.bw[0], a.bw[1]) : a.bw[0];
+    a.abytes = tc::kTileM * bw * 2;
+    a.bbytes = a.Ntile * bw * 2;
+    a.stages = tc::conv_stages((size_t)(a.abytes + a.bbytes), (size_t)mt * nt, a.Ktot / bw);
     int rc;
     for (int s = 0; s < 2; s++) {
         const int q = s < nsrc ? s : 0;
@@ -585,11 +602,12 @@ static int plan_batch(UNet& U, int B) {
         const uint16_t* z[2] = {U.dz[c.out], nullptr};
         const int Cz[2] = {c.cout, 0};
         if (!first && (rc = plan_conv(P.bwd, g, 9, 1, z, Cz, U.wbd + c.woff, c.cin))) return rc;
-        int per;
-        wgrad_splits(c, g.positions(), &per, &P.nsplit);
-        if ((size_t)P.nsplit * 9 * c.cin * c.cout > U.part_cap) return fail(PT_ERR_STATE, "U-Net: split workspace too small");
         P.nwg = ns;
         for (int s = 0; s < ns; s++) {
+            int per;
+            wgrad_splits(first ? 1 : 9, C[s], c.cout, g.positions(), &per, &P.nsplit[s]);
+            if ((size_t)P.nsplit[s] * 9 * c.cin * c.cout > U.part_cap)
+                return fail(PT_ERR_STATE, "U-Net: split workspace too small");
             WgradPlan& w = P.wg[s];
             tc::WgradArgs& a = w.a;
             a.g = g;
@@ -606,7 +624,10 @@ static int plan_batch(UNet& U, int B) {
             a.chunks = (int)((g.positions() + tc::kWgradK - 1) / tc::kWgradK);
             a.part = U.part;
             const int blocks = a.taps * (a.C / a.bwA), ablk = tc::kTileM / a.bwA;
-            w.grid = dim3((blocks + ablk - 1) / ablk, c.cout / a.Ntile, P.nsplit);
+            w.grid = dim3((blocks + ablk - 1) / ablk, c.cout / a.Ntile, P.nsplit[s]);
+            a.abytes = tc::kTileM * tc::kWgradK * 2;
+            a.bbytes = a.Ntile * tc::kWgradK * 2;
+            a.stages = tc::conv_stages((size_t)(a.abytes + a.bbytes), (size_t)w.grid.x * w.grid.y * w.grid.z, per);
             if ((rc = tensor_map(&w.A, t[s], C[s], g.positions(), a.bwA, tc::kWgradK)) ||
                 (rc = tensor_map(&w.B, U.dz[c.out], c.cout, g.positions(), a.bwB, tc::kWgradK)))
                 return rc;
@@ -616,9 +637,12 @@ static int plan_batch(UNet& U, int B) {
     return 0;
 }
 
+template <class Args>
+static size_t conv_smem(const Args& a) { return (size_t)a.stages * (size_t)(a.abytes + a.bbytes) + 1024; }
+
 template <class E>
 static int run_conv(UNet& U, const ConvPlan& P, const E& e) {
-    tc::k_conv_gemm<E><<<P.grid, tc::kConvThreads, tc::conv_smem_bytes(P.a.Ntile), U.st>>>(P.A[0], P.A[1], P.B[0], P.B[1],
+    tc::k_conv_gemm<E><<<P.grid, tc::kConvThreads, conv_smem(P.a), U.st>>>(P.A[0], P.A[1], P.B[0], P.B[1],
                                                                                        P.a, e, U.derr);
     return cuda_check(cudaGetLastError(), "k_conv_gemm");
 }
@@ -694,9 +718,10 @@ static int unet_backward(UNet& U, int B, float* loss) {
         // weights: split over positions, then a fixed-order reduction of the splits
         const int Mw = 9 * c.cin;
         for (int s = 0; s < P.nwg; s++)
-            tc::k_wgrad_gemm<<<P.wg[s].grid, tc::kConvThreads, tc::wgrad_smem_bytes(P.wg[s].a.Ntile), U.st>>>(
+            tc::k_wgrad_gemm<<<P.wg[s].grid, tc::kConvThreads, conv_smem(P.wg[s].a), U.st>>>(
                 P.wg[s].A, P.wg[s].B, P.wg[s].a, U.derr);
-        k_wgrad_reduce<<<nblk((size_t)Mw * c.cout, 256), 256, 0, U.st>>>(U.g + c.woff, U.part, P.nsplit, Mw, c.cout);
+        k_wgrad_reduce<<<nblk((size_t)Mw * c.cout, 256), 256, 0, U.st>>>(
+            U.g + c.woff, U.part, P.nsplit[0], P.nsplit[1], P.nwg > 1 ? P.wg[0].a.C : Mw, P.nwg > 1 ? c.cin : Mw, Mw, c.cout);
         CK(cudaGetLastError());
         if (c.src0 < 0) continue;  // the network input needs no gradient
         float* dx = c.mode == 2 ? U.dxcat[c.out] : U.dx;
