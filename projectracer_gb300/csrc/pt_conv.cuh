@@ -6,13 +6,19 @@
 // a tap and a block of channels is a plain [128 positions x 64 channels] box of a 2D tensor, and no
 // thread computes an im2col address; the padding positions cost (W+2)(H+1)/(W H) more rows, and are not
 // stored.  Threads that gathered the tiles through registers kept the tensor pipe at 2.5% of its rate.
-//   * k_conv_gemm (forward, backward-data): a CTA computes 128 positions x Ntile columns.  One thread
-//     issues the TMA loads of a chunk (one tap, 64 or 32 channels: A box and weight box, K-major,
-//     128- or 64-byte swizzle), one the MMAs (K = 16 each, taps and channels in ascending order, so an
-//     output's sum does not depend on the tiling), through a ring of stages with full/empty mbarriers;
-//     four warps read the accumulator from tensor memory and store.
-//   * k_wgrad_gemm: M = 128 rows of (tap, input channel), N = output channels, K = positions.  Both
-//     operands are the same boxes read with their channels as the leading dimension (MN-major).
+//   * k_conv_gemm (forward, backward-data): tiles of 128 positions x Ntile columns.  A box of 130 positions
+//     serves the three taps of a row: the swizzle goes by the shared-memory address, so an operand may
+//     start at any row of a box.  Two warps issue the TMA loads (activation boxes, weight boxes; K-major,
+//     128- or 64-byte swizzle), one the MMAs (K = 16 each, taps, then channels, in ascending order, so an
+//     output's sum does not depend on the tiling); four read the accumulator from tensor memory and store.
+//   * k_wgrad_gemm: M = (tap, input channel), N = output channels, K = positions.  The same boxes read
+//     with their channels as the leading dimension (MN-major): the taps of a row are one box at row
+//     offsets 0, 1 and 2, as blocks of M one position apart.
+// What bounds them: on large grids the issue of one MMA per 16 channels (N = 32 takes the 64 cycles that
+// reading the 128 rows takes) beside loads and stores; on small ones a chain of set-up, load latency,
+// MMAs and store, 7 us with the launch.  The forward convolutions of 8 images of 512 x 256: 1338 us with
+// a CTA per tile, a box per tap and single threads issuing, now 681; backward-data 1124 and 505, weight
+// gradients 1279 and 640.
 // Every wait is bounded; a timeout sets an error flag and the CTA leaves after its copies have landed.
 #pragma once
 #include <cuda.h>
@@ -22,7 +28,8 @@
 namespace pt {
 namespace tc {
 
-constexpr int kMaxStages = 10, kConvThreads = 192;  // warps 0-3: epilogue, 4: TMA, 5: MMA
+constexpr int kMaxRing = 12, kConvThreads = 224;  // warps 0-3: epilogue, 4 and 6: TMA, 5: MMA
+constexpr int kSms = 152, kWgradThreads = 192;  // warps 0-3: epilogue, 4: TMA, 5: MMA
 
 // shared-memory descriptor with a swizzle: layout 2 = 128-byte, 4 = 64-byte; strides in bytes
 __device__ __forceinline__ uint64_t smem_desc_sw(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
@@ -30,6 +37,9 @@ __device__ __forceinline__ uint64_t smem_desc_sw(uint32_t saddr, uint32_t lbo, u
 }
 __device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
@@ -62,12 +72,24 @@ struct PadGeo {
     __host__ __device__ int Hp() const { return H + 1; }
     __host__ __device__ size_t positions() const { return ((size_t)B * Hp() + 1) * Wp(); }
     __host__ __device__ size_t at(int b, int y, int x) const { return ((size_t)b * Hp() + y + 1) * Wp() + x + 1; }
-    // pixel of position p; false for padding
-    __device__ __forceinline__ bool pixel(int p, int& b, int& y, int& x) const {
-        const int row = p / Wp();
-        x = p - row * Wp() - 1;
-        b = row / Hp();
-        y = row - b * Hp() - 1;
+    // pixel of position p; false for padding (divisions as multiplications: exact for p < 2^31)
+    struct Div {
+        int d;
+        uint32_t m;
+        int sh;
+        explicit Div(int n) : d(n), m(0), sh(0) {
+            while ((1ll << sh) < n) sh++;
+            m = (uint32_t)(((1ull << (31 + sh)) + (unsigned)n - 1) / (unsigned)n);
+            sh--;
+        }
+        Div() = default;
+        __device__ __forceinline__ int operator()(int p) const { return (int)(__umulhi((uint32_t)p, m) >> sh); }
+    };
+    __device__ __forceinline__ bool pixel(int p, Div wp, Div hp, int& b, int& y, int& x) const {
+        const int row = wp(p);
+        x = p - row * wp.d - 1;
+        b = hp(row);
+        y = row - b * hp.d - 1;
         return b < B && y >= 0 && x >= 0 && x < W;
     }
 };
@@ -78,26 +100,97 @@ struct PadGeo {
 struct ConvArgs {
     PadGeo g;
     int taps, nsrc, C[2], bw[2], Ktot, N, Ntile, first, last;  // positions first .. last - 1
-    int stages, abytes, bbytes;                               // pipeline depth; operand bytes of a stage
+    PadGeo::Div wp, hp;  // by the padded width and height
+    int tiles, nt, nbuf;  // tiles, of which nt share their positions; accumulators in tensor memory
+    // pipeline: S stages of G blocks and nd taps of a row (3: one box of kBoxRows positions serves them, or 1),
+    // slots of abytes and bbytes; ctas: on an SM; keep: the weights stay for all tiles of a CTA
+    int S, G, nd, abytes, bbytes, ctas, keep;
 };
+constexpr int kBoxRows = kTileM + 2;
 
-// one role's failure ends the CTA: waits that follow return at once
+// one role's failure ends the CTA: the others leave their waits at their next look
 __device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, volatile int* bad) {
-    if (*bad) return false;
-    if (mbar_wait(bar, parity)) return true;
+    const uint32_t a = smem_u32(bar);
+    for (int it = 0; it < kWaitPolls; it++) {
+        if (mbar_try(a, parity)) return true;
+        if ((it & 15) == 15 && *bad) return false;
+    }
     *bad = 1;
     return false;
 }
 
-// Pipeline depth for stages of sbytes in a grid of `ctas`: with a CTA per SM at most, as deep as the
-// shared memory allows, since a chunk's load latency (1-2 us) is all there is; with more, four stages, so
-// that several CTAs share an SM and one's prologue and epilogue run beside the others' loads.
-static inline int conv_stages(size_t sbytes, size_t ctas, int chunks) {
-    const int most = (int)((220 * 1024) / sbytes);
-    int s = ctas <= 152 ? most : 4;
-    s = s < most ? s : most;
-    s = s < chunks ? s : chunks;
-    return s < kMaxStages ? (s > 1 ? s : 1) : kMaxStages;
+// The pipeline of a convolution of nblk blocks.  A grid of more tiles than SMs runs persistent CTAs with two
+// accumulators, so that one tile's stores overlap the next one's loads; as many on an SM as have three
+// stages, of a whole row of taps where it fits.  There the weights stay in shared memory where they leave
+// that room: all SMs reading the same 18 KB for every tile is a hot spot of L2 (32 -> 32 channels on a
+// million pixels: 48 us with them kept, 74 us without; four CTAs on an SM 48 us, three 52, two 64, one 105).
+// A smaller grid has an SM for each CTA, and the latency of its loads is all there is: the deepest ring.
+static inline void conv_stages(ConvArgs& a, int nblk) {
+    const int bw = a.nsrc > 1 && a.bw[1] > a.bw[0] ? a.bw[1] : a.bw[0];
+    const bool large = a.tiles > kSms;
+    a.bbytes = a.Ntile * bw * 2;
+    a.nbuf = a.Ntile <= 128 && large ? 2 : 1;
+    auto stages = [&](int k, int keep) {  // of k CTAs on an SM, which has 228 KB (1 KB reserved, 2.1 KB static each)
+        const int room = (k == 1 ? 220 : 228 / k - 4) * 1024 - (keep ? a.taps * nblk * a.bbytes : 0);
+        auto bytes = [&](int nd, int G) {
+            a.nd = nd;
+            a.G = G;
+            a.abytes = ((nd == 3 ? kBoxRows : kTileM) * bw * 2 + 1023) / 1024 * 1024;
+            return G * (a.abytes + (keep ? 0 : nd * a.bbytes));
+        };
+        int n;
+        if (a.taps != 9 || 2 * (n = bytes(3, nblk)) > room) {
+            int G = nblk;  // a divisor of nblk: three stages of it
+            while (nblk % G || (3 * bytes(1, G) > room && G > 1)) G--;
+            n = bytes(1, G);
+        }
+        a.keep = keep;
+        a.ctas = k;
+        a.S = room / n < kMaxRing ? room / n : kMaxRing;
+        return a.S;
+    };
+    if (!large) {
+        stages(1, 0);
+        const int steps = a.taps / a.nd * (nblk / a.G);
+        if (a.S > steps) a.S = steps;
+        return;
+    }
+    const int cols = (int)tmem_cols(a.nbuf * a.Ntile);
+    for (int keep = 1; keep >= 0; keep--)
+        for (int k = 4; k >= 1; k--)
+            if (k * cols <= 512 && (!keep || kSms * k % a.nt == 0) && stages(k, keep) >= (keep || k > 2 ? 3 : k)) return;
+}
+static inline size_t conv_smem(const ConvArgs& a) {
+    const int nblk = a.C[0] / a.bw[0] + (a.nsrc > 1 ? a.C[1] / a.bw[1] : 0), w = a.keep ? a.taps * nblk : a.S * a.nd * a.G;
+    return (size_t)a.S * a.G * a.abytes + (size_t)w * a.bbytes + 1024;
+}
+
+// barriers of a ring
+struct Ring {
+    uint64_t full[kMaxRing], empty[kMaxRing];
+    __device__ __forceinline__ void init(int n, int fills, int frees) {
+        for (int s = 0; s < n; s++) {
+            mbar_init(full + s, (uint32_t)fills);
+            mbar_init(empty + s, (uint32_t)frees);
+        }
+    }
+};
+// a position in a ring and the parity of its use
+struct RingPos {
+    int i = 0;
+    uint32_t parity;
+    __device__ __forceinline__ explicit RingPos(uint32_t p) : parity(p) {}
+    __device__ __forceinline__ void next(int n) {
+        if (++i == n) {
+            i = 0;
+            parity ^= 1u;
+        }
+    }
+};
+
+// after a failure: the loader at r waits for its copies in flight (bounded)
+__device__ __forceinline__ void drain(Ring& ring, const RingPos& r, int n) {
+    for (int s = 0; s < n; s++) mbar_wait(ring.full + s, s < r.i ? r.parity ^ 1u : r.parity);
 }
 
 // Epilogue E: void operator()(int p, int col0, const float (&v)[32]) for columns col0 .. col0 + 31 of
@@ -109,221 +202,317 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
                                                             const __grid_constant__ CUtensorMap mapB1, ConvArgs a, E epi,
                                                             int* err) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
+    __shared__ Ring ring, accs;  // stages; accumulators
+    __shared__ uint64_t done, wfull;
     __shared__ uint32_t tslot;
     __shared__ int bad;
+    __shared__ __align__(16) float sbias[256];
     unsigned char* const smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int p0 = a.first + blockIdx.x * kTileM, n0 = blockIdx.y * a.Ntile;
-    const uint32_t ncols = tmem_cols(a.Ntile);
-    const int S = a.stages;
-    const size_t sbytes = (size_t)(a.abytes + a.bbytes);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int S = a.S, G = a.G, nd = a.nd;
+    const uint32_t ncols = tmem_cols(a.nbuf * a.Ntile);
     if (tid == 0) {
         bad = 0;
-        for (int s = 0; s < S; s++) {
-            mbar_init(full + s, 1);
-            mbar_init(empty + s, 1);
-        }
+        ring.init(S, a.keep ? 1 : 2, 1);
+        accs.init(a.nbuf, 1, 4);
         mbar_init(&done, 1);
+        mbar_init(&wfull, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) tmem_alloc(&tslot, ncols);
+    epi.stage(sbias, a.N, tid);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t taddr = tslot;
-    const int nb0 = a.C[0] / a.bw[0], nb1 = a.nsrc > 1 ? a.C[1] / a.bw[1] : 0, nblk = nb0 + nb1, chunks = a.taps * nblk;
-    // One thread each drives the loads and the MMAs, so a chunk's instructions are a serial chain: counters
-    // instead of divisions (with them a chunk took 0.6 us).
-    if (warp == 4 && lane == 0) {
-        int k = 0, st = 0, dx = -1, shift = a.taps == 1 ? 0 : -a.g.Wp() - 1;
-        uint32_t parity = 1;  // of the stage's previous use; the first wait for a stage passes
+    const int bw0 = a.bw[0], bw1 = a.bw[1], nb0 = a.C[0] / bw0, nblk = nb0 + (a.nsrc > 1 ? a.C[1] / bw1 : 0);
+    const int rows = a.taps == 1 ? 1 : 3, steps = a.taps / nd, brows = nd == 3 ? kBoxRows : kTileM;
+    const uint32_t boff = (uint32_t)(G * a.abytes), sbytes = boff + (uint32_t)(a.keep ? 0 : G * nd * a.bbytes);
+    unsigned char* const wsm = smem + (size_t)S * sbytes;  // weights that stay
+    // The loads and the MMAs are serial chains of single instructions: whole warps run the loops, so that the
+    // operands stay in uniform registers, and one lane issues (by one thread alone a
+    // chunk of 64 channels took 650 cycles to load and 550 to multiply, now 150 each).
+    if (warp == 4) {  // activation boxes
+        RingPos r(1);  // the first wait for a stage passes
         bool go = true;
-        for (int tap = 0; tap < a.taps && go; tap++) {
-            for (int blk = 0; blk < nblk; blk++) {
-                if (!conv_wait(empty + st, parity, &bad)) {
-                    go = false;
-                    break;
+        for (int tile = blockIdx.x; tile < a.tiles && go; tile += gridDim.x) {
+            const int p0 = a.first + tile / a.nt * kTileM;
+            int pos = a.taps == 1 ? p0 : p0 - a.g.Wp() - 1, dx = 0;
+            for (int t = 0; t < steps && go; t++) {
+                for (int b0 = 0; b0 < nblk; b0 += G) {
+                    if (!(go = conv_wait(ring.empty + r.i, r.parity, &bad))) break;
+                    if (elect_one()) {
+                        unsigned char* sa = smem + r.i * sbytes;
+                        uint64_t* const bar = ring.full + r.i;
+                        const int k0 = min(max(nb0 - b0, 0), G);
+                        mbar_expect(bar, (uint32_t)(brows * 2 * (k0 * bw0 + (G - k0) * bw1)));
+                        for (int blk = b0; blk < b0 + G; blk++, sa += a.abytes)
+                            if (blk < nb0)
+                                tma_load_2d(sa, &mapA0, blk * bw0, pos, bar);
+                            else
+                                tma_load_2d(sa, &mapA1, (blk - nb0) * bw1, pos, bar);
+                    }
+                    __syncwarp();
+                    r.next(S);
                 }
-                const int src = blk >= nb0, bw = a.bw[src], ch = (src ? blk - nb0 : blk) * bw;
-                unsigned char* sa = smem + st * sbytes;
-                mbar_expect(full + st, (uint32_t)((kTileM + a.Ntile) * bw * 2));
-                tma_load_2d(sa, src ? &mapA1 : &mapA0, ch, p0 + shift, full + st);
-                tma_load_2d(sa + a.abytes, bw == a.bw[0] ? &mapB0 : &mapB1, k, n0, full + st);
-                k += bw;
-                if (++st == S) {
-                    st = 0;
-                    parity ^= 1u;
+                if (nd == 3 || dx == rows - 1) {
+                    pos += a.g.Wp() - dx;
+                    dx = 0;
+                } else {
+                    pos++;
+                    dx++;
                 }
             }
-            shift += dx < 1 ? 1 : a.g.Wp() - 2;
-            dx = dx < 1 ? dx + 1 : -1;
         }
-    } else if (warp == 5 && lane == 0) {
+        if (!go) drain(ring, r, S);
+    } else if (warp == 6 && a.keep) {
+        if (elect_one()) {
+            unsigned char* sb = wsm;
+            int x = 0;
+            mbar_expect(&wfull, (uint32_t)(a.Ntile * 2 * a.Ktot));
+            for (int q = 0; q < a.taps; q++)
+                for (int g = 0; g < nblk; g++, sb += a.bbytes)
+                    if (g < nb0 || bw1 == bw0) {
+                        tma_load_2d(sb, &mapB0, x, (int)blockIdx.x % a.nt * a.Ntile, &wfull);
+                        x += bw0;
+                    } else {
+                        tma_load_2d(sb, &mapB1, x, (int)blockIdx.x % a.nt * a.Ntile, &wfull);
+                        x += bw1;
+                    }
+        }
+        __syncwarp();
+        mbar_wait(&wfull, 0);  // the CTA does not leave before its copies have landed
+    } else if (warp == 6) {  // weight boxes
+        RingPos r(1);
+        bool go = true;
+        for (int tile = blockIdx.x; tile < a.tiles && go; tile += gridDim.x) {
+            const int n0 = tile % a.nt * a.Ntile;
+            int k = 0;
+            for (int t = 0; t < steps && go; t++)
+                for (int b0 = 0; b0 < nblk; b0 += G) {
+                    if (!(go = conv_wait(ring.empty + r.i, r.parity, &bad))) break;
+                    const int k0 = min(max(nb0 - b0, 0), G), kw = k0 * bw0 + (G - k0) * bw1;
+                    if (elect_one()) {
+                        unsigned char* sb = smem + r.i * sbytes + boff;
+                        uint64_t* const bar = ring.full + r.i;
+                        mbar_expect(bar, (uint32_t)(nd * a.Ntile * 2 * kw));
+                        int x = k;
+                        for (int q = 0; q < nd; q++)
+                            for (int g = 0; g < G; g++, sb += a.bbytes)
+                                if (g < k0 || bw1 == bw0) {
+                                    tma_load_2d(sb, &mapB0, x, n0, bar);
+                                    x += bw0;
+                                } else {
+                                    tma_load_2d(sb, &mapB1, x, n0, bar);
+                                    x += bw1;
+                                }
+                    }
+                    __syncwarp();
+                    k += nd * kw;
+                    r.next(S);
+                }
+        }
+        if (!go) drain(ring, r, S);
+    } else if (warp == 5) {
         const uint32_t idesc = idesc_bf16(a.Ntile);
         const uint64_t d64 = smem_desc_sw(0, 16, 1024, 2u), d32 = smem_desc_sw(0, 16, 512, 4u);
-        int st = 0, blk = 0;
-        uint32_t parity = 0, acc = 0;
-        for (int c = 0; c < chunks; c++) {
-            if (!conv_wait(full + st, parity, &bad)) break;
+        RingPos r(0), c(1);
+        bool go = !a.keep || conv_wait(&wfull, 0, &bad);
+        for (int tile = blockIdx.x; tile < a.tiles && go; tile += gridDim.x) {
+            const uint32_t t0 = taddr + (uint32_t)(c.i * a.Ntile);
+            uint32_t acc = 0, sw = smem_u32(wsm);
+            if (!(go = conv_wait(accs.empty + c.i, c.parity, &bad))) break;
             tc_fence_after();
-            const bool wide = a.bw[blk >= nb0] == 64;
-            const uint32_t sa = smem_u32(smem) + (uint32_t)(st * sbytes);
-            const uint64_t da = (wide ? d64 : d32) + (sa >> 4), db = da + (uint32_t)(a.abytes >> 4);
-#pragma unroll
-            for (int s = 0; s < 4; s++) {
-                if (s >= 2 && !wide) break;
-                mma_bf16(taddr, da + 2 * s, db + 2 * s, idesc, acc);  // 16 channels further: 32 bytes
-                acc = 1u;
-            }
-            mma_commit(empty + st);
-            if (++blk == nblk) blk = 0;
-            if (++st == S) {
-                st = 0;
-                parity ^= 1u;
-            }
+            for (int t = 0; t < steps && go; t++)
+                for (int b0 = 0; b0 < nblk; b0 += G) {
+                    if (!(go = conv_wait(ring.full + r.i, r.parity, &bad))) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t sa = smem_u32(smem) + r.i * sbytes;
+                        uint32_t sb = a.keep ? sw : sa + boff;
+                        for (int q = 0; q < nd; q++)
+                            for (int g = 0; g < G; g++, sb += (uint32_t)a.bbytes) {
+                                const bool wide = (b0 + g < nb0 ? bw0 : bw1) == 64;
+                                const uint64_t d0 = wide ? d64 : d32;
+                                const uint64_t da =
+                                    d0 + ((sa + (uint32_t)(g * a.abytes + q * (wide ? 128 : 64))) >> 4);
+                                const uint64_t db = d0 + (sb >> 4);
+                                mma_bf16(t0, da, db, idesc, acc | (uint32_t)(q + g));
+                                mma_bf16(t0, da + 2, db + 2, idesc, 1u);  // 16 channels further: 32 bytes
+                                if (wide) {
+                                    mma_bf16(t0, da + 4, db + 4, idesc, 1u);
+                                    mma_bf16(t0, da + 6, db + 6, idesc, 1u);
+                                }
+                            }
+                        mma_commit(ring.empty + r.i);
+                    }
+                    __syncwarp();
+                    acc = 1u;
+                    sw += (uint32_t)(nd * G * a.bbytes);
+                    r.next(S);
+                }
+            if (elect_one()) mma_commit(accs.full + c.i);
+            __syncwarp();
+            c.next(a.nbuf);
         }
-        mma_commit(&done);
-    }
-    __syncwarp();
-    if (warp < 4) {
-        const bool ok = conv_wait(&done, 0, &bad);
-        tc_fence_after();
-        const int p = p0 + warp * 32 + lane;
-        int b = 0, y = 0, x = 0;
-        const bool real = p < a.last && a.g.pixel(p, b, y, x);
-        for (int c0 = 0; c0 < a.Ntile; c0 += 32) {
-            float v[32];
-            tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (ok && real) epi(p, b, y, x, n0 + c0, v);
+        if (!go) {  // MMAs in flight read the stages
+            if (elect_one()) mma_commit(&done);
+            __syncwarp();
+            mbar_wait(&done, 0);
+        }
+    } else {
+        RingPos c(0);
+        for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
+            const int n0 = tile % a.nt * a.Ntile, p = a.first + tile / a.nt * kTileM + warp * 32 + lane;
+            int b = 0, y = 0, x = 0;
+            const bool real = p < a.last && a.g.pixel(p, a.wp, a.hp, b, y, x);
+            int ok = 0;
+            if (lane == 0) ok = conv_wait(accs.full + c.i, c.parity, &bad);  // one lane: polls take issue slots
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            tc_fence_after();
+            const uint32_t t0 = taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c.i * a.Ntile);
+            for (int c0 = 0; c0 < a.Ntile; c0 += 32) {
+                float v[32];
+                __syncwarp();
+                tmem_ld32(t0 + (uint32_t)c0, v);
+                if (c0 + 32 == a.Ntile) {  // the accumulator is free
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accs.empty + c.i);
+                }
+                if (real) epi(p, b, y, x, n0 + c0, v, sbias + n0 + c0);
+            }
+            c.next(a.nbuf);
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (bad && tid == 0) {
-        atomicOr(err, 1);
-        for (int s = 0; s < S; s++) mbar_wait(full + s, 0);  // copies still in flight (bounded)
-    }
+    if (bad && tid == 0) atomicOr(err, 1);
     if (warp == 5) tmem_dealloc(taddr, ncols);
 }
 
 // Weight gradient of one source tensor: part[z][kk][co] = sum over the split's positions of
-// in[p + shift(tap)][ci] dZ[p][co], kk = tap cin + c_off + ci.  A's 128 rows are `ablk` blocks of bwA
-// channels (2 x 64 or 4 x 32); block q of tile t is number t ablk + q of the taps x (C / bwA) blocks.
+// in[p + shift(tap)][ci] dZ[p][co], kk = tap cin + c_off + ci.  A CTA takes a block of bw channels and the
+// taps of one image row: per chunk of 128 positions a box of 132 positions, and dZ's boxes.  An accumulator
+// holds 128 / bw blocks of M, one position apart: 4 x 32 (taps -1, 0, 1, and one that is not stored) or
+// 2 x 64 (taps -1, 0, and in a second one tap 1).
 struct WgradArgs {
     PadGeo g;
-    int taps, C, bwA, c_off, cin, N, Ntile, bwB, per, chunks;  // per: chunks of 64 positions a split, of `chunks`
+    int taps, C, bw, c_off, cin, N, Ntile, bwB, per, chunks;  // per: chunks a split, of `chunks`
     int kk_max;  // rows kk >= kk_max are not stored (im2col padding)
-    int stages, abytes, bbytes;
+    int ncols;   // tensor-memory columns
+    int S, abytes, bbytes;  // stages of abytes (the box of positions) and bbytes
     float* part;
 };
-constexpr int kWgradK = 64;
+static inline size_t wgrad_smem(const WgradArgs& a) { return (size_t)a.S * (a.abytes + a.bbytes) + 1024; }
+constexpr int kWgradK = 128, kWgradBox = kWgradK + 4;
+// bytes of a box of positions, to a 1024-byte boundary
+__host__ __device__ constexpr int wgrad_box_bytes(int bw) { return (kWgradBox * bw * 2 + 1023) / 1024 * 1024; }
 // instruction descriptor with both operands MN-major
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) { return idesc_bf16(n) | (1u << 15) | (1u << 16); }
 
-__global__ void __launch_bounds__(kConvThreads) k_wgrad_gemm(const __grid_constant__ CUtensorMap mapA,
+__global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_constant__ CUtensorMap mapA,
                                                              const __grid_constant__ CUtensorMap mapB, WgradArgs a,
                                                              int* err) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
+    __shared__ Ring ring;
+    __shared__ uint64_t done;
     __shared__ uint32_t tslot;
     __shared__ int bad;
     unsigned char* const smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n0 = blockIdx.y * a.Ntile;
-    const uint32_t ncols = tmem_cols(a.Ntile);
-    const int S = a.stages;
-    const size_t sbytes = (size_t)(a.abytes + a.bbytes);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int n0 = blockIdx.y * a.Ntile, S = a.S;
+    const uint32_t sbytes = (uint32_t)(a.abytes + a.bbytes);
     if (tid == 0) {
         bad = 0;
-        for (int s = 0; s < S; s++) {
-            mbar_init(full + s, 1);
-            mbar_init(empty + s, 1);
-        }
+        ring.init(S, 1, 1);
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 5) tmem_alloc(&tslot, ncols);
+    if (warp == 5) tmem_alloc(&tslot, (uint32_t)a.ncols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t taddr = tslot;
     const int cbeg = blockIdx.z * a.per, cend = min(a.chunks, cbeg + a.per), n = max(0, cend - cbeg);
-    const int ablk = kTileM / a.bwA, nch = a.C / a.bwA, blocks = a.taps * nch, bblk = a.Ntile / a.bwB;
-    const uint32_t abox = (uint32_t)(kWgradK * a.bwA * 2), bbox = (uint32_t)(kWgradK * a.bwB * 2);
-    if (warp == 4 && lane == 0) {
-        int ch[4], shift[4];  // of the A blocks; past the last one: loaded, not stored
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int blk = min((int)blockIdx.x * ablk + q, blocks - 1), tap = blk / nch;
-            ch[q] = (blk - tap * nch) * a.bwA;
-            shift[q] = a.taps == 1 ? 0 : (tap / 3 - 1) * a.g.Wp() + (tap % 3 - 1);
-        }
-        int st = 0, p = cbeg * kWgradK;
-        uint32_t parity = 1;  // of the stage's previous use; the first wait for a stage passes
+    const int nch = a.C / a.bw, unit = blockIdx.x / nch, ch = (blockIdx.x - unit * nch) * a.bw;
+    const int bblk = a.Ntile / a.bwB, nacc = a.taps == 1 || a.bw == 32 ? 1 : 2;  // accumulators
+    const int shift = a.taps == 1 ? 0 : (unit - 1) * a.g.Wp() - 1;                // of tap -1 of the row
+    const uint32_t bbox = (uint32_t)(kWgradK * a.bwB * 2);
+    if (warp == 4) {
+        RingPos r(1);  // the first wait for a stage passes
+        int p = cbeg * kWgradK;
         for (int c = 0; c < n; c++, p += kWgradK) {
-            if (!conv_wait(empty + st, parity, &bad)) break;
-            unsigned char* sa = smem + st * sbytes;
-            mbar_expect(full + st, (uint32_t)ablk * abox + (uint32_t)bblk * bbox);
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (q < ablk) tma_load_2d(sa + q * abox, &mapA, ch[q], p + shift[q], full + st);
-            for (int q = 0; q < bblk; q++) tma_load_2d(sa + a.abytes + q * bbox, &mapB, n0 + q * a.bwB, p, full + st);
-            if (++st == S) {
-                st = 0;
-                parity ^= 1u;
+            if (!conv_wait(ring.empty + r.i, r.parity, &bad)) {
+                drain(ring, r, S);
+                break;
             }
+            unsigned char* sa = smem + r.i * sbytes;
+            if (elect_one()) {
+                mbar_expect(ring.full + r.i, (uint32_t)(kWgradBox * a.bw * 2) + (uint32_t)bblk * bbox);
+                tma_load_2d(sa, &mapA, ch, p + shift, ring.full + r.i);
+                for (int q = 0; q < bblk; q++)
+                    tma_load_2d(sa + a.abytes + q * bbox, &mapB, n0 + q * a.bwB, p, ring.full + r.i);
+            }
+            __syncwarp();
+            r.next(S);
         }
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 5) {
         const uint32_t idesc = idesc_bf16_mn(a.Ntile);
-        const uint32_t ra = (uint32_t)a.bwA * 2, rb = (uint32_t)a.bwB * 2;  // bytes of a position's block row
-        const uint64_t da0 = smem_desc_sw(0, abox, 8 * ra, a.bwA == 64 ? 2u : 4u);
-        const uint64_t db0 = smem_desc_sw(0, bbox, 8 * rb, a.bwB == 64 ? 2u : 4u);
-        int st = 0;
-        uint32_t parity = 0, acc = 0;
+        const uint32_t pa = (uint32_t)a.bw * 2, pb = (uint32_t)a.bwB * 2;  // bytes of a position
+        const uint64_t da0 = smem_desc_sw(0, pa, 8 * pa, a.bw == 64 ? 2u : 4u);  // blocks of M: one position apart
+        const uint64_t db0 = smem_desc_sw(0, bbox, 8 * pb, a.bwB == 64 ? 2u : 4u);
+        RingPos r(0);
+        uint32_t acc = 0;
         for (int c = 0; c < n; c++) {
-            if (!conv_wait(full + st, parity, &bad)) break;
+            if (!conv_wait(ring.full + r.i, r.parity, &bad)) break;
             tc_fence_after();
-            const uint32_t sa = smem_u32(smem) + (uint32_t)(st * sbytes);
-            const uint64_t da = da0 + (sa >> 4), db = db0 + ((sa + (uint32_t)a.abytes) >> 4);
+            const uint32_t sa = smem_u32(smem) + r.i * sbytes;
+            const uint64_t db = db0 + ((sa + (uint32_t)a.abytes) >> 4);
+            if (elect_one()) {
+                for (int h = 0; h < nacc; h++) {
+                    const uint64_t da = da0 + ((sa + 2 * h * pa) >> 4);
 #pragma unroll
-            for (int s = 0; s < kWgradK / 16; s++) {
-                mma_bf16(taddr, da + s * ra, db + s * rb, idesc, acc);  // 16 positions further
-                acc = 1u;
+                    for (int s = 0; s < kWgradK / 16; s++)  // 16 positions further
+                        mma_bf16(taddr + (uint32_t)(h * a.Ntile), da + s * pa, db + s * pb, idesc, acc | (s > 0));
+                }
+                mma_commit(ring.empty + r.i);
             }
-            mma_commit(empty + st);
-            if (++st == S) {
-                st = 0;
-                parity ^= 1u;
-            }
+            __syncwarp();
+            acc = 1u;
+            r.next(S);
         }
-        mma_commit(&done);
+        if (elect_one()) mma_commit(&done);
+        __syncwarp();
+        conv_wait(&done, 0, &bad);
+        tc_fence_before();
     }
-    __syncwarp();
+    __syncthreads();  // not a wait on the barrier by every thread: their polls took the driving threads' issue slots
     if (warp < 4) {
-        const bool ok = conv_wait(&done, 0, &bad);
+        const bool ok = !bad;
         tc_fence_after();
-        const int row = warp * 32 + lane, blk = blockIdx.x * ablk + row / a.bwA, tap = blk / nch;
-        const int kk = tap * a.cin + a.c_off + (blk - tap * nch) * a.bwA + row % a.bwA;
-        const bool real = blk < blocks && kk < a.kk_max;
-        for (int c0 = 0; c0 < a.Ntile; c0 += 32) {
-            float v[32];
-            tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (!ok || !real) continue;
-            float* o = a.part + ((size_t)blockIdx.z * a.kk_max + kk) * a.N + n0 + c0;
+        const int row = warp * 32 + lane, blk = row / a.bw, ci = ch + row - blk * a.bw;
+        for (int h = 0; h < nacc; h++) {
+            const int dx = blk + 2 * h;  // 0, 1, 2: taps -1, 0, 1
+            const int tap = a.taps == 1 ? 0 : 3 * unit + dx, kk = tap * a.cin + a.c_off + ci;
+            const bool real = (a.taps == 1 ? blk == 0 : dx < 3 && (h == 0 || blk == 0)) && kk < a.kk_max;
+            for (int c0 = 0; c0 < a.Ntile; c0 += 32) {
+                float v[32];
+                __syncwarp();
+                tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * a.Ntile + c0), v);
+                if (!ok || !real) continue;
+                float* o = a.part + ((size_t)blockIdx.z * a.kk_max + kk) * a.N + n0 + c0;
 #pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(o + j) = n > 0 ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3])
-                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4*>(o + j) = n > 0 ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3])
+                                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (bad && tid == 0) {
-        atomicOr(err, 1);
-        for (int s = 0; s < S; s++) mbar_wait(full + s, 0);  // copies still in flight (bounded)
-    }
-    if (warp == 5) tmem_dealloc(taddr, ncols);
+    if (bad && tid == 0) atomicOr(err, 1);
+    if (warp == 5) tmem_dealloc(taddr, (uint32_t)a.ncols);
 }
 
 }  // namespace tc

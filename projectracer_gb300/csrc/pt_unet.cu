@@ -104,21 +104,33 @@ __global__ void k_pool(uint16_t* __restrict__ o, const uint16_t* __restrict__ in
 
 // epilogue of the forward GEMM: bias, ReLU, BF16; the nearest-neighbour upsampled copy beside it
 // where the next layer reads that
+// 32 bytes in one store: whole sectors, where 16-byte stores of a row per thread are halves of them
+__device__ __forceinline__ void st32(void* p, const uint32_t (&h)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]),
+                 "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7])
+                 : "memory");
+}
 struct FwdEpi {
     uint16_t* out;
     const float* bias;
     int C;
     uint16_t* up;
     PadGeo gup;
-    __device__ __forceinline__ void operator()(int p, int b, int y, int x, int c0, const float (&v)[32]) const {
+    __device__ __forceinline__ void stage(float* sb, int n, int tid) const {
+        for (int c = tid; c < n; c += tc::kConvThreads) sb[c] = bias[c];
+    }
+    __device__ __forceinline__ void operator()(int p, int b, int y, int x, int c0, const float (&v)[32],
+                                               const float* sb) const {
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-            uint16_t h[8];
+        for (int j = 0; j < 32; j += 16) {
+            uint32_t h[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) h[e] = f2bf(fmaxf(v[j + e] + bias[c0 + j + e], 0.f));
-            st8(out + (size_t)p * C + c0 + j, h);
+            for (int e = 0; e < 8; e++)
+                h[e] = (uint32_t)f2bf(fmaxf(v[j + 2 * e] + sb[j + 2 * e], 0.f)) |
+                       (uint32_t)f2bf(fmaxf(v[j + 2 * e + 1] + sb[j + 2 * e + 1], 0.f)) << 16;
+            st32(out + (size_t)p * C + c0 + j, h);
             if (up)
-                for (int q = 0; q < 4; q++) st8(up + gup.at(b, 2 * y + (q >> 1), 2 * x + (q & 1)) * C + c0 + j, h);
+                for (int q = 0; q < 4; q++) st32(up + gup.at(b, 2 * y + (q >> 1), 2 * x + (q & 1)) * C + c0 + j, h);
         }
     }
 };
@@ -126,10 +138,16 @@ struct FwdEpi {
 struct DxEpi {
     float* dx;
     int N;
-    __device__ __forceinline__ void operator()(int p, int, int, int, int c0, const float (&v)[32]) const {
+    __device__ __forceinline__ void stage(float*, int, int) const {}
+    __device__ __forceinline__ void operator()(int p, int, int, int, int c0, const float (&v)[32], const float*) const {
         float* o = dx + (size_t)p * N + c0;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        for (int j = 0; j < 32; j += 8) {
+            uint32_t h[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) h[e] = __float_as_uint(v[j + e]);
+            st32(o + j, h);
+        }
     }
 };
 
@@ -153,23 +171,30 @@ __global__ void k_pack_weights(uint16_t* __restrict__ wbd, uint16_t* __restrict_
     }
 }
 
-// dW[co][kk] = sum_z part[z][kk][co], z ascending (loads of eight splits in flight); with two sources
-// the rows' channels below c0 have nsplit0 partial sums, the others nsplit1
-__global__ void k_wgrad_reduce(float* dW, const float* part, int nsplit0, int nsplit1, int c0, int cin, int M, int N) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= M * N) return;
+// dW[co][kk] = sum_z part[z][kk][co]: a warp adds every eighth split of 32 weights (eight loads in flight),
+// then the eight sums are added in order; with two sources the rows' channels below c0 have nsplit0 partial
+// sums, the others nsplit1
+__global__ void __launch_bounds__(256) k_wgrad_reduce(float* dW, const float* __restrict__ part, int nsplit0, int nsplit1,
+                                                      int c0, int cin, int M, int N) {
+    __shared__ float sh[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;  // N % 32 == 0
     const int kk = q / N, co = q % N, nsplit = kk % cin < c0 ? nsplit0 : nsplit1;
     const size_t ld = (size_t)M * N;
     float s = 0.f;
-    int z = 0;
-    for (; z + 8 <= nsplit; z += 8) {
+    int z = warp;
+    for (; z + 56 < nsplit; z += 64) {
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = part[(size_t)(z + j) * ld + q];
+        for (int j = 0; j < 8; j++) v[j] = part[(size_t)(z + 8 * j) * ld + q];
 #pragma unroll
         for (int j = 0; j < 8; j++) s += v[j];
     }
-    for (; z < nsplit; z++) s += part[(size_t)z * ld + q];
+    for (; z < nsplit; z += 8) s += part[(size_t)z * ld + q];
+    sh[warp][lane] = s;
+    __syncthreads();
+    if (warp) return;
+#pragma unroll
+    for (int j = 1; j < 8; j++) s += sh[j][lane];
     dW[(size_t)co * M + kk] = s;
 }
 
@@ -414,15 +439,21 @@ static int pack_weights(UNet& U) {
     return cuda_check(cudaGetLastError(), "k_pack_weights");
 }
 
-// Weight tiles' columns, and the splits over the positions of the weight gradient of a source of C channels:
-// about two CTAs per SM in all, and at least eight chunks each
-static int wgrad_ntile(int cout) { return std::min(cout, 128); }
-static void wgrad_splits(int taps, int C, int cout, size_t positions, int* per, int* ns) {
-    const int chunks = (int)((positions + tc::kWgradK - 1) / tc::kWgradK);
-    const int tiles = (taps * C + tc::kTileM - 1) / tc::kTileM * (cout / wgrad_ntile(cout));
-    const int n0 = std::max(1, std::min((chunks + 7) / 8, (304 + tiles - 1) / tiles));
-    *per = (chunks + n0 - 1) / n0;
-    *ns = (chunks + *per - 1) / *per;
+// The shape of a source's weight gradient: columns of a tile, CTAs over blocks of channels and image rows,
+// and the splits over the positions: one and a half CTAs per SM in all (1, 1.5 and 2 are within 3 % on
+// 8 images of 512 x 256), and at least four chunks each
+struct WgradShape {
+    int ntile, units, per, ns;
+};
+static WgradShape wgrad_shape(int taps, int C, int cout, size_t positions) {
+    WgradShape w;
+    w.ntile = std::min(cout, 128);
+    w.units = C / (C % 64 == 0 ? 64 : 32) * (taps == 1 ? 1 : 3);
+    const int chunks = (int)((positions + tc::kWgradK - 1) / tc::kWgradK), tiles = w.units * (cout / w.ntile);
+    const int n0 = std::max(1, std::min((chunks + 3) / 4, 228 / tiles));
+    w.per = (chunks + n0 - 1) / n0;
+    w.ns = (chunks + w.per - 1) / w.per;
+    return w;
 }
 
 static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
@@ -488,10 +519,9 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
         const int C0 = c.src0 < 0 ? kImCols : U.tch[c.src0], C1 = c.mode == 2 ? U.tch[c.src1] : 0;
         for (int B = 1; B <= maxB; B++)  // (a smaller batch may have more splits)
             for (int C : {C0, C1}) {
-                int per, ns;
                 if (C == 0) continue;
-                wgrad_splits(c.src0 < 0 ? 1 : 9, C, c.cout, U.geo(c.level, B).positions(), &per, &ns);
-                part = std::max(part, (size_t)ns * 9 * c.cin * c.cout);
+                const WgradShape w = wgrad_shape(c.src0 < 0 ? 1 : 9, C, c.cout, U.geo(c.level, B).positions());
+                part = std::max(part, (size_t)w.ns * 9 * c.cin * c.cout);
             }
     }
     bpart = (size_t)4 * 152 * 256;
@@ -501,7 +531,7 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
         (rc = ualloc(U, &U.dy, P0)) || (rc = ualloc(U, &U.tgt, P0)) || (rc = ualloc(U, &U.lpart, P0 / 256 + 1)) ||
         (rc = ualloc(U, &U.dx, dx)) || (rc = ualloc(U, &U.part, part)) || (rc = ualloc(U, &U.bpart, bpart)))
         return rc;
-    const int smax = 221 * 1024;  // conv_stages' bound and the alignment
+    const int smax = 221 * 1024;  // the rings' bound and the alignment
     CK(cudaFuncSetAttribute(tc::k_conv_gemm<FwdEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     CK(cudaFuncSetAttribute(tc::k_conv_gemm<DxEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     CK(cudaFuncSetAttribute(tc::k_wgrad_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
@@ -554,6 +584,8 @@ static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* 
                      int N) {
     tc::ConvArgs& a = P.a;
     a.g = g;
+    a.wp = PadGeo::Div(g.Wp());
+    a.hp = PadGeo::Div(g.Hp());
     a.taps = taps;
     a.nsrc = nsrc;
     a.N = N;
@@ -571,15 +603,15 @@ static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* 
     for (int f = nt + 1; f <= N / 32 && mt * nt < 152; f++)
         if (N % f == 0 && (N / f) % 32 == 0) nt = f;
     a.Ntile = N / nt;
-    P.grid = dim3(mt, nt);
-    const int bw = nsrc > 1 ? std::max(a.bw[0], a.bw[1]) : a.bw[0];
-    a.abytes = tc::kTileM * bw * 2;
-    a.bbytes = a.Ntile * bw * 2;
-    a.stages = tc::conv_stages((size_t)(a.abytes + a.bbytes), (size_t)mt * nt, a.Ktot / bw);
+    a.nt = nt;
+    a.tiles = mt * nt;
+    tc::conv_stages(a, C[0] / a.bw[0] + (nsrc > 1 ? C[1] / a.bw[1] : 0));
+    P.grid = dim3(std::min(a.tiles, tc::kSms * a.ctas));
+    const int brows = a.nd == 3 ? tc::kBoxRows : tc::kTileM;
     int rc;
     for (int s = 0; s < 2; s++) {
         const int q = s < nsrc ? s : 0;
-        if ((rc = tensor_map(&P.A[s], t[q], C[q], g.positions(), a.bw[q], tc::kTileM)) ||
+        if ((rc = tensor_map(&P.A[s], t[q], C[q], g.positions(), a.bw[q], brows)) ||
             (rc = tensor_map(&P.B[s], w, a.Ktot, N, a.bw[q], a.Ntile)))
             return rc;
     }
@@ -604,31 +636,31 @@ static int plan_batch(UNet& U, int B) {
         if (!first && (rc = plan_conv(P.bwd, g, 9, 1, z, Cz, U.wbd + c.woff, c.cin))) return rc;
         P.nwg = ns;
         for (int s = 0; s < ns; s++) {
-            int per;
-            wgrad_splits(first ? 1 : 9, C[s], c.cout, g.positions(), &per, &P.nsplit[s]);
-            if ((size_t)P.nsplit[s] * 9 * c.cin * c.cout > U.part_cap)
-                return fail(PT_ERR_STATE, "U-Net: split workspace too small");
             WgradPlan& w = P.wg[s];
             tc::WgradArgs& a = w.a;
+            const WgradShape sh = wgrad_shape(first ? 1 : 9, C[s], c.cout, g.positions());
+            P.nsplit[s] = sh.ns;
+            if ((size_t)sh.ns * 9 * c.cin * c.cout > U.part_cap)
+                return fail(PT_ERR_STATE, "U-Net: split workspace too small");
             a.g = g;
             a.taps = first ? 1 : 9;
             a.C = C[s];
-            a.bwA = C[s] % 64 == 0 ? 64 : 32;
+            a.bw = C[s] % 64 == 0 ? 64 : 32;
             a.c_off = s ? C[0] : 0;
             a.cin = first ? 9 * c.cin : c.cin;
             a.kk_max = 9 * c.cin;
             a.N = c.cout;
-            a.Ntile = wgrad_ntile(c.cout);
+            a.Ntile = sh.ntile;
             a.bwB = c.cout % 64 == 0 ? 64 : 32;
-            a.per = per;
+            a.per = sh.per;
             a.chunks = (int)((g.positions() + tc::kWgradK - 1) / tc::kWgradK);
-            a.part = U.part;
-            const int blocks = a.taps * (a.C / a.bwA), ablk = tc::kTileM / a.bwA;
-            w.grid = dim3((blocks + ablk - 1) / ablk, c.cout / a.Ntile, P.nsplit[s]);
-            a.abytes = tc::kTileM * tc::kWgradK * 2;
+            a.ncols = (int)tc::tmem_cols((first || a.bw == 32 ? 1 : 2) * a.Ntile);
+            a.abytes = tc::wgrad_box_bytes(a.bw);
             a.bbytes = a.Ntile * tc::kWgradK * 2;
-            a.stages = tc::conv_stages((size_t)(a.abytes + a.bbytes), (size_t)w.grid.x * w.grid.y * w.grid.z, per);
-            if ((rc = tensor_map(&w.A, t[s], C[s], g.positions(), a.bwA, tc::kWgradK)) ||
+            a.part = U.part;
+            w.grid = dim3(sh.units, c.cout / a.Ntile, sh.ns);
+            a.S = std::min(std::min(110 * 1024 / (a.abytes + a.bbytes), tc::kMaxRing), sh.per);  // two CTAs on an SM
+            if ((rc = tensor_map(&w.A, t[s], C[s], g.positions(), a.bw, tc::kWgradBox)) ||
                 (rc = tensor_map(&w.B, U.dz[c.out], c.cout, g.positions(), a.bwB, tc::kWgradK)))
                 return rc;
         }
@@ -637,13 +669,10 @@ static int plan_batch(UNet& U, int B) {
     return 0;
 }
 
-template <class Args>
-static size_t conv_smem(const Args& a) { return (size_t)a.stages * (size_t)(a.abytes + a.bbytes) + 1024; }
-
 template <class E>
 static int run_conv(UNet& U, const ConvPlan& P, const E& e) {
-    tc::k_conv_gemm<E><<<P.grid, tc::kConvThreads, conv_smem(P.a), U.st>>>(P.A[0], P.A[1], P.B[0], P.B[1],
-                                                                                       P.a, e, U.derr);
+    tc::k_conv_gemm<E><<<P.grid, tc::kConvThreads, tc::conv_smem(P.a), U.st>>>(P.A[0], P.A[1], P.B[0], P.B[1], P.a, e,
+                                                                                U.derr);
     return cuda_check(cudaGetLastError(), "k_conv_gemm");
 }
 
@@ -718,9 +747,9 @@ static int unet_backward(UNet& U, int B, float* loss) {
         // weights: split over positions, then a fixed-order reduction of the splits
         const int Mw = 9 * c.cin;
         for (int s = 0; s < P.nwg; s++)
-            tc::k_wgrad_gemm<<<P.wg[s].grid, tc::kConvThreads, conv_smem(P.wg[s].a), U.st>>>(
-                P.wg[s].A, P.wg[s].B, P.wg[s].a, U.derr);
-        k_wgrad_reduce<<<nblk((size_t)Mw * c.cout, 256), 256, 0, U.st>>>(
+            tc::k_wgrad_gemm<<<P.wg[s].grid, tc::kWgradThreads, tc::wgrad_smem(P.wg[s].a), U.st>>>(P.wg[s].A, P.wg[s].B,
+                                                                                                  P.wg[s].a, U.derr);
+        k_wgrad_reduce<<<(unsigned)(Mw * c.cout / 32), 256, 0, U.st>>>(
             U.g + c.woff, U.part, P.nsplit[0], P.nsplit[1], P.nwg > 1 ? P.wg[0].a.C : Mw, P.nwg > 1 ? c.cin : Mw, Mw, c.cout);
         CK(cudaGetLastError());
         if (c.src0 < 0) continue;  // the network input needs no gradient

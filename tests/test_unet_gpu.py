@@ -121,6 +121,11 @@ def test_unet_ragged_grids_match_the_oracle(nz, nx, B):
     net.close()
 
 
+def test_unet_grids_of_more_tiles_than_sms_match_the_oracle():
+    """Several tiles per thread block at the top level, one or two at the second: the bounds above."""
+    test_unet_ragged_grids_match_the_oracle(128, 160, 4)
+
+
 def test_unet_batches_below_the_maximum_see_nothing_of_earlier_ones():
     nz, nx = 24, 40
     rng = np.random.default_rng(1)
