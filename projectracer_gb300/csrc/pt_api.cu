@@ -240,6 +240,8 @@ static void engine_free(Engine& E) {
     for (double* p : {E.Ginv2, E.Mc2, E.RowB2})
         if (p) cudaFree(p);
     if (E.ipiv2) cudaFree(E.ipiv2);
+    for (void* p : {E.luw, E.luw2})
+        if (p) cudaFree(p);
     if (E.derr2) cudaFree(E.derr2);
     if (E.hflag2) cudaFreeHost(E.hflag2);
     if (E.ev_in) cudaEventDestroy(E.ev_in);

@@ -156,6 +156,7 @@ struct Engine {
     // top-of-step solve runs with the previous one, then copied into Mc/RowB/ipiv/Ginv
     double *Mc2 = nullptr, *RowB2 = nullptr, *Ginv2 = nullptr;
     int *ipiv2 = nullptr, *derr2 = nullptr, *hflag2 = nullptr;
+    void *luw = nullptr, *luw2 = nullptr;  // workspaces of the coarse LU on st and st2
     cudaStream_t st2 = nullptr;
     cudaEvent_t ev_in = nullptr, ev_fact = nullptr;
     bool fact_pending = false;

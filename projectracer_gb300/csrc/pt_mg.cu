@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "pt_bandlu.cuh"
 #include "pt_cluster.cuh"
 #include "pt_consts.cuh"
 #include "pt_exact.cuh"
@@ -1026,82 +1027,6 @@ __global__ void k_coarse_matrix(double* M, Geo g, int l, int kl, int ku, int n, 
 #undef MB
 }
 
-// DGBTF2: unblocked band LU with partial pivoting, one CTA (band in global memory / L2)
-__global__ void __launch_bounds__(1024) k_band_lu(double* ab, int* ipiv, int n, int kl, int ku, int* err) {
-    const int ldab = 2 * kl + ku + 1, kv = ku + kl;
-    __shared__ int s_jp, s_ju, s_nz;
-    const int tid = threadIdx.x, nt = blockDim.x;
-#define AB(r, c) ab[(size_t)((r) - 1) + (size_t)((c) - 1) * (size_t)ldab]
-    for (int j = ku + 2; j <= (kv < n ? kv : n); j++)
-        for (int i = kv - j + 2 + tid; i <= kl; i += nt) AB(i, j) = 0.0;
-    if (tid == 0) s_ju = 1;
-    __syncthreads();
-    for (int j = 1; j <= n; j++) {
-        if (j + kv <= n)
-            for (int i = 1 + tid; i <= kl; i += nt) AB(i, j + kv) = 0.0;
-        const int km = kl < n - j ? kl : n - j;
-        // pivot: first index of the maximum |a| in AB(kv+1..kv+1+km, j).  A NaN never wins the
-        // comparison; the search starts from row 1 so the index stays inside the band even for a
-        // column of NaNs, which is then reported like a zero pivot.
-        if (tid < 32) {
-            double best = -1.0;
-            int bi = 1 << 30;
-            for (int i = 1 + tid; i <= km + 1; i += 32) {
-                double a = fabs(AB(kv + i, j));
-                if (a > best) { best = a; bi = i; }
-            }
-            if (bi > km + 1) bi = 1;
-            for (int o = 16; o > 0; o >>= 1) {
-                double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-            }
-            if (tid == 0) {
-                s_jp = bi;
-                ipiv[j - 1] = bi + j - 1;
-                const double piv = AB(kv + bi, j);
-                s_nz = (piv != 0.0 && piv == piv);
-                if (s_nz) {
-                    int jue = j + ku + bi - 1 < n ? j + ku + bi - 1 : n;
-                    if (jue > s_ju) s_ju = jue;
-                } else {
-                    atomicCAS(err, 0, j);
-                }
-            }
-        }
-        __syncthreads();
-        const int jp = s_jp, ju = s_ju;
-        if (s_nz) {
-            if (jp != 1) {
-                for (int t = tid; t <= ju - j; t += nt) {
-                    size_t a0 = (size_t)(kv + jp - 1) + (size_t)(j - 1) * ldab + (size_t)t * (ldab - 1);
-                    size_t b0 = (size_t)kv + (size_t)(j - 1) * ldab + (size_t)t * (ldab - 1);
-                    double x = ab[a0];
-                    ab[a0] = ab[b0];
-                    ab[b0] = x;
-                }
-                __syncthreads();
-            }
-            if (km > 0) {
-                const double rp = 1.0 / AB(kv + 1, j);
-                for (int i = 1 + tid; i <= km; i += nt) AB(kv + 1 + i, j) = AB(kv + 1 + i, j) * rp;
-                __syncthreads();
-                const int ncol = ju - j;
-                for (int e = tid; e < ncol * km; e += nt) {
-                    int jj = e / km + 1, i = e % km + 1;
-                    double y = ab[(size_t)(kv - 1) + (size_t)j * ldab + (size_t)(jj - 1) * (ldab - 1)];
-                    if (y != 0.0) {
-                        size_t a0 = (size_t)kv + (size_t)j * ldab + (size_t)(jj - 1) * (ldab - 1) + (size_t)(i - 1);
-                        ab[a0] = ab[a0] + AB(kv + 1 + i, j) * (-1.0 * y);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-#undef AB
-}
-
 // DGBTRS (forward substitution with the row interchanges and L, back substitution with U) on one
 // right-hand side.  The substitutions are sequential over the n columns, so one warp carries
 // them, its lanes splitting each column's band update; the band columns (and pivots) a chunk of
@@ -1328,8 +1253,7 @@ static int coarse_factor(Engine& E) {
     CK(cudaMemsetAsync(E.derr, 0, sizeof(int), E.st));
     PT_COUNT(), k_coarse_matrix<<<nblk(n, 128), 128, 0, E.st>>>(E.Mc, E.gl[L], L, E.kl, E.ku, n, E.RowB, E.cfg.Vbc,
                                                     E.cfg.ivis, E.vis[L], E.vx[L], E.vz[L], E.vxz[L], E.vxxmzz[L], E.derr);
-    PT_COUNT(), k_band_lu<<<1, 1024, 0, E.st>>>(E.Mc, E.ipiv, n, E.kl, E.ku, E.derr);
-    CKL("coarse LU");
+    if (int rc = bandlu::factor(E.Mc, E.ipiv, n, E.kl, E.ku, bandlu::work_of(E.luw, E.kl), E.derr, E.st)) return rc;
     int h = 0;
     CK(cudaMemcpyAsync(&h, E.derr, sizeof(int), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
@@ -1343,15 +1267,15 @@ static int coarse_factor(Engine& E) {
 }
 
 // Mixed precision: build the coarse matrix, its LU and inverse for the viscosity just computed
-// on st into the second buffer set on st2, overlapped with the solve that follows on st (the LU
-// runs on one SM).  coarse_resolve copies the result into the live buffers.
+// on st into the second buffer set on st2, overlapped with the solve that follows on st (the
+// LU's panels run on one SM, the columns they reach on a SM each for a few us).  coarse_resolve copies the result into the live buffers.
 static int coarse_factor_async(Engine& E, const VisLevels& V) {
     const int L = E.grids, n = E.ngc;
     CK(cudaMemsetAsync(E.derr2, 0, sizeof(int), E.st2));
     PT_COUNT(), k_coarse_matrix<<<nblk(n, 128), 128, 0, E.st2>>>(E.Mc2, E.gl[L], L, E.kl, E.ku, n, E.RowB2, E.cfg.Vbc,
                                                      E.cfg.ivis, V.vis[L], V.vx[L], V.vz[L], V.vxz[L], V.vxxmzz[L],
                                                      E.derr2);
-    PT_COUNT(), k_band_lu<<<1, 1024, 0, E.st2>>>(E.Mc2, E.ipiv2, n, E.kl, E.ku, E.derr2);
+    if (int rc = bandlu::factor(E.Mc2, E.ipiv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, E.kl), E.derr2, E.st2)) return rc;
     PT_COUNT(), k_band_inverse<<<nblk(n, kInvWarps), 32 * kInvWarps, inv_smem(n, E.kl, E.ku), E.st2>>>(
         E.Mc2, E.ipiv2, E.Ginv2, n, E.kl, E.ku);
     CKL("async coarse factorisation");
@@ -1725,6 +1649,7 @@ int mg_alloc(Engine& E) {
     if (int rc = alloc(&E.Bc, E.ngc)) return rc;
     if (int rc = alloc(&E.RowB, E.ngc)) return rc;
     CK(cudaMalloc(&E.ipiv, sizeof(int) * E.ngc));
+    CK(cudaMalloc(&E.luw, bandlu::work_bytes(E.kl)));
     const size_t smem = sizeof(double) * (size_t)E.ngc;
     if (smem > 220 * 1024) return fail(PT_ERR_CONFIG, "coarsest grid too large for the banded solve");
     if (band_solve_smem(E.ngc, E.kl, E.ku) > 220 * 1024)
@@ -1743,6 +1668,7 @@ int mg_alloc(Engine& E) {
         CK(cudaMalloc(&E.Mc2, sizeof(double) * (size_t)ldab * E.ngc));
         CK(cudaMalloc(&E.RowB2, sizeof(double) * (size_t)E.ngc));
         CK(cudaMalloc(&E.ipiv2, sizeof(int) * (size_t)E.ngc));
+        CK(cudaMalloc(&E.luw2, bandlu::work_bytes(E.kl)));
         CK(cudaMalloc(&E.derr2, sizeof(int)));
         CK(cudaMallocHost(&E.hflag2, sizeof(int)));
         *E.hflag2 = 0;
