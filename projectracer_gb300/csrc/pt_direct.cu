@@ -309,33 +309,11 @@ __global__ void __launch_bounds__(kLuThreads) k_direct_lu(double* ab, int* ipiv,
 // column-by-column DGBTRS; zero entries are divided and propagated too, like the optimized BLAS of
 // the shipped run (psi = -0 on the non-corner wall nodes of its snapshots).
 //
-// The column steps are sequential, so one CTA carries them.  Every element of b has one owner
-// thread (element i: thread (i - 1) mod kDsThreads), which alone writes it: in a column step each
-// thread applies the column to the elements it owns, and the value the next step needs first (the
-// pivot row's b for the forward step, the next x = b / U_jj for the back substitution) is
-// published by its owner, so a step needs one barrier.
-//   * b stays in global memory; the elements a step touches (j .. j+kl forward, j-k .. j back)
-//     live in a window of W shared-memory slots (W a power of two >= k + 4, element i in slot
-//     (i - 1) mod W).  An element enters two steps before its first use: its owner loads it into
-//     a register one step, stores it into its slot the next.  An element is written back by its
-//     owner in the step it becomes final (forward: when swapped into b(j); back: as x).
-//   * The band columns stream through a ring of AHEAD + 1 shared-memory slots, filled by
-//     cp.async AHEAD columns ahead of their step (16-byte copies from the 16-byte boundary at or
-//     below the column's first entry; the column sits at offset s0 & 1 in its slot).
-// On this part a step is bound by the SM's FP64 pipe: forward kl, backward kl + ku
-// multiply-subtract pairs.  AHEAD = 8 where that ring fits, else 2.
-constexpr int kDsThreads = 256;
-static __host__ __device__ int direct_slot_len(int kl, int ku) { return (kl + ku + 3) & ~1; }
-static int direct_window(int kl, int ku) {
-    int w = 64;
-    while (w < kl + ku + 4) w *= 2;
-    return w;
-}
-static size_t direct_solve_smem(int kl, int ku, int ahead) {
-    return sizeof(double) * ((size_t)(ahead + 1) * (size_t)direct_slot_len(kl, ku) + (size_t)direct_window(kl, ku) + 4) +
-           sizeof(int) * (size_t)(ahead + 1);
-}
-
+// The column steps are sequential, so one CTA carries them.  An FP64 instruction takes its scheduler 64 to
+// 76 cycles for a warp, alone or behind another one, so a step's chain counts in those: the forward step is
+// bound by the SM's FP64 rate (2 kl operations, 300 of the 500 cycles at kl = 303) and its barrier, the back
+// substitution by the chain of its diagonal (quotient, product and difference: 650 cycles).
+constexpr int kDsRows = 960;  // row threads of the forward substitution at most
 __device__ __forceinline__ void ds_cp16(void* dst, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
@@ -350,145 +328,256 @@ __device__ __forceinline__ void ds_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// copies band entries [s0, s0 + len) into a slot from the even index at or below s0 (the slot
-// then holds entry s0 at position s0 & 1); every thread commits one group, empty or not
-__device__ __forceinline__ void ds_issue(double* slot, const double* ab, size_t s0, int len, bool live, int tid) {
-    if (live) {
-        const size_t a0 = s0 & ~(size_t)1;
-        const int pairs = (int)((s0 - a0) + (size_t)len + 1) >> 1;
-        for (int q = tid; q < pairs; q += kDsThreads) ds_cp16(slot + 2 * q, ab + a0 + 2 * (size_t)q);
+// Products, sums and differences in the form of a fused multiply-add, each rounded once as they are: the
+// unit takes a warp's DFMA every 16 cycles, its DMUL or DADD every 19.  (Kernel arguments, so that the
+// compiler does not turn them back.)
+struct FmaForms {
+    double zero = -0.0, one = 1.0, minus = -1.0;
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, zero); }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(b, one, a); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, minus, a); }
+};
+
+// Forward substitution: for j = 1 .. n-1, b(j) <-> b(ipiv(j)), then b(j+1 .. j+lm) += L(., j) * (-b(j)).
+// Element i of b stays in a register of thread (i - 1) mod (blockDim - 64), as its register
+// ((i - 1) / that) mod RPT, from kl + 1 steps before it is final at the latest; a step's
+// multipliers are read a step ahead.  The values that the next step interchanges are published by their
+// owners, so a step has one barrier.  A warp loads its next 32 elements when its last one became final.
+// The last two warps stream the columns of L and the pivots through a ring of kDsAhead + 1 slots (16-byte
+// copies from the boundary at or below a column's first entry); kDsAhead = 8, or 4 for bands of more
+// than 2 kDsRows.
+// n = 10201, kl = 303: 4.8 ms with b in shared memory, 2.7 now.
+static __host__ __device__ int direct_slot_len(int kl) { return (kl + 3) & ~1; }
+static size_t direct_forward_smem(int kl, int ahead) {
+    return sizeof(double) * (size_t)(ahead + 1) * (size_t)direct_slot_len(kl) + sizeof(int) * (size_t)(ahead + 1);
+}
+template <int RPT, int kDsAhead>
+__global__ void __launch_bounds__(1024, 1) k_direct_forward(const double* __restrict__ ab, const int* __restrict__ ipiv,
+                                                         double* bg, int n, int kl, int ku, FmaForms F) {
+    constexpr int kRing = kDsAhead + 1;
+    extern __shared__ __align__(16) double dsm[];
+    __shared__ double pubT[2], pubS[2];
+    const int SL = direct_slot_len(kl), ldab = 2 * kl + ku + 1, kd = kl + ku + 1;
+    int* ipr = reinterpret_cast<int*>(dsm + (size_t)kRing * SL);
+    const int tid = threadIdx.x, lane = tid & 31, nt = (int)blockDim.x - 64, M = RPT * nt;
+    if (tid >= nt) {  // loaders: column c's multipliers AB(kd+1 .. kd+kl, c) and its pivot
+        const int t = tid - nt;
+        auto issue = [&](int c, int slot) {
+            if (c <= n - 1) {
+                const size_t s0 = (size_t)kd + (size_t)(c - 1) * (size_t)ldab, a0 = s0 & ~(size_t)1;
+                const int pairs = (int)((s0 - a0) + (size_t)kl + 1) >> 1;
+                double* d = dsm + (size_t)slot * SL;
+                if (t == 0) ds_cp4(ipr + slot, ipiv + (c - 1));
+                for (int q = t; q < pairs; q += 64) ds_cp16(d + 2 * q, ab + a0 + 2 * (size_t)q);
+            }
+            ds_commit();
+        };
+        for (int c = 1; c <= kDsAhead; c++) issue(c, c);  // (kDsAhead < kRing)
+        ds_wait<kDsAhead - 2>();                          // columns 1 and 2
+        __syncthreads();
+        __syncthreads();
+        int slot = kDsAhead;
+        for (int j = 1; j <= n - 1; j++) {
+            if (++slot == kRing) slot = 0;
+            issue(j + kDsAhead, slot);  // into the slot of column j - 1
+            ds_wait<kDsAhead - 2>();    // column j + 2
+            __syncthreads();
+        }
+        return;
     }
-    ds_commit();
+    double v[RPT], nx[RPT], L[RPT];
+    int own[RPT];  // the element
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        own[r] = 1 + tid + r * nt;
+        v[r] = own[r] <= n ? bg[own[r] - 1] : 0.0;
+        nx[r] = own[r] + M <= n ? bg[own[r] + M - 1] : 0.0;
+    }
+    __syncthreads();
+    int slot = 1, par = kd & 1, l = n >= 2 ? ipr[1] : 1;
+    const double* col = dsm + (size_t)slot * SL + par;  // element i's multiplier of column j at col[i - j - 1]
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        if (own[r] == l) pubT[1] = v[r];
+        if (own[r] == 1) pubS[1] = v[r];
+        const int o = own[r] - 1;
+        L[r] = o >= 1 && o <= kl ? col[o - 1] : 0.0;
+    }
+    __syncthreads();
+    for (int j = 1; j <= n - 1; j++) {
+        const double T = pubT[j & 1], S = pubS[j & 1];
+        if (++slot == kRing) slot = 0;
+        par ^= ldab & 1;
+        const int l1 = j + 1 <= n - 1 ? ipr[slot] : j + 1;
+        col = dsm + (size_t)slot * SL + par;
+        const double temp = -T;  // -1.0 * T, exactly
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+            const int o = own[r] - j;
+            if (own[r] == l && l != j) v[r] = S;
+            const double u = F.add(v[r], F.mul(L[r], temp));
+            if (o >= 1 && o <= kl) v[r] = u;
+            if (own[r] == l1) pubT[(j + 1) & 1] = v[r];
+            if (own[r] == j + 1) pubS[(j + 1) & 1] = v[r];
+            if (o == 0) {  // final for the forward substitution
+                bg[j - 1] = T;
+                v[r] = nx[r];
+                own[r] += M;
+            }
+            const int o1 = own[r] - j - 1;
+            L[r] = o1 >= 1 && o1 <= kl ? col[o1 - 1] : 0.0;
+            // the warp's last element became final: its next ones
+            if (__any_sync(0xffffffffu, o == 0 && lane == 31)) nx[r] = own[r] + M <= n ? bg[own[r] + M - 1] : 0.0;
+        }
+        l = l1;
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < RPT; r++)
+        if (own[r] == n) bg[n - 1] = v[r];
 }
 
-template <int kDsAhead>
-__global__ void __launch_bounds__(kDsThreads, 1) k_direct_solve(const double* __restrict__ ab, const int* __restrict__ ipiv,
-                                                               double* __restrict__ bg, int n, int kl, int ku, int W) {
-    constexpr int kDsRing = kDsAhead + 1;
-    extern __shared__ __align__(16) double dsm[];
-    const int SL = direct_slot_len(kl, ku), mask = W - 1;
-    double* ring = dsm;                                  // kDsRing slots of SL doubles
-    double* win = ring + (size_t)kDsRing * SL;           // W: the window of b
-    double* pub = win + W;                               // [4]: published values, by step parity
-    int* ipr = reinterpret_cast<int*>(pub + 4);          // pivots of the columns in the ring
-    const int ldab = 2 * kl + ku + 1, kd = kl + ku + 1, kp1 = kl + ku + 1, k = kl + ku;
-    const int tid = threadIdx.x;
-    auto B = [&](int i) -> double& { return win[(i - 1) & mask]; };
-    // the first element >= a that this thread owns
-    auto first_owned = [&](int a) {
-        int r = (tid - (a - 1)) % kDsThreads;
-        if (r < 0) r += kDsThreads;
-        return a + r;
-    };
-    auto owns = [&](int i) { return (i - 1) % kDsThreads == tid; };
-    double pend = 0.0;  // the element this thread loaded for the window, stored the next step
-    int pend_i = 0;
+// f(kernel, threads, shared memory) for a band: a thread per element of the window (kl + 2), up to four
+// elements per thread for wide bands, whose ring is shorter
+template <class F>
+static int direct_forward_of(int kl, F f) {
+    const int rpt = kl + 2 <= kDsRows ? 1 : kl + 2 <= 2 * kDsRows ? 2 : 4;
+    const int threads = ((kl + 2 + rpt - 1) / rpt + 31) / 32 * 32 + 64;
+    return rpt == 1 ? f(k_direct_forward<1, 8>, threads, direct_forward_smem(kl, 8))
+         : rpt == 2 ? f(k_direct_forward<2, 8>, threads, direct_forward_smem(kl, 8))
+                    : f(k_direct_forward<4, 4>, threads, direct_forward_smem(kl, 4));
+}
 
-    // ---- forward: for j = 1 .. n-1, b(j) <-> b(ipiv(j)), then b(j+1 .. j+lm) += L(., j) * (-b(j));
-    // the window holds b(j .. j+kl) at step j
-    auto issue_fwd = [&](int c) {  // column c's multipliers AB(kd+1 .. kd+kl, c) and its pivot
-        const bool live = c <= n - 1;
-        double* slot = ring + (size_t)(c % kDsRing) * SL;
-        if (live && tid == 0) ds_cp4(ipr + c % kDsRing, ipiv + (c - 1));
-        ds_issue(slot, ab, (size_t)kd + (size_t)(c - 1) * (size_t)ldab, kl, live, tid);
-    };
-    for (int c = 1; c <= kDsAhead; c++) issue_fwd(c);
-    for (int i = 1 + tid; i <= n && i <= kl + 1; i += kDsThreads) B(i) = bg[i - 1];
-    if (kl + 2 <= n && owns(kl + 2)) {  // needed from step 2
-        pend = bg[kl + 1];
-        pend_i = kl + 2;
-    }
-    ds_wait<kDsAhead - 1>();  // column 1
-    __syncthreads();
-    if (n >= 2 && tid == 0) {
-        pub[1] = B(ipr[1 % kDsRing]);  // the value the first step swaps into b(1)
-        pub[3] = B(1);
-    }
-    for (int j = 1; j <= n - 1; j++) {
-        ds_wait<kDsAhead - 2>();  // columns j and j + 1
-        __syncthreads();
-        if (pend_i) {  // b(j + kl + 1), first used in step j + 1
-            B(pend_i) = pend;
-            pend_i = 0;
-        }
-        const int sl = j % kDsRing;
-        const double* L = ring + (size_t)sl * SL + (((size_t)kd + (size_t)(j - 1) * (size_t)ldab) & 1);
-        const int l = ipr[sl];
-        const double T = pub[j & 1], S = pub[2 + (j & 1)];
-        if (owns(j)) {
-            B(j) = T;
-            bg[j - 1] = T;  // final for the forward substitution
-        }
-        if (l != j && owns(l)) B(l) = S;
-        const double temp = -T;  // -1.0 * T, exactly
-        const int lm = kl < n - j ? kl : n - j;
-        for (int i = first_owned(j + 1); i <= j + lm; i += kDsThreads) B(i) = B(i) + L[i - j - 1] * temp;
-        if (j + 1 <= n - 1) {
-            const int l1 = ipr[(j + 1) % kDsRing];
-            if (owns(l1)) pub[(j + 1) & 1] = B(l1);
-            if (owns(j + 1)) pub[2 + ((j + 1) & 1)] = B(j + 1);
-        }
-        const int f = j + kl + 2;  // first used in step j + 2
-        if (f <= n && owns(f)) {
-            pend = bg[f - 1];
-            pend_i = f;
-        }
-        issue_fwd(j + kDsAhead);
-    }
-    if (owns(n)) bg[n - 1] = B(n);
-    __syncthreads();  // the forward results in bg are visible to the whole CTA
+// b / d, correctly rounded, from r = 1 / d (Markstein, IBM J. Res. Dev. 34 (1990): a quotient within an ulp,
+// corrected once with its exact residual and a correctly rounded reciprocal, is the rounded quotient; two
+// corrections bring b r there).  Five dependent operations where a division takes nine.  For exponents that
+// keep every intermediate a normal number: in_range(b, 800) and in_range(d, 100).
+__device__ __forceinline__ bool in_range(double v, int bits) {  // 2^-bits <= |v| < 2^bits
+    return ((unsigned)__double2hiint(v) >> 20 & 0x7ffu) - (unsigned)(1023 - bits) < 2u * (unsigned)bits;
+}
+__device__ __forceinline__ double quotient(double b, double d, double r) {
+    double q = __dmul_rn(b, r);
+    q = __fma_rn(__fma_rn(-d, q, b), r, q);
+    return __fma_rn(__fma_rn(-d, q, b), r, q);
+}
 
-    // ---- back substitution: for j = n .. 1, x = b(j) / U(j,j), b(j) = x, b(i0 .. j-1) -= x U(., j)
-    // (step m handles column j = n - m + 1); the window holds b(j-k .. j) at step j
-    auto issue_bwd = [&](int m) {  // column n - m + 1: AB(1 .. kp1, j)
-        const int c = n - m + 1;
-        ds_issue(ring + (size_t)(m % kDsRing) * SL, ab, (size_t)(c - 1) * (size_t)ldab, kp1, c >= 1, tid);
+// Back substitution: for j = n .. 1, x = b(j) / U(j,j), b(j) = x, b(i0 .. j-1) -= x U(., j), in blocks of 32
+// columns, on a cluster of four CTAs (one FP64 unit serves an SM's warps in turn, so the chain of the
+// diagonal is kept from the rows beyond it):
+//   * Warp 0 of CTA 0 solves block q (lane t holds row e - t).
+//   * Warp 1 holds the rows of block q + 1: it applies the columns of block q - 1, then those of block q as
+//     they are solved (it is a few columns behind, and one at the block's end).
+//   * Warp 2 fetches the next block's triangle and takes the reciprocals of its diagonal.
+//   * The other CTAs apply the columns of block q - 1 to the rows beyond.  Subtracting x times a zero of U
+//     changes nothing but the sign of a zero: where all 32 entries of a column are zeros (the fill-in of
+//     interchanges that did not happen: half the band) and no element of b is -0, they skip the FP64
+//     instructions.
+// n = 10201, k = 606: 10.7 ms in one CTA with a barrier per column, 3.8 now.
+constexpr int kBackThreads = 256, kBackCtas = 4, kBackWarps = (kBackCtas - 1) * kBackThreads / 32;
+__device__ __forceinline__ void named_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__global__ void __cluster_dims__(kBackCtas, 1, 1) __launch_bounds__(kBackThreads, 1)
+    k_direct_back(const double* __restrict__ ab, double* bg, int n, int kl, int ku, FmaForms F) {
+    __shared__ double xs[2][32], hand[32], rec[2][32], tri[2][32][32];  // tri[.][s][t] = U(e - t, e - s)
+    __shared__ unsigned fast[2];
+    const int ldab = 2 * kl + ku + 1, k = kl + ku;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)blockIdx.x;
+    // U(i, j), 0 outside the band
+    auto U = [&](int i, int j) {
+        return i >= 1 && j >= 1 && i >= j - k && i <= j ? ab[(size_t)(j - 1) * (size_t)ldab + (size_t)(k + i - j)] : 0.0;
     };
-    auto ucol = [&](int m) {
-        const int c = n - m + 1;
-        return ring + (size_t)(m % kDsRing) * SL + (((size_t)(c - 1) * (size_t)ldab) & 1);
+    auto fetch = [&](int e, int buf) {
+        double t[32];
+#pragma unroll
+        for (int s = 0; s < 32; s++) t[s] = s <= lane ? U(e - lane, e - s) : 0.0;
+#pragma unroll
+        for (int s = 0; s < 32; s++) tri[buf][s][lane] = t[s];
+        __syncwarp();
+        const double d = tri[buf][lane][lane];
+        rec[buf][lane] = 1.0 / d;
+        const unsigned plain = __ballot_sync(0xffffffffu, in_range(d, 100));
+        if (lane == 0) fast[buf] = plain;
     };
-    for (int m = 1; m <= kDsAhead; m++) issue_bwd(m);
-    pend_i = 0;
-    for (int i = n - tid; i >= 1 && i >= n - k; i -= kDsThreads) B(i) = bg[i - 1];
-    if (n - k - 1 >= 1 && owns(n - k - 1)) {  // needed from step j = n - 1
-        pend = bg[n - k - 2];
-        pend_i = n - k - 1;
-    }
-    ds_wait<kDsAhead - 1>();  // column n
+    // the columns e .. e - 31, whose solutions the lanes hold, applied to v = b(i)
+    auto apply = [&](double& v, int i, int e, double x) {
+        double u[32];
+        unsigned some = 0;
+#pragma unroll
+        for (int s = 0; s < 32; s++) u[s] = U(i, e - s);
+#pragma unroll
+        for (int s = 0; s < 32; s++) some |= (unsigned)((__double_as_longlong(u[s]) << 1) != 0) << s;
+        const bool odd = __double_as_longlong(v) == (long long)0x8000000000000000ull ||
+                         ((unsigned)__double2hiint(x) & 0x7ff00000u) == 0x7ff00000u;
+        some = __any_sync(0xffffffffu, odd) ? 0xffffffffu : __reduce_or_sync(0xffffffffu, some);
+#pragma unroll
+        for (int s = 0; s < 32; s++)
+            if (some >> s & 1u) {
+                const double w = F.sub(v, F.mul(__shfl_sync(0xffffffffu, x, s), u[s]));
+                if (i >= 1 && e - s >= 1 && i >= e - s - k) v = w;
+            }
+    };
+    double vb = rank == 0 && warp == 0 && n - lane >= 1 ? bg[n - lane - 1] : 0.0;
+    if (rank == 0 && warp == 2) fetch(n, 0);
     __syncthreads();
-    if (owns(n)) {
-        const double x = B(n) / ucol(1)[kp1 - 1];
-        B(n) = x;
-        bg[n - 1] = x;
-        pub[1] = x;
+    int buf = 0;
+    for (int e = n; e >= 1; e -= 32, buf ^= 1) {
+        if (rank > 0) {
+            if (e < n) {
+                const double x = __ldcg(bg + (e + 32 - lane - 1));
+                for (int g = e - 64 - 32 * ((rank - 1) * (kBackThreads / 32) + warp); g >= 1 && g >= e + 1 - k;
+                     g -= 32 * kBackWarps) {
+                    const int i = g - lane;
+                    double v = i >= 1 ? __ldcg(bg + i - 1) : 1.0;
+                    apply(v, i, e + 32, x);
+                    if (i >= 1) bg[i - 1] = v;
+                }
+            }
+        } else if (warp == 0) {
+            double u = tri[buf][0][lane], d = tri[buf][0][0], r = rec[buf][0], mine = 0.0;
+            const unsigned plain = fast[buf];
+#pragma unroll
+            for (int s = 0; s < 32; s++) {
+                const double un = tri[buf][(s + 1) & 31][lane], dn = tri[buf][(s + 1) & 31][(s + 1) & 31],
+                             rn = rec[buf][(s + 1) & 31];
+                if (e - s >= 1) {
+                    const double t = __shfl_sync(0xffffffffu, vb, s);
+                    const double x = in_range(t, 800) && (plain >> s & 1u) ? quotient(t, d, r) : t / d;
+                    xs[buf][s] = x;
+                    if (lane == s) mine = x;
+                    const double w = vb - x * u;
+                    if (lane > s && lane - s <= k) vb = w;
+                }
+                u = un;
+                d = dn;
+                r = rn;
+                // warp 1 follows in pieces of 16, 8, 4, 2, 1 and 1 columns
+                if (s == 15 || s == 23 || s == 27 || s == 29 || s == 30 || s == 31) {
+                    __syncwarp();
+                    named_arrive(s == 15 ? 1 : s == 23 ? 2 : s == 27 ? 3 : s == 29 ? 4 : s == 30 ? 5 : 6);
+                }
+            }
+            if (e - lane >= 1) bg[e - lane - 1] = mine;
+        } else if (warp == 1) {
+            const int i = e - 32 - lane;
+            double v = i >= 1 ? __ldcg(bg + i - 1) : 0.0;
+            if (e < n) apply(v, i, e + 32, xs[buf ^ 1][lane]);
+            double u[32];
+#pragma unroll
+            for (int s = 0; s < 32; s++) u[s] = U(i, e - s);
+#pragma unroll
+            for (int s = 0; s < 32; s++) {
+                if (s == 0 || s == 16 || s == 24 || s == 28 || s == 30 || s == 31)
+                    named_sync(s == 0 ? 1 : s == 16 ? 2 : s == 24 ? 3 : s == 28 ? 4 : s == 30 ? 5 : 6);
+                const double w = v - xs[buf][s] * u[s];
+                if (i >= 1 && e - s >= 1 && i >= e - s - k) v = w;
+            }
+            hand[lane] = v;
+        } else if (warp == 2) {
+            if (e > 32) fetch(e - 32, buf ^ 1);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0 && warp == 0) vb = hand[lane];
     }
-    for (int m = 1; m <= n; m++) {
-        const int j = n - m + 1;
-        ds_wait<kDsAhead - 2>();  // columns j and j - 1
-        __syncthreads();
-        if (pend_i) {  // b(j - k - 1), first used in step j - 1
-            B(pend_i) = pend;
-            pend_i = 0;
-        }
-        const double* U = ucol(m);
-        const double x = pub[m & 1];
-        const int lo = kp1 - j, i0 = 1 > j - k ? 1 : j - k;
-        for (int i = first_owned(i0); i <= j - 1; i += kDsThreads) B(i) = B(i) - x * U[lo + i - 1];
-        if (j >= 2 && owns(j - 1)) {
-            const double x1 = B(j - 1) / ucol(m + 1)[kp1 - 1];
-            B(j - 1) = x1;
-            bg[j - 2] = x1;
-            pub[(m + 1) & 1] = x1;
-        }
-        const int f = j - k - 2;  // first used in step j - 2
-        if (f >= 1 && owns(f)) {
-            pend = bg[f - 1];
-            pend_i = f;
-        }
-        issue_bwd(m + kDsAhead);
-    }
-    ds_wait<0>();
 }
 
 // buoyancy (momentum.f90:258-289): Bvec(p) = (Ra_T T_x - Ra_C C_x) r(p) on interior nodes, 0 on
@@ -581,13 +670,14 @@ int direct_alloc(Engine& E) {
     E.dkl = kl;
     E.dku = ku;
     E.dn = n;
-    // the substitution kernel keeps its window of b and its column ring in shared memory
-    E.dahead = direct_solve_smem(kl, ku, 8) <= 227 * 1024 ? 8 : 2;
-    if (direct_solve_smem(kl, ku, E.dahead) > 227 * 1024)
+    // the forward substitution keeps its ring of columns in shared memory and its window of b in registers
+    if (kl + 2 > 4 * kDsRows)
         return fail(PT_ERR_CONFIG, "direct solve: the band is too wide for the banded substitution kernel");
-    const int smem = (int)direct_solve_smem(kl, ku, E.dahead);
-    if (E.dahead == 8) CK(cudaFuncSetAttribute(k_direct_solve<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    else CK(cudaFuncSetAttribute(k_direct_solve<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (int rc = direct_forward_of(kl, [&](auto kernel, int, size_t smem) {
+            return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                              "direct solve");
+        }))
+        return rc;
     CK(cudaMalloc(&E.dMB, sizeof(double) * (size_t)ldab * (size_t)n));
     CK(cudaMalloc(&E.dRow, sizeof(double) * (size_t)n));
     CK(cudaMalloc(&E.dB, sizeof(double) * (size_t)n));
@@ -673,10 +763,12 @@ int direct_solve(Engine& E, pt_solve_info* info) {
     const int n = E.dn, kl = E.dkl, ku = E.dku;
     PT_COUNT(), k_direct_rhs<<<nblk(n, 128), 128, 0, E.st>>>(E.dB, E.Tbuoy, E.Cbuoy, E.dRow, E.g1, n, E.cfg.comp,
                                                             E.cfg.RaT, E.cfg.RaC);
-    const size_t smem = direct_solve_smem(kl, ku, E.dahead);
-    const int W = direct_window(kl, ku);
-    if (E.dahead == 8) PT_COUNT(), k_direct_solve<8><<<1, kDsThreads, smem, E.st>>>(E.dMB, E.dipiv, E.dB, n, kl, ku, W);
-    else PT_COUNT(), k_direct_solve<2><<<1, kDsThreads, smem, E.st>>>(E.dMB, E.dipiv, E.dB, n, kl, ku, W);
+    if (int rc = direct_forward_of(kl, [&](auto kernel, int threads, size_t smem) {
+            PT_COUNT(), kernel<<<1, threads, smem, E.st>>>(E.dMB, E.dipiv, E.dB, n, kl, ku, FmaForms());
+            return cuda_check(cudaGetLastError(), "k_direct_forward");
+        }))
+        return rc;
+    PT_COUNT(), k_direct_back<<<kBackCtas, kBackThreads, 0, E.st>>>(E.dMB, E.dB, n, kl, ku, FmaForms());
     PT_COUNT(), k_direct_scatter<<<nblk(n, 128), 128, 0, E.st>>>(E.SF, E.dB, E.g1, E.K.nx, E.K.nz);
     PT_COUNT(), k_direct_images_x<<<nblk(3 * (E.K.nz + 1), 128), 128, 0, E.st>>>(E.SF, E.g1, E.K.nx, E.K.nz);
     PT_COUNT(), k_direct_images_z<<<nblk(3 * (E.K.nx + 7), 128), 128, 0, E.st>>>(E.SF, E.g1, E.K.nx, E.K.nz,
