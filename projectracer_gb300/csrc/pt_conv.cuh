@@ -15,14 +15,15 @@
 //     with their channels as the leading dimension (MN-major): the taps of a row are one box at row
 //     offsets 0, 1 and 2, as blocks of M one position apart.
 // What bounds them: on large grids the issue of one MMA per 16 channels (N = 32 takes the 64 cycles that
-// reading the 128 rows takes) beside loads and stores; on small ones a chain of set-up, load latency,
-// MMAs and store, 7 us with the launch.  The forward convolutions of 8 images of 512 x 256: 1338 us with
+// reading the 128 rows takes) beside loads and stores; on small ones a chain of load latency, MMAs and
+// store (set-up and weight loads run while the kernel before ends).  The forward convolutions of 8 images of 512 x 256: 1338 us with
 // a CTA per tile, a box per tap and single threads issuing, now 681; backward-data 1124 and 505, weight
 // gradients 1279 and 640.
 // Every wait is bounded; a timeout sets an error flag and the CTA leaves after its copies have landed.
 #pragma once
 #include <cuda.h>
 
+#include "pt_launch.cuh"
 #include "pt_tc.cuh"
 
 namespace pt {
@@ -224,6 +225,9 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // everything above, and the weights, does not depend on the kernel before this one (a parameter update
+    // is at least two launches back, and a kernel lets its successor start once its predecessor has ended)
+    if (warp != 6) pdl_begin();
     const uint32_t taddr = tslot;
     const int bw0 = a.bw[0], bw1 = a.bw[1], nb0 = a.C[0] / bw0, nblk = nb0 + (a.nsrc > 1 ? a.C[1] / bw1 : 0);
     const int rows = a.taps == 1 ? 1 : 3, steps = a.taps / nd, brows = nd == 3 ? kBoxRows : kTileM;
@@ -433,6 +437,7 @@ __global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_begin();
     const uint32_t taddr = tslot;
     const int cbeg = blockIdx.z * a.per, cend = min(a.chunks, cbeg + a.per), n = max(0, cend - cbeg);
     const int nch = a.C / a.bw, unit = blockIdx.x / nch, ch = (blockIdx.x - unit * nch) * a.bw;

@@ -12,6 +12,7 @@
 #include "pt_internal.h"
 #include "../../include/ptgpu_unet.h"
 #include "pt_conv.cuh"
+#include "pt_launch.cuh"
 #include <cuda_bf16.h>
 
 namespace pt {
@@ -55,6 +56,7 @@ constexpr int kImCols = 64;  // columns of the first layer's im2col rows: 36 val
 // the network input, NCHW FP32, as im2col rows in BF16 at the padded positions: 8 columns a thread
 // (columns 40..63 stay zero from allocation)
 __global__ void k_im2col(uint16_t* __restrict__ o, const float* __restrict__ x, PadGeo g) {
+    pdl_begin();
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x, n = (size_t)g.B * g.H * g.W;
     if (q >= 5 * n) return;
     const int j = (int)(q / n);
@@ -87,6 +89,7 @@ __device__ __forceinline__ bool octet(size_t q, const PadGeo& g, int C, int& b, 
 
 // 2x2 average of a tensor at twice the resolution, ((a+b)+c)+d in FP32
 __global__ void k_pool(uint16_t* __restrict__ o, const uint16_t* __restrict__ in, PadGeo g, PadGeo gf, int C) {
+    pdl_begin();
     int b, y, x, c;
     if (!octet((size_t)blockIdx.x * blockDim.x + threadIdx.x, g, C, b, y, x, c)) return;
     const uint16_t* p = in + gf.at(b, 2 * y, 2 * x) * C + c;
@@ -171,31 +174,44 @@ __global__ void k_pack_weights(uint16_t* __restrict__ wbd, uint16_t* __restrict_
     }
 }
 
-// dW[co][kk] = sum_z part[z][kk][co]: a warp adds every eighth split of 32 weights (eight loads in flight),
-// then the eight sums are added in order; with two sources the rows' channels below c0 have nsplit0 partial
-// sums, the others nsplit1
-__global__ void __launch_bounds__(256) k_wgrad_reduce(float* dW, const float* __restrict__ part, int nsplit0, int nsplit1,
-                                                      int c0, int cin, int M, int N) {
+// All layers' weight gradients from the splits' partial sums, dW[co][kk] = sum_z part[z][kk][co]: a warp adds
+// every eighth split of 32 weights (eight loads in flight), then the eight sums are added in order; with two
+// sources the rows' channels below c0 have ns0 partial sums, the others ns1.  One launch for the network:
+// a launch per layer lasted longer than its reads.
+struct ReduceArgs {
+    struct Layer {
+        float* dW;
+        const float* part;
+        int ns0, ns1, c0, cin, M, N, block0;  // block0: its first block
+    } l[14];
+};
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const __grid_constant__ ReduceArgs a) {
+    pdl_begin();
     __shared__ float sh[8][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;  // N % 32 == 0
-    const int kk = q / N, co = q % N, nsplit = kk % cin < c0 ? nsplit0 : nsplit1;
-    const size_t ld = (size_t)M * N;
+    int li = 13;
+    while (li > 0 && (int)blockIdx.x < a.l[li].block0) li--;
+    const ReduceArgs::Layer& L = a.l[li];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = ((int)blockIdx.x - L.block0) * 32 + lane, kk = q / L.N, co = q - kk * L.N;  // N % 32 == 0
+    const int ns = kk % L.cin < L.c0 ? L.ns0 : L.ns1;
+    const size_t ld = (size_t)L.M * L.N;
+    const float* part = L.part + q;
     float s = 0.f;
     int z = warp;
-    for (; z + 56 < nsplit; z += 64) {
+    for (; z + 56 < ns; z += 64) {
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = part[(size_t)(z + 8 * j) * ld + q];
+        for (int j = 0; j < 8; j++) v[j] = part[(size_t)(z + 8 * j) * ld];
 #pragma unroll
         for (int j = 0; j < 8; j++) s += v[j];
     }
-    for (; z < nsplit; z += 8) s += part[(size_t)z * ld + q];
+    for (; z < ns; z += 8) s += part[(size_t)z * ld];
     sh[warp][lane] = s;
     __syncthreads();
     if (warp) return;
 #pragma unroll
     for (int j = 1; j < 8; j++) s += sh[j][lane];
-    dW[(size_t)co * M + kk] = s;
+    L.dW[(size_t)co * L.M + kk] = s;
 }
 
 // Gradient of a layer's pre-activation as a GEMM operand, dZ = dY masked by Y > 0 in BF16, and per-block
@@ -207,7 +223,7 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(float* dW, const float* __
 //   out     the output layer: dy w[c]; the partial sums of its own weights' gradients too
 // One pass over the tensor, bound by its bytes (FP32 in, two BF16 tensors in and out).
 enum { kDzPlain = 0, kDzPooled, kDzUp, kDzOut };
-constexpr int kDzThreads = 256;
+constexpr int kDzThreads = 256, kDzBlocks = 4 * tc::kSms;
 struct DzArgs {
     PadGeo g, g2;  // of the layer, and of the other resolution (pooled: coarse, up: fine)
     int C;
@@ -222,6 +238,7 @@ struct DzArgs {
 };
 template <int MODE>
 __global__ void __launch_bounds__(kDzThreads) k_dz(DzArgs a) {
+    pdl_begin();
     constexpr int NV = MODE == kDzOut ? 2 : 1;
     __shared__ float sh[NV * 8][kDzThreads + 1];
     __shared__ float shb[kDzThreads];
@@ -295,18 +312,33 @@ __global__ void __launch_bounds__(kDzThreads) k_dz(DzArgs a) {
         a.part[(size_t)blockIdx.x * nout + o] = s;
     }
 }
-// out[c] = sum over blocks of part[block][off + c]: a warp a column, fixed order
-__global__ void k_colsum(float* out, const float* part, int blocks, int ld, int off, int n) {
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (c >= n) return;
+// All layers' bias gradients (and the output layer's weights and bias) from the blocks' partial sums: a warp
+// per column, lanes over blocks, then a fixed shuffle tree
+struct ColsumArgs {
+    struct Layer {
+        float* out;
+        const float* part;
+        int blocks, ld, off, n, col0;  // col0: its first column among all
+    } l[15];
+    int total;
+};
+__global__ void __launch_bounds__(128) k_colsum(const __grid_constant__ ColsumArgs a) {
+    pdl_begin();
+    const int col = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (col >= a.total) return;
+    int li = 14;
+    while (li > 0 && col < a.l[li].col0) li--;
+    const ColsumArgs::Layer& L = a.l[li];
+    const int c = col - L.col0;
     float s = 0.f;
-    for (int b = lane; b < blocks; b += 32) s += part[(size_t)b * ld + off + c];
+    for (int b = lane; b < L.blocks; b += 32) s += L.part[(size_t)b * L.ld + L.off + c];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[c] = s;
+    if (lane == 0) L.out[c] = s;
 }
 
 // 1x1 output convolution (linear, FP32 out)
 __global__ void k_out_fwd(float* y, const uint16_t* d, const float* w, const float* b, PadGeo g) {
+    pdl_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= g.B * g.H * g.W) return;
     const int x = p % g.W, r = p / g.W;
@@ -323,6 +355,7 @@ __global__ void k_out_fwd(float* y, const uint16_t* d, const float* w, const flo
 }
 // loss = mean (y - t)^2; dy = 2 (y - t) / P; per-block partial sums of (y - t)^2
 __global__ void k_mse(float* dy, float* lpart, const float* y, const float* t, int P) {
+    pdl_begin();
     __shared__ float sh[256];
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     float e = 0.f;
@@ -399,7 +432,7 @@ struct UNet {
     float *dx = nullptr, *dxcat[14] = {};  // a view's gradient; of the concatenated views, kept for the skips
     float *xin = nullptr, *y = nullptr, *dy = nullptr, *tgt = nullptr, *lpart = nullptr, *part = nullptr,
           *bpart = nullptr;
-    size_t part_cap = 0;
+    size_t part_cap = 0, part_off[14] = {}, bpart_off[15] = {};  // of a layer's partial sums in part, in bpart
     int planB = 0;  // batch size of the plans
     LayerPlan plan[14];
     int* derr = nullptr;
@@ -454,6 +487,21 @@ static WgradShape wgrad_shape(int taps, int C, int cout, size_t positions) {
     w.per = (chunks + n0 - 1) / n0;
     w.ns = (chunks + w.per - 1) / w.per;
     return w;
+}
+
+// where the layers' partial sums of a batch lie in U.part; their total
+static size_t layout_partials(UNet& U, int B) {
+    size_t n = 0;
+    for (size_t li = 0; li < U.L.size(); li++) {
+        const UConv& c = U.L[li];
+        const int C0 = c.src0 < 0 ? kImCols : U.tch[c.src0], C1 = c.mode == 2 ? U.tch[c.src1] : 0;
+        int ns = 0;
+        for (int C : {C0, C1})
+            if (C) ns = std::max(ns, wgrad_shape(c.src0 < 0 ? 1 : 9, C, c.cout, U.geo(c.level, B).positions()).ns);
+        U.part_off[li] = n;
+        n += (size_t)ns * 9 * c.cin * c.cout;
+    }
+    return n;
 }
 
 static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
@@ -516,15 +564,13 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
         } else {
             dx = std::max(dx, n(c.level, c.cin));
         }
-        const int C0 = c.src0 < 0 ? kImCols : U.tch[c.src0], C1 = c.mode == 2 ? U.tch[c.src1] : 0;
-        for (int B = 1; B <= maxB; B++)  // (a smaller batch may have more splits)
-            for (int C : {C0, C1}) {
-                if (C == 0) continue;
-                const WgradShape w = wgrad_shape(c.src0 < 0 ? 1 : 9, C, c.cout, U.geo(c.level, B).positions());
-                part = std::max(part, (size_t)w.ns * 9 * c.cin * c.cout);
-            }
     }
-    bpart = (size_t)4 * 152 * 256;
+    for (int B = 1; B <= maxB; B++)  // (a smaller batch may have more splits)
+        part = std::max(part, layout_partials(U, B));
+    for (size_t li = 0; li < U.L.size(); li++) {
+        U.bpart_off[li] = bpart;
+        bpart += (size_t)kDzBlocks * (li == 13 ? 2 * U.L[li].cout + 1 : U.L[li].cout);
+    }
     U.part_cap = part;
     const size_t P0 = (size_t)maxB * H * W;
     if ((rc = ualloc(U, &U.im, n(0, kImCols))) || (rc = ualloc(U, &U.xin, P0 * 4)) || (rc = ualloc(U, &U.y, P0)) ||
@@ -621,6 +667,7 @@ static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* 
 static int plan_batch(UNet& U, int B) {
     if (U.planB == B) return 0;
     U.planB = 0;
+    if (layout_partials(U, B) > U.part_cap) return fail(PT_ERR_STATE, "U-Net: split workspace too small");
     int rc;
     for (size_t li = 0; li < U.L.size(); li++) {
         const UConv& c = U.L[li];
@@ -640,8 +687,6 @@ static int plan_batch(UNet& U, int B) {
             tc::WgradArgs& a = w.a;
             const WgradShape sh = wgrad_shape(first ? 1 : 9, C[s], c.cout, g.positions());
             P.nsplit[s] = sh.ns;
-            if ((size_t)sh.ns * 9 * c.cin * c.cout > U.part_cap)
-                return fail(PT_ERR_STATE, "U-Net: split workspace too small");
             a.g = g;
             a.taps = first ? 1 : 9;
             a.C = C[s];
@@ -657,7 +702,7 @@ static int plan_batch(UNet& U, int B) {
             a.ncols = (int)tc::tmem_cols((first || a.bw == 32 ? 1 : 2) * a.Ntile);
             a.abytes = tc::wgrad_box_bytes(a.bw);
             a.bbytes = a.Ntile * tc::kWgradK * 2;
-            a.part = U.part;
+            a.part = U.part + U.part_off[li];
             w.grid = dim3(sh.units, c.cout / a.Ntile, sh.ns);
             a.S = std::min(std::min(110 * 1024 / (a.abytes + a.bbytes), tc::kMaxRing), sh.per);  // two CTAs on an SM
             if ((rc = tensor_map(&w.A, t[s], C[s], g.positions(), a.bw, tc::kWgradBox)) ||
@@ -671,9 +716,8 @@ static int plan_batch(UNet& U, int B) {
 
 template <class E>
 static int run_conv(UNet& U, const ConvPlan& P, const E& e) {
-    tc::k_conv_gemm<E><<<P.grid, tc::kConvThreads, tc::conv_smem(P.a), U.st>>>(P.A[0], P.A[1], P.B[0], P.B[1], P.a, e,
-                                                                                U.derr);
-    return cuda_check(cudaGetLastError(), "k_conv_gemm");
+    return launch_pdl("k_conv_gemm", tc::k_conv_gemm<E>, P.grid, dim3(tc::kConvThreads), tc::conv_smem(P.a), U.st, P.A[0],
+                      P.A[1], P.B[0], P.B[1], P.a, e, U.derr);
 }
 
 // network input already in U.xin (device, NCHW FP32); output in U.y ([B][H][W] FP32).
@@ -682,25 +726,25 @@ static int unet_forward(UNet& U, int B, cudaEvent_t* ev = nullptr) {
     const size_t P0 = (size_t)B * U.H * U.W;
     int rc;
     if ((rc = plan_batch(U, B))) return rc;
-    k_im2col<<<nblk(P0 * 5, 256), 256, 0, U.st>>>(U.im, U.xin, U.geo(0, B));
-    CK(cudaGetLastError());
+    if ((rc = launch_pdl("k_im2col", k_im2col, dim3(nblk(P0 * 5, 256)), dim3(256), 0, U.st, U.im, U.xin, U.geo(0, B))))
+        return rc;
     int li = 0;
     if (ev) CK(cudaEventRecord(ev[0], U.st));
     for (auto& c : U.L) {
         if (c.mode == 1) {
             const PadGeo g = U.geo(c.level, B);
             const size_t n = (size_t)B * g.H * g.W * (c.cin / 8);
-            k_pool<<<nblk(n, 256), 256, 0, U.st>>>(U.pool[c.src0], U.act[c.src0], g, U.geo(c.level - 1, B), c.cin);
-            CK(cudaGetLastError());
+            if ((rc = launch_pdl("k_pool", k_pool, dim3(nblk(n, 256)), dim3(256), 0, U.st, U.pool[c.src0], U.act[c.src0], g,
+                                 U.geo(c.level - 1, B), c.cin)))
+                return rc;
         }
         const FwdEpi e{U.act[c.out], U.w32 + c.boff, c.cout, U.up[c.out], U.geo(c.level > 0 ? c.level - 1 : 0, B)};
         if ((rc = run_conv(U, U.plan[li].fwd, e))) return rc;
         li++;
         if (ev) CK(cudaEventRecord(ev[li], U.st));
     }
-    k_out_fwd<<<nblk(P0, 128), 128, 0, U.st>>>(U.y, U.act[13], U.w32 + U.out_w, U.w32 + U.out_b, U.geo(0, B));
-    CK(cudaGetLastError());
-    return 0;
+    return launch_pdl("k_out_fwd", k_out_fwd, dim3(nblk(P0, 128)), dim3(128), 0, U.st, U.y, U.act[13], U.w32 + U.out_w,
+                      U.w32 + U.out_b, U.geo(0, B));
 }
 
 static int gemm_error(UNet& U) {
@@ -711,7 +755,11 @@ static int gemm_error(UNet& U) {
     return 0;
 }
 
-// dZ of the layer that produced tensor t from where its gradient lies, and that layer's bias gradient
+static int dz_blocks(const UNet& U, const UConv& c, int B) {
+    const size_t oct = (size_t)B * (U.H >> c.level) * (U.W >> c.level) * (c.cout / 8);
+    return (int)std::min<size_t>(nblk(oct, 4 * kDzThreads), kDzBlocks);
+}
+// dZ of the layer that produced tensor t from where its gradient lies, and the partial sums of its bias gradient
 template <int MODE>
 static int run_dz(UNet& U, int t, int B, DzArgs a) {
     const UConv& c = U.L[t];  // (tensor t is layer t's output)
@@ -719,15 +767,8 @@ static int run_dz(UNet& U, int t, int B, DzArgs a) {
     a.C = c.cout;
     a.Y = U.act[t];
     a.dZ = U.dz[t];
-    a.part = U.bpart;
-    const size_t oct = (size_t)B * a.g.H * a.g.W * (c.cout / 8);
-    const int blocks = (int)std::min<size_t>(nblk(oct, 4 * kDzThreads), 4 * 152);
-    k_dz<MODE><<<blocks, kDzThreads, 0, U.st>>>(a);
-    const int ld = MODE == kDzOut ? 2 * c.cout + 1 : c.cout;
-    k_colsum<<<nblk(c.cout, 4), 128, 0, U.st>>>(U.g + c.boff, U.bpart, blocks, ld, 0, c.cout);
-    if (MODE == kDzOut)  // (the output layer's weights and bias lie next to each other)
-        k_colsum<<<nblk(c.cout + 1, 4), 128, 0, U.st>>>(U.g + U.out_w, U.bpart, blocks, ld, c.cout, c.cout + 1);
-    return cuda_check(cudaGetLastError(), "k_dz");
+    a.part = U.bpart + U.bpart_off[t];
+    return launch_pdl("k_dz", k_dz<MODE>, dim3(dz_blocks(U, c, B)), dim3(kDzThreads), 0, U.st, a);
 }
 
 // gradients of the MSE loss against U.tgt into U.g; loss on the host
@@ -735,8 +776,8 @@ static int unet_backward(UNet& U, int B, float* loss) {
     const int P0 = B * U.H * U.W;
     const int nb = (int)nblk(P0, 256);
     int rc;
-    k_mse<<<nb, 256, 0, U.st>>>(U.dy, U.lpart, U.y, U.tgt, P0);
-    CK(cudaGetLastError());
+    ReduceArgs red{};
+    if ((rc = launch_pdl("k_mse", k_mse, dim3(nb), dim3(256), 0, U.st, U.dy, U.lpart, U.y, U.tgt, P0))) return rc;
     DzArgs o{};
     o.dx = U.dy;
     o.w = U.w32 + U.out_w;
@@ -744,14 +785,14 @@ static int unet_backward(UNet& U, int B, float* loss) {
     for (int li = (int)U.L.size() - 1; li >= 0; li--) {
         const UConv& c = U.L[li];
         const LayerPlan& P = U.plan[li];
-        // weights: split over positions, then a fixed-order reduction of the splits
-        const int Mw = 9 * c.cin;
+        // weights: split over positions; the splits are added at the end, for all layers
+        const int M = 9 * c.cin;
+        red.l[li] = {U.g + c.woff, U.part + U.part_off[li], P.nsplit[0], P.nsplit[1], P.nwg > 1 ? P.wg[0].a.C : M,
+                     P.nwg > 1 ? c.cin : M, M, c.cout, 0};
         for (int s = 0; s < P.nwg; s++)
-            tc::k_wgrad_gemm<<<P.wg[s].grid, tc::kWgradThreads, tc::wgrad_smem(P.wg[s].a), U.st>>>(P.wg[s].A, P.wg[s].B,
-                                                                                                  P.wg[s].a, U.derr);
-        k_wgrad_reduce<<<(unsigned)(Mw * c.cout / 32), 256, 0, U.st>>>(
-            U.g + c.woff, U.part, P.nsplit[0], P.nsplit[1], P.nwg > 1 ? P.wg[0].a.C : Mw, P.nwg > 1 ? c.cin : Mw, Mw, c.cout);
-        CK(cudaGetLastError());
+            if ((rc = launch_pdl("k_wgrad_gemm", tc::k_wgrad_gemm, P.wg[s].grid, dim3(tc::kWgradThreads),
+                                 tc::wgrad_smem(P.wg[s].a), U.st, P.wg[s].A, P.wg[s].B, P.wg[s].a, U.derr)))
+                return rc;
         if (c.src0 < 0) continue;  // the network input needs no gradient
         float* dx = c.mode == 2 ? U.dxcat[c.out] : U.dx;
         if ((rc = run_conv(U, P.bwd, DxEpi{dx, c.cin}))) return rc;
@@ -775,12 +816,32 @@ static int unet_backward(UNet& U, int B, float* loss) {
         }
         if (rc) return rc;
     }
+    int blocks = 0, cols = 0;
+    ColsumArgs sum{};
+    for (int li = 0; li < 14; li++) {
+        const UConv& c = U.L[li];
+        red.l[li].block0 = blocks;
+        blocks += red.l[li].M * red.l[li].N / 32;
+        sum.l[li] = {U.g + c.boff, U.bpart + U.bpart_off[li], dz_blocks(U, c, B), li == 13 ? 2 * c.cout + 1 : c.cout, 0,
+                     c.cout, cols};
+        cols += c.cout;
+    }
+    // (the output layer's weights and bias lie next to each other)
+    sum.l[14] = sum.l[13];
+    sum.l[14].out = U.g + U.out_w;
+    sum.l[14].off = U.L[13].cout;
+    sum.l[14].n = U.L[13].cout + 1;
+    sum.l[14].col0 = cols;
+    sum.total = cols + sum.l[14].n;
+    if ((rc = launch_pdl("k_wgrad_reduce", k_wgrad_reduce, dim3(blocks), dim3(256), 0, U.st, red)) ||
+        (rc = launch_pdl("k_colsum", k_colsum, dim3(nblk(sum.total, 4)), dim3(128), 0, U.st, sum)))
+        return rc;
     std::vector<float> lp(nb);
     CK(cudaMemcpyAsync(lp.data(), U.lpart, sizeof(float) * nb, cudaMemcpyDeviceToHost, U.st));
     if ((rc = gemm_error(U))) return rc;
-    double sum = 0.0;
-    for (float a : lp) sum += a;
-    if (loss) *loss = (float)(sum / P0);
+    double err = 0.0;
+    for (float a : lp) err += a;
+    if (loss) *loss = (float)(err / P0);
     return 0;
 }
 
