@@ -1,4 +1,5 @@
-// pt_bandlu.cuh -- LU of the coarse band matrix with partial pivoting (DGBTF2's operations, in panels).
+// pt_bandlu.cuh -- LU of the coarse band matrix with partial pivoting (DGBTF2's operations, in panels), and its
+// explicit inverse.
 //
 // A panel of kPanel columns is factored by one CTA in shared memory (k_band_panel), then every column to
 // its right that the panel reaches takes the panel's row interchanges, multipliers and updates in a CTA of
@@ -9,6 +10,7 @@
 // pivot search, reciprocal, scaling and the update of the next column.
 // n = 2145, kl = ku = 99: 26 -> 3.2 ms; n = 561, kl = ku = 51: 2.2 -> 0.9 ms.
 #pragma once
+#include "pt_fp64.cuh"
 #include "pt_launch.cuh"
 
 namespace pt {
@@ -16,19 +18,28 @@ namespace bandlu {
 
 constexpr int kPanel = 16;
 
-// what a panel leaves for the columns to its right: multipliers L[jj][r] in the rows' final order (r counts
-// from the panel's first row), perm[r] = the row that ends at r, and the last column it reaches (1-based,
-// the running maximum)
+// what panels leave for the columns to their right and for the inverse: per panel multipliers L[jj][r] in the
+// rows' final order (r counts from the panel's first row), perm[r] = the row that ends at r, and top, the
+// first row in which its columns of U have an entry; and the last column reached so far (1-based)
 struct Work {
     double* L;
-    int *perm, *ju;
+    int *perm, *top, *ju;
+    int LD;  // kl + kPanel
+    __host__ __device__ double* l(int panel) const { return L + (size_t)panel * kPanel * LD; }
+    __host__ __device__ int* p(int panel) const { return perm + (size_t)panel * LD; }
 };
-static inline size_t work_bytes(int kl) { return sizeof(double) * kPanel * (kl + kPanel) + sizeof(int) * (kl + kPanel + 1); }
-static inline Work work_of(void* base, int kl) {
+static inline int panels(int n) { return (n + kPanel - 1) / kPanel; }
+static inline size_t work_bytes(int n, int kl) {
+    const size_t rows = (size_t)panels(n) * (kl + kPanel);
+    return sizeof(double) * kPanel * rows + sizeof(int) * (rows + panels(n) + 1);
+}
+static inline Work work_of(void* base, int n, int kl) {
     Work w;
+    w.LD = kl + kPanel;
     w.L = static_cast<double*>(base);
-    w.perm = reinterpret_cast<int*>(w.L + (size_t)kPanel * (kl + kPanel));
-    w.ju = w.perm + kl + kPanel;
+    w.perm = reinterpret_cast<int*>(w.L + (size_t)panels(n) * kPanel * w.LD);
+    w.top = w.perm + (size_t)panels(n) * w.LD;
+    w.ju = w.top + panels(n);
     return w;
 }
 static inline int row_threads(int kl) { return (kl + kPanel + 31) / 32 * 32; }
@@ -151,8 +162,8 @@ __global__ void __launch_bounds__(512) k_band_panel(double* ab, int* ipiv, int n
     if (warp < nw) {
 #pragma unroll
         for (int c = 0; c < kPanel; c++)
-            if (r < R) w.L[(size_t)c * LD + r] = r > c && (usable >> c & 1u) ? v[c] : 0.0;
-        if (r < R) w.perm[r] = id;
+            if (r < R) w.l(j0 / kPanel)[(size_t)c * LD + r] = r > c && (usable >> c & 1u) ? v[c] : 0.0;
+        if (r < R) w.p(j0 / kPanel)[r] = id;
     } else if (lane == 0) {
         *w.ju = max(*w.ju, ju);
     }
@@ -168,15 +179,16 @@ __global__ void __launch_bounds__(512) k_band_trail(double* ab, int n, int kl, i
     double* const col = ab + (size_t)c * ldab + kv + j0 - c;  // row j0 + r at col[r], stored from r >= r0
     const int r0 = c - kv - j0;
     auto load = [&](int r) {
-        const int q = w.perm[r];
+        const int q = w.p(j0 / kPanel)[r];
         return q >= r0 ? col[q] : 0.0;
     };
     double t = lane < kPanel ? load(lane) : 0.0, v = tid >= kPanel && tid < R ? load(tid) : 0.0;
     double lt[kPanel], lv[kPanel];
+    const double* const wl = w.l(j0 / kPanel);
 #pragma unroll
     for (int jj = 0; jj < kPanel; jj++) {
-        lt[jj] = lane < kPanel ? w.L[(size_t)jj * LD + lane] : 0.0;
-        lv[jj] = tid >= kPanel && tid < R ? w.L[(size_t)jj * LD + tid] : 0.0;
+        lt[jj] = lane < kPanel ? wl[(size_t)jj * LD + lane] : 0.0;
+        lv[jj] = tid >= kPanel && tid < R ? wl[(size_t)jj * LD + tid] : 0.0;
     }
     __syncthreads();
 #pragma unroll
@@ -206,6 +218,207 @@ static int factor(double* ab, int* ipiv, int n, int kl, int ku, const Work& w, i
             return rc;
     }
     return 0;
+}
+
+// ---- explicit inverse G = (P L U)^{-1}, row-major, so that the coarse solve is a coalesced GEMV
+
+// the first row in which a panel's columns of U have an entry (kv rows above the diagonal are stored, of
+// which interchanges that did not happen leave the upper kl zero)
+__global__ void k_band_top(const double* ab, int n, int kl, int ku, Work w) {
+    const int ldab = 2 * kl + ku + 1, kv = ku + kl, j0 = blockIdx.x * kPanel;
+    __shared__ int top;
+    if (threadIdx.x == 0) top = j0;
+    __syncthreads();
+    for (int c = j0; c < min(j0 + kPanel, n); c++)
+        for (int i = max(0, c - kv) + threadIdx.x; i < j0; i += blockDim.x)
+            if (nonzero(ab[(size_t)c * ldab + kv + i - c])) {
+                atomicMin(&top, i);
+                break;  // (a thread's rows ascend)
+            }
+    __syncthreads();
+    if (threadIdx.x == 0) w.top[blockIdx.x] = top;
+}
+
+// COLS columns of G per CTA: unit vectors through the panels' interchanges, multipliers and updates, then
+// back through U, the operations of the column-by-column DGBTRS in the same order for every element.  Per
+// panel the kPanel x kPanel triangle is solved with a lane per row (two columns per warp), the other rows
+// with COLS / 4 threads per row, four columns each.  The window of rows that a panel reaches is in shared
+// memory, twice for the forward pass, whose interchanges permute it.
+// What bounds it is the FP64 rate (n^2 (kl / 2 + ku) multiply-subtract pairs): n = 2145, kl = ku = 99:
+// 11.2 ms with a warp per column (a division per column and step, partly filled warps, the zeros of U
+// above its entries), 6.5 now; n = 561, kl = ku = 51: 0.65 before and now.
+constexpr int kInvThreads = 256, kInvCols = 4;  // columns of a thread
+static inline int pow2_above(int v) {
+    int w = 32;
+    while (w < v) w *= 2;
+    return w;
+}
+static inline size_t inverse_smem(int kl, int ku, int cols) {
+    const int f = 2 * pow2_above(kl + 2 * kPanel), b = pow2_above(kl + ku + 2 * kPanel);
+    return sizeof(double) * (size_t)(f > b ? f : b) * cols;
+}
+template <int COLS>
+__global__ void __launch_bounds__(kInvThreads, 2) k_band_inverse(const double* __restrict__ ab, double* G, int n, int kl, int ku,
+                                                            Work w, int tops, int WF, int WB, FmaForms F) {
+    constexpr int H = COLS / kInvCols;  // threads per row
+    extern __shared__ __align__(16) double win[];
+    __shared__ __align__(16) double ys[kPanel][COLS];
+    __shared__ double ut[2][kPanel][kPanel], rec[2][kPanel];  // ut[.][jj][r] = U(j0 + r, j0 + jj)
+    const int ldab = 2 * kl + ku + 1, kv = ku + kl, LD = w.LD, np = (n + kPanel - 1) / kPanel;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = blockIdx.x * COLS;
+    const int row = lane & 15, col = 2 * warp + (lane >> 4);  // of the triangle: warps below COLS / 2
+    const bool tri = warp < COLS / 2, live = tri && c0 + col < n;
+    const int h4 = (tid % H) * kInvCols;
+
+    // forward
+    const int ps = max(0, (c0 - LD + kPanel) / kPanel);  // the first panel that reaches row c0
+    for (int q = tid; q < min(ps * kPanel, n) * COLS; q += kInvThreads)
+        if (c0 + q % COLS < n) G[(size_t)(q / COLS) * n + c0 + q % COLS] = 0.0;
+    double* A = win;                      // the panel's window, row i in slot i mod WF
+    double* B = win + (size_t)WF * COLS;  // the next one's
+    auto enter = [&](double* W, int from, int to) {
+        for (int q = from * COLS + tid; q < to * COLS; q += kInvThreads)
+            W[(size_t)(q / COLS & (WF - 1)) * COLS + q % COLS] = q / COLS == c0 + q % COLS ? 1.0 : 0.0;
+    };
+    enter(A, ps * kPanel, min(n, ps * kPanel + LD));
+    __syncthreads();
+    for (int p = ps; p < np; p++) {
+        const int j0 = p * kPanel, R = min(LD, n - j0), nb = min(kPanel, n - j0);
+        const double* const L = w.l(p);
+        const int* const perm = w.p(p);
+        double l[kPanel];
+        int it = tid;  // item: row kPanel + it / H, columns h4 ..
+        const int items = max(0, R - kPanel) * H;
+        auto load = [&](int r) {
+#pragma unroll
+            for (int jj = 0; jj < kPanel; jj++) l[jj] = L[(size_t)jj * LD + r];
+        };
+        if (tri) {
+            double t = row < nb ? A[(size_t)((j0 + perm[row]) & (WF - 1)) * COLS + col] : 0.0;
+            if (row < nb) load(row);
+#pragma unroll
+            for (int jj = 0; jj < kPanel; jj++) {
+                const double y = __shfl_sync(0xffffffffu, t, jj + (lane & 16));
+                const double u = F.add(t, F.mul(l[jj], -y));
+                if (row > jj && row < nb) t = u;
+            }
+            ys[row][col] = t;
+            if (live && row < nb) G[(size_t)(j0 + row) * n + c0 + col] = t;
+        }
+        if (it < items) load(kPanel + it / H);
+        __syncthreads();
+        for (; it < items; it += kInvThreads) {
+            const int r = kPanel + it / H;
+            if (it != tid) load(r);
+            const double* a = A + (size_t)((j0 + perm[r]) & (WF - 1)) * COLS + h4;
+            double v[kInvCols];
+#pragma unroll
+            for (int c = 0; c < kInvCols; c++) v[c] = a[c];
+#pragma unroll
+            for (int jj = 0; jj < kPanel; jj++) {
+                const volatile double* y = &ys[jj][h4];  // (volatile: 64 values loaded ahead would fill the registers)
+#pragma unroll
+                for (int c = 0; c < kInvCols; c++) v[c] = F.add(v[c], F.mul(l[jj], -y[c]));
+            }
+            double* b = B + (size_t)((j0 + r) & (WF - 1)) * COLS + h4;
+#pragma unroll
+            for (int c = 0; c < kInvCols; c++) b[c] = v[c];
+        }
+        enter(B, min(n, j0 + LD), min(n, j0 + kPanel + LD));
+        __syncthreads();
+        double* const x = A;
+        A = B;
+        B = x;
+    }
+
+    // back: row i in slot i mod WB
+    auto fetch = [&](int p, int buf) {  // a panel's triangle: threads 0 .. 255, (jj, r)
+        const int jj = tid / kPanel, r = tid % kPanel, j = p * kPanel + jj;
+        const double u = j < n && r <= jj ? ab[(size_t)j * ldab + kv + r - jj] : 1.0;
+        ut[buf][jj][r] = u;
+        if (r == jj) rec[buf][jj] = 1.0 / u;
+    };
+    int lo = max(0, (np - 1) * kPanel - kv);  // rows lo .. are in the window
+    for (int q = lo * COLS + tid; q < n * COLS; q += kInvThreads)
+        win[(size_t)(q / COLS & (WB - 1)) * COLS + q % COLS] = c0 + q % COLS < n ? G[(size_t)(q / COLS) * n + c0 + q % COLS] : 0.0;
+    fetch(np - 1, 0);
+    __syncthreads();
+    for (int p = np - 1, buf = 0; p >= 0; p--, buf ^= 1) {
+        const int j0 = p * kPanel, nb = min(kPanel, n - j0), top = tops ? w.top[p] : max(0, j0 - kv);
+        double u[kPanel];
+        auto load = [&](int i) {
+#pragma unroll
+            for (int jj = 0; jj < kPanel; jj++)
+                u[jj] = j0 + jj < n && i >= j0 + jj - kv ? ab[(size_t)(j0 + jj) * ldab + kv + i - j0 - jj] : 0.0;
+        };
+        // rows that enter for the next panel
+        const int next = max(0, j0 - kPanel - kv), entering = (lo - next) * COLS;
+        double e = 0.0;
+        if (tid < entering && c0 + tid % COLS < n) e = G[(size_t)(next + tid / COLS) * n + c0 + tid % COLS];
+        int it = tid;  // item: row top + it / H
+        const int items = (j0 - top) * H;
+        if (it < items) load(top + it / H);
+        if (tri) {
+            double t = row < nb ? win[(size_t)((j0 + row) & (WB - 1)) * COLS + col] : 0.0;
+#pragma unroll
+            for (int jj = kPanel - 1; jj >= 0; jj--) {
+                if (jj >= nb) continue;
+                const double y = __shfl_sync(0xffffffffu, t, jj + (lane & 16)), d = ut[buf][jj][jj];
+                double x = y;
+                if (nonzero(y)) x = in_range(y, 800) && in_range(d, 100) ? quotient(y, d, rec[buf][jj]) : y / d;
+                __syncwarp();
+                const double s = F.sub(t, F.mul(x, ut[buf][jj][row]));
+                if (row < jj) t = s;
+                if (row == jj) t = x;
+            }
+            ys[row][col] = row < nb ? t : 0.0;
+            if (live && row < nb) G[(size_t)(j0 + row) * n + c0 + col] = t;
+        }
+        if (p > 0) fetch(p - 1, buf ^ 1);
+        __syncthreads();
+        for (; it < items; it += kInvThreads) {
+            const int i = top + it / H;
+            if (it != tid) load(i);
+            double* a = win + (size_t)(i & (WB - 1)) * COLS + h4;
+            double v[kInvCols];
+#pragma unroll
+            for (int c = 0; c < kInvCols; c++) v[c] = a[c];
+#pragma unroll
+            for (int jj = kPanel - 1; jj >= 0; jj--) {
+                const volatile double* y = &ys[jj][h4];
+#pragma unroll
+                for (int c = 0; c < kInvCols; c++) v[c] = F.sub(v[c], F.mul(y[c], u[jj]));
+            }
+#pragma unroll
+            for (int c = 0; c < kInvCols; c++) a[c] = v[c];
+        }
+        if (tid < entering) win[(size_t)((next + tid / COLS) & (WB - 1)) * COLS + tid % COLS] = e;
+        lo = next;
+        __syncthreads();
+    }
+}
+
+// eight columns per CTA where that leaves more than one CTA per SM, else four
+static int inverse(const double* ab, double* G, int n, int kl, int ku, const Work& w, cudaStream_t st) {
+    const int WF = pow2_above(kl + 2 * kPanel), WB = pow2_above(kl + ku + 2 * kPanel);
+    const int tops = n > 256;  // (a launch costs more than a small band's zeros)
+    if (tops) PT_COUNT(), k_band_top<<<panels(n), 128, 0, st>>>(ab, n, kl, ku, w);
+    if (n > 8 * 152)
+        PT_COUNT(), k_band_inverse<8><<<(n + 7) / 8, kInvThreads, inverse_smem(kl, ku, 8), st>>>(ab, G, n, kl, ku, w, tops,
+                                                                                              WF, WB, FmaForms());
+    else
+        PT_COUNT(), k_band_inverse<4><<<(n + 3) / 4, kInvThreads, inverse_smem(kl, ku, 4), st>>>(ab, G, n, kl, ku, w, tops,
+                                                                                              WF, WB, FmaForms());
+    return cuda_check(cudaGetLastError(), "k_band_inverse");
+}
+static int inverse_setup(int kl, int ku) {
+    if (int rc = cuda_check(cudaFuncSetAttribute(k_band_inverse<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)inverse_smem(kl, ku, 4)),
+                            "coarse inverse"))
+        return rc;
+    return cuda_check(cudaFuncSetAttribute(k_band_inverse<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)inverse_smem(kl, ku, 8)),
+                      "coarse inverse");
 }
 
 }  // namespace bandlu

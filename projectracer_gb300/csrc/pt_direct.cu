@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "pt_fp64.cuh"
 #include "pt_consts.cuh"
 
 namespace pt {
@@ -328,16 +329,6 @@ __device__ __forceinline__ void ds_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Products, sums and differences in the form of a fused multiply-add, each rounded once as they are: the
-// unit takes a warp's DFMA every 16 cycles, its DMUL or DADD every 19.  (Kernel arguments, so that the
-// compiler does not turn them back.)
-struct FmaForms {
-    double zero = -0.0, one = 1.0, minus = -1.0;
-    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, zero); }
-    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(b, one, a); }
-    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, minus, a); }
-};
-
 // Forward substitution: for j = 1 .. n-1, b(j) <-> b(ipiv(j)), then b(j+1 .. j+lm) += L(., j) * (-b(j)).
 // Element i of b stays in a register of thread (i - 1) mod (blockDim - 64), as its register
 // ((i - 1) / that) mod RPT, from kl + 1 steps before it is final at the latest; a step's
@@ -446,19 +437,6 @@ static int direct_forward_of(int kl, F f) {
     return rpt == 1 ? f(k_direct_forward<1, 8>, threads, direct_forward_smem(kl, 8))
          : rpt == 2 ? f(k_direct_forward<2, 8>, threads, direct_forward_smem(kl, 8))
                     : f(k_direct_forward<4, 4>, threads, direct_forward_smem(kl, 4));
-}
-
-// b / d, correctly rounded, from r = 1 / d (Markstein, IBM J. Res. Dev. 34 (1990): a quotient within an ulp,
-// corrected once with its exact residual and a correctly rounded reciprocal, is the rounded quotient; two
-// corrections bring b r there).  Five dependent operations where a division takes nine.  For exponents that
-// keep every intermediate a normal number: in_range(b, 800) and in_range(d, 100).
-__device__ __forceinline__ bool in_range(double v, int bits) {  // 2^-bits <= |v| < 2^bits
-    return ((unsigned)__double2hiint(v) >> 20 & 0x7ffu) - (unsigned)(1023 - bits) < 2u * (unsigned)bits;
-}
-__device__ __forceinline__ double quotient(double b, double d, double r) {
-    double q = __dmul_rn(b, r);
-    q = __fma_rn(__fma_rn(-d, q, b), r, q);
-    return __fma_rn(__fma_rn(-d, q, b), r, q);
 }
 
 // Back substitution: for j = n .. 1, x = b(j) / U(j,j), b(j) = x, b(i0 .. j-1) -= x U(., j), in blocks of 32

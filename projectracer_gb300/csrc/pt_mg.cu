@@ -1091,83 +1091,6 @@ __global__ void __launch_bounds__(kBsThreads) k_band_solve(const double* ab, con
     for (int q = tid; q < n; q += kBsThreads) bg[q] = b[q];
 }
 
-// Explicit inverse of the factored coarse matrix, G = (P L U)^{-1}.  Warp w of a block carries
-// column c = 4 blockIdx.x + w through the forward/back substitution of k_band_solve (DGBTRS
-// restated) on the unit vector e_c, its lanes splitting each step's band update.  The four warps
-// share the band columns, staged through shared memory kInvChunk at a time; each column vector
-// lives in shared memory.  G is row-major, so the per-cycle coarse solve is a coalesced GEMV.
-constexpr int kInvWarps = 4, kInvChunk = 16;
-__host__ __device__ constexpr size_t inv_smem(int n, int kl, int ku) {
-    return sizeof(double) * ((size_t)kInvChunk * (kl + ku + 1) + (size_t)kInvWarps * n) + sizeof(int) * kInvChunk;
-}
-__global__ void __launch_bounds__(32 * kInvWarps) k_band_inverse(const double* ab, const int* ipiv, double* G, int n,
-                                                                 int kl, int ku) {
-    extern __shared__ double sm[];
-    const int ldab = 2 * kl + ku + 1, kd = ku + kl + 1, k = kl + ku, kp1 = k + 1;
-    double* band = sm;                                           // kInvChunk x kp1
-    double* y = band + (size_t)kInvChunk * kp1 + (size_t)(threadIdx.x >> 5) * n;
-    int* piv = reinterpret_cast<int*>(sm + (size_t)kInvChunk * kp1 + (size_t)kInvWarps * n);
-    const int lane = threadIdx.x & 31, c = blockIdx.x * kInvWarps + (threadIdx.x >> 5);
-    const bool active = c < n;  // inactive warps still join every __syncthreads
-#define AB(r, cc) ab[(size_t)((r) - 1) + (size_t)((cc) - 1) * (size_t)ldab]
-    if (active)
-        for (int q = lane; q < n; q += 32) y[q] = (q == c) ? 1.0 : 0.0;
-    // forward: L with the row interchanges
-    for (int j0 = 1; j0 <= n - 1; j0 += kInvChunk) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < kInvChunk * kl; t += blockDim.x) {
-            const int jj = j0 + t / kl, i = t % kl + 1;
-            band[(size_t)(t / kl) * kl + (i - 1)] = (jj <= n - 1 && i <= n - jj) ? AB(kd + i, jj) : 0.0;
-        }
-        for (int t = threadIdx.x; t < kInvChunk; t += blockDim.x) piv[t] = (j0 + t <= n - 1) ? ipiv[j0 + t - 1] : 0;
-        __syncthreads();
-        if (!active) continue;
-        const int jend = min(n - 1, j0 + kInvChunk - 1);
-        for (int j = j0; j <= jend; j++) {
-            const int lm = kl < n - j ? kl : n - j, l = piv[j - j0];
-            if (l != j && lane == 0) {
-                const double tt = y[l - 1];
-                y[l - 1] = y[j - 1];
-                y[j - 1] = tt;
-            }
-            __syncwarp();
-            const double bj = y[j - 1];
-            if (bj != 0.0) {
-                const double temp = -1.0 * bj;
-                const double* bc = band + (size_t)(j - j0) * kl;
-                for (int i = 1 + lane; i <= lm; i += 32) y[j + i - 1] = y[j + i - 1] + bc[i - 1] * temp;
-            }
-            __syncwarp();
-        }
-    }
-    // backward: U (band rows 1..kp1 of each column), columns n..1
-    for (int j1 = n; j1 >= 1; j1 -= kInvChunk) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < kInvChunk * kp1; t += blockDim.x) {
-            const int jj = j1 - t / kp1, r = t % kp1 + 1;
-            band[(size_t)(t / kp1) * kp1 + (r - 1)] = (jj >= 1) ? AB(r, jj) : 0.0;
-        }
-        __syncthreads();
-        if (!active) continue;
-        const int jend = max(1, j1 - kInvChunk + 1);
-        for (int j = j1; j >= jend; j--) {
-            const double* bc = band + (size_t)(j1 - j) * kp1;  // bc[r - 1] = AB(r, j)
-            const double bj = y[j - 1];
-            if (bj != 0.0) {
-                const double x = bj / bc[kp1 - 1];
-                __syncwarp();
-                if (lane == 0) y[j - 1] = x;
-                const int l = kp1 - j, i0 = 1 > j - k ? 1 : j - k;
-                for (int i = j - 1 - lane; i >= i0; i -= 32) y[i - 1] = y[i - 1] - x * bc[l + i - 1];
-            }
-            __syncwarp();
-        }
-    }
-#undef AB
-    if (active)
-        for (int q = lane; q < n; q += 32) G[(size_t)q * n + c] = y[q];
-}
-
 // coarse solve through the explicit inverse: b = RowB * RHS on interior nodes (0 on the
 // boundary), x = G b (one warp per row, lanes stride the row, fixed-order shuffle reduction),
 // scattered into the level array.
@@ -1253,15 +1176,13 @@ static int coarse_factor(Engine& E) {
     CK(cudaMemsetAsync(E.derr, 0, sizeof(int), E.st));
     PT_COUNT(), k_coarse_matrix<<<nblk(n, 128), 128, 0, E.st>>>(E.Mc, E.gl[L], L, E.kl, E.ku, n, E.RowB, E.cfg.Vbc,
                                                     E.cfg.ivis, E.vis[L], E.vx[L], E.vz[L], E.vxz[L], E.vxxmzz[L], E.derr);
-    if (int rc = bandlu::factor(E.Mc, E.ipiv, n, E.kl, E.ku, bandlu::work_of(E.luw, E.kl), E.derr, E.st)) return rc;
+    if (int rc = bandlu::factor(E.Mc, E.ipiv, n, E.kl, E.ku, bandlu::work_of(E.luw, n, E.kl), E.derr, E.st)) return rc;
     int h = 0;
     CK(cudaMemcpyAsync(&h, E.derr, sizeof(int), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
     if (h) return fail(PT_ERR_SINGULAR_COARSE, "coarse banded LU: zero row or pivot");
     if (E.Ginv) {
-        PT_COUNT(), k_band_inverse<<<nblk(n, kInvWarps), 32 * kInvWarps, inv_smem(n, E.kl, E.ku), E.st>>>(
-            E.Mc, E.ipiv, E.Ginv, n, E.kl, E.ku);
-        CKL("k_band_inverse");
+        if (int rc = bandlu::inverse(E.Mc, E.Ginv, n, E.kl, E.ku, bandlu::work_of(E.luw, n, E.kl), E.st)) return rc;
     }
     return 0;
 }
@@ -1275,10 +1196,8 @@ static int coarse_factor_async(Engine& E, const VisLevels& V) {
     PT_COUNT(), k_coarse_matrix<<<nblk(n, 128), 128, 0, E.st2>>>(E.Mc2, E.gl[L], L, E.kl, E.ku, n, E.RowB2, E.cfg.Vbc,
                                                      E.cfg.ivis, V.vis[L], V.vx[L], V.vz[L], V.vxz[L], V.vxxmzz[L],
                                                      E.derr2);
-    if (int rc = bandlu::factor(E.Mc2, E.ipiv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, E.kl), E.derr2, E.st2)) return rc;
-    PT_COUNT(), k_band_inverse<<<nblk(n, kInvWarps), 32 * kInvWarps, inv_smem(n, E.kl, E.ku), E.st2>>>(
-        E.Mc2, E.ipiv2, E.Ginv2, n, E.kl, E.ku);
-    CKL("async coarse factorisation");
+    if (int rc = bandlu::factor(E.Mc2, E.ipiv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, n, E.kl), E.derr2, E.st2)) return rc;
+    if (int rc = bandlu::inverse(E.Mc2, E.Ginv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, n, E.kl), E.st2)) return rc;
     CK(cudaMemcpyAsync(E.hflag2, E.derr2, sizeof(int), cudaMemcpyDeviceToHost, E.st2));
     E.fact_pending = true;
     return 0;
@@ -1649,7 +1568,7 @@ int mg_alloc(Engine& E) {
     if (int rc = alloc(&E.Bc, E.ngc)) return rc;
     if (int rc = alloc(&E.RowB, E.ngc)) return rc;
     CK(cudaMalloc(&E.ipiv, sizeof(int) * E.ngc));
-    CK(cudaMalloc(&E.luw, bandlu::work_bytes(E.kl)));
+    CK(cudaMalloc(&E.luw, bandlu::work_bytes(E.ngc, E.kl)));
     const size_t smem = sizeof(double) * (size_t)E.ngc;
     if (smem > 220 * 1024) return fail(PT_ERR_CONFIG, "coarsest grid too large for the banded solve");
     if (band_solve_smem(E.ngc, E.kl, E.ku) > 220 * 1024)
@@ -1660,15 +1579,17 @@ int mg_alloc(Engine& E) {
     CK(cudaFuncSetAttribute(k_coarse_apply_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // explicit coarse inverse (both precisions): the coarse solve becomes a GEMV spread over the
     // SMs instead of two sequential banded substitutions on one warp of this part's narrow FP64
-    // pipe; n^2 doubles, kept while it is small next to the level arrays (n <= 4096: <= 134 MB)
-    if (!E.cfg.reference_rounding && E.ngc <= 4096 && inv_smem(E.ngc, E.kl, E.ku) <= 200 * 1024) {
+    // pipe; n^2 doubles, kept while it is small next to the level arrays (n <= 4096: <= 134 MB) and
+    // the band is narrow next to n (the bound's second part, 16 band columns and 4 vectors in 200 KB,
+    // is where the inverse has always ended)
+    if (!E.cfg.reference_rounding && E.ngc <= 4096 && 16 * (E.kl + E.ku + 1) + 4 * E.ngc <= 25 * 1024) {
         CK(cudaMalloc(&E.Ginv, sizeof(double) * (size_t)E.ngc * E.ngc));
         E.bytes_allocated += sizeof(double) * (size_t)E.ngc * E.ngc;
         CK(cudaMalloc(&E.Ginv2, sizeof(double) * (size_t)E.ngc * E.ngc));
         CK(cudaMalloc(&E.Mc2, sizeof(double) * (size_t)ldab * E.ngc));
         CK(cudaMalloc(&E.RowB2, sizeof(double) * (size_t)E.ngc));
         CK(cudaMalloc(&E.ipiv2, sizeof(int) * (size_t)E.ngc));
-        CK(cudaMalloc(&E.luw2, bandlu::work_bytes(E.kl)));
+        CK(cudaMalloc(&E.luw2, bandlu::work_bytes(E.ngc, E.kl)));
         CK(cudaMalloc(&E.derr2, sizeof(int)));
         CK(cudaMallocHost(&E.hflag2, sizeof(int)));
         *E.hflag2 = 0;
@@ -1691,8 +1612,7 @@ int mg_alloc(Engine& E) {
         CK(cudaEventCreateWithFlags(&E.ev_in, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&E.ev_fact, cudaEventDisableTiming));
         E.bytes_allocated += sizeof(double) * ((size_t)E.ngc * E.ngc + (size_t)ldab * E.ngc + E.ngc);
-        CK(cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_smem(E.ngc, E.kl, E.ku)));
+        if (int rc = bandlu::inverse_setup(E.kl, E.ku)) return rc;
     }
     return cluster_setup_d(E);
 }
