@@ -20,6 +20,7 @@
 #include <utility>
 
 #include "pt_consts.cuh"
+#include "pt_fp64.cuh"
 
 namespace pt {
 
@@ -172,27 +173,55 @@ __global__ void k_scatter(const int32_t* __restrict__ cell, int64_t n, const int
     if (c >= 0) list[start[c] + base + __popc(group & ((1u << lane) - 1u))] = (int32_t)t;
 }
 
-// ascending tracer IDs inside each cell (insertion sort: cells hold a few dozen tracers)
-__global__ void k_sort_cells(int32_t* list, const int32_t* start, const int32_t* count, int ncell) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
+// Ascending tracer IDs inside each cell: a warp per cell takes up to 32 kSortRegs IDs into registers, and an
+// ID's place is the number of smaller ones.  (A thread per cell that inserted them in global memory took
+// 141 us for 100 x 100 cells of 60; now 20.)  Fuller cells are sorted by one lane.
+constexpr int kSortRegs = 8, kCellsPerWarp = 10;
+__global__ void __launch_bounds__(256) k_sort_cells(int32_t* list, const int32_t* __restrict__ start,
+                                                  const int32_t* __restrict__ count, int ncell) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (c >= ncell) return;
-    int b = start[c], n = count[c];
-    for (int a = 1; a < n; a++) {
-        int32_t key = list[b + a];
-        int j = a - 1;
-        while (j >= 0 && list[b + j] > key) {
-            list[b + j + 1] = list[b + j];
-            j--;
-        }
-        list[b + j + 1] = key;
+    const int n = count[c];
+    int32_t* const l = list + start[c];
+    if (n > 32 * kSortRegs) {
+        if (lane == 0)
+            for (int a = 1; a < n; a++) {
+                const int32_t key = l[a];
+                int j = a - 1;
+                while (j >= 0 && l[j] > key) {
+                    l[j + 1] = l[j];
+                    j--;
+                }
+                l[j + 1] = key;
+            }
+        return;
     }
+    int32_t key[kSortRegs];
+    int rank[kSortRegs] = {};
+#pragma unroll
+    for (int q = 0; q < kSortRegs; q++) key[q] = 32 * q + lane < n ? l[32 * q + lane] : INT_MAX;
+#pragma unroll
+    for (int q = 0; q < kSortRegs; q++) {
+        if (32 * q >= n) break;
+        const int m = min(32, n - 32 * q);
+        for (int t = 0; t < m; t++) {
+            const int32_t k = __shfl_sync(0xffffffffu, key[q], t);
+#pragma unroll
+            for (int u = 0; u < kSortRegs; u++) rank[u] += k < key[u];
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kSortRegs; q++)
+        if (32 * q + lane < n) l[rank[q]] = key[q];
 }
 
-__device__ __forceinline__ double shape1(double x, int i, double h, double inv, int exact) {
-    double d = fabs(__dsub_rn(x, __dmul_rn((double)i, h)));
-    double q = exact ? __dmul_rn(d, inv) : __ddiv_rn(d, h);
-    double a = __dsub_rn(1.0, q);
-    return a > 0.0 ? a : 0.0;
+__device__ __forceinline__ double shape1(double x, double node, double h, double inv, int exact, const FmaForms& F) {
+    const double d = fabs(F.sub(x, node));
+    const double q = exact ? F.mul(d, inv) : (in_range(d, 800) || __double_as_longlong(d) == 0) && in_range(h, 100) ? quotient(d, h, inv) : __ddiv_rn(d, h);
+    const double a = F.sub(1.0, q);
+    const long long bits = __double_as_longlong(a);
+    return bits > 0 && bits <= 0x7ff0000000000000ll ? a : 0.0;  // a > 0
 }
 
 // per-cell partial sums for the 3x3 nodes around the cell; planes of ncell: [q*9 + dz*3 + dx]
@@ -201,51 +230,62 @@ __device__ __forceinline__ double shape1(double x, int i, double h, double inv, 
 // shape sum of the type-1 tracers (count_type_real(1)) and that of the type-0 tracers
 // (count_type_real(0)); a tracer of the other type leaves a plane's partial unchanged (+0.0 and
 // x 1.0 are exact), so the sums are those of the reference's per-type loops in ID order.
+// Three lanes per cell, a row dz of nodes each; lane d forms the shape functions of column and row d and
+// the columns' go round by shuffle.  Bound by the SM's FP64 unit, which the instructions of a thread per
+// cell left to one CTA's warps on half of the SMs (100 x 100 cells of 60: 357 us, now 186).
 template <bool OG>
-__global__ void k_cell_partials(const double* __restrict__ r, const double* __restrict__ s,
+__global__ void __launch_bounds__(128) k_cell_partials(const double* __restrict__ r, const double* __restrict__ s,
                                 const double* __restrict__ Tt, const double* __restrict__ Ct,
                                 const int32_t* __restrict__ list, const int32_t* __restrict__ start,
                                 const int32_t* __restrict__ count, int ncell, double* __restrict__ P,
-                                int comp) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
+                                int comp, FmaForms F) {
+    const int lane = threadIdx.x & 31, d = lane % 3, l0 = lane - d;
+    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kCellsPerWarp + lane / 3;
+    const bool live = lane < 3 * kCellsPerWarp && c < ncell;
     const int nx1 = cK.nx + 1;
-    int ci = c % nx1, ck = c / nx1;
-    double aT[9], aC[9], aS[9];
-#pragma unroll
-    for (int q = 0; q < 9; q++) { aT[q] = 0.0; aC[q] = 0.0; aS[q] = 0.0; }
-    int b = start[c], n = count[c];
-    for (int a = 0; a < n; a++) {
-        int32_t t = list[b + a];
-        double rr = r[t], ss = s[t], tv = Tt[t], cv = comp ? Ct[t] : 0.0;
+    const int ck = live ? c / nx1 : 0, ci = live ? c - ck * nx1 : 0;
+    const double xn = __dmul_rn((double)(ci + d - 1), cK.dr), zn = __dmul_rn((double)(ck + d - 1), cK.ds);
+    double aT[3] = {}, aC[3] = {}, aS[3] = {};
+    const int b = live ? start[c] : 0, n = live ? count[c] : 0, most = __reduce_max_sync(0xffffffffu, n);
+    // the next tracer's values are in flight, and the ID of the one after it
+    int32_t t1 = 1 < n ? list[b + 1] : -1;
+    double r1 = 0.0, s1 = 0.0, T1 = 0.0, C1 = 0.0;
+    auto load = [&](int32_t t) {
+        r1 = t >= 0 ? r[t] : 0.0;
+        s1 = t >= 0 ? s[t] : 0.0;
+        T1 = t >= 0 ? Tt[t] : 0.0;
+        C1 = t >= 0 && comp ? Ct[t] : 0.0;
+    };
+    load(n > 0 ? list[b] : -1);
+    for (int a = 0; a < most; a++) {
+        const bool has = a < n;
+        const double rr = r1, ss = s1, tv = T1, cv = C1;
+        load(t1);
+        t1 = a + 2 < n ? list[b + a + 2] : -1;
         const bool type1 = OG && cv != 0.0;
-        double wx[3], wz[3];
+        const double wx = shape1(rr, xn, cK.dr, cK.inv_dr, cK.exact_div, F);
+        const double wz = shape1(ss, zn, cK.ds, cK.inv_ds, cK.exact_div, F);
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            wx[d] = shape1(rr, ci + d - 1, cK.dr, cK.inv_dr, cK.exact_div);
-            wz[d] = shape1(ss, ck + d - 1, cK.ds, cK.inv_ds, cK.exact_div);
-        }
-#pragma unroll
-        for (int dz = 0; dz < 3; dz++)
-#pragma unroll
-            for (int dx = 0; dx < 3; dx++) {
-                double S = __dmul_rn(wx[dx], wz[dz]);
-                int q = dz * 3 + dx;
-                aT[q] = __dadd_rn(aT[q], __dmul_rn(tv, S));
-                if (OG) {
-                    if (type1) aC[q] = __dadd_rn(aC[q], S);
-                    else aS[q] = __dadd_rn(aS[q], S);
-                } else {
-                    aC[q] = __dadd_rn(aC[q], __dmul_rn(cv, S));
-                    aS[q] = __dadd_rn(aS[q], S);
-                }
+        for (int dx = 0; dx < 3; dx++) {
+            const double S = F.mul(__shfl_sync(0xffffffffu, wx, (l0 + dx) & 31), wz);
+            if (!has) continue;
+            aT[dx] = F.add(aT[dx], F.mul(tv, S));
+            if (OG) {
+                if (type1) aC[dx] = F.add(aC[dx], S);
+                else aS[dx] = F.add(aS[dx], S);
+            } else {
+                if (comp) aC[dx] = F.add(aC[dx], F.mul(cv, S));
+                aS[dx] = F.add(aS[dx], S);
             }
+        }
     }
+    if (!live) return;
 #pragma unroll
-    for (int q = 0; q < 9; q++) {
-        P[(size_t)q * ncell + c] = aT[q];
-        P[(size_t)(9 + q) * ncell + c] = aC[q];
-        P[(size_t)(18 + q) * ncell + c] = aS[q];
+    for (int dx = 0; dx < 3; dx++) {
+        const size_t q = (size_t)(3 * d + dx) * ncell + c;
+        P[q] = aT[dx];
+        P[q + (size_t)9 * ncell] = aC[dx];
+        P[q + (size_t)18 * ncell] = aS[dx];
     }
 }
 
@@ -628,10 +668,10 @@ static int project_with(Engine& E, const ProjScratch& W, const double* r, const 
             int32_t* cursor = W.scan_tmp + nb + 32;
             CK(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (size_t)ncell, E.st));
             PT_COUNT(), k_scatter<<<nblk(n, 256), 256, 0, E.st>>>(W.tcell, n, W.cstart, cursor, W.clist);
-            PT_COUNT(), k_sort_cells<<<nblk(ncell, 128), 128, 0, E.st>>>(W.clist, W.cstart, W.ccount, ncell);
+            PT_COUNT(), k_sort_cells<<<nblk(ncell, 8), 256, 0, E.st>>>(W.clist, W.cstart, W.ccount, ncell);
             const bool og = E.cfg.discrete_types != 0;
-            PT_COUNT(), (og ? k_cell_partials<true> : k_cell_partials<false>)<<<nblk(ncell, 128), 128, 0, E.st>>>(
-                r, s, Tt, E.Ctr, W.clist, W.cstart, W.ccount, ncell, W.cpart, E.cfg.comp);
+            PT_COUNT(), (og ? k_cell_partials<true> : k_cell_partials<false>)<<<nblk(ncell, 2 * kCellsPerWarp), 64, 0, E.st>>>(
+                r, s, Tt, E.Ctr, W.clist, W.cstart, W.ccount, ncell, W.cpart, E.cfg.comp, FmaForms());
             PT_COUNT(), (og ? k_node_sums<true> : k_node_sums<false>)<<<grid, 128, 0, E.st>>>(
                 W.cpart, W.ccount, ncell, E.Tratio, E.Cnew, E.nempty, E.g1, E.cfg.comp);
         }
