@@ -172,7 +172,7 @@ __global__ void k_fill(double* a, double v, size_t n) {
     if (q < n) a[q] = v;
 }
 
-// ---- band LU over the whole GPU
+// ---- band LU over the whole GPU, for bands too wide for the panel LU (a thread per row of the band)
 struct LuShared {
     unsigned count, gen;  // grid barrier
     int jp, ju, nz;       // this column's pivot offset, reach and pivot-is-usable flag
@@ -661,6 +661,10 @@ int direct_alloc(Engine& E) {
     CK(cudaMalloc(&E.dB, sizeof(double) * (size_t)n));
     CK(cudaMalloc(&E.dipiv, sizeof(int) * (size_t)n));
     CK(cudaMalloc(&E.dlu, sizeof(LuShared)));
+    if (band_lu_fits(kl)) {
+        CK(cudaMalloc(&E.dluw, band_lu_bytes(n, kl)));
+        E.bytes_allocated += band_lu_bytes(n, kl);
+    }
     CK(cudaMalloc(&E.dluerr, 2 * sizeof(int)));
     E.bytes_allocated += sizeof(double) * ((size_t)ldab + 2) * (size_t)n + sizeof(int) * (size_t)n;
     // Matrix_element for every (stencil point, image signs, row kind)
@@ -683,11 +687,12 @@ int direct_alloc(Engine& E) {
 }
 
 void direct_free(Engine& E) {
-    for (void* p : {(void*)E.dMB, (void*)E.dRow, (void*)E.dB, (void*)E.dipiv, (void*)E.dlu, (void*)E.dluerr})
+    for (void* p : {(void*)E.dMB, (void*)E.dRow, (void*)E.dB, (void*)E.dipiv, (void*)E.dlu, (void*)E.dluerr, E.dluw})
         if (p) cudaFree(p);
     E.dMB = E.dRow = E.dB = nullptr;
     E.dipiv = E.dluerr = nullptr;
     E.dlu = nullptr;
+    E.dluw = nullptr;
 }
 
 // build_SF_matrix: assembly, equilibration and factorisation (once: the isoviscous operator does
@@ -705,22 +710,26 @@ static int direct_factor(Engine& E) {
     CK(cudaMemcpyAsync(&h, E.derr, sizeof(int), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
     if (h) return fail(PT_ERR_SINGULAR_COARSE, "direct solve: DGBEQU found a zero row");
-    // one CTA per SM, all resident (cooperative launch)
-    int dev = 0, sms = 0, per = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_direct_lu, kLuThreads, 0));
-    if (per < 1) return fail(PT_ERR_CUDA, "direct solve: the LU kernel cannot be resident");
-    double* ab = E.dMB;
-    int* ipiv = E.dipiv;
-    int* lu_err = E.dluerr;
-    int nn = n, kkl = kl, kku = ku;
-    LuShared* sh = reinterpret_cast<LuShared*>(E.dlu);
-    void* args[] = {&ab, &ipiv, &nn, &kkl, &kku, &lu_err, &sh};
-    PT_COUNT();
-    CK(cudaLaunchCooperativeKernel((void*)k_direct_lu, dim3(sms), dim3(kLuThreads), args, 0, E.st));
+    if (E.dluw) {  // n = 16641, kl = ku = 387: 95 ms, 209 in the cooperative kernel
+        if (int rc = band_lu(E.dMB, E.dipiv, n, kl, ku, E.dluw, E.dluerr + 1, E.st)) return rc;
+    } else {
+        // one CTA per SM, all resident (cooperative launch)
+        int dev = 0, sms = 0, per = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_direct_lu, kLuThreads, 0));
+        if (per < 1) return fail(PT_ERR_CUDA, "direct solve: the LU kernel cannot be resident");
+        double* ab = E.dMB;
+        int* ipiv = E.dipiv;
+        int* lu_err = E.dluerr;
+        int nn = n, kkl = kl, kku = ku;
+        LuShared* sh = reinterpret_cast<LuShared*>(E.dlu);
+        void* args[] = {&ab, &ipiv, &nn, &kkl, &kku, &lu_err, &sh};
+        PT_COUNT();
+        CK(cudaLaunchCooperativeKernel((void*)k_direct_lu, dim3(sms), dim3(kLuThreads), args, 0, E.st));
+    }
     int hl[2] = {0, 0};
-    CK(cudaMemcpyAsync(hl, lu_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, E.st));
+    CK(cudaMemcpyAsync(hl, E.dluerr, 2 * sizeof(int), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
     if (hl[0] & 8) return fail(PT_ERR_ITER_CAP, "direct solve: LU grid barrier timed out");
     if (hl[1]) return fail(PT_ERR_SINGULAR_COARSE, "direct solve: DGBTRF found a zero pivot");

@@ -111,6 +111,7 @@ struct Engine {
     // direct banded solve (cfg.direct, pt_direct.cu): band matrix and LU, row factors, right-hand
     // side, pivots, the LU kernel's barrier state and error words
     int dn = 0, dkl = 0, dku = 0;
+    void* dluw = nullptr;  // workspace of the panel LU (bands that it takes)
     double *dMB = nullptr, *dRow = nullptr, *dB = nullptr;
     int *dipiv = nullptr, *dluerr = nullptr;
     void* dlu = nullptr;
@@ -341,6 +342,10 @@ int c_to_types(Engine& E, const double* c, int32_t* dev_types);
 void io_release(Engine& E);
 
 // direct banded solve (pt_direct.cu)
+// band LU in panels (pt_mg.cu): in, out: LAPACK band storage; err: the first column without a usable pivot
+bool band_lu_fits(int kl);
+size_t band_lu_bytes(int n, int kl);
+int band_lu(double* ab, int* ipiv, int n, int kl, int ku, void* work, int* err, cudaStream_t st);
 int direct_alloc(Engine& E);
 void direct_free(Engine& E);
 int direct_solve(Engine& E, pt_solve_info* info);  // momentum.f90:258-317, 636-653

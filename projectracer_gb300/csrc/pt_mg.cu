@@ -1170,6 +1170,13 @@ __global__ void k_coarse_scatter(double* E, const double* B, Geo g, int nxc, int
     E[g.at((p - 1) / N, (p - 1) % N)] = B[p - 1];
 }
 
+// the panel LU for the direct solve's band (pt_direct.cu)
+bool band_lu_fits(int kl) { return bandlu::row_threads(kl) + 32 <= 512; }
+size_t band_lu_bytes(int n, int kl) { return bandlu::work_bytes(n, kl); }
+int band_lu(double* ab, int* ipiv, int n, int kl, int ku, void* work, int* err, cudaStream_t st) {
+    return bandlu::factor(ab, ipiv, n, kl, ku, bandlu::work_of(work, n, kl), err, st);
+}
+
 static int coarse_factor(Engine& E) {
     PhaseTimer tf(E, PH_FACTOR);
     const int L = E.grids, n = E.ngc;
