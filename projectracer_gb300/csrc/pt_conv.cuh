@@ -126,13 +126,14 @@ __device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, volati
 // that room: all SMs reading the same 18 KB for every tile is a hot spot of L2 (32 -> 32 channels on a
 // million pixels: 48 us with them kept, 74 us without; four CTAs on an SM 48 us, three 52, two 64, one 105).
 // A smaller grid has an SM for each CTA, and the latency of its loads is all there is: the deepest ring.
-static inline void conv_stages(ConvArgs& a, int nblk) {
+static inline void conv_stages(ConvArgs& a, int nblk, bool sums) {
     const int bw = a.nsrc > 1 && a.bw[1] > a.bw[0] ? a.bw[1] : a.bw[0];
     const bool large = a.tiles > kSms;
     a.bbytes = a.Ntile * bw * 2;
     a.nbuf = a.Ntile <= 128 && large ? 2 : 1;
-    auto stages = [&](int k, int keep) {  // of k CTAs on an SM, which has 228 KB (1 KB reserved, 2.1 KB static each)
-        const int room = (k == 1 ? 220 : 228 / k - 4) * 1024 - (keep ? a.taps * nblk * a.bbytes : 0);
+    auto stages = [&](int k, int keep) {  // of k CTAs on an SM, which has 228 KB (1 KB reserved, 2.1 KB static each, 5.1 with
+        // column sums)
+        const int room = (k == 1 ? 220 : 228 / k - (sums ? 8 : 4)) * 1024 - (keep ? a.taps * nblk * a.bbytes : 0);
         auto bytes = [&](int nd, int G) {
             a.nd = nd;
             a.G = G;
@@ -194,8 +195,9 @@ __device__ __forceinline__ void drain(Ring& ring, const RingPos& r, int n) {
     for (int s = 0; s < n; s++) mbar_wait(ring.full + s, s < r.i ? r.parity ^ 1u : r.parity);
 }
 
-// Epilogue E: void operator()(int p, int col0, const float (&v)[32]) for columns col0 .. col0 + 31 of
-// position p (called for real pixels with their coordinates)
+// Epilogue E: void operator()(p, b, y, x, col0, v, bias) for columns col0 .. col0 + 31 of position p (called
+// for real pixels with their coordinates); with kSums: void sums(p, real, col0, v, sum) by whole warps,
+// which adds its lanes' masked values to sum[col0 ..], and part[CTA][column] for the CTA's sums
 template <class E>
 __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constant__ CUtensorMap mapA0,
                                                             const __grid_constant__ CUtensorMap mapA1,
@@ -208,6 +210,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
     __shared__ uint32_t tslot;
     __shared__ int bad;
     __shared__ __align__(16) float sbias[256];
+    __shared__ float sacc[E::kSums ? 4 * 256 : 1];  // column sums of the epilogue's warps
     unsigned char* const smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int S = a.S, G = a.G, nd = a.nd;
@@ -222,6 +225,8 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
     }
     if (warp == 5) tmem_alloc(&tslot, ncols);
     epi.stage(sbias, a.N, tid);
+    if (E::kSums)
+        for (int q = tid; q < 4 * 256; q += kConvThreads) sacc[q] = 0.f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -384,13 +389,17 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_gemm(const __grid_constan
                     __syncwarp();
                     if (lane == 0) mbar_arrive(accs.empty + c.i);
                 }
-                if (real) epi(p, b, y, x, n0 + c0, v, sbias + n0 + c0);
+                if (E::kSums) epi.sums(p, real, n0 + c0, v, sacc + warp * 256);
+                else if (real) epi(p, b, y, x, n0 + c0, v, sbias + n0 + c0);
             }
             c.next(a.nbuf);
         }
     }
     tc_fence_before();
     __syncthreads();
+    if (E::kSums)
+        for (int c = tid; c < a.N; c += kConvThreads)
+            epi.part[(size_t)blockIdx.x * a.N + c] = ((sacc[c] + sacc[256 + c]) + sacc[512 + c]) + sacc[768 + c];
     if (bad && tid == 0) atomicOr(err, 1);
     if (warp == 5) tmem_dealloc(taddr, ncols);
 }

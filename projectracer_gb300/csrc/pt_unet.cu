@@ -114,6 +114,8 @@ __device__ __forceinline__ void st32(void* p, const uint32_t (&h)[8]) {
                  : "memory");
 }
 struct FwdEpi {
+    static constexpr bool kSums = false;
+    static constexpr float* part = nullptr;
     uint16_t* out;
     const float* bias;
     int C;
@@ -136,9 +138,12 @@ struct FwdEpi {
                 for (int q = 0; q < 4; q++) st32(up + gup.at(b, 2 * y + (q >> 1), 2 * x + (q & 1)) * C + c0 + j, h);
         }
     }
+    __device__ __forceinline__ void sums(int, bool, int, const float (&)[32], float*) const {}
 };
 // epilogue of the backward-data GEMM: the view's gradient in FP32 at the padded positions
 struct DxEpi {
+    static constexpr bool kSums = false;
+    static constexpr float* part = nullptr;
     float* dx;
     int N;
     __device__ __forceinline__ void stage(float*, int, int) const {}
@@ -151,6 +156,51 @@ struct DxEpi {
             for (int e = 0; e < 8; e++) h[e] = __float_as_uint(v[j + e]);
             st32(o + j, h);
         }
+    }
+    __device__ __forceinline__ void sums(int, bool, int, const float (&)[32], float*) const {}
+};
+// epilogue of the backward-data GEMM of a view that is a layer's output itself: that layer's dZ (the
+// gradient masked by Y > 0, in BF16) and the column sums of its bias gradient, without a pass over the
+// gradient in FP32
+struct DzEpi {
+    static constexpr bool kSums = true;
+    const uint16_t* Y;
+    uint16_t* dZ;
+    int C;
+    float* part;
+    __device__ __forceinline__ void stage(float*, int, int) const {}
+    __device__ __forceinline__ void operator()(int, int, int, int, int, const float (&)[32], const float*) const {}
+    __device__ __forceinline__ void sums(int p, bool real, int c0, const float (&v)[32], float* sum) const {
+        const size_t o = (size_t)p * C + c0;
+        float g[32];
+#pragma unroll
+        for (int j = 0; j < 32; j += 16) {
+            float y[16];
+            if (real) {
+                float (&y0)[8] = reinterpret_cast<float (&)[8]>(y[0]);
+                float (&y1)[8] = reinterpret_cast<float (&)[8]>(y[8]);
+                unpack8(ld8(Y + o + j), y0);
+                unpack8(ld8(Y + o + j + 8), y1);
+            }
+#pragma unroll
+            for (int e = 0; e < 16; e++) g[j + e] = real && y[e] > 0.f ? v[j + e] : 0.f;
+            uint32_t h[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) h[e] = (uint32_t)f2bf(g[j + 2 * e]) | (uint32_t)f2bf(g[j + 2 * e + 1]) << 16;
+            if (real) st32(dZ + o + j, h);
+        }
+        // lane l: the sum of column l over the warp's rows (halves exchanged, then quarters, ...)
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+            const bool up = lane & w;
+#pragma unroll
+            for (int j = 0; j < w; j++) {
+                const float other = __shfl_xor_sync(0xffffffffu, up ? g[j] : g[j + w], w);
+                g[j] = (up ? g[j + w] : g[j]) + other;
+            }
+        }
+        sum[c0 + lane] += g[0];
     }
 };
 
@@ -217,12 +267,11 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const __grid_constant__ Re
 // Gradient of a layer's pre-activation as a GEMM operand, dZ = dY masked by Y > 0 in BF16, and per-block
 // partial sums of its bias gradient (of the FP32 dY).  dY is where the gradient of the view that read
 // the layer's output comes from:
-//   plain   the view's gradient itself
 //   pooled  the skip connection's share plus a quarter of the pooled pixel's
 //   up      the sum of the four fine pixels, ((a+b)+c)+d
 //   out     the output layer: dy w[c]; the partial sums of its own weights' gradients too
 // One pass over the tensor, bound by its bytes (FP32 in, two BF16 tensors in and out).
-enum { kDzPlain = 0, kDzPooled, kDzUp, kDzOut };
+enum { kDzPooled, kDzUp, kDzOut };
 constexpr int kDzThreads = 256, kDzBlocks = 4 * tc::kSms;
 struct DzArgs {
     PadGeo g, g2;  // of the layer, and of the other resolution (pooled: coarse, up: fine)
@@ -256,9 +305,7 @@ __global__ void __launch_bounds__(kDzThreads) k_dz(DzArgs a) {
             const float4 u = *reinterpret_cast<const float4*>(f), w = *reinterpret_cast<const float4*>(f + 4);
             v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
         };
-        if (MODE == kDzPlain) {
-            load(a.dx + p * a.ldx + c, g);
-        } else if (MODE == kDzPooled) {
+        if (MODE == kDzPooled) {
             float d[8];
             load(a.skip + p * a.lds + a.offs + c, g);
             load(a.dx + a.g2.at(b, y >> 1, x >> 1) * a.ldx + c, d);
@@ -561,7 +608,7 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
             if ((rc = ualloc(U, &U.up[c.src0], n(c.level, U.tch[c.src0]))) ||
                 (rc = ualloc(U, &U.dxcat[c.out], n(c.level, c.cin))))
                 return rc;
-        } else {
+        } else if (c.mode == 1) {
             dx = std::max(dx, n(c.level, c.cin));
         }
     }
@@ -580,6 +627,7 @@ static int unet_build(UNet& U, int H, int W, int maxB, uint64_t seed) {
     const int smax = 221 * 1024;  // the rings' bound and the alignment
     CK(cudaFuncSetAttribute(tc::k_conv_gemm<FwdEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     CK(cudaFuncSetAttribute(tc::k_conv_gemm<DxEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+    CK(cudaFuncSetAttribute(tc::k_conv_gemm<DzEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     CK(cudaFuncSetAttribute(tc::k_wgrad_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     return 0;
 }
@@ -627,7 +675,7 @@ static int view_sources(const UNet& U, const UConv& c, const uint16_t* (&t)[2], 
 // one convolution GEMM: sources t (C channels each), weights w [N][Ktot], over the positions of g.  The
 // column tile is the largest that still gives every SM a CTA (at least 32 columns).
 static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* const* t, const int* C, const uint16_t* w,
-                     int N) {
+                     int N, bool sums) {
     tc::ConvArgs& a = P.a;
     a.g = g;
     a.wp = PadGeo::Div(g.Wp());
@@ -651,7 +699,7 @@ static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* 
     a.Ntile = N / nt;
     a.nt = nt;
     a.tiles = mt * nt;
-    tc::conv_stages(a, C[0] / a.bw[0] + (nsrc > 1 ? C[1] / a.bw[1] : 0));
+    tc::conv_stages(a, C[0] / a.bw[0] + (nsrc > 1 ? C[1] / a.bw[1] : 0), sums);
     P.grid = dim3(std::min(a.tiles, tc::kSms * a.ctas));
     const int brows = a.nd == 3 ? tc::kBoxRows : tc::kTileM;
     int rc;
@@ -677,10 +725,11 @@ static int plan_batch(UNet& U, int B) {
         int C[2];
         const int ns = view_sources(U, c, t, C);
         const bool first = c.src0 < 0;
-        if ((rc = plan_conv(P.fwd, g, first ? 1 : 9, ns, t, C, first ? U.w0 : U.wbf + c.woff, c.cout))) return rc;
+        if ((rc = plan_conv(P.fwd, g, first ? 1 : 9, ns, t, C, first ? U.w0 : U.wbf + c.woff, c.cout, false)))
+            return rc;
         const uint16_t* z[2] = {U.dz[c.out], nullptr};
         const int Cz[2] = {c.cout, 0};
-        if (!first && (rc = plan_conv(P.bwd, g, 9, 1, z, Cz, U.wbd + c.woff, c.cin))) return rc;
+        if (!first && (rc = plan_conv(P.bwd, g, 9, 1, z, Cz, U.wbd + c.woff, c.cin, c.mode == 0))) return rc;
         P.nwg = ns;
         for (int s = 0; s < ns; s++) {
             WgradPlan& w = P.wg[s];
@@ -782,6 +831,8 @@ static int unet_backward(UNet& U, int B, float* loss) {
     o.dx = U.dy;
     o.w = U.w32 + U.out_w;
     if ((rc = run_dz<kDzOut>(U, 13, B, o))) return rc;
+    int bsums[14] = {};  // rows of a layer's bias partial sums
+    bsums[13] = dz_blocks(U, U.L[13], B);
     for (int li = (int)U.L.size() - 1; li >= 0; li--) {
         const UConv& c = U.L[li];
         const LayerPlan& P = U.plan[li];
@@ -794,14 +845,19 @@ static int unet_backward(UNet& U, int B, float* loss) {
                                  tc::wgrad_smem(P.wg[s].a), U.st, P.wg[s].A, P.wg[s].B, P.wg[s].a, U.derr)))
                 return rc;
         if (c.src0 < 0) continue;  // the network input needs no gradient
+        if (c.mode == 0) {
+            const DzEpi e{U.act[c.src0], U.dz[c.src0], c.cin, U.bpart + U.bpart_off[c.src0]};
+            if ((rc = run_conv(U, P.bwd, e))) return rc;
+            bsums[c.src0] = (int)P.bwd.grid.x;
+            continue;
+        }
         float* dx = c.mode == 2 ? U.dxcat[c.out] : U.dx;
         if ((rc = run_conv(U, P.bwd, DxEpi{dx, c.cin}))) return rc;
         DzArgs a{};
         a.dx = dx;
         a.ldx = c.cin;
-        if (c.mode == 0) {
-            rc = run_dz<kDzPlain>(U, c.src0, B, a);
-        } else if (c.mode == 2) {
+        bsums[c.src0] = dz_blocks(U, U.L[c.src0], B);
+        if (c.mode == 2) {
             a.g2 = U.geo(c.level, B);
             rc = run_dz<kDzUp>(U, c.src0, B, a);
         } else {  // the skip connection's share was left by the layer that concatenates this tensor
@@ -822,7 +878,7 @@ static int unet_backward(UNet& U, int B, float* loss) {
         const UConv& c = U.L[li];
         red.l[li].block0 = blocks;
         blocks += red.l[li].M * red.l[li].N / 32;
-        sum.l[li] = {U.g + c.boff, U.bpart + U.bpart_off[li], dz_blocks(U, c, B), li == 13 ? 2 * c.cout + 1 : c.cout, 0,
+        sum.l[li] = {U.g + c.boff, U.bpart + U.bpart_off[li], bsums[li], li == 13 ? 2 * c.cout + 1 : c.cout, 0,
                      c.cout, cols};
         cols += c.cout;
     }
