@@ -53,38 +53,64 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
 
 constexpr int kImCols = 64;  // columns of the first layer's im2col rows: 36 values (tap, channel), zeros
 
-// the network input, NCHW FP32, as im2col rows in BF16 at the padded positions: 8 columns a thread
-// (columns 40..63 stay zero from allocation)
-__global__ void k_im2col(uint16_t* __restrict__ o, const float* __restrict__ x, PadGeo g) {
+// 32 bytes in one store: whole sectors, where 16-byte stores of a row per thread are halves of them
+__device__ __forceinline__ void st32(void* p, const uint32_t (&h)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]),
+                 "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7])
+                 : "memory");
+}
+// the network input, NCHW FP32, as im2col rows in BF16 at the padded positions, a pixel per thread (columns
+// 40..63 stay zero from allocation).  Bound by its 128-byte rows: with a thread per 8 columns, half-sector
+// stores and 64-bit divisions 77 us for 8 images of 512 x 256, now 33.
+__global__ void __launch_bounds__(256) k_im2col(uint16_t* __restrict__ o, const float* __restrict__ x, PadGeo g) {
     pdl_begin();
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x, n = (size_t)g.B * g.H * g.W;
-    if (q >= 5 * n) return;
-    const int j = (int)(q / n);
-    size_t r = q - j * n;
-    const int px = (int)(r % g.W);
-    r /= g.W;
-    const int py = (int)(r % g.H), b = (int)(r / g.H);
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;  // (positions fit in 31 bits)
+    if (q >= (unsigned)g.B * g.H * g.W) return;
+    const unsigned row = q / (unsigned)g.W;
+    const int px = (int)(q - row * (unsigned)g.W), b = (int)(row / (unsigned)g.H), py = (int)(row - (unsigned)(b * g.H));
+    const size_t plane = (size_t)g.H * g.W;
+    const float* in = x + (size_t)b * 4 * plane + (size_t)py * g.W + px;
+    float v[40];  // 4 tap + channel
+#pragma unroll
+    for (int t = 0; t < 9; t++) {
+        const int y = py + t / 3 - 1, xx = px + t % 3 - 1;
+        const bool in_image = y >= 0 && y < g.H && xx >= 0 && xx < g.W;
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            v[4 * t + c] = in_image ? in[c * plane + (ptrdiff_t)(t / 3 - 1) * g.W + (t % 3 - 1)] : 0.f;
+    }
+#pragma unroll
+    for (int c = 36; c < 40; c++) v[c] = 0.f;
+    uint16_t* const out = o + g.at(b, py, px) * kImCols;
+#pragma unroll
+    for (int j = 0; j < 32; j += 16) {
+        uint32_t h[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) h[e] = (uint32_t)f2bf(v[j + 2 * e]) | (uint32_t)f2bf(v[j + 2 * e + 1]) << 16;
+        st32(out + j, h);
+    }
     uint16_t h[8];
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const int tap = 2 * j + e / 4, c = e % 4, y = py + tap / 3 - 1, xx = px + tap % 3 - 1;
-        float v = 0.f;
-        if (tap < 9 && y >= 0 && y < g.H && xx >= 0 && xx < g.W) v = x[(((size_t)b * 4 + c) * g.H + y) * g.W + xx];
-        h[e] = f2bf(v);
-    }
-    st8(o + g.at(b, py, px) * kImCols + 8 * j, h);
+    for (int e = 0; e < 8; e++) h[e] = f2bf(v[32 + e]);
+    st8(out + 32, h);
 }
 
-// pixel and channel octet of element q of a batch's real pixels, pixels within octets of a row adjacent
+// pixel and channel octet of element q of a batch's real pixels, pixels within octets of a row adjacent; in
+// 32 bits where q fits (64-bit divisions are several times as long)
+template <class I>
+__device__ __forceinline__ bool octet_of(I q, const PadGeo& g, int C, int& b, int& y, int& x, int& c) {
+    const I noct = (I)(C >> 3), W = (I)g.W, H = (I)g.H;
+    I r = q / noct;
+    c = (int)(q - r * noct) * 8;
+    const I row = r / W;
+    x = (int)(r - row * W);
+    const I im = row / H;
+    y = (int)(row - im * H);
+    b = (int)im;
+    return im < (I)g.B;
+}
 __device__ __forceinline__ bool octet(size_t q, const PadGeo& g, int C, int& b, int& y, int& x, int& c) {
-    const int noct = C >> 3;
-    c = (int)(q % noct) * 8;
-    size_t r = q / noct;
-    x = (int)(r % g.W);
-    r /= g.W;
-    y = (int)(r % g.H);
-    b = (int)(r / g.H);
-    return b < g.B;
+    return q >> 32 ? octet_of(q, g, C, b, y, x, c) : octet_of((unsigned)q, g, C, b, y, x, c);
 }
 
 // 2x2 average of a tensor at twice the resolution, ((a+b)+c)+d in FP32
@@ -107,12 +133,6 @@ __global__ void k_pool(uint16_t* __restrict__ o, const uint16_t* __restrict__ in
 
 // epilogue of the forward GEMM: bias, ReLU, BF16; the nearest-neighbour upsampled copy beside it
 // where the next layer reads that
-// 32 bytes in one store: whole sectors, where 16-byte stores of a row per thread are halves of them
-__device__ __forceinline__ void st32(void* p, const uint32_t (&h)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]),
-                 "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7])
-                 : "memory");
-}
 struct FwdEpi {
     static constexpr bool kSums = false;
     static constexpr float* part = nullptr;
@@ -225,9 +245,10 @@ __global__ void k_pack_weights(uint16_t* __restrict__ wbd, uint16_t* __restrict_
 }
 
 // All layers' weight gradients from the splits' partial sums, dW[co][kk] = sum_z part[z][kk][co]: a warp adds
-// every eighth split of 32 weights (eight loads in flight), then the eight sums are added in order; with two
-// sources the rows' channels below c0 have ns0 partial sums, the others ns1.  One launch for the network:
-// a launch per layer lasted longer than its reads.
+// every eighth split of 128 weights (four a lane, four loads in flight), then the eight sums are added in
+// order; with two sources the rows' channels below c0 have ns0 partial sums, the others ns1.  One launch for
+// the network: a launch per layer lasted longer than its reads.  8 images of 512 x 256: 114 us with one weight
+// a lane, now 51.
 struct ReduceArgs {
     struct Layer {
         float* dW;
@@ -235,33 +256,44 @@ struct ReduceArgs {
         int ns0, ns1, c0, cin, M, N, block0;  // block0: its first block
     } l[14];
 };
+constexpr int kReduce = 128;  // weights of a block (a layer's count, 9 cin cout, is a multiple)
 __global__ void __launch_bounds__(256) k_wgrad_reduce(const __grid_constant__ ReduceArgs a) {
     pdl_begin();
-    __shared__ float sh[8][32];
+    __shared__ float4 sh[8][32];
     int li = 13;
     while (li > 0 && (int)blockIdx.x < a.l[li].block0) li--;
     const ReduceArgs::Layer& L = a.l[li];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int q = ((int)blockIdx.x - L.block0) * 32 + lane, kk = q / L.N, co = q - kk * L.N;  // N % 32 == 0
+    const int q = ((int)blockIdx.x - L.block0) * kReduce + 4 * lane, kk = q / L.N, co = q - kk * L.N;  // N % 32 == 0
     const int ns = kk % L.cin < L.c0 ? L.ns0 : L.ns1;
     const size_t ld = (size_t)L.M * L.N;
     const float* part = L.part + q;
-    float s = 0.f;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](const float4& v) {
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+    };
     int z = warp;
-    for (; z + 56 < ns; z += 64) {
-        float v[8];
+    for (; z + 24 < ns; z += 32) {
+        float4 v[4];
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = part[(size_t)(z + 8 * j) * ld];
+        for (int j = 0; j < 4; j++) v[j] = *reinterpret_cast<const float4*>(part + (size_t)(z + 8 * j) * ld);
 #pragma unroll
-        for (int j = 0; j < 8; j++) s += v[j];
+        for (int j = 0; j < 4; j++) add(v[j]);
     }
-    for (; z < ns; z += 8) s += part[(size_t)z * ld];
+    for (; z < ns; z += 8) add(*reinterpret_cast<const float4*>(part + (size_t)z * ld));
     sh[warp][lane] = s;
     __syncthreads();
     if (warp) return;
 #pragma unroll
-    for (int j = 1; j < 8; j++) s += sh[j][lane];
-    L.dW[(size_t)co * L.M + kk] = s;
+    for (int j = 1; j < 8; j++) add(sh[j][lane]);
+    float* const o = L.dW + (size_t)co * L.M + kk;
+    o[0] = s.x;
+    o[L.M] = s.y;
+    o[2 * L.M] = s.z;
+    o[3 * L.M] = s.w;
 }
 
 // Gradient of a layer's pre-activation as a GEMM operand, dZ = dY masked by Y > 0 in BF16, and per-block
@@ -775,7 +807,7 @@ static int unet_forward(UNet& U, int B, cudaEvent_t* ev = nullptr) {
     const size_t P0 = (size_t)B * U.H * U.W;
     int rc;
     if ((rc = plan_batch(U, B))) return rc;
-    if ((rc = launch_pdl("k_im2col", k_im2col, dim3(nblk(P0 * 5, 256)), dim3(256), 0, U.st, U.im, U.xin, U.geo(0, B))))
+    if ((rc = launch_pdl("k_im2col", k_im2col, dim3(nblk(P0, 256)), dim3(256), 0, U.st, U.im, U.xin, U.geo(0, B))))
         return rc;
     int li = 0;
     if (ev) CK(cudaEventRecord(ev[0], U.st));
@@ -877,7 +909,7 @@ static int unet_backward(UNet& U, int B, float* loss) {
     for (int li = 0; li < 14; li++) {
         const UConv& c = U.L[li];
         red.l[li].block0 = blocks;
-        blocks += red.l[li].M * red.l[li].N / 32;
+        blocks += red.l[li].M * red.l[li].N / kReduce;
         sum.l[li] = {U.g + c.boff, U.bpart + U.bpart_off[li], bsums[li], li == 13 ? 2 * c.cout + 1 : c.cout, 0,
                      c.cout, cols};
         cols += c.cout;
