@@ -424,9 +424,27 @@ __host__ __device__ constexpr int wgrad_box_bytes(int bw) { return (kWgradBox * 
 // instruction descriptor with both operands MN-major
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) { return idesc_bf16(n) | (1u << 15) | (1u << 16); }
 
-__global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_constant__ CUtensorMap mapA,
-                                                             const __grid_constant__ CUtensorMap mapB, WgradArgs a,
-                                                             int* err) {
+// The weight gradients of all layers in one launch: they depend on nothing of each other, and on a small grid
+// one layer's CTAs fill part of the chip for 7 us (gradients of 3 images of 136 x 72: 500 us with a launch per
+// layer and source, now 414).  first: a problem's first CTA; gx, gy: its CTAs over
+// blocks of channels and rows, and over tiles of N.
+constexpr int kMaxWgrads = 17;
+struct WgradGroup {
+    struct Problem {
+        CUtensorMap A, B;
+        WgradArgs a;
+        int first, gx, gy;
+    } p[kMaxWgrads];
+    int n, ctas;
+    size_t smem;
+};
+__global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_constant__ WgradGroup group, int* err) {
+    int pi = group.n - 1;
+    while (pi > 0 && (int)blockIdx.x < group.p[pi].first) pi--;
+    const WgradGroup::Problem& P = group.p[pi];
+    const WgradArgs& a = P.a;
+    const int cta = (int)blockIdx.x - P.first, bz = cta / (P.gx * P.gy), bxy = cta - bz * P.gx * P.gy, by = bxy / P.gx,
+              bx = bxy - by * P.gx;
     extern __shared__ unsigned char smem_raw[];
     __shared__ Ring ring;
     __shared__ uint64_t done;
@@ -434,7 +452,7 @@ __global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_const
     __shared__ int bad;
     unsigned char* const smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int n0 = blockIdx.y * a.Ntile, S = a.S;
+    const int n0 = by * a.Ntile, S = a.S;
     const uint32_t sbytes = (uint32_t)(a.abytes + a.bbytes);
     if (tid == 0) {
         bad = 0;
@@ -448,8 +466,8 @@ __global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_const
     tc_fence_after();
     pdl_begin();
     const uint32_t taddr = tslot;
-    const int cbeg = blockIdx.z * a.per, cend = min(a.chunks, cbeg + a.per), n = max(0, cend - cbeg);
-    const int nch = a.C / a.bw, unit = blockIdx.x / nch, ch = (blockIdx.x - unit * nch) * a.bw;
+    const int cbeg = bz * a.per, cend = min(a.chunks, cbeg + a.per), n = max(0, cend - cbeg);
+    const int nch = a.C / a.bw, unit = bx / nch, ch = (bx - unit * nch) * a.bw;
     const int bblk = a.Ntile / a.bwB, nacc = a.taps == 1 || a.bw == 32 ? 1 : 2;  // accumulators
     const int shift = a.taps == 1 ? 0 : (unit - 1) * a.g.Wp() - 1;                // of tap -1 of the row
     const uint32_t bbox = (uint32_t)(kWgradK * a.bwB * 2);
@@ -464,9 +482,9 @@ __global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_const
             unsigned char* sa = smem + r.i * sbytes;
             if (elect_one()) {
                 mbar_expect(ring.full + r.i, (uint32_t)(kWgradBox * a.bw * 2) + (uint32_t)bblk * bbox);
-                tma_load_2d(sa, &mapA, ch, p + shift, ring.full + r.i);
+                tma_load_2d(sa, &P.A, ch, p + shift, ring.full + r.i);
                 for (int q = 0; q < bblk; q++)
-                    tma_load_2d(sa + a.abytes + q * bbox, &mapB, n0 + q * a.bwB, p, ring.full + r.i);
+                    tma_load_2d(sa + a.abytes + q * bbox, &P.B, n0 + q * a.bwB, p, ring.full + r.i);
             }
             __syncwarp();
             r.next(S);
@@ -515,7 +533,7 @@ __global__ void __launch_bounds__(kWgradThreads) k_wgrad_gemm(const __grid_const
                 __syncwarp();
                 tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * a.Ntile + c0), v);
                 if (!ok || !real) continue;
-                float* o = a.part + ((size_t)blockIdx.z * a.kk_max + kk) * a.N + n0 + c0;
+                float* o = a.part + ((size_t)bz * a.kk_max + kk) * a.N + n0 + c0;
 #pragma unroll
                 for (int j = 0; j < 32; j += 4)
                     *reinterpret_cast<float4*>(o + j) = n > 0 ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3])

@@ -487,15 +487,9 @@ struct ConvPlan {
     tc::ConvArgs a;
     dim3 grid;
 };
-struct WgradPlan {
-    CUtensorMap A, B;
-    tc::WgradArgs a;
-    dim3 grid;
-};
 struct LayerPlan {
     ConvPlan fwd, bwd;
-    WgradPlan wg[2];
-    int nwg = 0, nsplit[2] = {};
+    int nwg = 0, nsplit[2] = {}, c0 = 0;  // weight gradient: sources, their splits, the first one's channels
 };
 
 struct UNet {
@@ -514,6 +508,7 @@ struct UNet {
     size_t part_cap = 0, part_off[14] = {}, bpart_off[15] = {};  // of a layer's partial sums in part, in bpart
     int planB = 0;  // batch size of the plans
     LayerPlan plan[14];
+    tc::WgradGroup wg;
     int* derr = nullptr;
     cudaStream_t st = nullptr;
     std::vector<void*> owned;
@@ -747,6 +742,8 @@ static int plan_conv(ConvPlan& P, PadGeo g, int taps, int nsrc, const uint16_t* 
 static int plan_batch(UNet& U, int B) {
     if (U.planB == B) return 0;
     U.planB = 0;
+    U.wg.n = U.wg.ctas = 0;
+    U.wg.smem = 0;
     if (layout_partials(U, B) > U.part_cap) return fail(PT_ERR_STATE, "U-Net: split workspace too small");
     int rc;
     for (size_t li = 0; li < U.L.size(); li++) {
@@ -763,8 +760,9 @@ static int plan_batch(UNet& U, int B) {
         const int Cz[2] = {c.cout, 0};
         if (!first && (rc = plan_conv(P.bwd, g, 9, 1, z, Cz, U.wbd + c.woff, c.cin, c.mode == 0))) return rc;
         P.nwg = ns;
+        P.c0 = C[0];
         for (int s = 0; s < ns; s++) {
-            WgradPlan& w = P.wg[s];
+            tc::WgradGroup::Problem& w = U.wg.p[U.wg.n++];
             tc::WgradArgs& a = w.a;
             const WgradShape sh = wgrad_shape(first ? 1 : 9, C[s], c.cout, g.positions());
             P.nsplit[s] = sh.ns;
@@ -784,8 +782,12 @@ static int plan_batch(UNet& U, int B) {
             a.abytes = tc::wgrad_box_bytes(a.bw);
             a.bbytes = a.Ntile * tc::kWgradK * 2;
             a.part = U.part + U.part_off[li];
-            w.grid = dim3(sh.units, c.cout / a.Ntile, sh.ns);
+            w.first = U.wg.ctas;
+            w.gx = sh.units;
+            w.gy = c.cout / a.Ntile;
+            U.wg.ctas += w.gx * w.gy * sh.ns;
             a.S = std::min(std::min(110 * 1024 / (a.abytes + a.bbytes), tc::kMaxRing), sh.per);  // two CTAs on an SM
+            U.wg.smem = std::max(U.wg.smem, tc::wgrad_smem(a));
             if ((rc = tensor_map(&w.A, t[s], C[s], g.positions(), a.bw, tc::kWgradBox)) ||
                 (rc = tensor_map(&w.B, U.dz[c.out], c.cout, g.positions(), a.bwB, tc::kWgradK)))
                 return rc;
@@ -870,12 +872,8 @@ static int unet_backward(UNet& U, int B, float* loss) {
         const LayerPlan& P = U.plan[li];
         // weights: split over positions; the splits are added at the end, for all layers
         const int M = 9 * c.cin;
-        red.l[li] = {U.g + c.woff, U.part + U.part_off[li], P.nsplit[0], P.nsplit[1], P.nwg > 1 ? P.wg[0].a.C : M,
+        red.l[li] = {U.g + c.woff, U.part + U.part_off[li], P.nsplit[0], P.nsplit[1], P.nwg > 1 ? P.c0 : M,
                      P.nwg > 1 ? c.cin : M, M, c.cout, 0};
-        for (int s = 0; s < P.nwg; s++)
-            if ((rc = launch_pdl("k_wgrad_gemm", tc::k_wgrad_gemm, P.wg[s].grid, dim3(tc::kWgradThreads),
-                                 tc::wgrad_smem(P.wg[s].a), U.st, P.wg[s].A, P.wg[s].B, P.wg[s].a, U.derr)))
-                return rc;
         if (c.src0 < 0) continue;  // the network input needs no gradient
         if (c.mode == 0) {
             const DzEpi e{U.act[c.src0], U.dz[c.src0], c.cin, U.bpart + U.bpart_off[c.src0]};
@@ -921,7 +919,9 @@ static int unet_backward(UNet& U, int B, float* loss) {
     sum.l[14].n = U.L[13].cout + 1;
     sum.l[14].col0 = cols;
     sum.total = cols + sum.l[14].n;
-    if ((rc = launch_pdl("k_wgrad_reduce", k_wgrad_reduce, dim3(blocks), dim3(256), 0, U.st, red)) ||
+    if ((rc = launch_pdl("k_wgrad_gemm", tc::k_wgrad_gemm, dim3(U.wg.ctas), dim3(tc::kWgradThreads), U.wg.smem, U.st, U.wg,
+                         U.derr)) ||
+        (rc = launch_pdl("k_wgrad_reduce", k_wgrad_reduce, dim3(blocks), dim3(256), 0, U.st, red)) ||
         (rc = launch_pdl("k_colsum", k_colsum, dim3(nblk(sum.total, 4)), dim3(128), 0, U.st, sum)))
         return rc;
     std::vector<float> lp(nb);
