@@ -547,17 +547,20 @@ static int pack_weights(UNet& U) {
 }
 
 // The shape of a source's weight gradient: columns of a tile, CTAs over blocks of channels and image rows,
-// and the splits over the positions: one and a half CTAs per SM in all (1, 1.5 and 2 are within 3 % on
-// 8 images of 512 x 256), and at least four chunks each
+// and the splits over the positions: 304 over every 128 of the layer's 9 cin rows, and at least eight chunks
+// each.  (The layers share a launch, so a layer alone need not fill the chip: a third as many splits or half as
+// many again change the time for 8 images of 512 x 256 by 1 %.  An accumulator's rounding error grows with its
+// chain: these lengths are those of the GEMM that gathered its tiles, and the gradients of 12 batches agree
+// with its own to 4e-7 to 9e-7, where other lengths leave 4e-6 to 6e-5.)
 struct WgradShape {
     int ntile, units, per, ns;
 };
-static WgradShape wgrad_shape(int taps, int C, int cout, size_t positions) {
+static WgradShape wgrad_shape(int taps, int cin, int C, int cout, size_t positions) {
     WgradShape w;
     w.ntile = std::min(cout, 128);
     w.units = C / (C % 64 == 0 ? 64 : 32) * (taps == 1 ? 1 : 3);
-    const int chunks = (int)((positions + tc::kWgradK - 1) / tc::kWgradK), tiles = w.units * (cout / w.ntile);
-    const int n0 = std::max(1, std::min((chunks + 3) / 4, 228 / tiles));
+    const int chunks = (int)((positions + tc::kWgradK - 1) / tc::kWgradK), rows = (9 * cin + 127) / 128;
+    const int n0 = std::max(1, std::min((chunks + 7) / 8, 304 / rows));
     w.per = (chunks + n0 - 1) / n0;
     w.ns = (chunks + w.per - 1) / w.per;
     return w;
@@ -571,7 +574,7 @@ static size_t layout_partials(UNet& U, int B) {
         const int C0 = c.src0 < 0 ? kImCols : U.tch[c.src0], C1 = c.mode == 2 ? U.tch[c.src1] : 0;
         int ns = 0;
         for (int C : {C0, C1})
-            if (C) ns = std::max(ns, wgrad_shape(c.src0 < 0 ? 1 : 9, C, c.cout, U.geo(c.level, B).positions()).ns);
+            if (C) ns = std::max(ns, wgrad_shape(c.src0 < 0 ? 1 : 9, c.cin, C, c.cout, U.geo(c.level, B).positions()).ns);
         U.part_off[li] = n;
         n += (size_t)ns * 9 * c.cin * c.cout;
     }
@@ -764,7 +767,7 @@ static int plan_batch(UNet& U, int B) {
         for (int s = 0; s < ns; s++) {
             tc::WgradGroup::Problem& w = U.wg.p[U.wg.n++];
             tc::WgradArgs& a = w.a;
-            const WgradShape sh = wgrad_shape(first ? 1 : 9, C[s], c.cout, g.positions());
+            const WgradShape sh = wgrad_shape(first ? 1 : 9, c.cin, C[s], c.cout, g.positions());
             P.nsplit[s] = sh.ns;
             a.g = g;
             a.taps = first ? 1 : 9;
@@ -840,7 +843,7 @@ static int gemm_error(UNet& U) {
 
 static int dz_blocks(const UNet& U, const UConv& c, int B) {
     const size_t oct = (size_t)B * (U.H >> c.level) * (U.W >> c.level) * (c.cout / 8);
-    return (int)std::min<size_t>(nblk(oct, 4 * kDzThreads), kDzBlocks);
+    return (int)std::min<size_t>(nblk(oct, kDzThreads), kDzBlocks);
 }
 // dZ of the layer that produced tensor t from where its gradient lies, and the partial sums of its bias gradient
 template <int MODE>
