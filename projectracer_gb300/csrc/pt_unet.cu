@@ -141,11 +141,17 @@ struct FwdEpi {
     int C;
     uint16_t* up;
     PadGeo gup;
+    // the last layer: the 1x1 output convolution (linear, FP32 out), its weights and bias, [B][H][W] of g
+    float* y;
+    const float *ow, *ob;
+    PadGeo g;
     __device__ __forceinline__ void stage(float* sb, int n, int tid) const {
         for (int c = tid; c < n; c += tc::kConvThreads) sb[c] = bias[c];
+        if (y && tid <= 32) sb[32 + tid] = tid < 32 ? ow[tid] : ob[0];  // (n = 32)
     }
-    __device__ __forceinline__ void operator()(int p, int b, int y, int x, int c0, const float (&v)[32],
+    __device__ __forceinline__ void operator()(int p, int b, int py, int x, int c0, const float (&v)[32],
                                                const float* sb) const {
+        float s = y ? sb[64] : 0.f;
 #pragma unroll
         for (int j = 0; j < 32; j += 16) {
             uint32_t h[8];
@@ -154,9 +160,13 @@ struct FwdEpi {
                 h[e] = (uint32_t)f2bf(fmaxf(v[j + 2 * e] + sb[j + 2 * e], 0.f)) |
                        (uint32_t)f2bf(fmaxf(v[j + 2 * e + 1] + sb[j + 2 * e + 1], 0.f)) << 16;
             st32(out + (size_t)p * C + c0 + j, h);
+            if (y)
+#pragma unroll
+                for (int c = 0; c < 16; c++) s += bf2f((uint16_t)(h[c >> 1] >> (16 * (c & 1)))) * sb[32 + j + c];
             if (up)
-                for (int q = 0; q < 4; q++) st32(up + gup.at(b, 2 * y + (q >> 1), 2 * x + (q & 1)) * C + c0 + j, h);
+                for (int q = 0; q < 4; q++) st32(up + gup.at(b, 2 * py + (q >> 1), 2 * x + (q & 1)) * C + c0 + j, h);
         }
+        if (y) y[((size_t)b * g.H + py) * g.W + x] = s;
     }
     __device__ __forceinline__ void sums(int, bool, int, const float (&)[32], float*) const {}
 };
@@ -415,23 +425,6 @@ __global__ void __launch_bounds__(128) k_colsum(const __grid_constant__ ColsumAr
     if (lane == 0) L.out[c] = s;
 }
 
-// 1x1 output convolution (linear, FP32 out)
-__global__ void k_out_fwd(float* y, const uint16_t* d, const float* w, const float* b, PadGeo g) {
-    pdl_begin();
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= g.B * g.H * g.W) return;
-    const int x = p % g.W, r = p / g.W;
-    const uint16_t* in = d + g.at(r / g.H, r % g.H, x) * 32;
-    float s = b[0];
-#pragma unroll
-    for (int c = 0; c < 32; c += 8) {
-        float f[8];
-        unpack8(ld8(in + c), f);
-#pragma unroll
-        for (int j = 0; j < 8; j++) s += f[j] * w[c + j];
-    }
-    y[p] = s;
-}
 // loss = mean (y - t)^2; dy = 2 (y - t) / P; per-block partial sums of (y - t)^2
 __global__ void k_mse(float* dy, float* lpart, const float* y, const float* t, int P) {
     pdl_begin();
@@ -824,13 +817,13 @@ static int unet_forward(UNet& U, int B, cudaEvent_t* ev = nullptr) {
                                  U.geo(c.level - 1, B), c.cin)))
                 return rc;
         }
-        const FwdEpi e{U.act[c.out], U.w32 + c.boff, c.cout, U.up[c.out], U.geo(c.level > 0 ? c.level - 1 : 0, B)};
+        const FwdEpi e{U.act[c.out], U.w32 + c.boff, c.cout, U.up[c.out], U.geo(c.level > 0 ? c.level - 1 : 0, B),
+                       c.out == 13 ? U.y : nullptr, U.w32 + U.out_w, U.w32 + U.out_b, U.geo(0, B)};
         if ((rc = run_conv(U, U.plan[li].fwd, e))) return rc;
         li++;
         if (ev) CK(cudaEventRecord(ev[li], U.st));
     }
-    return launch_pdl("k_out_fwd", k_out_fwd, dim3(nblk(P0, 128)), dim3(128), 0, U.st, U.y, U.act[13], U.w32 + U.out_w,
-                      U.w32 + U.out_b, U.geo(0, B));
+    return 0;
 }
 
 static int gemm_error(UNet& U) {
