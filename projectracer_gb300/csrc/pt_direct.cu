@@ -14,10 +14,11 @@
 // The band LU is the reference's unblocked algorithm (the LAPACK DGBTF2 that its DGBTRF call runs
 // at these band widths): for each column, a pivot search, a row interchange over the columns the
 // pivot reaches, the column scaled by the pivot's reciprocal, and a rank-1 update of the trailing
-// kl x (ju - j) block.  The update is spread over the whole GPU: one cooperative kernel, one CTA per
-// SM, the column steps separated by grid barriers (bounded spins that report a timeout instead of
-// waiting forever).  Every element sees the same operations in the same order as in DGBTF2 and this
-// file is compiled with --fmad=false, so the factors round exactly like the reference's.
+// kl x (ju - j) block.  Bands of up to 464 sub-diagonals are factored in panels (pt_bandlu.cuh); for wider ones
+// the update is spread over the whole GPU: one cooperative kernel, one CTA per SM, the column steps separated by
+// grid barriers (bounded spins that report a timeout instead of waiting forever).  Either way every element sees
+// the same operations in the same order as in DGBTF2 and both files are compiled with --fmad=false, so the
+// factors round exactly like the reference's.
 #include <cmath>
 #include <cstring>
 

@@ -27,3 +27,20 @@ def test_solves_on_coarse_grids_of_every_remainder_match_the_oracle(nx, nz, roun
     # the bound of the solve's other comparisons with the oracle: sums that differ in the last bits
     assert rel_err(e.get(eng.F_SF), o.get(7)) < 1e-10
     e.close()
+
+
+# two levels only, so that the inverse takes eight columns a CTA: 49 x 33 = 1617 nodes (a last panel of one
+# column, a last CTA of one) and 41 x 33 = 1353 (nine columns, one)
+@pytest.mark.parametrize("nx,nz", [(96, 64), (80, 64)])
+def test_solves_with_two_levels_match_the_oracle(nx, nz):
+    cfg, st = small_case("chem", nx=nx, nz=nz)
+    cfg.grids = 2
+    o = Oracle(cfg, iterate=1, nparts=0)
+    o.load_restart(st["xg"], st["zg"], st["T"], st["Cnew"], st["SF"], st["rtr"], st["str"], st["Ctr"], st["Ttr"])
+    e = eng.Engine(cfg)
+    e.upload(st)
+    info = e.solve_psi()
+    o.solve_psi()
+    assert info["cycles"] == int(o.scalar("cycles"))
+    assert rel_err(e.get(eng.F_SF), o.get(7)) < 1e-10
+    e.close()
