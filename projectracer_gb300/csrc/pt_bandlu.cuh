@@ -246,7 +246,8 @@ __global__ void k_band_top(const double* ab, int n, int kl, int ku, Work w) {
 // memory, twice for the forward pass, whose interchanges permute it.
 // What bounds it is the FP64 rate (n^2 (kl / 2 + ku) multiply-subtract pairs): n = 2145, kl = ku = 99:
 // 11.2 ms with a warp per column (a division per column and step, partly filled warps, the zeros of U
-// above its entries), 6.5 now; n = 561, kl = ku = 51: 0.65 before and now.
+// above its entries), 6.5 now; n = 561, kl = ku = 51: 0.65 before and now.  A grid of fewer CTAs than groups
+// of columns takes them in turn (see inverse).
 constexpr int kInvThreads = 256, kInvCols = 4;  // columns of a thread
 static inline int pow2_above(int v) {
     int w = 32;
@@ -265,160 +266,209 @@ __global__ void __launch_bounds__(kInvThreads, 2) k_band_inverse(const double* _
     __shared__ __align__(16) double ys[kPanel][COLS];
     __shared__ double ut[2][kPanel][kPanel], rec[2][kPanel];  // ut[.][jj][r] = U(j0 + r, j0 + jj)
     const int ldab = 2 * kl + ku + 1, kv = ku + kl, LD = w.LD, np = (n + kPanel - 1) / kPanel;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = blockIdx.x * COLS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = lane & 15, col = 2 * warp + (lane >> 4);  // of the triangle: warps below COLS / 2
-    const bool tri = warp < COLS / 2, live = tri && c0 + col < n;
+    const bool tri = warp < COLS / 2;
     const int h4 = (tid % H) * kInvCols;
 
-    // forward
-    const int ps = max(0, (c0 - LD + kPanel) / kPanel);  // the first panel that reaches row c0
-    for (int q = tid; q < min(ps * kPanel, n) * COLS; q += kInvThreads)
-        if (c0 + q % COLS < n) G[(size_t)(q / COLS) * n + c0 + q % COLS] = 0.0;
-    double* A = win;                      // the panel's window, row i in slot i mod WF
-    double* B = win + (size_t)WF * COLS;  // the next one's
-    auto enter = [&](double* W, int from, int to) {
-        for (int q = from * COLS + tid; q < to * COLS; q += kInvThreads)
-            W[(size_t)(q / COLS & (WF - 1)) * COLS + q % COLS] = q / COLS == c0 + q % COLS ? 1.0 : 0.0;
-    };
-    enter(A, ps * kPanel, min(n, ps * kPanel + LD));
-    __syncthreads();
-    for (int p = ps; p < np; p++) {
-        const int j0 = p * kPanel, R = min(LD, n - j0), nb = min(kPanel, n - j0);
-        const double* const L = w.l(p);
-        const int* const perm = w.p(p);
-        double l[kPanel];
-        int it = tid;  // item: row kPanel + it / H, columns h4 ..
-        const int items = max(0, R - kPanel) * H;
-        auto load = [&](int r) {
-#pragma unroll
-            for (int jj = 0; jj < kPanel; jj++) l[jj] = L[(size_t)jj * LD + r];
-        };
-        if (tri) {
-            double t = row < nb ? A[(size_t)((j0 + perm[row]) & (WF - 1)) * COLS + col] : 0.0;
-            if (row < nb) load(row);
-#pragma unroll
-            for (int jj = 0; jj < kPanel; jj++) {
-                const double y = __shfl_sync(0xffffffffu, t, jj + (lane & 16));
-                const double u = F.add(t, F.mul(l[jj], -y));
-                if (row > jj && row < nb) t = u;
-            }
-            ys[row][col] = t;
-            if (live && row < nb) G[(size_t)(j0 + row) * n + c0 + col] = t;
-        }
-        if (it < items) load(kPanel + it / H);
-        __syncthreads();
-        for (; it < items; it += kInvThreads) {
-            const int r = kPanel + it / H;
-            if (it != tid) load(r);
-            const double* a = A + (size_t)((j0 + perm[r]) & (WF - 1)) * COLS + h4;
-            double v[kInvCols];
-#pragma unroll
-            for (int c = 0; c < kInvCols; c++) v[c] = a[c];
-#pragma unroll
-            for (int jj = 0; jj < kPanel; jj++) {
-                const volatile double* y = &ys[jj][h4];  // (volatile: 64 values loaded ahead would fill the registers)
-#pragma unroll
-                for (int c = 0; c < kInvCols; c++) v[c] = F.add(v[c], F.mul(l[jj], -y[c]));
-            }
-            double* b = B + (size_t)((j0 + r) & (WF - 1)) * COLS + h4;
-#pragma unroll
-            for (int c = 0; c < kInvCols; c++) b[c] = v[c];
-        }
-        enter(B, min(n, j0 + LD), min(n, j0 + kPanel + LD));
-        __syncthreads();
-        double* const x = A;
-        A = B;
-        B = x;
-    }
+    for (int c0 = blockIdx.x * COLS; c0 < n; c0 += gridDim.x * COLS) {
+        const bool live = tri && c0 + col < n;
 
-    // back: row i in slot i mod WB
-    auto fetch = [&](int p, int buf) {  // a panel's triangle: threads 0 .. 255, (jj, r)
-        const int jj = tid / kPanel, r = tid % kPanel, j = p * kPanel + jj;
-        const double u = j < n && r <= jj ? ab[(size_t)j * ldab + kv + r - jj] : 1.0;
-        ut[buf][jj][r] = u;
-        if (r == jj) rec[buf][jj] = 1.0 / u;
-    };
-    int lo = max(0, (np - 1) * kPanel - kv);  // rows lo .. are in the window
-    for (int q = lo * COLS + tid; q < n * COLS; q += kInvThreads)
-        win[(size_t)(q / COLS & (WB - 1)) * COLS + q % COLS] = c0 + q % COLS < n ? G[(size_t)(q / COLS) * n + c0 + q % COLS] : 0.0;
-    fetch(np - 1, 0);
-    __syncthreads();
-    for (int p = np - 1, buf = 0; p >= 0; p--, buf ^= 1) {
-        const int j0 = p * kPanel, nb = min(kPanel, n - j0), top = tops ? w.top[p] : max(0, j0 - kv);
-        double u[kPanel];
-        auto load = [&](int i) {
-#pragma unroll
-            for (int jj = 0; jj < kPanel; jj++)
-                u[jj] = j0 + jj < n && i >= j0 + jj - kv ? ab[(size_t)(j0 + jj) * ldab + kv + i - j0 - jj] : 0.0;
+        // forward
+        const int ps = max(0, (c0 - LD + kPanel) / kPanel);  // the first panel that reaches row c0
+        for (int q = tid; q < min(ps * kPanel, n) * COLS; q += kInvThreads)
+            if (c0 + q % COLS < n) G[(size_t)(q / COLS) * n + c0 + q % COLS] = 0.0;
+        double* A = win;                      // the panel's window, row i in slot i mod WF
+        double* B = win + (size_t)WF * COLS;  // the next one's
+        auto enter = [&](double* W, int from, int to) {
+            for (int q = from * COLS + tid; q < to * COLS; q += kInvThreads)
+                W[(size_t)(q / COLS & (WF - 1)) * COLS + q % COLS] = q / COLS == c0 + q % COLS ? 1.0 : 0.0;
         };
-        // rows that enter for the next panel
-        const int next = max(0, j0 - kPanel - kv), entering = (lo - next) * COLS;
-        double e = 0.0;
-        if (tid < entering && c0 + tid % COLS < n) e = G[(size_t)(next + tid / COLS) * n + c0 + tid % COLS];
-        int it = tid;  // item: row top + it / H
-        const int items = (j0 - top) * H;
-        if (it < items) load(top + it / H);
-        if (tri) {
-            double t = row < nb ? win[(size_t)((j0 + row) & (WB - 1)) * COLS + col] : 0.0;
-#pragma unroll
-            for (int jj = kPanel - 1; jj >= 0; jj--) {
-                if (jj >= nb) continue;
-                const double y = __shfl_sync(0xffffffffu, t, jj + (lane & 16)), d = ut[buf][jj][jj];
-                double x = y;
-                if (nonzero(y)) x = in_range(y, 800) && in_range(d, 100) ? quotient(y, d, rec[buf][jj]) : y / d;
-                __syncwarp();
-                const double s = F.sub(t, F.mul(x, ut[buf][jj][row]));
-                if (row < jj) t = s;
-                if (row == jj) t = x;
-            }
-            ys[row][col] = row < nb ? t : 0.0;
-            if (live && row < nb) G[(size_t)(j0 + row) * n + c0 + col] = t;
-        }
-        if (p > 0) fetch(p - 1, buf ^ 1);
+        enter(A, ps * kPanel, min(n, ps * kPanel + LD));
         __syncthreads();
-        for (; it < items; it += kInvThreads) {
-            const int i = top + it / H;
-            if (it != tid) load(i);
-            double* a = win + (size_t)(i & (WB - 1)) * COLS + h4;
-            double v[kInvCols];
-#pragma unroll
-            for (int c = 0; c < kInvCols; c++) v[c] = a[c];
-#pragma unroll
-            for (int jj = kPanel - 1; jj >= 0; jj--) {
-                const volatile double* y = &ys[jj][h4];
-#pragma unroll
-                for (int c = 0; c < kInvCols; c++) v[c] = F.sub(v[c], F.mul(y[c], u[jj]));
+        for (int p = ps; p < np; p++) {
+            const int j0 = p * kPanel, R = min(LD, n - j0), nb = min(kPanel, n - j0);
+            const double* const L = w.l(p);
+            const int* const perm = w.p(p);
+            double l[kPanel];
+            int it = tid;  // item: row kPanel + it / H, columns h4 ..
+            const int items = max(0, R - kPanel) * H;
+            auto load = [&](int r) {
+    #pragma unroll
+                for (int jj = 0; jj < kPanel; jj++) l[jj] = L[(size_t)jj * LD + r];
+            };
+            if (tri) {
+                double t = row < nb ? A[(size_t)((j0 + perm[row]) & (WF - 1)) * COLS + col] : 0.0;
+                if (row < nb) load(row);
+    #pragma unroll
+                for (int jj = 0; jj < kPanel; jj++) {
+                    const double y = __shfl_sync(0xffffffffu, t, jj + (lane & 16));
+                    const double u = F.add(t, F.mul(l[jj], -y));
+                    if (row > jj && row < nb) t = u;
+                }
+                ys[row][col] = t;
+                if (live && row < nb) G[(size_t)(j0 + row) * n + c0 + col] = t;
             }
-#pragma unroll
-            for (int c = 0; c < kInvCols; c++) a[c] = v[c];
+            if (it < items) load(kPanel + it / H);
+            __syncthreads();
+            for (; it < items; it += kInvThreads) {
+                const int r = kPanel + it / H;
+                if (it != tid) load(r);
+                const double* a = A + (size_t)((j0 + perm[r]) & (WF - 1)) * COLS + h4;
+                double v[kInvCols];
+    #pragma unroll
+                for (int c = 0; c < kInvCols; c++) v[c] = a[c];
+    #pragma unroll
+                for (int jj = 0; jj < kPanel; jj++) {
+                    const volatile double* y = &ys[jj][h4];  // (volatile: 64 values loaded ahead would fill the registers)
+    #pragma unroll
+                    for (int c = 0; c < kInvCols; c++) v[c] = F.add(v[c], F.mul(l[jj], -y[c]));
+                }
+                double* b = B + (size_t)((j0 + r) & (WF - 1)) * COLS + h4;
+    #pragma unroll
+                for (int c = 0; c < kInvCols; c++) b[c] = v[c];
+            }
+            enter(B, min(n, j0 + LD), min(n, j0 + kPanel + LD));
+            __syncthreads();
+            double* const x = A;
+            A = B;
+            B = x;
         }
-        if (tid < entering) win[(size_t)((next + tid / COLS) & (WB - 1)) * COLS + tid % COLS] = e;
-        lo = next;
+
+        // back: row i in slot i mod WB
+        auto fetch = [&](int p, int buf) {  // a panel's triangle: threads 0 .. 255, (jj, r)
+            const int jj = tid / kPanel, r = tid % kPanel, j = p * kPanel + jj;
+            const double u = j < n && r <= jj ? ab[(size_t)j * ldab + kv + r - jj] : 1.0;
+            ut[buf][jj][r] = u;
+            if (r == jj) rec[buf][jj] = 1.0 / u;
+        };
+        int lo = max(0, (np - 1) * kPanel - kv);  // rows lo .. are in the window
+        for (int q = lo * COLS + tid; q < n * COLS; q += kInvThreads)
+            win[(size_t)(q / COLS & (WB - 1)) * COLS + q % COLS] = c0 + q % COLS < n ? G[(size_t)(q / COLS) * n + c0 + q % COLS] : 0.0;
+        fetch(np - 1, 0);
         __syncthreads();
+        for (int p = np - 1, buf = 0; p >= 0; p--, buf ^= 1) {
+            const int j0 = p * kPanel, nb = min(kPanel, n - j0), top = tops ? w.top[p] : max(0, j0 - kv);
+            double u[kPanel];
+            auto load = [&](int i) {
+    #pragma unroll
+                for (int jj = 0; jj < kPanel; jj++)
+                    u[jj] = j0 + jj < n && i >= j0 + jj - kv ? ab[(size_t)(j0 + jj) * ldab + kv + i - j0 - jj] : 0.0;
+            };
+            // rows that enter for the next panel
+            const int next = max(0, j0 - kPanel - kv), entering = (lo - next) * COLS;
+            double e = 0.0;
+            if (tid < entering && c0 + tid % COLS < n) e = G[(size_t)(next + tid / COLS) * n + c0 + tid % COLS];
+            int it = tid;  // item: row top + it / H
+            const int items = (j0 - top) * H;
+            if (it < items) load(top + it / H);
+            if (tri) {
+                double t = row < nb ? win[(size_t)((j0 + row) & (WB - 1)) * COLS + col] : 0.0;
+    #pragma unroll
+                for (int jj = kPanel - 1; jj >= 0; jj--) {
+                    if (jj >= nb) continue;
+                    const double y = __shfl_sync(0xffffffffu, t, jj + (lane & 16)), d = ut[buf][jj][jj];
+                    double x = y;
+                    if (nonzero(y)) x = in_range(y, 800) && in_range(d, 100) ? quotient(y, d, rec[buf][jj]) : y / d;
+                    __syncwarp();
+                    const double s = F.sub(t, F.mul(x, ut[buf][jj][row]));
+                    if (row < jj) t = s;
+                    if (row == jj) t = x;
+                }
+                ys[row][col] = row < nb ? t : 0.0;
+                if (live && row < nb) G[(size_t)(j0 + row) * n + c0 + col] = t;
+            }
+            if (p > 0) fetch(p - 1, buf ^ 1);
+            __syncthreads();
+            for (; it < items; it += kInvThreads) {
+                const int i = top + it / H;
+                if (it != tid) load(i);
+                double* a = win + (size_t)(i & (WB - 1)) * COLS + h4;
+                double v[kInvCols];
+    #pragma unroll
+                for (int c = 0; c < kInvCols; c++) v[c] = a[c];
+    #pragma unroll
+                for (int jj = kPanel - 1; jj >= 0; jj--) {
+                    const volatile double* y = &ys[jj][h4];
+    #pragma unroll
+                    for (int c = 0; c < kInvCols; c++) v[c] = F.sub(v[c], F.mul(y[c], u[jj]));
+                }
+    #pragma unroll
+                for (int c = 0; c < kInvCols; c++) a[c] = v[c];
+            }
+            if (tid < entering) win[(size_t)((next + tid / COLS) & (WB - 1)) * COLS + tid % COLS] = e;
+            lo = next;
+            __syncthreads();
+        }
     }
 }
 
-// eight columns per CTA where that leaves more than one CTA per SM, else four
-static int inverse(const double* ab, double* G, int n, int kl, int ku, const Work& w, cudaStream_t st) {
+// Eight columns per CTA where that leaves more than one CTA per SM, else four.
+// clusters = 0: a CTA per group of columns, the whole chip.  Otherwise (beside the solves of another stream) that
+// many clusters of kInvCluster CTAs, one CTA an SM: the CTAs are independent, the clusters only keep them on a
+// few GPCs.  Two CTAs fill an SM's registers, and one on every SM leaves no 16 SMs of a GPC to the cycle's cluster
+// kernels (pt_cluster.cuh), so a solve that met the whole-chip form waited for its end: with n = 2145 one of
+// 1.6 ms took 5.0 (2048x1024), one of 0.62 took 2.95 (1024x512, five levels); beside six clusters (10.6 ms
+// instead of 6.1) 2.0 and 0.72.
+constexpr int kInvCluster = 16;
+constexpr size_t kInvAlone = 116 * 1024;  // shared memory that a second CTA does not find on an SM
+static inline size_t inverse_smem_alone(int kl, int ku, int cols) {
+    const size_t b = inverse_smem(kl, ku, cols);
+    return b > kInvAlone ? b : kInvAlone;
+}
+static inline int inverse_cols(int n) { return n > 8 * 152 ? 8 : 4; }
+static int inverse(const double* ab, double* G, int n, int kl, int ku, const Work& w, cudaStream_t st, int clusters = 0) {
     const int WF = pow2_above(kl + 2 * kPanel), WB = pow2_above(kl + ku + 2 * kPanel);
     const int tops = n > 256;  // (a launch costs more than a small band's zeros)
     if (tops) PT_COUNT(), k_band_top<<<panels(n), 128, 0, st>>>(ab, n, kl, ku, w);
-    if (n > 8 * 152)
-        PT_COUNT(), k_band_inverse<8><<<(n + 7) / 8, kInvThreads, inverse_smem(kl, ku, 8), st>>>(ab, G, n, kl, ku, w, tops,
-                                                                                              WF, WB, FmaForms());
-    else
-        PT_COUNT(), k_band_inverse<4><<<(n + 3) / 4, kInvThreads, inverse_smem(kl, ku, 4), st>>>(ab, G, n, kl, ku, w, tops,
-                                                                                              WF, WB, FmaForms());
-    return cuda_check(cudaGetLastError(), "k_band_inverse");
+    const int cols = inverse_cols(n), groups = (n + cols - 1) / cols;
+    const auto kernel = cols == 8 ? k_band_inverse<8> : k_band_inverse<4>;
+    if (clusters == 0) {
+        PT_COUNT(), kernel<<<groups, kInvThreads, inverse_smem(kl, ku, cols), st>>>(ab, G, n, kl, ku, w, tops, WF, WB,
+                                                                                 FmaForms());
+        return cuda_check(cudaGetLastError(), "k_band_inverse");
+    }
+    const int need = (groups + kInvCluster - 1) / kInvCluster;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {kInvCluster, 1, 1};
+    cfg.gridDim = dim3(kInvCluster * (need < clusters ? need : clusters));
+    cfg.blockDim = dim3(kInvThreads);
+    cfg.dynamicSmemBytes = inverse_smem_alone(kl, ku, cols);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    PT_COUNT();
+    return cuda_check(cudaLaunchKernelEx(&cfg, kernel, ab, G, n, kl, ku, w, tops, WF, WB, FmaForms()), "k_band_inverse");
 }
-static int inverse_setup(int kl, int ku) {
-    if (int rc = cuda_check(cudaFuncSetAttribute(k_band_inverse<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)inverse_smem(kl, ku, 4)),
+// *clusters: as many as can run at once, less one, so that a cycle's cluster finds its SMs; 0 where that leaves none
+static int inverse_setup(int n, int kl, int ku, int* clusters) {
+    const int cols = inverse_cols(n);
+    const auto kernel = cols == 8 ? k_band_inverse<8> : k_band_inverse<4>;
+    const size_t smem = inverse_smem_alone(kl, ku, cols);
+    if (int rc = cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                             "coarse inverse"))
         return rc;
-    return cuda_check(cudaFuncSetAttribute(k_band_inverse<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)inverse_smem(kl, ku, 8)),
-                      "coarse inverse");
+    if (int rc = cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                            "coarse inverse"))
+        return rc;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {kInvCluster, 1, 1};
+    cfg.gridDim = dim3(kInvCluster);
+    cfg.blockDim = dim3(kInvThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        fit = 0;
+    }
+    *clusters = fit > 1 ? fit - 1 : 0;
+    return 0;
 }
 
 }  // namespace bandlu

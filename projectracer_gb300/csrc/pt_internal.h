@@ -158,6 +158,7 @@ struct Engine {
     double *Mc2 = nullptr, *RowB2 = nullptr, *Ginv2 = nullptr;
     int *ipiv2 = nullptr, *derr2 = nullptr, *hflag2 = nullptr;
     void *luw = nullptr, *luw2 = nullptr;  // workspaces of the coarse LU on st and st2
+    int side_clusters = 0;                 // clusters of the worker's inverse on st2 (0: the whole chip)
     cudaStream_t st2 = nullptr;
     cudaEvent_t ev_in = nullptr, ev_fact = nullptr;
     bool fact_pending = false;

@@ -1195,8 +1195,9 @@ static int coarse_factor(Engine& E) {
 }
 
 // Mixed precision: build the coarse matrix, its LU and inverse for the viscosity just computed
-// on st into the second buffer set on st2, overlapped with the solve that follows on st (the
-// LU's panels run on one SM, the columns they reach on a SM each for a few us).  coarse_resolve copies the result into the live buffers.
+// on st into the second buffer set on st2, overlapped with the solves that follow on st (the
+// LU's panels run on one SM, the columns they reach on an SM each for a few us; the inverse on
+// E.side_clusters clusters).  coarse_resolve copies the result into the live buffers.
 static int coarse_factor_async(Engine& E, const VisLevels& V) {
     const int L = E.grids, n = E.ngc;
     CK(cudaMemsetAsync(E.derr2, 0, sizeof(int), E.st2));
@@ -1204,7 +1205,9 @@ static int coarse_factor_async(Engine& E, const VisLevels& V) {
                                                      E.cfg.ivis, V.vis[L], V.vx[L], V.vz[L], V.vxz[L], V.vxxmzz[L],
                                                      E.derr2);
     if (int rc = bandlu::factor(E.Mc2, E.ipiv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, n, E.kl), E.derr2, E.st2)) return rc;
-    if (int rc = bandlu::inverse(E.Mc2, E.Ginv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, n, E.kl), E.st2)) return rc;
+    if (int rc = bandlu::inverse(E.Mc2, E.Ginv2, n, E.kl, E.ku, bandlu::work_of(E.luw2, n, E.kl), E.st2,
+                                 E.side_clusters))
+        return rc;
     CK(cudaMemcpyAsync(E.hflag2, E.derr2, sizeof(int), cudaMemcpyDeviceToHost, E.st2));
     E.fact_pending = true;
     return 0;
@@ -1231,7 +1234,8 @@ static void coarse_levels_worker(Engine* Ep) {
 // Joins the worker and moves its levels into the cycle's arrays (after st2's work, in stream
 // order); the factorisation follows in coarse_resolve.  Unless `wait`, only a worker whose work
 // has completed on the device is joined: the solves of this time level keep the previous coarse
-// levels until then (a preconditioner, O(dt) older), so the worker never delays a solve.
+// levels until then (a preconditioner, O(dt) older), so a solve waits for no worker; it shares the
+// SMs with the worker's kernels.
 static int coarse_join(Engine& E, bool wait) {
     if (!E.job_active) return 0;
     if (!wait && !(E.job_done.load() && cudaEventQuery(E.ev_fact) == cudaSuccess)) {
@@ -1619,7 +1623,16 @@ int mg_alloc(Engine& E) {
         CK(cudaEventCreateWithFlags(&E.ev_in, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&E.ev_fact, cudaEventDisableTiming));
         E.bytes_allocated += sizeof(double) * ((size_t)E.ngc * E.ngc + (size_t)ldab * E.ngc + E.ngc);
-        if (int rc = bandlu::inverse_setup(E.kl, E.ku)) return rc;
+        if (int rc = bandlu::inverse_setup(E.ngc, E.kl, E.ku, &E.side_clusters)) return rc;
+        // On few SMs the worker's inverse takes longer, which costs nothing while it ends within the time step (a
+        // new time level waits for it).  Its work is n^2 (kl / 2 + ku) multiply-subtract pairs; a mixed step takes
+        // some 5 ms and 1 ms for every 65,000 nodes.  Steps with the whole chip and with six clusters, ms:
+        // 256x128 n = 561 (2.4e7) 6.0, 5.7; 384x192 n = 1225 (1.7e8) 8.7, 7.8; 1024x512 n = 2145 (6.8e8) 18.3,
+        // 17.7; 2048x1024 n = 2145 36.5, 34.5; past the line 256x128 n = 2145 11.2, 14.2; 512x256 n = 2145 12.7,
+        // 15.2; 1280x640 n = 3321 (2.0e9) 31.8, 40.8 (there the worker is the longer path, and a solve that
+        // meets its inverse still waits)
+        const double work = (double)E.ngc * E.ngc * (0.5 * E.kl + E.ku);
+        if (work > 2e8 + 1e3 * (double)(E.K.nx - 1) * (double)(E.K.nz - 1)) E.side_clusters = 0;
     }
     return cluster_setup_d(E);
 }
