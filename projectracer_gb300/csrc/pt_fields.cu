@@ -3,8 +3,9 @@
 //
 // Compiled with --fmad=false: every operation rounds exactly as the reference's Fortran
 // expression (same association order), so these kernels reproduce the CPU oracle bit for bit and
-// the data-dependent smoother loop counts match (the statistics are the exception: their sums run
-// in a fixed tree, not in the reference's serial order).  All are HBM-bound stencils or reductions.
+// the data-dependent smoother loop counts match (the statistics do so where the solve rounds like the
+// reference, with reference_rounding or direct; elsewhere their sums run in a fixed tree).  All are
+// HBM-bound stencils or reductions.
 #include <cmath>
 #include <cstring>
 
@@ -402,6 +403,9 @@ int stability_dt(Engine& E, double* dt) {
 // not depend on the launch.  The trapezoid rule is taken as (sum f - (f_first + f_last) / 2) dr,
 // which needs each node's value once.  One thread per row and one thread for the tail took
 // 20.7 ms at 1024x512 and 1.5 ms at 128x128 (GB300, host time of the call); this takes 0.16 and 0.06 ms.
+// SERIAL (where the solve rounds like the reference): the reference's sums, 0.5 (f_i + f_{i+1}) h added in
+// ascending order; the CTA forms the terms, one thread a sum adds them: 0.35 ms at 1024x512 and
+// 0.05 at 128x128, the additions one after the other at some 64 cycles.
 constexpr int kStatsRow = 7;  // per row: T, C, u^2+w^2, Ra/conduct/vis, empty, fewest, most tracers
 constexpr int kStatsThreads = 256;
 
@@ -430,6 +434,37 @@ __device__ __forceinline__ void stats_block(double (&a)[NS], int& lo, int& hi) {
         }
 }
 
+// f of thread 32 q, q < NQ: the sum over the intervals i < n of 0.5 (v_i + v_{i+1}) h of value q in ascending
+// order; value(i, v) forms the values at node i
+template <int NQ, int NT, class Value>
+__device__ __forceinline__ void stats_serial(double (&sh)[4][NT], int n, double h, const Value& value, double& f) {
+    const int tid = threadIdx.x;
+    f = 0.0;
+    for (int i0 = 0; i0 < n; i0 += NT - 1) {
+        const int i = i0 + tid;
+        double v[NQ];
+        if (i <= n) {
+            value(i, v);
+#pragma unroll
+            for (int q = 0; q < NQ; q++) sh[q][tid] = v[q];
+        }
+        __syncthreads();
+        const bool term = tid < NT - 1 && i < n;
+        if (term)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) v[q] = 0.5 * (v[q] + sh[q][tid + 1]) * h;
+        __syncthreads();
+        if (term)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) sh[q][tid] = v[q];
+        __syncthreads();
+        if ((tid & 31) == 0 && tid < 32 * NQ)
+            for (int j = 0; j < min(NT - 1, n - i0); j++) f = f + sh[tid >> 5][j];
+        __syncthreads();
+    }
+}
+
+template <bool SERIAL>
 __global__ void __launch_bounds__(kStatsThreads) k_stats_rows(const double* T, const double* C, const double* u,
                                                               const double* w, const double* cd, const double* vis,
                                                               const int32_t* nempty, Geo g, double* rows) {
@@ -437,22 +472,38 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats_rows(const double* T, c
     double a[5] = {0, 0, 0, 0, 0};  // T, C, u^2+w^2, Ra/conduct/vis, empty
     int lo = 0x7fffffff, hi = -0x7fffffff;
     for (int i = threadIdx.x; i <= nx; i += kStatsThreads) {
-        const size_t o = g.at(i, k);
-        const double end = (i == 0 || i == nx) ? 0.5 : 1.0;
-        const double uu = u[o], ww = w[o];
-        a[0] += end * T[o];
-        a[1] += end * C[o];
-        a[2] += end * (uu * uu + ww * ww);
-        a[3] += end * (cK.RaT / cd[o] / vis[o]);
+        if (!SERIAL) {
+            const size_t o = g.at(i, k);
+            const double end = (i == 0 || i == nx) ? 0.5 : 1.0;
+            const double uu = u[o], ww = w[o];
+            a[0] += end * T[o];
+            a[1] += end * C[o];
+            a[2] += end * (uu * uu + ww * ww);
+            a[3] += end * (cK.RaT / cd[o] / vis[o]);
+        }
         const int n = nempty[(size_t)k * (nx + 1) + i];
         a[4] += n == 0 ? 1.0 : 0.0;
         lo = min(lo, n);
         hi = max(hi, n);
     }
     stats_block<5, kStatsThreads>(a, lo, hi);
-    if (threadIdx.x != 0) return;
     double* r = rows + (size_t)kStatsRow * k;
-    for (int q = 0; q < 4; q++) r[q] = a[q] * cK.dr;
+    if constexpr (SERIAL) {
+        __shared__ double sh[4][kStatsThreads];
+        double f;
+        stats_serial<4>(sh, nx, cK.dr, [&](int i, double* v) {
+            const size_t o = g.at(i, k);
+            const double uu = u[o], ww = w[o];
+            v[0] = T[o];
+            v[1] = C[o];
+            v[2] = uu * uu + ww * ww;
+            v[3] = cK.RaT / cd[o] / vis[o];
+        }, f);
+        if ((threadIdx.x & 31) == 0 && threadIdx.x < 128) r[threadIdx.x >> 5] = f;
+    }
+    if (threadIdx.x != 0) return;
+    if (!SERIAL)
+        for (int q = 0; q < 4; q++) r[q] = a[q] * cK.dr;
     r[4] = a[4];
     r[5] = (double)lo;
     r[6] = (double)hi;
@@ -491,6 +542,7 @@ __device__ __forceinline__ double stats_strain(const double* u, const double* w,
 // momentum.f90:73-92; for the direct solve from the velocities: compute_strain_rate_invariant,
 // momentum.f90:1-34) and the tracer counts
 constexpr int kStatsTail = 512;
+template <bool SERIAL>
 __global__ void __launch_bounds__(kStatsTail) k_stats_tail(const double* rows, const double* T, const double* u,
                                                            const double* w, const double* cd, const double* E1, Geo g,
                                                            double* out, int kent, int direct) {
@@ -499,25 +551,34 @@ __global__ void __launch_bounds__(kStatsTail) k_stats_tail(const double* rows, c
     int lo = 0x7fffffff, hi = -0x7fffffff;
     for (int k = tid; k <= nz; k += kStatsTail) {
         const double* r = rows + (size_t)kStatsRow * k;
-        const double end = (k == 0 || k == nz) ? 0.5 : 1.0;
-        for (int q = 0; q < 4; q++) a[q] += end * r[q];
-        if (k >= kent) a[4] += ((k == kent && kent < nz) || k == nz ? (kent < nz ? 0.5 : 0.0) : 1.0) * r[1];
+        if (!SERIAL) {
+            const double end = (k == 0 || k == nz) ? 0.5 : 1.0;
+            for (int q = 0; q < 4; q++) a[q] += end * r[q];
+            if (k >= kent) a[4] += ((k == kent && kent < nz) || k == nz ? (kent < nz ? 0.5 : 0.0) : 1.0) * r[1];
+        }
         a[9] += r[4];
         lo = min(lo, (int)r[5]);
         hi = max(hi, (int)r[6]);
     }
     double smax = -1.0 / 0.0;
-    for (int i = tid; i <= nx; i += kStatsTail) {
-        const double end = (i == 0 || i == nx) ? 0.5 : 1.0;
+    auto walls = [&](int i, double* v) {
         double t1 = 0.0, t2 = 0.0;
         for (int j = -2; j <= 2; j++) t1 = t1 + cK.D1[3 + j] * T[g.at(i, nz + j)];
         for (int j = -2; j <= 2; j++) t2 = t2 + cK.D1[3 + j] * T[g.at(i, j)];
-        const double tzs = qdiv(t1, cK.ds, cK.inv_ds), tzb = qdiv(t2, cK.ds, cK.inv_ds);
+        const double tzs = qdiv(t1, cK.ds, cK.inv_ds), tzb = qdiv(t2, cK.ds, cK.inv_ds);  // (the reference's / 1.0 is exact)
         const double uu = u[g.at(i, nz)], ww = w[g.at(i, nz)];
-        a[5] += end * -(cd[g.at(i, nz)] * tzs);
-        a[6] += end * T[g.at(i, 0)];
-        a[7] += end * -(cd[g.at(i, 0)] * tzb);
-        a[8] += end * (uu * uu + ww * ww);
+        v[0] = -(cd[g.at(i, nz)] * tzs);
+        v[1] = T[g.at(i, 0)];
+        v[2] = -(cd[g.at(i, 0)] * tzb);
+        v[3] = uu * uu + ww * ww;
+    };
+    for (int i = tid; i <= nx; i += kStatsTail) {
+        if (!SERIAL) {
+            const double end = (i == 0 || i == nx) ? 0.5 : 1.0;
+            double v[4];
+            walls(i, v);
+            for (int q = 0; q < 4; q++) a[5 + q] += end * v[q];
+        }
         const double s = stats_strain(u, w, E1, g, i, direct);
         if (s > smax) smax = s;
     }
@@ -525,6 +586,19 @@ __global__ void __launch_bounds__(kStatsTail) k_stats_tail(const double* rows, c
     __shared__ double ssm[kStatsTail / 32];
     if ((tid & 31) == 0) ssm[tid >> 5] = smax;
     stats_block<10, kStatsTail>(a, lo, hi);  // (its barrier orders ssm too)
+    if constexpr (SERIAL) {
+        __shared__ double sh[4][kStatsTail];
+        double f;
+        const bool one = (tid & 31) == 0 && tid < 128;
+        stats_serial<4>(sh, nz, cK.ds, [&](int k, double* v) {
+            for (int q = 0; q < 4; q++) v[q] = rows[(size_t)kStatsRow * k + q];
+        }, f);
+        if (one) out[tid >> 5] = f;
+        stats_serial<1>(sh, nz - kent, cK.ds, [&](int k, double* v) { v[0] = rows[(size_t)kStatsRow * (kent + k) + 1]; }, f);
+        if (tid == 0) out[4] = f;
+        stats_serial<4>(sh, nx, cK.dr, walls, f);
+        if (one) out[5 + (tid >> 5)] = f;
+    }
     if (tid != 0) return;
     for (int q = 1; q < kStatsTail / 32; q++) smax = fmax(smax, ssm[q]);
     double d, q1, q2, q3, q4;
@@ -536,8 +610,10 @@ __global__ void __launch_bounds__(kStatsTail) k_stats_tail(const double* rows, c
     q3 = -qdiv(cd[g.at(nx, 0)] * d, cK.ds, cK.inv_ds);
     d = 0; for (int j = -2; j <= 2; j++) d = d + cK.D1[3 + j] * T[g.at(0, j)];
     q4 = -qdiv(cd[g.at(0, 0)] * d, cK.ds, cK.inv_ds);
-    for (int q = 0; q < 5; q++) out[q] = a[q] * cK.ds;  // integrals of T, C, u^2+w^2, Ra/conduct/vis, C above kent
-    for (int q = 5; q < 9; q++) out[q] = a[q] * cK.dr;  // Nu_top, T bottom, Nu_bot, mobility
+    if (!SERIAL) {
+        for (int q = 0; q < 5; q++) out[q] = a[q] * cK.ds;  // integrals of T, C, u^2+w^2, Ra/conduct/vis, C above kent
+        for (int q = 5; q < 9; q++) out[q] = a[q] * cK.dr;  // Nu_top, T bottom, Nu_bot, mobility
+    }
     out[9] = smax;
     out[10] = q1; out[11] = q2; out[12] = q3; out[13] = q4;
     out[14] = a[9]; out[15] = (double)lo; out[16] = (double)hi;
@@ -547,11 +623,12 @@ int stats(Engine& E, pt_stats_row* o) {
     double* rows = E.red;
     int nz = E.K.nz;
     const double* C = E.cfg.comp ? E.Cnew : E.T;
-    PT_COUNT(), k_stats_rows<<<nz + 1, kStatsThreads, 0, E.st>>>(E.T, C, E.u, E.w, E.cond, E.vis[1], E.nempty, E.g1,
-                                                                 rows);
+    const bool serial = E.cfg.reference_rounding || E.cfg.direct;
+    const auto row_sums = serial ? k_stats_rows<true> : k_stats_rows<false>;
+    const auto tail = serial ? k_stats_tail<true> : k_stats_tail<false>;
+    PT_COUNT(), row_sums<<<nz + 1, kStatsThreads, 0, E.st>>>(E.T, C, E.u, E.w, E.cond, E.vis[1], E.nempty, E.g1, rows);
     double* out = rows + kStatsRow * (nz + 1) + 8;
-    PT_COUNT(), k_stats_tail<<<1, kStatsTail, 0, E.st>>>(rows, E.T, E.u, E.w, E.cond, E.err[1], E.g1, out, E.kent,
-                                                         E.cfg.direct);
+    PT_COUNT(), tail<<<1, kStatsTail, 0, E.st>>>(rows, E.T, E.u, E.w, E.cond, E.err[1], E.g1, out, E.kent, E.cfg.direct);
     CKL("stats");
     CK(cudaMemcpyAsync(E.hscal, out, 17 * sizeof(double), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));

@@ -44,3 +44,29 @@ def test_stats_row_is_the_trapezoid_rule(nx, nz, dent):
     assert s["entrainment"] == pytest.approx(ent, rel=tol, abs=1e-300)
     assert (s["empty_cells"], s["tracer_min"], s["tracer_max"]) == (int((n == 0).sum()), int(n.min()), int(n.max()))
     e.close()
+
+
+# rows and columns below, at and past the terms that a CTA adds at a time (255 columns, 511 rows or columns)
+@pytest.mark.parametrize("kind,nx,nz,direct", [("iso", 64, 64, 0), ("iso", 64, 64, 1), ("iso", 100, 100, 1),
+                                               ("chem", 256, 32, 0), ("chem", 520, 40, 0), ("chem", 40, 520, 0)])
+def test_stats_row_has_the_oracles_bits_where_the_solve_rounds_like_it(kind, nx, nz, direct):
+    """Every column of the isoviscous runs, whose psi has the oracle's bits; of the others the columns that
+    psi does not enter."""
+    from oracle.ptref import Oracle
+
+    cfg, _ = small_case(kind, nx=nx, nz=nz, tpc=4)
+    cfg.aspect, cfg.direct = nx / nz, direct
+    cfg.reference_rounding = 1 - direct
+    if kind == "chem":
+        cfg.tolerance = 1e-2
+    st = make_state(cfg, 4, noise=1e-3)
+    o = Oracle(cfg, iterate=1 - direct, nparts=0)
+    o.load_restart(st["xg"], st["zg"], st["T"], st["Cnew"], st["SF"], st["rtr"], st["str"], st["Ctr"], st["Ttr"])
+    o.solve_psi()
+    e = eng.Engine(cfg)
+    e.upload(st)
+    e.solve_psi()
+    a, b = e.stats(), o.stats()
+    e.close()
+    names = list(b) if kind == "iso" else ["Tavg", "RaT_avg", "Nu", "Nu_bot", "q1", "q2", "q3", "q4", "empty_cells"]
+    assert {k: a[k] for k in names} == {k: b[k] for k in names}
