@@ -316,6 +316,10 @@ __global__ void __launch_bounds__(kLuThreads) k_direct_lu(double* ab, int* ipiv,
 // bound by the SM's FP64 rate (2 kl operations, 300 of the 500 cycles at kl = 303) and its barrier, the back
 // substitution by the chain of its diagonal (quotient, product and difference: 650 cycles).
 constexpr int kDsRows = 960;  // row threads of the forward substitution at most
+// Widest band that pt_init accepts, kl + ku (nz up to 1157): the documented bound of the interface, at which
+// three columns and a window of 8192 elements in shared memory fill an SM.  The forward substitution alone,
+// with its window in registers, would take kl + 2 = 4 kDsRows.
+constexpr int kDsBand = 6950;
 __device__ __forceinline__ void ds_cp16(void* dst, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
@@ -649,8 +653,7 @@ int direct_alloc(Engine& E) {
     E.dkl = kl;
     E.dku = ku;
     E.dn = n;
-    // the forward substitution keeps its ring of columns in shared memory and its window of b in registers
-    if (kl + 2 > 4 * kDsRows)
+    if (kl + ku > kDsBand || kl + 2 > 4 * kDsRows)
         return fail(PT_ERR_CONFIG, "direct solve: the band is too wide for the banded substitution kernel");
     if (int rc = direct_forward_of(kl, [&](auto kernel, int, size_t smem) {
             return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),

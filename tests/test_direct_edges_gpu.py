@@ -12,3 +12,21 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("nx,nz", [(8, 8), (24, 16), (8, 12), (32, 320)])
 def test_direct_solve_matches_oracle_at_block_edges(nx, nz):
     same_bits(nx, nz)
+
+
+def test_bands_past_the_documented_bound_are_refused():
+    """kl + ku = 6 (nz + 1) up to 6,950: nz = 1152 is accepted, 1168 refused (both with nz / 16 rows on the
+    coarsest of four halvings)."""
+    from projectracer_gb300 import engine as eng
+    from projectracer_gb300.config import PT_PREC_FP64, workload
+
+    cfg, _ = workload("C1", 1.0, PT_PREC_FP64)
+    cfg.nx, cfg.direct, cfg.mingrid = 32, 1, 2
+    for nz in (1168, 1152):
+        cfg.nz, cfg.aspect, cfg.ntr = nz, 32 / nz, 32 * nz
+        if nz == 1168:
+            with pytest.raises(eng.PtError, match="band is too wide") as ex:
+                eng.Engine(cfg)
+            assert ex.value.code == -1
+        else:
+            eng.Engine(cfg).close()
