@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "pt_consts.cuh"
+#include "pt_internal.h"
 
 namespace pt {
 namespace cl {
@@ -176,7 +177,9 @@ struct Visit {
     unsigned char flags;
 };
 enum { kRestrict = 1, kProlong = 2, kZero = 4, kResidual = 8, kCoarse = 16 };
-constexpr int kMaxVisits = 48;
+constexpr int kMaxVisits = 64;  // as many as a schedule has entries: a run is never cut
+static_assert(kMaxVisits >= sizeof(Engine::multi) / sizeof(int) && kMaxVisits >= sizeof(Engine::mmulti) / sizeof(int),
+              "a run holds every entry of a level schedule");
 
 // the launch of one cluster; at: one attribute
 static inline void cluster_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, size_t smem, cudaStream_t st) {

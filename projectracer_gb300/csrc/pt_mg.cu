@@ -1395,7 +1395,7 @@ static int cluster_setup_d(Engine& E) {
 // the entries p.. of the schedule on levels ctop.. as one launch; *last receives the last of them
 static int cluster_run_d(Engine& E, const int* multi, int nsteps, int p, int* last) {
     DRun R{};
-    for (; p <= nsteps && multi[p] >= E.ctop && R.nv < cl::kMaxVisits; p++) {
+    for (; p <= nsteps && multi[p] >= E.ctop; p++) {
         const int l = multi[p];
         cl::Visit& v = R.v[R.nv++];
         v.level = (signed char)l;

@@ -1199,7 +1199,7 @@ static int launch_run_f(Engine& E, FRun& R, bool coarse_smoother, const double* 
 static int cluster_run_f(Engine& E, int p, const double* r1, int* last) {
     FRun R{};
     const int* multi = E.mmulti;
-    for (; p <= E.mnsteps && R.nv < cl::kMaxVisits; p++) {
+    for (; p <= E.mnsteps; p++) {
         const int l = multi[p];
         if (l < E.ctop || (l == E.grids && !E.ccoarse)) break;
         cl::Visit& v = R.v[R.nv++];
