@@ -1084,6 +1084,9 @@ static int cluster_setup_f(Engine& E) {
     E.ctop = E.grids + 1;
     E.csolo = E.grids + 1;
     E.cl1 = E.ccoarse = E.coarse_solo = false;
+#ifdef PT_STAGE_KERNELS  // a build for comparison: a kernel per stage on every level
+    return 0;
+#endif
     if (E.cfg.Nmulti != 1) return 0;
     for (int l = 1; l < E.grids; l++) {
         Stencil<float> f;

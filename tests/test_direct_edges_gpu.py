@@ -30,3 +30,28 @@ def test_bands_past_the_documented_bound_are_refused():
             assert ex.value.code == -1
         else:
             eng.Engine(cfg).close()
+
+
+def test_wide_bands_take_four_elements_per_thread():
+    """kl = 3 (640 + 1) = 1923, past twice the row threads, with the shorter ring: psi has the oracle's bits."""
+    import numpy as np
+
+    from oracle.ptref import Oracle
+    from projectracer_gb300 import engine as eng
+    from projectracer_gb300.config import PT_PREC_FP64, workload
+    from projectracer_gb300.inputs import make_state
+
+    cfg, _ = workload("C1", 1.0, PT_PREC_FP64)
+    cfg.nx, cfg.nz, cfg.aspect, cfg.mingrid = 8, 640, 8 / 640, 1  # (a coarsest grid that pt_init takes)
+    cfg.direct, cfg.ntr = 1, 8 * 640 * 4
+    st = make_state(cfg, 3)
+    e = eng.Engine(cfg)
+    e.upload(st)
+    e.solve_psi()
+    e.solve_psi()
+    sf = e.get(eng.F_SF)
+    e.close()
+    o = Oracle(cfg, iterate=0, nparts=0)
+    o.load_restart(st["xg"], st["zg"], st["T"], st["Cnew"], st["SF"], st["rtr"], st["str"], st["Ctr"], st["Ttr"])
+    o.solve_psi()
+    assert np.array_equal(sf.view(np.int64), o.get(7).view(np.int64))
