@@ -173,47 +173,58 @@ __global__ void k_scatter(const int32_t* __restrict__ cell, int64_t n, const int
     if (c >= 0) list[start[c] + base + __popc(group & ((1u << lane) - 1u))] = (int32_t)t;
 }
 
-// Ascending tracer IDs inside each cell: a warp per cell takes up to 32 kSortRegs IDs into registers, and an
-// ID's place is the number of smaller ones.  (A thread per cell that inserted them in global memory took
-// 141 us for 100 x 100 cells of 60; now 20.)  Fuller cells are sorted by one lane.
+// Ascending tracer IDs inside each cell: LANES lanes per cell take up to LANES kSortRegs IDs into registers, and
+// an ID's place is the number of smaller ones; fuller cells are sorted by one lane.  Bound by the chain of a
+// warp's loads and its count of warps: 4 lanes up to a mean of 8 tracers per cell, 8 up to 24, 32 above, each
+// below the others there.  Time in us on 525,825 cells, lanes 1 (inserting in global memory), 4, 8, 32, by the
+// mean: 4: 24, 16, 24, 65; 8: 49, 24, 28, 73; 16: 131, 59, 53, 92; 24: 288, 160, 86, 120; 48: 1116, 976, 330,
+// 240.  100 x 100 cells of 60: 141 with one lane, 20 with 32.
 constexpr int kSortRegs = 8, kCellsPerWarp = 10;
-__global__ void __launch_bounds__(256) k_sort_cells(int32_t* list, const int32_t* __restrict__ start,
-                                                  const int32_t* __restrict__ count, int ncell) {
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (c >= ncell) return;
-    const int n = count[c];
-    int32_t* const l = list + start[c];
-    if (n > 32 * kSortRegs) {
-        if (lane == 0)
-            for (int a = 1; a < n; a++) {
-                const int32_t key = l[a];
-                int j = a - 1;
-                while (j >= 0 && l[j] > key) {
-                    l[j + 1] = l[j];
-                    j--;
-                }
-                l[j + 1] = key;
-            }
-        return;
-    }
-    int32_t key[kSortRegs];
-    int rank[kSortRegs] = {};
+template <int LANES, int R>
+__device__ __forceinline__ void rank_sort(int32_t* l, int n, int most, int sub) {
+    int32_t key[R];
+    int rank[R] = {};
 #pragma unroll
-    for (int q = 0; q < kSortRegs; q++) key[q] = 32 * q + lane < n ? l[32 * q + lane] : INT_MAX;
+    for (int q = 0; q < R; q++) key[q] = LANES * q + sub < n ? l[LANES * q + sub] : INT_MAX;
 #pragma unroll
-    for (int q = 0; q < kSortRegs; q++) {
-        if (32 * q >= n) break;
-        const int m = min(32, n - 32 * q);
+    for (int q = 0; q < R; q++) {
+        const int m = min(LANES, most - LANES * q);
         for (int t = 0; t < m; t++) {
-            const int32_t k = __shfl_sync(0xffffffffu, key[q], t);
+            const int32_t k = __shfl_sync(0xffffffffu, key[q], t, LANES);
 #pragma unroll
-            for (int u = 0; u < kSortRegs; u++) rank[u] += k < key[u];
+            for (int u = 0; u < R; u++) rank[u] += k < key[u];
         }
     }
     __syncwarp();
 #pragma unroll
-    for (int q = 0; q < kSortRegs; q++)
-        if (32 * q + lane < n) l[rank[q]] = key[q];
+    for (int q = 0; q < R; q++)
+        if (LANES * q + sub < n) l[rank[q]] = key[q];
+}
+template <int LANES>
+__global__ void __launch_bounds__(256) k_sort_cells(int32_t* list, const int32_t* __restrict__ start,
+                                                  const int32_t* __restrict__ count, int ncell) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = (int)(t / LANES), sub = (int)(t % LANES);
+    const bool live = c < ncell;
+    const int total = live ? count[c] : 0, n = total <= LANES * kSortRegs ? total : 0;
+    int32_t* const l = list + (live ? start[c] : 0);
+    if (total > n && sub == 0)
+        for (int a = 1; a < total; a++) {
+            const int32_t key = l[a];
+            int j = a - 1;
+            while (j >= 0 && l[j] > key) {
+                l[j + 1] = l[j];
+                j--;
+            }
+            l[j + 1] = key;
+        }
+    __syncwarp();
+    const int most = __reduce_max_sync(0xffffffffu, n);  // of the warp's cells
+    if (most <= 1) return;
+    if (most <= LANES) rank_sort<LANES, 1>(l, n, most, sub);
+    else if (most <= 2 * LANES) rank_sort<LANES, 2>(l, n, most, sub);
+    else if (most <= 4 * LANES) rank_sort<LANES, 4>(l, n, most, sub);
+    else rank_sort<LANES, 8>(l, n, most, sub);
 }
 
 __device__ __forceinline__ double shape1(double x, double node, double h, double inv, int exact, const FmaForms& F) {
@@ -668,7 +679,9 @@ static int project_with(Engine& E, const ProjScratch& W, const double* r, const 
             int32_t* cursor = W.scan_tmp + nb + 32;
             CK(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (size_t)ncell, E.st));
             PT_COUNT(), k_scatter<<<nblk(n, 256), 256, 0, E.st>>>(W.tcell, n, W.cstart, cursor, W.clist);
-            PT_COUNT(), k_sort_cells<<<nblk(ncell, 8), 256, 0, E.st>>>(W.clist, W.cstart, W.ccount, ncell);
+            const int lanes = n <= 8 * (int64_t)ncell ? 4 : n <= 24 * (int64_t)ncell ? 8 : 32;
+            const auto sort_cells = lanes == 4 ? k_sort_cells<4> : lanes == 8 ? k_sort_cells<8> : k_sort_cells<32>;
+            PT_COUNT(), sort_cells<<<nblk(ncell, 256 / lanes), 256, 0, E.st>>>(W.clist, W.cstart, W.ccount, ncell);
             const bool og = E.cfg.discrete_types != 0;
             PT_COUNT(), (og ? k_cell_partials<true> : k_cell_partials<false>)<<<nblk(ncell, 2 * kCellsPerWarp), 64, 0, E.st>>>(
                 r, s, Tt, E.Ctr, W.clist, W.cstart, W.ccount, ncell, W.cpart, E.cfg.comp, FmaForms());

@@ -33,3 +33,29 @@ def test_projection_of_uneven_cells_is_bit_exact(kind, nx, nz):
     if cfg.comp:
         assert np.array_equal(e.get(eng.F_CNEW), o.get(4))
     e.close()
+
+
+# tracers per cell on each side of the sort's widths (4 lanes up to a mean of 8 per cell, 8 up to 24, 32 above)
+# and cells at and past what each width holds in registers (32, 64 and 256)
+@pytest.mark.parametrize("tpc", [1, 7, 9, 25, 28])
+def test_projection_is_bit_exact_at_every_width_of_the_sort(tpc):
+    cfg, st = small_case("chem", nx=40, nz=24, tpc=tpc)
+    n = len(st["rtr"])
+    order = np.random.default_rng(2).permutation(n)
+    for k in ("rtr", "str", "Ttr", "Ctr"):
+        st[k] = np.ascontiguousarray(st[k][order])
+    at, sizes = 0, (300, 70, 65, 64, 33, 32, 9, 8)
+    for q, size in enumerate(sizes):  # cells (3 + 4 q, 5) get `size` tracers more
+        st["rtr"][at:at + size] = (3 + 4 * q) * cfg.aspect / 40
+        st["str"][at:at + size] = 5 / 24
+        at += size
+    o = Oracle(cfg, iterate=1, nparts=0)
+    o.load_restart(st["xg"], st["zg"], st["T"], st["Cnew"], st["SF"], st["rtr"], st["str"], st["Ctr"], st["Ttr"])
+    e = eng.Engine(cfg)
+    e.upload(st)
+    counts = o.get(11)
+    assert np.array_equal(e.get(eng.F_NEMPTY), counts) and counts[5, 3:32:4].min() >= 8 and counts.max() >= 300
+    g, r = e.get(eng.F_TRATIO), o.get(eng.F_TRATIO)
+    assert np.array_equal(g[1:-1, 1:-1], r[1:-1, 1:-1])
+    assert np.array_equal(e.get(eng.F_CNEW), o.get(4))
+    e.close()
