@@ -4,11 +4,12 @@
 // A panel of kPanel columns is factored by one CTA in shared memory (k_band_panel), then every column to
 // its right that the panel reaches takes the panel's row interchanges, multipliers and updates in a CTA of
 // its own (k_band_trail).  Every element sees the operations of the column-by-column DGBTF2 in the same
-// order (interchanges permute rows, updates by ascending pivot column), so the factors are the same
-// bit for bit; one CTA that updated the whole trailing block column by column was bound by its SM's FP64
+// order (interchanges permute rows, updates by ascending pivot column), so the factors of a finite matrix
+// have the same bits; where DGBTF2 leaves an element alone, k_band_trail may add a product with a multiplier
+// of zero, which turns a -0 into +0, and an infinite row spreads as NaN.  One CTA that updated the whole trailing block column by column was bound by its SM's FP64
 // rate (two multiply-subtract pairs a cycle).  What bounds it now is the chain of a panel's columns:
 // pivot search, reciprocal, scaling and the update of the next column.
-// n = 2145, kl = ku = 99: 26 -> 3.2 ms; n = 561, kl = ku = 51: 2.2 -> 0.9 ms.
+// n = 2145, kl = ku = 99: 26 -> 3.2 ms; n = 561, kl = ku = 51: 2.2 -> 1.1 ms.
 #pragma once
 #include "pt_fp64.cuh"
 #include "pt_launch.cuh"
@@ -246,7 +247,7 @@ __global__ void k_band_top(const double* ab, int n, int kl, int ku, Work w) {
 // memory, twice for the forward pass, whose interchanges permute it.
 // What bounds it is the FP64 rate (n^2 (kl / 2 + ku) multiply-subtract pairs): n = 2145, kl = ku = 99:
 // 11.2 ms with a warp per column (a division per column and step, partly filled warps, the zeros of U
-// above its entries), 6.5 now; n = 561, kl = ku = 51: 0.65 before and now.  A grid of fewer CTAs than groups
+// above its entries), 6.1 now; n = 561, kl = ku = 51: 0.65 before and now.  A grid of fewer CTAs than groups
 // of columns takes them in turn (see inverse).
 constexpr int kInvThreads = 256, kInvCols = 4;  // columns of a thread
 static inline int pow2_above(int v) {

@@ -73,7 +73,8 @@ struct PadGeo {
     __host__ __device__ int Hp() const { return H + 1; }
     __host__ __device__ size_t positions() const { return ((size_t)B * Hp() + 1) * Wp(); }
     __host__ __device__ size_t at(int b, int y, int x) const { return ((size_t)b * Hp() + y + 1) * Wp() + x + 1; }
-    // pixel of position p; false for padding (divisions as multiplications: exact for p < 2^31)
+    // pixel of position p; false for padding (divisions as products with the divisor's reciprocal rounded up,
+    // Granlund and Montgomery, PLDI 1994: exact for p < 2^31)
     struct Div {
         int d;
         uint32_t m;

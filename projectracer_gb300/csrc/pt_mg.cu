@@ -1361,7 +1361,8 @@ int mg_setup_solve(Engine& E) {
 }
 
 // levels ctop.. run in one cluster, where their nodes fit its arrays and the coarsest solve is a small
-// product with the explicit inverse
+// product with the explicit inverse (us a cycle in the cluster and with a kernel per stage: 256x64, n = 297 1003,
+// 1893; 256x128, n = 561 1377, 1926; at n = 1089 682 and 790, which the limit of 700 leaves out)
 static int cluster_setup_d(Engine& E) {
     E.ctop = E.grids + 1;
     if (E.cfg.precision != PT_PREC_FP64 || E.cfg.Nmulti != 1 || !E.res_int || !E.Ginv || E.ngc > 700) return 0;

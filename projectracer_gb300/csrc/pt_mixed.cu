@@ -1120,9 +1120,12 @@ static int cluster_setup_f(Engine& E) {
     while (E.ctop > 2 && (E.ctop - 1 == E.grids || fits(E.ctop - 1))) E.ctop--;
     if (E.ctop >= E.grids) E.ctop = E.grids + 1;  // nothing but the coarsest level
     E.cl1 = fits(1);
-    // the coarse solve inside the cluster: n^2 FP64 products on 16 SMs against 152 and a launch
+    // the coarse solve inside the cluster: n^2 FP64 products on 16 SMs against 152 and a launch; us a cycle inside
+    // and outside: n = 297 118, 118; 561 130, 131; 1089 131, 107
     E.ccoarse = E.Ginv && E.ngc <= 700;
-    E.coarse_solo = E.ccoarse && E.ngc <= 90;  // n^2 products on one SM against one exchange
+    // n^2 products on one SM against one exchange; us a cycle, solo and not: n = 25 119, 123; 121 115, 114 (and
+    // the inverse of 127 would fill the shared memory)
+    E.coarse_solo = E.ccoarse && E.ngc <= 90;
     // levels whose nodes fit one CTA's threads, 512 nodes, need no exchange between CTAs: each CTA
     // walks them for itself.  The way back up must be in the same launch.
     E.csolo = E.grids;
